@@ -285,9 +285,11 @@ static int mul_mat_chunks(dc_ctx* ctx, const dc_weight* w, const float* x_dev, i
     const int K = (int)w->K, N = (int)w->N;
     for (int m0 = 0; m0 < M; m0 += DC_MAX_T) {
         const int T = M - m0 < DC_MAX_T ? M - m0 : DC_MAX_T;
-        DC_TRY(dc_launch_quantize_q8k(ctx, x_dev + (size_t)m0 * K, T, K, q8));
+        const float* x = x_dev + (size_t)m0 * K;
+        const bool own = dc_rows_quantise(T, K);
+        if (!own) DC_TRY(dc_launch_quantize_q8k(ctx, x, T, K, q8, true));
         dc_gemv_seg seg = {w->dev, w->type, N, (int)w->row_bytes, y_dev + (size_t)m0 * N, N};
-        DC_TRY(dc_launch_gemv(ctx, &seg, 1, DC_EPI_STORE, q8, T, K, nullptr));
+        DC_TRY(dc_launch_gemv(ctx, &seg, 1, DC_EPI_STORE, q8, T, K, nullptr, nullptr, nullptr, own ? x : nullptr));
     }
     return DC_B200_OK;
 }
@@ -304,7 +306,7 @@ static int check_mul_mat_args(dc_ctx* ctx, const dc_weight* w, const void* x, in
 // Bytes of the quantised-activation scratch of one MUL_MAT with M token rows.
 static size_t mul_mat_act_bytes(dc_ctx* ctx, const dc_weight* w, int M) {
     if (M >= ctx->gemm_tc_min_rows && dc_gemm_tc_supports(w)) return dc_gemm_tc_act_bytes(M, (int)w->K);
-    return (size_t)DC_MAX_T * (w->K / DC_QK_K) * DC_Q8K_BYTES;
+    return (size_t)DC_MAX_T * (w->K / DC_QK_K) * DC_Q8F_BYTES;
 }
 
 // Prompt-sized inputs take the tensor-core kernel (cb_gemv_batched_custom serves M up to 4096 on the CPU,
@@ -354,7 +356,7 @@ int dc_b200_mul_mat_block_sums(dc_ctx* ctx, const dc_weight* w, const float* x_h
     cudaSetDevice(ctx->device);
     const int K = (int)w->K, nb = K / DC_QK_K;
     const size_t xb = ((size_t)M * K * 4 + 255) & ~(size_t)255;
-    const size_t qb = ((size_t)M * nb * DC_Q8K_BYTES + 255) & ~(size_t)255;
+    const size_t qb = ((size_t)M * nb * DC_Q8F_BYTES + 255) & ~(size_t)255;
     const size_t ib = ((size_t)M * w->N * nb * 4 + 255) & ~(size_t)255;
     const size_t yb = ((size_t)M * w->N * 4 + 255) & ~(size_t)255;
     uint8_t* s = dc_scratch(ctx, xb + qb + 2 * ib + yb);
@@ -363,7 +365,7 @@ int dc_b200_mul_mat_block_sums(dc_ctx* ctx, const dc_weight* w, const float* x_h
     int32_t* Md = (int32_t*)(s + xb + qb + ib);
     float* yd = (float*)(s + xb + qb + 2 * ib);
     DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(s, x_host, (size_t)M * K * 4, cudaMemcpyHostToDevice, ctx->stream), "H2D x"));
-    DC_TRY(dc_launch_quantize_q8k(ctx, (const float*)s, M, K, s + xb));
+    DC_TRY(dc_launch_quantize_q8k(ctx, (const float*)s, M, K, s + xb, true));
     // the production GEMV kernel itself, asked to store the integer sums it forms on the way
     dc_gemv_seg seg = {w->dev, w->type, (int)w->N, (int)w->row_bytes, yd, (int)w->N};
     DC_TRY(dc_launch_gemv(ctx, &seg, 1, DC_EPI_STORE, s + xb, M, K, nullptr, Id, w->type == DC_TYPE_Q4_K ? Md : nullptr));

@@ -22,6 +22,12 @@
 
 using namespace dc;
 
+#define DC_TRY(expr)                       \
+    do {                                   \
+        int st_ = (expr);                  \
+        if (st_ != DC_B200_OK) return st_; \
+    } while (0)
+
 #define ATT_MAX_GROUP 8  // query heads per kv head
 #define ATT_TILE 32      // keys per score tile (two KV blocks)
 
@@ -41,7 +47,7 @@ struct AttnParams {
     float* part_d;               // [T][n_head][nsplit]
     int* tickets;                // [T][n_kv], zeroed once, self-resetting
     float* out;                  // optional [T][n_head][128]
-    uint8_t* q8_out;             // optional Q8_K rows of out
+    uint8_t* q8_out;             // optional Q8_K rows of out, blocks in fragment order
 };
 
 __device__ __forceinline__ void split_range(int pos, int split, int nsplit, int& n_blk, int& b0, int& b1) {
@@ -215,7 +221,7 @@ __device__ __forceinline__ void attn_merge_tail(const AttnParams& p, int t, int 
             *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
         }
         if (p.q8_out)
-            quantize_block_q8k_regs(v, p.q8_out + ((size_t)t * (p.n_head / 2) + kvh * (g / 2) + pb2) * DC_Q8K_BYTES, lane);
+            quantize_block_q8f_regs(v, p.q8_out + ((size_t)t * (p.n_head / 2) + kvh * (g / 2) + pb2) * DC_Q8F_BYTES, lane);
     }
 }
 
@@ -490,6 +496,406 @@ __global__ void __launch_bounds__(128) k_attn_pv_run(const AttnParams p) {
     attn_merge_tail(p, t, kvh, g, tid, warp, lane, s_last);
 }
 
+// ------------------------------------------------------- one kernel, a cluster per (token, kv head)
+// What bounds decode attention at these lengths is not its bytes (4.7 MB of K and V at 2304 keys: 0.7 us of HBM) but the chain of
+// global round trips between score, P.V and merge kernels.  Here the CTAs of a cluster share a sequence's blocks and exchange
+// block maxima and partial sums through each other's shared memory: K and V rows of earlier positions are copied to shared memory while
+// this kernel still waits for its predecessor, scores never leave the SM, and the merge reads all partials at once.
+// The running-maximum chain is the reference's: a block's exponents are taken against the largest score up to that block.  What the
+// reference multiplies onto its accumulator block by block (alpha) is multiplied onto the exponentials of the blocks before instead,
+// within a CTA; across CTAs the partials are scaled in the merge.
+// With `fuse.qkv` the kernel also norms and rotates the q heads (every CTA its own copy) and writes the new token's K and V rows
+// (k_qknorm_rope_kv); the tokens of such a step belong to different sequences.
+#define AC_THREADS 256
+#define AC_CAP 32              // KV blocks a CTA holds at most (a lane each)
+
+__device__ __forceinline__ uint32_t ac_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void ac_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ac_peer(const float* mine, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(mine)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ac_peer4(const float* mine, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(mine)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+// d = a * b + d on two floats at a time (each rounded once, as two fmaf would)
+__device__ __forceinline__ void ac_fma2(float2& d, float2 a, float2 b) {
+    asm("{\n.reg .b64 ra, rb, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nmov.b64 rd, {%0, %1};\n"
+        "fma.rn.f32x2 rd, ra, rb, rd;\nmov.b64 {%0, %1}, rd;\n}"
+        : "+f"(d.x), "+f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+// place of the 16-byte piece i of a key's K row: eight lanes (two keys x four pieces) fall on distinct banks
+__device__ __forceinline__ int ac_piece(int key, int i) { return key * 256 + ((i ^ ((key & 1) << 2)) << 4); }
+__device__ __forceinline__ void ac_copy16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// place of (key, head) among the scores: eight heads together, eight floats more per block so that four blocks fall on distinct banks
+__device__ __forceinline__ int ac_at(int key, int h) { return key * 8 + (key >> 4) * 8 + h; }
+
+// One head of 128 values by one warp: RMSNorm (w4 given) and rotation of interleaved pairs (c given), as k_qknorm_rope_kv.
+__device__ __forceinline__ float4 ac_norm_rope(const float* src, bool norm, float4 w4, bool turn, float4 c, float eps, int lane) {
+    const float4 v4 = __ldcg(reinterpret_cast<const float4*>(src) + lane);
+    float v[4] = {v4.x, v4.y, v4.z, v4.w};
+    if (norm) {
+        double ss = (double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2] + (double)v[3] * v[3];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float mean = (float)(ss / 128.0);
+        const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+        v[0] = __fmul_rn(__fmul_rn(v[0], scale), w4.x);
+        v[1] = __fmul_rn(__fmul_rn(v[1], scale), w4.y);
+        v[2] = __fmul_rn(__fmul_rn(v[2], scale), w4.z);
+        v[3] = __fmul_rn(__fmul_rn(v[3], scale), w4.w);
+    }
+    if (turn) {
+        const float a0 = __fsub_rn(__fmul_rn(v[0], c.x), __fmul_rn(v[1], c.y)), a1 = __fadd_rn(__fmul_rn(v[0], c.y), __fmul_rn(v[1], c.x));
+        const float b0 = __fsub_rn(__fmul_rn(v[2], c.z), __fmul_rn(v[3], c.w)), b1 = __fadd_rn(__fmul_rn(v[2], c.w), __fmul_rn(v[3], c.z));
+        v[0] = a0; v[1] = a1; v[2] = b0; v[3] = b1;
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ uint2 ac_half4(float4 v) {
+    const __half2 lo = __halves2half2(__float2half_rn(v.x), __float2half_rn(v.y)), hi = __halves2half2(__float2half_rn(v.z), __float2half_rn(v.w));
+    uint2 r;
+    r.x = *reinterpret_cast<const uint32_t*>(&lo);
+    r.y = *reinterpret_cast<const uint32_t*>(&hi);
+    return r;
+}
+
+// C: CTAs of a cluster.  hs: clusters that share a kv head's query heads.
+template <int C>
+__global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams p, const dc_attn_fuse fuse, const int cap, const int hs) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* sKV = smem;                                           // K rows, after the scores V rows, after P.V partial sums: [key][256]
+    float* sP = reinterpret_cast<float*>(sKV + max(cap * DC_KV_BLOCK * 256, 4 * ATT_MAX_GROUP * 128 * 4));   // scores, then weighted exponentials, see ac_at
+    float* sQ = sP + cap * (DC_KV_BLOCK + 1) * 8;                  // [head][128]
+    float* sPart = sQ + ATT_MAX_GROUP * 128;                       // [head][128], read by the other CTAs
+    float* sBm = sPart + ATT_MAX_GROUP * 128;                      // [block][head]: block maximum, then the maximum to take exponents against
+    float* sW = sBm + cap * 8;                                     // [block][head]: product of the alphas of this CTA's later blocks
+    float* sMax = sW + cap * 8;                                    // [head], read by the other CTAs, as are the next two
+    float* sDen = sMax + 8;
+    float* sProd = sDen + 8;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = (int)ac_rank(), kvh = blockIdx.x / (C * hs), part = blockIdx.x / C % hs, t = blockIdx.y, g = p.n_head / p.n_kv / hs;
+    const int head0 = (kvh * hs + part) * g;                       // first of this cluster's query heads
+    pdl_launch_dependents();
+    const int sid = p.seq_ids[t];
+    const int32_t* table = p.block_tables + (size_t)sid * p.max_blocks;
+    const size_t row = (size_t)p.n_kv * 128;                       // elements per token
+    const uint32_t aKV = smem_u32(sKV);
+    // K rows of keys [from, to), of which this CTA's first is k0
+    auto load_k = [&](int k0, int from, int to) {
+        for (int key = from + (tid >> 4); key < to; key += AC_THREADS / 16) {
+            const size_t off = ((size_t)table[key / DC_KV_BLOCK] * DC_KV_BLOCK + key % DC_KV_BLOCK) * row + kvh * 128 + (tid & 15) * 8;
+            ac_copy16(aKV + ac_piece(key - k0, tid & 15), p.k_arena + off);
+        }
+    };
+    // positions, sequence ids and block tables were settled before this step began, and rows of earlier positions are not written
+    // during it (in an eager chain of steps the position may still be the previous step's here: everything is looked at again after
+    // the wait)
+    const int pos0 = p.positions[t];
+    int stable = pos0;
+    if (!fuse.qkv)
+        for (int u = 0; u < p.T; ++u)
+            if (p.seq_ids[u] == sid) stable = min(stable, p.positions[u]);
+    int n_blk, b0, b1;
+    split_range(pos0, rank, C, n_blk, b0, b1);
+    const bool early = pos0 >= 0 && b1 - b0 <= cap;
+    if (early) load_k(b0 * DC_KV_BLOCK, b0 * DC_KV_BLOCK, min(b1 * DC_KV_BLOCK, stable));
+    auto turn_at = [&](int ps) {
+        const int rp = ps < 0 ? 0 : (fuse.max_pos > 0 && ps >= fuse.max_pos) ? fuse.max_pos - 1 : ps;
+        return reinterpret_cast<const float4*>(fuse.cos_sin + (size_t)rp * 128)[lane];
+    };
+    float4 qw = make_float4(0.f, 0.f, 0.f, 0.f), kw = qw, turn = qw;
+    if (fuse.qkv) {
+        if (fuse.qn_w) qw = reinterpret_cast<const float4*>(fuse.qn_w)[lane];
+        if (fuse.kn_w) kw = reinterpret_cast<const float4*>(fuse.kn_w)[lane];
+        turn = turn_at(pos0);
+    }
+    pdl_wait();
+    const int pos = *reinterpret_cast<const volatile int32_t*>(p.positions + t);
+    split_range(pos, rank, C, n_blk, b0, b1);
+    const int k0 = b0 * DC_KV_BLOCK, nbl = b1 - b0, keys = max(0, min(pos + 1, b1 * DC_KV_BLOCK) - k0);
+    {
+        const bool same = early && pos == pos0;
+        if (!same) asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        load_k(k0, same ? max(k0, stable) : k0, k0 + keys - (fuse.qkv && k0 + keys == pos + 1 ? 1 : 0));
+    }
+    uint2 new_v = make_uint2(0u, 0u);     // the new token's V row (warp 7), which has to wait for the K rows to go
+    const bool mine = fuse.qkv && keys > 0 && k0 + keys == pos + 1;
+    if (fuse.qkv) {
+        const float* src = fuse.qkv + (size_t)t * (p.n_head + 2 * p.n_kv) * 128;
+        if (pos != pos0) turn = turn_at(pos);
+        if (warp < g) reinterpret_cast<float4*>(sQ + warp * 128)[lane] = ac_norm_rope(src + (head0 + warp) * 128, fuse.qn_w != nullptr, qw, true, turn, fuse.eps, lane);
+        if (mine && warp >= 6) {       // the new token's rows: to the cache and to this CTA's tiles
+            const bool is_k = warp == 6;
+            const float4 v = ac_norm_rope(src + (p.n_head + (is_k ? 0 : p.n_kv) + kvh) * 128, is_k && fuse.kn_w, kw, is_k, turn, fuse.eps, lane);
+            const uint2 hv = ac_half4(v);
+            const size_t off = ((size_t)table[pos / DC_KV_BLOCK] * DC_KV_BLOCK + pos % DC_KV_BLOCK) * row + kvh * 128 + 4 * lane;
+            if (part == 0) *reinterpret_cast<uint2*>(const_cast<__half*>(is_k ? p.k_arena : p.v_arena) + off) = hv;
+            if (is_k) *reinterpret_cast<uint2*>(sKV + ac_piece(pos - k0, lane >> 1) + 8 * (lane & 1)) = hv;
+            else new_v = hv;
+        }
+    } else {
+        for (int i = tid; i < g * 32; i += AC_THREADS) reinterpret_cast<float4*>(sQ)[i] = reinterpret_cast<const float4*>(p.q + ((size_t)t * p.n_head + head0) * 128)[i];
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // ---- scores: four lanes per key, lane `sub` takes the 16-byte pieces 4 i + sub of the row
+    for (int key = tid >> 2; key < nbl * DC_KV_BLOCK; key += AC_THREADS / 4) {
+        const int sub = tid & 3;
+        if (key < keys) {
+            float2 kf[16];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 u = *reinterpret_cast<const uint4*>(sKV + ac_piece(key, 4 * i + sub));
+                const __half2* h2 = reinterpret_cast<const __half2*>(&u);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) kf[4 * i + j] = __half22float2(h2[j]);
+            }
+            const uint32_t quad = 0xFu << (lane & ~3);
+            for (int h0 = 0; h0 < g; h0 += 4) {      // four heads at a time: independent chains (heads past the last are read as the last)
+                float2 d[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) d[h] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        const float4* q4 = reinterpret_cast<const float4*>(sQ + min(h0 + h, g - 1) * 128 + (4 * i + sub) * 8);
+                        const float4 a = q4[0], b = q4[1];
+                        ac_fma2(d[h], make_float2(a.x, a.y), kf[4 * i]);
+                        ac_fma2(d[h], make_float2(a.z, a.w), kf[4 * i + 1]);
+                        ac_fma2(d[h], make_float2(b.x, b.y), kf[4 * i + 2]);
+                        ac_fma2(d[h], make_float2(b.z, b.w), kf[4 * i + 3]);
+                    }
+                float mine = 0.0f;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    float dot = d[h].x + d[h].y;
+                    dot += __shfl_xor_sync(quad, dot, 1);
+                    dot += __shfl_xor_sync(quad, dot, 2);
+                    if (h == sub) mine = dot;
+                }
+                if (h0 + sub < g) sP[ac_at(key, h0 + sub)] = __fmul_rn(mine, p.scale);
+            }
+        } else {
+            for (int h = sub; h < g; h += 4) sP[ac_at(key, h)] = -INFINITY;
+        }
+    }
+    __syncthreads();
+    // the V rows follow into the same memory while the block maxima make their way
+    for (int key = tid >> 4; key < keys - (mine ? 1 : 0); key += AC_THREADS / 16) {
+        const int at = k0 + key;
+        const size_t off = ((size_t)table[at / DC_KV_BLOCK] * DC_KV_BLOCK + at % DC_KV_BLOCK) * row + kvh * 128 + (tid & 15) * 8;
+        ac_copy16(aKV + key * 256 + (tid & 15) * 16, p.v_arena + off);
+    }
+    if (mine && warp == 7) *reinterpret_cast<uint2*>(sKV + (pos - k0) * 256 + 8 * lane) = new_v;
+    for (int i = tid; i < nbl * 8; i += AC_THREADS) {
+        const int bl = i >> 3, h = i & 7;
+        if (h < g) {
+            float mx = -1e30f;  // the reference's m_block starts at -1e30
+#pragma unroll
+            for (int k = 0; k < DC_KV_BLOCK; ++k) mx = fmaxf(mx, sP[ac_at(bl * DC_KV_BLOCK + k, h)]);
+            sBm[i] = mx;
+        }
+    }
+    __syncthreads();
+    // ---- the chain: warp h, lane = block
+    float incl = -1e30f, excl = -1e30f;
+    if (warp < g) {
+        if (lane < nbl) incl = sBm[lane * 8 + warp];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl = fmaxf(incl, u);
+        }
+        excl = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) excl = -1e30f;
+        if (lane == 31) sMax[warp] = incl;
+    }
+    ac_sync();
+    if (warp < g) {
+        float m0 = lane < rank ? ac_peer(sMax + warp, lane) : -1e30f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+        const float m_new = fmaxf(m0, incl);
+        const float alpha = lane < nbl ? fast_exp_fma(fmaxf(m0, excl) - m_new) : 1.0f;
+        float after = alpha;   // inclusive product from this block on
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float u = __shfl_down_sync(0xffffffffu, after, o);
+            if (lane + o < 32) after *= u;
+        }
+        float later = __shfl_down_sync(0xffffffffu, after, 1);
+        if (lane == 31) later = 1.0f;
+        if (lane < nbl) {
+            sBm[lane * 8 + warp] = m_new;
+            sW[lane * 8 + warp] = later;
+        }
+        if (lane == 0) sProd[warp] = after;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < nbl * DC_KV_BLOCK * 8; i += AC_THREADS) {
+        const int key = i >> 3, h = i & 7, c = (key >> 4) * 8 + h;
+        if (h < g) {
+            const float s = sP[ac_at(key, h)];
+            sP[ac_at(key, h)] = s == -INFINITY ? 0.0f : __fmul_rn(fast_exp_fma(s - sBm[c]), sW[c]);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (warp < g) {
+        float den = 0.0f;
+        for (int key = lane; key < keys; key += 32) den += sP[ac_at(key, warp)];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+        if (lane == 0) sDen[warp] = den;
+    }
+    // ---- P.V: four groups of threads take every fourth key, a thread two dimensions of all heads
+    {
+        const int kg = tid >> 6, dp = tid & 63;
+        float2 a0[4], a1[4];   // head pairs, of the first and the second dimension
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a0[i] = a1[i] = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+        for (int key = kg; key < keys; key += 4) {
+            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(sKV + key * 256 + dp * 4));
+            const float4* pp = reinterpret_cast<const float4*>(sP + ac_at(key, 0));
+            const float4 x = pp[0], y = pp[1];
+            const float2 vx = make_float2(v.x, v.x), vy = make_float2(v.y, v.y);
+            ac_fma2(a0[0], make_float2(x.x, x.y), vx);
+            ac_fma2(a1[0], make_float2(x.x, x.y), vy);
+            if (g > 2) {
+                ac_fma2(a0[1], make_float2(x.z, x.w), vx);
+                ac_fma2(a1[1], make_float2(x.z, x.w), vy);
+            }
+            if (g > 4) {
+                ac_fma2(a0[2], make_float2(y.x, y.y), vx);
+                ac_fma2(a1[2], make_float2(y.x, y.y), vy);
+            }
+            if (g > 6) {
+                ac_fma2(a0[3], make_float2(y.z, y.w), vx);
+                ac_fma2(a1[3], make_float2(y.z, y.w), vy);
+            }
+        }
+        __syncthreads();      // V has been read
+        float* red = reinterpret_cast<float*>(sKV) + kg * ATT_MAX_GROUP * 128 + 2 * dp;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (2 * i < g) {
+                *reinterpret_cast<float2*>(red + (2 * i) * 128) = make_float2(a0[i].x, a1[i].x);
+                *reinterpret_cast<float2*>(red + (2 * i + 1) * 128) = make_float2(a0[i].y, a1[i].y);
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < g * 128; i += AC_THREADS) {
+        const float* red = reinterpret_cast<const float*>(sKV) + i;
+        sPart[i] = (red[0] + red[ATT_MAX_GROUP * 128]) + (red[2 * ATT_MAX_GROUP * 128] + red[3 * ATT_MAX_GROUP * 128]);
+    }
+    ac_sync();      // (also: every thread of this CTA is done with the key groups' sums)
+    // ---- merge: CTA r writes the head pair r, the 256 values of one Q8_K block of the o-projection's input.  A warp takes C / 8 ranks'
+    // partials, times the alphas of all ranks after; the warps' sums meet in shared memory.
+    float* sSum = reinterpret_cast<float*>(sKV);                   // [warp][256], then [warp][2] denominators (the key groups' sums are done with)
+    if (rank < g / 2) {
+        const int head = 2 * rank + (lane >> 4), d0 = (lane & 15) * 8;
+        constexpr int R = C / 8;
+        float4 a[R], c[R];
+        float dd[R], pr = 1.0f;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            a[r] = ac_peer4(sPart + head * 128 + d0, warp * R + r);
+            c[r] = ac_peer4(sPart + head * 128 + d0 + 4, warp * R + r);
+            dd[r] = ac_peer(sDen + head, warp * R + r);
+        }
+        if ((lane & 15) < C) pr = ac_peer(sProd + head, lane & 15);            // lane of a half: the product of that rank's alphas
+        float after = pr;                                                      // of this rank and all later ones
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const float u = __shfl_down_sync(0xffffffffu, after, o, 16);
+            if ((lane & 15) + o < 16) after *= u;
+        }
+        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, den = 0.0f;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int next = warp * R + r + 1;
+            const float suffix = __shfl_sync(0xffffffffu, after, (lane & 16) + (next & 15));
+            const float f = next < C ? suffix : 1.0f;
+            den += dd[r] * f;
+            v[0] += a[r].x * f; v[1] += a[r].y * f; v[2] += a[r].z * f; v[3] += a[r].w * f;
+            v[4] += c[r].x * f; v[5] += c[r].y * f; v[6] += c[r].z * f; v[7] += c[r].w * f;
+        }
+        float4* o = reinterpret_cast<float4*>(sSum + warp * 256 + lane * 8);
+        o[0] = make_float4(v[0], v[1], v[2], v[3]);
+        o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        if ((lane & 15) == 0) sSum[8 * 256 + warp * 2 + (lane >> 4)] = den;
+    }
+    __syncthreads();
+    if (rank < g / 2 && warp == 0) {
+        const int head = 2 * rank + (lane >> 4), d0 = (lane & 15) * 8;
+        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, den = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const float4* o = reinterpret_cast<const float4*>(sSum + w * 256 + lane * 8);
+            const float4 x = o[0], y = o[1];
+            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+            v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+            den += sSum[8 * 256 + w * 2 + (lane >> 4)];
+        }
+        const float inv = (den > 0.0f && isfinite(den)) ? __fdiv_rn(1.0f, __fadd_rn(den, 1e-6f)) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] *= inv;
+        if (p.out) {
+            float* o = p.out + ((size_t)t * p.n_head + head0 + head) * 128 + d0;
+            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        }
+        if (p.q8_out) quantize_block_q8f_regs(v, p.q8_out + ((size_t)t * (p.n_head / 2) + head0 / 2 + rank) * DC_Q8F_BYTES, lane);
+    }
+    ac_sync();      // nobody leaves while its shared memory is read
+}
+
+static size_t attn_cluster_smem(int cap) {
+    const size_t k = (size_t)cap * DC_KV_BLOCK * 256, red = 4 * ATT_MAX_GROUP * 128 * 4;
+    return (k > red ? k : red) + ((size_t)cap * (DC_KV_BLOCK + 1) * 8 + 2 * ATT_MAX_GROUP * 128 + (size_t)cap * 16 + 24) * 4;
+}
+bool dc_attn_cluster_ok(int max_blocks) { return max_blocks <= 16 * AC_CAP; }
+
+template <int C>
+static int launch_attn_cluster(dc_ctx* ctx, const AttnParams& p, const dc_attn_fuse& fuse, int max_blocks) {
+    const void* f = (const void*)k_attn_cluster<C>;
+    const int cap = (max_blocks + C - 1) / C, g = p.n_head / p.n_kv;
+    const size_t smem = attn_cluster_smem(cap);
+    DC_TRY(dc_kernel_setup(ctx, f, (int)attn_cluster_smem(AC_CAP), "cudaFuncSetAttribute(k_attn_cluster)"));
+    if (C > 8) {       // more than the portable eight, which the device has to allow
+        static std::mutex mu;
+        static bool done[64];
+        std::lock_guard<std::mutex> lk(mu);
+        const int d = ctx->device & 63;
+        if (!done[d]) DC_TRY(dc_check_cuda(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "clusters of sixteen"));
+        done[d] = true;
+    }
+    // few tokens: two clusters share a kv head's query heads, as long as there is an SM for every CTA
+    const int hs = g % 4 == 0 && 2 * p.T * p.n_kv * C <= 128 ? 2 : 1;
+    return dc_launch_cluster(ctx, "k_attn_cluster", k_attn_cluster<C>, dim3(p.n_kv * hs * C, p.T), dim3(AC_THREADS), smem, C, p, fuse, cap, hs);
+}
+
 size_t dc_attention_scratch_bytes(int T, int n_head, int n_kv, int max_blocks, int nsplit) {
     size_t n = 0;
     n += (size_t)T * n_head * max_blocks * DC_KV_BLOCK * 4 + 256;  // scores
@@ -505,7 +911,7 @@ size_t dc_attention_scratch_bytes(int T, int n_head, int n_kv, int max_blocks, i
 int dc_launch_attention(dc_ctx* ctx, const float* q, const void* k_arena, const void* v_arena,
                         const int32_t* block_tables, int max_blocks, const int32_t* seq_ids, const int32_t* positions,
                         int T, int n_head, int n_kv, float scale, int nsplit, const dc_attn_scratch* sc, float* out,
-                        uint8_t* q8_out) {
+                        uint8_t* q8_out, const dc_attn_fuse* fuse) {
     const int g = n_kv > 0 ? n_head / n_kv : 0;
     if (n_kv < 1 || n_head % n_kv || g > ATT_MAX_GROUP || (g & 1))
         return dc_fail(ctx, DC_B200_UNSUPPORTED, "attention: n_head=%d n_kv=%d not supported (group must be even, <= 8)", n_head, n_kv);
@@ -529,6 +935,15 @@ int dc_launch_attention(dc_ctx* ctx, const float* q, const void* k_arena, const 
     p.tickets = sc->tickets;
     p.out = out;
     p.q8_out = q8_out;
+    // The cluster's shared memory holds all keys of a sequence up to a length; longer ones take the split kernels.  Clusters of sixteen
+    // halve a CTA's share but only one fits into a group of SMs: they pay for up to eight clusters, or where eight CTAs cannot hold the keys
+    // (16 Q / 8 KV heads, 512 keys, 4 tokens: 11 us a launch with eight, 26 us with sixteen).
+    if (dc_attn_cluster_ok(max_blocks)) {
+        const dc_attn_fuse none = {};
+        if (max_blocks > 8 * AC_CAP || T * n_kv <= 8) return launch_attn_cluster<16>(ctx, p, fuse ? *fuse : none, max_blocks);
+        return launch_attn_cluster<8>(ctx, p, fuse ? *fuse : none, max_blocks);
+    }
+    if (fuse) return dc_fail(ctx, DC_B200_UNSUPPORTED, "attention: %d blocks a sequence do not fit the fused kernel", max_blocks);
     int st = dc_launch(ctx, "k_attn_scores", k_attn_scores, dim3(nsplit, n_kv, T), dim3(128), 0, p);
     if (st != DC_B200_OK) return st;
     // runs short enough for the kernel that keeps a whole run's scores in shared memory

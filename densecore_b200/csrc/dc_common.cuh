@@ -11,6 +11,7 @@
 #define DC_Q4K_BYTES 144
 #define DC_Q6K_BYTES 210
 #define DC_Q8K_BYTES 292
+#define DC_Q8F_BYTES 320   // a Q8_K block in fragment order, see quantize_block_q8f_regs
 #define DC_KV_BLOCK 16   // core/include/densecore/memory/kv_cache.h:50
 #define DC_MAX_T 16      // tokens per step (kMaxSmallBatchColsHard, core/src/llm/matmul/userdata.h:14)
 #define DC_TYPE_F32 0
@@ -259,13 +260,36 @@ __device__ __forceinline__ void quantize_block_q8k_regs(const float (&v)[8], uin
     if ((lane & 3) == 0) o32[65 + (lane >> 2)] = bw;
     if (lane == 0) o32[0] = __float_as_uint(d);
 }
+// The same block in the order in which the integer tensor instructions of the row kernels (dc_rows.cuh) take it: four runs of 80 bytes, one
+// per thread of a fragment's group of four.  Run t holds word t (four codes) of the block's sixteen 16-value groups, ordered [half][group of the
+// quadrant][quadrant], so that a lane's operands are 16-byte loads.  The runs' last 16 bytes hold the low and the high bytes of the eight
+// 32-value sums (run 0) and the block scale (run 1); those of runs 2 and 3 are not used.  With 320 bytes between rows and 80 between
+// runs eight neighbouring lanes' 16-byte loads fall on distinct banks of shared memory, to which blocks are copied as they are.
+__device__ __forceinline__ void quantize_block_q8f_regs(const float (&v)[8], uint8_t* __restrict__ out, int lane) {
+    uint32_t w0, w1, bw;
+    float d;
+    q8k_block_core(v, lane, w0, w1, bw, d);
+    // words 2 lane and 2 lane + 1: 32-value quadrant lane / 4, group lane / 2 % 2 of it, words 2 (lane % 2) and the next
+    uint32_t* o = reinterpret_cast<uint32_t*>(out) + 40 * (lane & 1) + (lane >> 4) * 8 + ((lane >> 1) & 1) * 4 + ((lane >> 2) & 3);
+    o[0] = w0;
+    o[20] = w1;
+    if ((lane & 3) == 0) {
+        const int s = lane >> 2, sum = (int)(int16_t)(bw & 0xFFFF) + (int)(int16_t)(bw >> 16), lo = (int)(int8_t)(sum & 0xFF);
+        out[64 + s] = (uint8_t)lo;
+        out[72 + s] = (uint8_t)((sum - lo) >> 8);
+    }
+    if (lane == 0) *reinterpret_cast<float*>(out + 144) = d;
+}
+// FRAG: in fragment order.
+template <bool FRAG = false>
 __device__ __forceinline__ void quantize_block_q8k_warp(const float* __restrict__ x, uint8_t* __restrict__ out,
                                                         int lane) {
     float v[8];
     const float4 a = reinterpret_cast<const float4*>(x)[2 * lane];
     const float4 b = reinterpret_cast<const float4*>(x)[2 * lane + 1];
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    quantize_block_q8k_regs(v, out, lane);
+    if (FRAG) quantize_block_q8f_regs(v, out, lane);
+    else quantize_block_q8k_regs(v, out, lane);
 }
 
 // ------------------------------------------------------- activations

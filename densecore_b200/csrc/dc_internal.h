@@ -69,16 +69,20 @@ struct dc_gemv_seg {
 };
 enum { DC_EPI_STORE = 0, DC_EPI_ACC = 1, DC_EPI_SWIGLU = 2 };
 
-// y = W x for T <= 16 tokens whose Q8_K activations are at act_q8 (row stride K/256*292).
+// y = W x for T <= 16 tokens whose Q8_K activations are at act_q8 in fragment order (row stride K/256*320).
 // n_seg 1..3 segments share the activations.  DC_EPI_SWIGLU: seg[0]=gate, seg[1]=up,
 // result silu(gate.x)*(up.x) stored to seg[0].out.  argmax (optional, [T] u64 keys,
 // zeroed by the caller) receives the packed (value,row) maximum of the stored rows.
+// act_f32 (instead of act_q8): the rows before quantisation, which then is part of the kernel; pays where T * K / 256 blocks are few.
 // dump_I / dump_M (parity checks, single segment): receive the exact int32 block sums the kernel forms,
 // [T][n_rows][K/256] (M for Q4_K only).
 DC_PART int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, const uint8_t* act_q8, int T, int K,
-                   unsigned long long* argmax, int32_t* dump_I = nullptr, int32_t* dump_M = nullptr);
-// rows x K f32 -> native Q8_K blocks (row stride K/256*292)
-DC_PART int dc_launch_quantize_q8k(dc_ctx* ctx, const float* x, int rows, int K, uint8_t* out);
+                   unsigned long long* argmax, int32_t* dump_I = nullptr, int32_t* dump_M = nullptr, const float* act_f32 = nullptr);
+// whether k_rows quantises its T rows itself (act_f32): each of its eight warps then has three blocks at most to quantise, about 1 us,
+// against a launch of the chain
+static inline bool dc_rows_quantise(int T, int K) { return T * (K / 256) <= 24; }
+// rows x K f32 -> native Q8_K blocks (row stride K/256*292), or blocks in fragment order (row stride K/256*320)
+DC_PART int dc_launch_quantize_q8k(dc_ctx* ctx, const float* x, int rows, int K, uint8_t* out, bool frag = false);
 // Tensor-core MUL_MAT for many token rows (gemm_tc.cu): activations quantised into 64-token tiles, then
 // out[slot * ldo + row] for every weight row; tile_expert (optional, device) picks an expert matrix per tile.
 DC_PART size_t dc_gemm_tc_act_bytes(int n_slots, int K);
@@ -113,6 +117,13 @@ int dc_launch_argmax_finish(dc_ctx* ctx, unsigned long long* keys, int T, int32_
 int dc_launch_argmax_rows(dc_ctx* ctx, const float* logits, int rows, int n, int32_t* out);
 
 // ---- attn.cu ----
+// What the attention kernel of a decode step does beside attention (qkv given): per-head norm, rotation and cache write of the rows of
+// the fused projection [T][n_head*128 | n_kv*128 | n_kv*128], as dc_launch_qknorm_rope_kv; every token of another sequence.
+struct dc_attn_fuse {
+    const float *qkv, *qn_w, *kn_w, *cos_sin;
+    int max_pos;
+    float eps;
+};
 struct dc_attn_scratch {
     float* scores;    // [T][n_head][max_blocks*16]
     float* bmax;      // [T][n_head][max_blocks]
@@ -125,7 +136,9 @@ DC_PART void dc_attn_scratch_bind(dc_attn_scratch* sc, uint8_t* base, int T, int
 DC_PART int dc_launch_attention(dc_ctx* ctx, const float* q, const void* k_arena, const void* v_arena,
                         const int32_t* block_tables, int max_blocks, const int32_t* seq_ids, const int32_t* positions,
                         int T, int n_head, int n_kv, float scale, int nsplit, const dc_attn_scratch* sc, float* out,
-                        uint8_t* q8_out);
+                        uint8_t* q8_out, const dc_attn_fuse* fuse = nullptr);
+// whether sequences of so many KV blocks take the one-kernel form, which is what `fuse` needs
+DC_PART bool dc_attn_cluster_ok(int max_blocks);
 
 // ---- moe.cu ----
 // causal attention of a prompt chunk (positions pos0 .. pos0 + n - 1 of one sequence) on the tensor cores
@@ -146,15 +159,28 @@ struct dc_moe_route {
 // (core/src/llm/moe/native.cpp:610-676); DC_ROUTE_SOFTMAX = softmax over all experts, top-k on the
 // probabilities with strict '>', renormalise (core/src/moe/moe_routing.cpp:53-101).
 enum { DC_ROUTE_STABLE = 0, DC_ROUTE_SOFTMAX = 1 };
+// Given: the router norms the residual rows x itself (xn is not read) and writes their Q8_K blocks in fragment order.  Every CTA norms
+// all rows, so this is for few tokens.
+struct dc_route_norm {
+    const float *x, *w;
+    float eps;
+    uint8_t* q8_out;
+};
 DC_PART int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_expert, int T, int top_k, float scale,
-                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode = DC_ROUTE_STABLE);
+                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode = DC_ROUTE_STABLE, const dc_route_norm* norm = nullptr);
 // the same routing for any number of tokens (prompt chunks): logits [T][E], ids and weights [T][top_k]
 int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, int T, int top_k, float scale, float* logits,
                              int32_t* ids, float* weights, int mode);
 // carves a dc_moe_route for (T, E, top_k) out of a byte buffer; returns bytes used
 DC_PART size_t dc_moe_route_bind(dc_moe_route* rt, uint8_t* base, int T, int E, int top_k);
+// whether the down projection quantises its rows itself: a CTA then has few blocks to quantise, and a launch of the chain goes away
+static inline bool dc_moe_quantise_in_down(int T) { return T <= 4; }
 DC_PART int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weight* w1, const uint8_t* act_q8,
-                     int act_rows, int T, int top_k, int e_base, const dc_moe_route* rt, float* out);
+                     int T, int top_k, int e_base, const dc_moe_route* rt, float* out, const float* act_f32 = nullptr);
+// x += the experts' weighted sum (as dc_launch_moe_combine), then RMSNorm (xn_out, optional) and Q8_K blocks in
+// fragment order (q8_out, optional), one kernel
+DC_PART int dc_launch_moe_combine_norm(dc_ctx* ctx, const float* dn, const int32_t* ids, const float* weights, int T, int top_k, int H, float* x,
+                               const float* norm_w, float eps, float* xn_out, uint8_t* q8_out);
 DC_PART int dc_launch_moe_combine(dc_ctx* ctx, const float* dn, const int32_t* ids, const float* weights, int T, int top_k,
                           int H, int ep_lo, int ep_hi, float* out);
 

@@ -68,6 +68,7 @@ int dc_launch_embed(dc_ctx* ctx, const dc_weight* w, const int32_t* tokens, int 
 }
 
 // ------------------------------------------------------ RMSNorm + Q8_K
+// (blocks in fragment order).
 // One CTA per token.  x (+= add, if given) -> y = x / sqrt(mean(x^2)+eps) * w
 // (core/src/llm/graph/decoder.cpp:268), then Q8_K blocks of y
 // (core/src/kernels/hwy/hwy_moe_quant.cc:103-144).  xn_out / q8_out optional.
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_q8k(float* __restrict__ x, cons
     if (q8_out) {
         const int nb = H / DC_QK_K;
         for (int b = warp; b < nb; b += 8)
-            quantize_block_q8k_warp(sx + b * DC_QK_K, q8_out + ((size_t)t * nb + b) * DC_Q8K_BYTES, lane);
+            quantize_block_q8k_warp<true>(sx + b * DC_QK_K, q8_out + ((size_t)t * nb + b) * DC_Q8F_BYTES, lane);
     }
 }
 

@@ -165,9 +165,9 @@ static int alloc_step_buffers(dc_model* m) {
     DC_TRY(dev_alloc(ctx, &b.attn_mem, att_bytes));
     dc_attn_scratch_bind(&b.attn, b.attn_mem, (int)T, c.n_head, c.n_kv_head, m->kv.max_blocks_per_seq, m->nsplit);
     DC_TRY(dc_check_cuda(ctx, cudaMemsetAsync(b.attn.tickets, 0, T * c.n_head * 4, ctx->stream), "memset"));
-    DC_TRY(dev_alloc(ctx, &b.q8_x, T * (H / 256) * 292));
-    DC_TRY(dev_alloc(ctx, &b.q8_attn, T * (QD / 256) * 292));
-    DC_TRY(dev_alloc(ctx, &b.q8_h, A * (F / 256) * 292));
+    DC_TRY(dev_alloc(ctx, &b.q8_x, T * (H / 256) * DC_Q8F_BYTES));
+    DC_TRY(dev_alloc(ctx, &b.q8_attn, T * (QD / 256) * DC_Q8F_BYTES));
+    DC_TRY(dev_alloc(ctx, &b.q8_h, A * (F / 256) * DC_Q8F_BYTES));
     DC_TRY(dev_alloc(ctx, &b.history, (size_t)DC_HISTORY_CAP * T));
     DC_TRY(dev_alloc(ctx, &b.history_len, 1));
     if (c.n_expert > 0) {
@@ -192,8 +192,8 @@ static int alloc_step_buffers(dc_model* m) {
 }
 
 // ------------------------------------------------------------- one step
-// lm_mode: 0 no logits, 1 last row only, 2 every row.
-static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback) {
+// lm_mode: 0 no logits, 1 last row only, 2 every row.  chunk: the tokens are neighbours in one sequence, not one each of several.
+static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool chunk) {
     const dc_model_config& c = m->cfg;
     dc_ctx* ctx = m->ctx;
     dc_step_buffers& b = m->buf;
@@ -218,13 +218,20 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback) {
         }                                                               \
         launches += (n);                                                \
     } while (0)
-    const double q8x = (double)T * (H / 256) * 292, xb = (double)T * H * 4;
+    const double q8x = (double)T * (H / 256) * DC_Q8F_BYTES, xb = (double)T * H * 4;
     L(DC_K_EMBED, m->tok_embd->row_bytes * T + xb, 1, dc_launch_embed(ctx, m->tok_embd, b.tokens, T, b.x));
     const float* pending = nullptr;  // MoE output of the previous layer, added in the next norm
+    bool split = false;              // the previous layer's expert outputs wait for their weighted sum
+    const bool sum_in_norm = E > 0 && c.ep_size == 1;
     for (int il = 0; il < c.n_layer; ++il) {
         dc_layer& Ly = m->layers[il];
-        L(DC_K_RMSNORM, xb + q8x + H * 4, 1,
-          dc_launch_rmsnorm_q8k(ctx, b.x, pending, (const float*)Ly.attn_norm->dev, T, H, c.rms_eps, nullptr, b.q8_x));
+        if (split)
+            L(DC_K_COMBINE, (double)T * top_k * H * 4 + xb + q8x, 1,
+              dc_launch_moe_combine_norm(ctx, b.dn, b.route.ids, b.route.weights, T, top_k, H, b.x, (const float*)Ly.attn_norm->dev, c.rms_eps, nullptr, b.q8_x));
+        else
+            L(DC_K_RMSNORM, xb + q8x + H * 4, 1,
+              dc_launch_rmsnorm_q8k(ctx, b.x, pending, (const float*)Ly.attn_norm->dev, T, H, c.rms_eps, nullptr, b.q8_x));
+        split = false;
         pending = nullptr;
         if (m->dbg_x)
             DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(m->dbg_x + (size_t)il * DC_MAX_T * H, b.x, (size_t)T * H * 4, cudaMemcpyDeviceToDevice, ctx->stream), "capture"));
@@ -237,34 +244,46 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback) {
           dc_launch_gemv(ctx, qkv, 3, DC_EPI_STORE, b.q8_x, T, H, nullptr));
         __half* ka = m->kv.k_arena + m->kv.layer_elems * il;
         __half* va = m->kv.v_arena + m->kv.layer_elems * il;
-        L(DC_K_QKROPE, (double)T * QKV * 4 * 2, 1,
-          dc_launch_qknorm_rope_kv(ctx, b.qkv, Ly.q_norm ? (const float*)Ly.q_norm->dev : nullptr,
-                                   Ly.k_norm ? (const float*)Ly.k_norm->dev : nullptr, b.cos_sin, c.max_ctx, b.positions,
-                                   b.seq_ids, m->kv.d_tables, m->kv.max_blocks_per_seq, ka, va, c.n_head, c.n_kv_head,
-                                   c.rms_eps, T, b.q));
+        const dc_attn_fuse fuse = {b.qkv, Ly.q_norm ? (const float*)Ly.q_norm->dev : nullptr, Ly.k_norm ? (const float*)Ly.k_norm->dev : nullptr,
+                                   b.cos_sin, c.max_ctx, c.rms_eps};
+        // one kernel where a token's attention does not read rows that the same step writes
+        const bool one = dc_attn_cluster_ok(m->kv.max_blocks_per_seq) && (!chunk || T == 1);
+        if (!one)
+            L(DC_K_QKROPE, (double)T * QKV * 4 * 2, 1,
+              dc_launch_qknorm_rope_kv(ctx, b.qkv, fuse.qn_w, fuse.kn_w, b.cos_sin, c.max_ctx, b.positions,
+                                       b.seq_ids, m->kv.d_tables, m->kv.max_blocks_per_seq, ka, va, c.n_head, c.n_kv_head,
+                                       c.rms_eps, T, b.q));
         // KV bytes depend on the context length; filled in by the caller of the profile
-        L(DC_K_ATTENTION, 0.0, 2,
+        L(DC_K_ATTENTION, 0.0, dc_attn_cluster_ok(m->kv.max_blocks_per_seq) ? 1 : 2,
           dc_launch_attention(ctx, b.q, ka, va, m->kv.d_tables, m->kv.max_blocks_per_seq, b.seq_ids, b.positions, T,
-                              c.n_head, c.n_kv_head, scale, m->nsplit, &b.attn, nullptr, b.q8_attn));
+                              c.n_head, c.n_kv_head, scale, m->nsplit, &b.attn, nullptr, b.q8_attn, one ? &fuse : nullptr));
         dc_gemv_seg wo = {Ly.wo->dev, Ly.wo->type, H, (int)Ly.wo->row_bytes, b.x, H};
-        L(DC_K_GEMV_O, (double)Ly.wo->bytes + (double)T * (QD / 256) * 292 + 2 * xb, 1,
+        L(DC_K_GEMV_O, (double)Ly.wo->bytes + (double)T * (QD / 256) * DC_Q8F_BYTES + 2 * xb, 1,
           dc_launch_gemv(ctx, &wo, 1, DC_EPI_ACC, b.q8_attn, T, QD, nullptr));
-        L(DC_K_RMSNORM, xb * (E > 0 ? 2 : 1) + q8x + H * 4, 1,
-          dc_launch_rmsnorm_q8k(ctx, b.x, nullptr, (const float*)Ly.ffn_norm->dev, T, H, c.rms_eps,
-                                E > 0 ? b.xn : nullptr, b.q8_x));
+        // few tokens: the router norms them itself
+        const dc_route_norm rn = {b.x, (const float*)Ly.ffn_norm->dev, c.rms_eps, b.q8_x};
+        const bool norm_in_router = E > 0 && T <= 4 && (size_t)T * H * 4 <= 128 * 1024;
+        if (!norm_in_router)
+            L(DC_K_RMSNORM, xb * (E > 0 ? 2 : 1) + q8x + H * 4, 1,
+              dc_launch_rmsnorm_q8k(ctx, b.x, nullptr, (const float*)Ly.ffn_norm->dev, T, H, c.rms_eps,
+                                    E > 0 ? b.xn : nullptr, b.q8_x));
         if (E > 0) {
             const int A = T * top_k, F = c.expert_ffn;
             // distinct experts hit: top_k for one token; for T > 1 the host only knows the bound
             const double U = T == 1 ? top_k : (A < E ? A : E);
             const double local = (double)(ep_hi - ep_lo) / E;
             L(DC_K_ROUTER, (double)Ly.router->bytes + xb, 1,
-              dc_launch_router(ctx, Ly.router, b.xn, E, T, top_k, c.routed_scale, ep_lo, ep_hi, &b.route, m->route_mode));
+              dc_launch_router(ctx, Ly.router, b.xn, E, T, top_k, c.routed_scale, ep_lo, ep_hi, &b.route, m->route_mode, norm_in_router ? &rn : nullptr));
             L(DC_K_MOE_GATEUP, U * local * 2.0 * F * Ly.gate_exps->row_bytes + q8x + (double)A * F * 4, 1,
-              dc_launch_moe_mm(ctx, true, Ly.gate_exps, Ly.up_exps, b.q8_x, T, T, top_k, ep_lo, &b.route, b.h));
-            L(DC_K_QUANT_H, (double)A * F * 4 + (double)A * (F / 256) * 292, 1,
-              dc_launch_quantize_q8k(ctx, b.h, A, F, b.q8_h));
-            L(DC_K_MOE_DOWN, U * local * H * Ly.down_exps->row_bytes + (double)A * (F / 256) * 292 + (double)A * H * 4, 1,
-              dc_launch_moe_mm(ctx, false, Ly.down_exps, nullptr, b.q8_h, A, T, top_k, ep_lo, &b.route, b.dn));
+              dc_launch_moe_mm(ctx, true, Ly.gate_exps, Ly.up_exps, b.q8_x, T, top_k, ep_lo, &b.route, b.h));
+            const bool own = dc_moe_quantise_in_down(T);
+            if (!own)
+                L(DC_K_QUANT_H, (double)A * F * 4 + (double)A * (F / 256) * DC_Q8F_BYTES, 1,
+                  dc_launch_quantize_q8k(ctx, b.h, A, F, b.q8_h, true));
+            L(DC_K_MOE_DOWN, U * local * H * Ly.down_exps->row_bytes + (double)A * (F / 256) * DC_Q8F_BYTES + (double)A * H * 4, 1,
+              dc_launch_moe_mm(ctx, false, Ly.down_exps, nullptr, b.q8_h, T, top_k, ep_lo, &b.route, b.dn, own ? b.h : nullptr));
+            split = sum_in_norm && il + 1 < c.n_layer;
+            if (split) continue;
             L(DC_K_COMBINE, (double)A * H * 4 + xb, 1,
               dc_launch_moe_combine(ctx, b.dn, b.route.ids, b.route.weights, T, top_k, H, ep_lo, ep_hi, b.moe_out));
             if (c.ep_size > 1) L(DC_K_ALLREDUCE, xb, 1, dc_ep_allreduce(m, b.moe_out, (size_t)T * H));
@@ -276,23 +295,25 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback) {
             };
             L(DC_K_FFN_GATEUP, (double)Ly.ffn_gate->bytes + Ly.ffn_up->bytes + q8x + (double)T * c.ffn * 4, 1,
               dc_launch_gemv(ctx, gu, 2, DC_EPI_SWIGLU, b.q8_x, T, H, nullptr));
-            L(DC_K_QUANT_H, (double)T * c.ffn * 4 + (double)T * (c.ffn / 256) * 292, 1,
-              dc_launch_quantize_q8k(ctx, b.h, T, c.ffn, b.q8_h));
+            const bool own = dc_rows_quantise(T, c.ffn);
+            if (!own)
+                L(DC_K_QUANT_H, (double)T * c.ffn * 4 + (double)T * (c.ffn / 256) * DC_Q8F_BYTES, 1,
+                  dc_launch_quantize_q8k(ctx, b.h, T, c.ffn, b.q8_h, true));
             dc_gemv_seg dw = {Ly.ffn_down->dev, Ly.ffn_down->type, H, (int)Ly.ffn_down->row_bytes, b.x, H};
-            L(DC_K_FFN_DOWN, (double)Ly.ffn_down->bytes + (double)T * (c.ffn / 256) * 292 + 2 * xb, 1,
-              dc_launch_gemv(ctx, &dw, 1, DC_EPI_ACC, b.q8_h, T, c.ffn, nullptr));
+            L(DC_K_FFN_DOWN, (double)Ly.ffn_down->bytes + (double)T * (c.ffn / 256) * DC_Q8F_BYTES + 2 * xb, 1,
+              dc_launch_gemv(ctx, &dw, 1, DC_EPI_ACC, b.q8_h, T, c.ffn, nullptr, nullptr, nullptr, own ? b.h : nullptr));
         }
     }
     if (lm_mode != 0) {
         const int rows = lm_mode == 1 ? 1 : T, first = lm_mode == 1 ? T - 1 : 0;
-        L(DC_K_RMSNORM, (double)rows * H * 4 * 2 + (double)rows * (H / 256) * 292, 1,
+        L(DC_K_RMSNORM, (double)rows * H * 4 * 2 + (double)rows * (H / 256) * DC_Q8F_BYTES, 1,
           dc_launch_rmsnorm_q8k(ctx, b.x + (size_t)first * H, pending ? pending + (size_t)first * H : nullptr,
                                 (const float*)m->out_norm->dev, rows, H, c.rms_eps, nullptr, b.q8_x));
         if (m->dbg_x)
             DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(m->dbg_x + ((size_t)c.n_layer * DC_MAX_T + first) * H, b.x + (size_t)first * H, (size_t)rows * H * 4, cudaMemcpyDeviceToDevice, ctx->stream), "capture"));
         const dc_weight* out_w = c.tie_embeddings ? m->tok_embd : m->output;
         dc_gemv_seg lm = {out_w->dev, out_w->type, c.vocab, (int)out_w->row_bytes, b.logits, c.vocab};
-        L(DC_K_LM_HEAD, (double)out_w->bytes + (double)rows * (H / 256) * 292 + (double)rows * c.vocab * 4, 1,
+        L(DC_K_LM_HEAD, (double)out_w->bytes + (double)rows * (H / 256) * DC_Q8F_BYTES + (double)rows * c.vocab * 4, 1,
           dc_launch_gemv(ctx, &lm, 1, DC_EPI_STORE, b.q8_x, rows, H, b.argmax_keys));
         L(DC_K_ARGMAX, 64.0, 1,
           dc_launch_argmax_finish(ctx, b.argmax_keys, rows, b.out_tokens, feedback ? b.tokens : nullptr,
@@ -308,9 +329,9 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback) {
 // chunk: the T tokens are consecutive positions of one sequence (otherwise one token each of T sequences).
 static int run_forward(dc_model* m, int T, int lm_mode, bool feedback, bool chunk = false) {
     dc_ctx* ctx = m->ctx;
-    auto enqueue = [&]() { return m->stack ? dc_stack_enqueue_small(m, T, chunk, lm_mode, feedback) : enqueue_forward(m, T, lm_mode, feedback); };
+    auto enqueue = [&]() { return m->stack ? dc_stack_enqueue_small(m, T, chunk, lm_mode, feedback) : enqueue_forward(m, T, lm_mode, feedback, chunk); };
     if (!m->use_graphs || m->dbg_x) return enqueue();
-    const int key = T * 8 + lm_mode * 2 + (feedback ? 1 : 0) + (m->stack && chunk ? 1024 : 0);
+    const int key = T * 8 + lm_mode * 2 + (feedback ? 1 : 0) + (chunk && (m->stack || T > 1) ? 1024 : 0);
     auto it = m->graphs.find(key);
     if (it == m->graphs.end()) {
         // one eager pass first: it sets kernel attributes, which is not allowed while capturing
@@ -355,11 +376,12 @@ static int upload_step_inputs(dc_model* m, const int32_t* tokens, const int32_t*
     return DC_B200_OK;
 }
 
-// The persistent kernel serves decode steps of MoE models.  With two or more streams every phase is bound
-// by instruction issue and the per-op kernels (more resident warps per SM) are faster (measured: 1116 vs
-// 1284 us per step at 2 streams, 1546 vs 2059 at 4, 8-layer cut), so the default sends one stream to it.
+// The persistent kernel serves decode steps of MoE models where it is asked for (use_mega 2), and one stream of an expert-parallel
+// model, whose ranks exchange expert outputs inside it.  Elsewhere the per-op kernels are faster: its seven grid barriers a layer cost
+// more than seven launches that overlap, and its row dots stay on dp4a.  (8-layer cut, 2048 tokens of context, us a step: one stream
+// 681 persistent, 518 per-op; four 2059 and 935.)
 static bool mega_ok(dc_model* m, int T) {
-    if (m->stack || !m->use_mega || (m->use_mega == 1 && T > 1)) return false;
+    if (m->stack || !m->use_mega || (m->use_mega == 1 && (T > 1 || m->cfg.ep_size == 1))) return false;
     MegaParams p;
     const char* why = "";
     return dc_mega_plan(m, T, &p, &why);

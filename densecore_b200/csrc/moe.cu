@@ -4,15 +4,15 @@
 //   k_router      router logits (F32 matmul, core/src/llm/graph/decoder.cpp:2265),
 //                 stable top-k + weights (core/src/llm/moe/native.cpp:610-676),
 //                 token->expert bucketing (core/src/moe/moe_routing.cpp:534-603)
-//   k_moe_mm<PAIR> gate/up + SwiGLU for every (distinct expert, row), each expert's
+//   k_moe_rows<PAIR> gate/up + SwiGLU for every (distinct expert, row), each expert's
 //                 weights read once for all its tokens (native.cpp:3929-4345)
-//   k_moe_mm      down projection per assignment (native.cpp:3051-3295)
+//   k_moe_rows    down projection per assignment (native.cpp:3051-3295)
 //   k_moe_combine weighted sum in the reference's order
 //                 (cpu_backend_moe_ops.cpp:1578-1597, moe_routing.cpp:647-676)
 #include "dc_common.cuh"
 #include "dc_internal.h"
 #include "dc_launch.cuh"
-#include "dc_stream.cuh"
+#include "dc_rows.cuh"
 
 using namespace dc;
 
@@ -35,6 +35,7 @@ struct RouterParams {
     int32_t* uexp;        // [E]   distinct local experts, ascending
     int32_t* uoff;        // [E+1] offsets into uassign
     int32_t* uassign;     // [T*top_k] assignment indices t*top_k+k, grouped by expert, routing order inside
+    dc_route_norm norm;   // x given: rows still to be normed
 };
 
 __device__ __forceinline__ unsigned long long route_key(float v, int id) {
@@ -155,10 +156,61 @@ __device__ __forceinline__ void route_token(const RouterParams& p, int t, int la
     }
 }
 
+// Routing of all T tokens by the whole CTA (DC_ROUTE_STABLE): an expert's place among a token's experts is the number of keys above its
+// own, so all experts find theirs at once; route_token's rounds of warp-wide maxima took 4.6 us a token.  Same picks, same weights.
+// s_key: 256 keys; s_sel: T * top_k picked logits.
+__device__ __forceinline__ void route_all_stable(const RouterParams& p, unsigned long long* s_key, float* s_sel, int32_t* s_ids) {
+    const int tid = threadIdx.x, per = p.E <= 32 ? 8 : p.E <= 64 ? 4 : p.E <= 128 ? 2 : 1;     // tokens at a time
+    const int width = 256 / per, slot = tid / width, e = tid % width;
+    for (int t0 = 0; t0 < p.T; t0 += per) {
+        const int t = t0 + slot;
+        const bool in = t < p.T && e < p.E;
+        const float v = in ? __ldcg(p.logits + (size_t)t * p.E + e) : 0.0f;
+        const unsigned long long key = in ? route_key(v, e) : 0ull;      // a real key is never 0
+        s_key[tid] = key;
+        __syncthreads();
+        if (in) {
+            int above = 0;
+            const unsigned long long* k = s_key + slot * width;
+#pragma unroll 8
+            for (int f = 0; f < p.E; ++f) above += k[f] > key;
+            if (above < p.top_k) {
+                const uint32_t ku = (uint32_t)(key >> 32);
+                s_sel[t * p.top_k + above] = __uint_as_float((ku & 0x80000000u) ? (ku & 0x7FFFFFFFu) : ~ku);    // (-0 became +0)
+                s_ids[t * p.top_k + above] = e;
+                p.ids[t * p.top_k + above] = e;
+            }
+        }
+        __syncthreads();
+    }
+    // weights over the selected experts only (native.cpp:649-674)
+    for (int i = tid; i < p.T * p.top_k; i += 256) {
+        const float* sel = s_sel + i / p.top_k * p.top_k;
+        float mx = -INFINITY;
+        bool finite = true;
+        for (int k = 0; k < p.top_k; ++k) {
+            finite = finite && isfinite(sel[k]);
+            if (isfinite(sel[k]) && sel[k] > mx) mx = sel[k];
+        }
+        float den = 0.0f, own = 0.0f;
+        if (finite && isfinite(mx)) {
+            for (int k = 0; k < p.top_k; ++k) {
+                const float w = expf(sel[k] - mx);
+                if (k == i % p.top_k) own = w;
+                den += w;
+            }
+        }
+        const bool ok = den > 0.0f && isfinite(den);
+        p.weights[i] = __fmul_rn(ok ? __fdiv_rn(own, den) : __fdiv_rn(1.0f, (float)p.top_k), p.scale);
+    }
+}
+
 __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     __shared__ int s_last;
     __shared__ float s_prob[8][MOE_MAX_E];
     __shared__ int32_t s_ids[DC_MAX_T * MOE_MAX_K];
+    __shared__ unsigned long long s_key[256];
+    __shared__ float s_sel[DC_MAX_T * MOE_MAX_K];
     __shared__ int s_wsum_a[8], s_wsum_c[8];
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -176,7 +228,54 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
                          : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
+    float4 nw[2] = {};      // norm weights, which are older than the previous kernel too
+    if (p.norm.x) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if ((int)threadIdx.x + 256 * j < p.H / 4) nw[j] = reinterpret_cast<const float4*>(p.norm.w)[threadIdx.x + 256 * j];
+    }
     pdl_wait();
+    const float* xn = p.xn;
+    if (p.norm.x) {
+        // every CTA norms all rows (k_rmsnorm_q8k's arithmetic) into shared memory; the blocks to quantise are shared out
+        extern __shared__ __align__(16) float s_xn[];
+        __shared__ double s_ss[8][4];
+        float4* sx4 = reinterpret_cast<float4*>(s_xn);
+        const int n4 = p.H / 4;
+        for (int t = 0; t < p.T; ++t) {
+            const float4* xr = reinterpret_cast<const float4*>(p.norm.x + (size_t)t * p.H);
+            double ss = 0.0;
+            for (int i0 = 0; i0 < n4; i0 += 512) {       // two loads in flight
+                const int i = i0 + threadIdx.x, k = i + 256;
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = i < n4 ? __ldcg(xr + i) : zero, b = k < n4 ? __ldcg(xr + k) : zero;
+                if (i < n4) sx4[t * n4 + i] = a;
+                if (k < n4) sx4[t * n4 + k] = b;
+                ss += ((double)a.x * a.x + (double)a.y * a.y) + ((double)a.z * a.z + (double)a.w * a.w);
+                ss += ((double)b.x * b.x + (double)b.y * b.y) + ((double)b.z * b.z + (double)b.w * b.w);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0) s_ss[warp][t] = ss;
+        }
+        __syncthreads();
+        for (int t = 0; t < p.T; ++t) {
+            double tot = 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tot += s_ss[i][t];
+            const float mean = (float)(tot / (double)p.H);
+            const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.norm.eps)));
+            for (int i = threadIdx.x, j = 0; i < n4; i += 256, ++j) {
+                const float4 v = sx4[t * n4 + i], w = j < 2 ? nw[j] : reinterpret_cast<const float4*>(p.norm.w)[i];
+                sx4[t * n4 + i] = make_float4(__fmul_rn(__fmul_rn(v.x, scale), w.x), __fmul_rn(__fmul_rn(v.y, scale), w.y),
+                                              __fmul_rn(__fmul_rn(v.z, scale), w.z), __fmul_rn(__fmul_rn(v.w, scale), w.w));
+            }
+        }
+        __syncthreads();
+        const int nb = p.H / DC_QK_K;
+        for (int i = warp * gridDim.x + blockIdx.x; i < p.T * nb; i += 8 * gridDim.x)
+            quantize_block_q8k_warp<true>(s_xn + i * DC_QK_K, p.norm.q8_out + (size_t)i * DC_Q8F_BYTES, lane);
+        xn = s_xn;
+    }
     if (p.wr) {
         __shared__ float s_part[8][DC_MAX_T];
         const int e = blockIdx.x * 2 + (warp >> 2), quarter = warp & 3;
@@ -196,7 +295,7 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
 #pragma unroll
                 for (int t = 0; t < DC_MAX_T; ++t) {
                     if (t < p.T) {
-                        const float4* x4 = reinterpret_cast<const float4*>(p.xn + (size_t)t * p.H + quarter * seg);
+                        const float4* x4 = reinterpret_cast<const float4*>(xn + (size_t)t * p.H + quarter * seg);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const int i = i0 + j * 32 + lane;
@@ -242,8 +341,10 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     __syncthreads();
     if (!s_last) return;
 
-    // ---- stable top-k per token, one warp per token
-    for (int t = warp; t < p.T; t += 8) route_token(p, t, lane, s_prob[warp], s_ids);
+    // ---- top-k per token
+    if (p.mode == DC_ROUTE_STABLE) route_all_stable(p, s_key, s_sel, s_ids);
+    else
+        for (int t = warp; t < p.T; t += 8) route_token(p, t, lane, s_prob[warp], s_ids);
     __syncthreads();
     // ---- bucketing: thread e owns expert e
     const int A = p.T * p.top_k;
@@ -292,61 +393,60 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
 }
 
 // ------------------------------------------- router over a prompt chunk
-// The same arithmetic as k_router for any number of tokens: logits by CTAs of two experts x sixteen tokens
-// (four warps per expert, a quarter of the row each, lane partials chained by fma in the same element order,
-// butterfly sum, quarters added pairwise), then one warp per token for the selection.  No bucketing: the
-// chunk's assignments are grouped by k_moe_group.
+// The same arithmetic as k_router for any number of tokens, bit for bit: four warps per expert, a quarter of the row each, lane partials
+// chained by fma in the same element order, butterfly sum, quarters added pairwise.  A warp keeps the partials of four experts x eight
+// tokens, so that twelve 16-byte loads feed 128 multiply-adds (the first form, two experts x sixteen tokens a CTA with one expert a warp,
+// read every token's row 64 times over: 194 us for 2048 tokens, 128 experts and 2048 columns, at 5 % of the multiply-adds' rate).
+// Its 32 sums over the lanes take 31 exchanges: each step halves the sums that a lane still holds, and adds the same pairs
+// as a butterfly of every sum would.  No bucketing: the chunk's assignments are grouped by k_moe_group.
+#define RB_E 4     // experts of a warp
+#define RB_T 8     // tokens of a warp
 __global__ void __launch_bounds__(256) k_router_logits_batched(const RouterParams p) {
-    __shared__ float s_part[8][DC_MAX_T];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.x * 2 + (warp >> 2), quarter = warp & 3, seg = p.H / 4;
-    const int t0 = blockIdx.y * DC_MAX_T, tn = min(DC_MAX_T, p.T - t0);
-    float acc[DC_MAX_T];
+    __shared__ float s_part[8][RB_E * RB_T];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quarter = warp & 3, seg = p.H / 4;
+    const int e0 = (blockIdx.x * 2 + (warp >> 2)) * RB_E, t0 = blockIdx.y * RB_T;
+    float acc[RB_E * RB_T];
 #pragma unroll
-    for (int t = 0; t < DC_MAX_T; ++t) acc[t] = 0.0f;
-    if (e < p.E) {
-        const float4* w4 = reinterpret_cast<const float4*>(p.wr + (size_t)e * p.H + quarter * seg);
-        for (int i0 = 0; i0 < seg / 4; i0 += 128) {
-            float4 wv[4];
+    for (int i = 0; i < RB_E * RB_T; ++i) acc[i] = 0.0f;
+    const float4 *w4[RB_E], *x4[RB_T];   // (experts and tokens past the end are read as the last one)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = i0 + j * 32 + lane;
-                wv[j] = i < seg / 4 ? w4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int e = 0; e < RB_E; ++e) w4[e] = reinterpret_cast<const float4*>(p.wr + (size_t)min(e0 + e, p.E - 1) * p.H + quarter * seg);
+#pragma unroll
+    for (int t = 0; t < RB_T; ++t) x4[t] = reinterpret_cast<const float4*>(p.xn + (size_t)min(t0 + t, p.T - 1) * p.H + quarter * seg);
+    for (int i = lane; i < seg / 4; i += 32) {
+        float4 w[RB_E], x[RB_T];
+#pragma unroll
+        for (int e = 0; e < RB_E; ++e) w[e] = w4[e][i];
+#pragma unroll
+        for (int t = 0; t < RB_T; ++t) x[t] = x4[t][i];
+#pragma unroll
+        for (int e = 0; e < RB_E; ++e)
+#pragma unroll
+            for (int t = 0; t < RB_T; ++t) {
+                float& a = acc[e * RB_T + t];
+                a = fmaf(w[e].x, x[t].x, a);
+                a = fmaf(w[e].y, x[t].y, a);
+                a = fmaf(w[e].z, x[t].z, a);
+                a = fmaf(w[e].w, x[t].w, a);
             }
+    }
+    // after the step over lane bit o a lane holds the sums whose index has that bit as its own lane number has
 #pragma unroll
-            for (int t = 0; t < DC_MAX_T; ++t) {
-                if (t < tn) {
-                    const float4* x4 = reinterpret_cast<const float4*>(p.xn + (size_t)(t0 + t) * p.H + quarter * seg);
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool upper = lane & o;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int i = i0 + j * 32 + lane;
-                        if (i < seg / 4) {
-                            const float4 xv = x4[i];
-                            acc[t] = fmaf(wv[j].x, xv.x, acc[t]);
-                            acc[t] = fmaf(wv[j].y, xv.y, acc[t]);
-                            acc[t] = fmaf(wv[j].z, xv.z, acc[t]);
-                            acc[t] = fmaf(wv[j].w, xv.w, acc[t]);
-                        }
-                    }
-                }
-            }
+        for (int i = 0; i < o; ++i) {
+            const float mine = upper ? acc[i + o] : acc[i], other = upper ? acc[i] : acc[i + o];
+            acc[i] = mine + __shfl_xor_sync(0xffffffffu, other, o);
         }
     }
-#pragma unroll
-    for (int t = 0; t < DC_MAX_T; ++t) {
-        if (t < tn) {
-            float v = acc[t];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) s_part[warp][t] = v;
-        }
-    }
+    s_part[warp][lane] = acc[0];
     __syncthreads();
-    if (threadIdx.x < 2 * tn) {
-        const int which = threadIdx.x / tn, t = threadIdx.x % tn, ee = blockIdx.x * 2 + which;
-        if (ee < p.E)
-            p.logits[(size_t)(t0 + t) * p.E + ee] = (s_part[which * 4][t] + s_part[which * 4 + 1][t]) +
-                                                    (s_part[which * 4 + 2][t] + s_part[which * 4 + 3][t]);
+    if (threadIdx.x < 2 * RB_E * RB_T) {
+        const int which = threadIdx.x >> 5, i = threadIdx.x & 31;
+        const int e = (blockIdx.x * 2 + which) * RB_E + i / RB_T, t = t0 + i % RB_T;
+        if (e < p.E && t < p.T)
+            p.logits[(size_t)t * p.E + e] = (s_part[which * 4][i] + s_part[which * 4 + 1][i]) + (s_part[which * 4 + 2][i] + s_part[which * 4 + 3][i]);
     }
 }
 
@@ -378,7 +478,7 @@ int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, 
     p.logits = logits;
     p.ids = ids;
     p.weights = weights;
-    k_router_logits_batched<<<dim3((E + 1) / 2, (T + DC_MAX_T - 1) / DC_MAX_T), 256, 0, ctx->stream>>>(p);
+    k_router_logits_batched<<<dim3((E + 2 * RB_E - 1) / (2 * RB_E), (T + RB_T - 1) / RB_T), 256, 0, ctx->stream>>>(p);
     {
         const int st = dc_check_cuda(ctx, cudaGetLastError(), "k_router_logits_batched");
         if (st != DC_B200_OK) return st;
@@ -388,128 +488,77 @@ int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, 
 }
 
 // --------------------------------------------------- expert matmul kernel
-// NSTAGE: pipeline depth per warp.  Fewer, smaller rings let more CTAs share an SM: the row decode is
-// bound by instruction issue, so resident warps matter more than bytes in flight per warp.
-template <int NT, bool PAIR, int NSTAGE>
-__global__ void __launch_bounds__(DC_WARPS * 32) k_moe_mm(const MoeMMParams p) {
+// Down projection (PAIR false): the routing was final before this kernel could start (the gate/up kernel lets its successor start only
+// after its own wait, and so does the quantiser between the two, an ordinary launch), so the expert rows can be requested while this
+// kernel still waits for its predecessor's output.  Gate/up: the expert ids come from the router kernel just before.
+template <int TYPE, int NP, bool ONE, bool PAIR>
+__global__ void __launch_bounds__(RW_THREADS, NP > 4 ? 1 : TYPE == DC_TYPE_Q4_K ? 3 : 2) k_moe_rows(const RowsParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem) + warp * NSTAGE;
-    uint8_t* act_base = smem + DC_WARPS * DC_NSTAGE * 8;
-    const size_t act_bytes = (ActSmem::bytes(p.act_rows, p.K) + 127) & ~(size_t)127;
-    uint8_t* bufs = act_base + act_bytes + (size_t)warp * NSTAGE * p.stage_bytes;
-    WarpPipe<NSTAGE> pipe;
-    pipe.init(bufs, bars, p.stage_bytes, p.err);
-    pdl_launch_dependents();
-    MoeStream<NSTAGE, PAIR> st;
-    if (PAIR) {
-        pdl_wait();  // expert ids come from the router kernel just before: nothing can be fetched earlier
-        st.begin(p, *p.n_active, blockIdx.x * DC_WARPS + warp, gridDim.x * DC_WARPS);
-        st.prefill(p, pipe, lane);
-    } else {
-        // down projection: the routing was final before the gate/up kernel ran, and the kernel just before
-        // this one (the quantiser of h, an ordinary launch) started only after gate/up had completed, so
-        // the expert rows can be requested while this kernel still waits for the quantiser's output
-        st.begin(p, *p.n_active, blockIdx.x * DC_WARPS + warp, gridDim.x * DC_WARPS);
-        st.prefill(p, pipe, lane);
-        pdl_wait();
-    }
-    ActSmem act;
-    act.bind(act_base, p.act_rows, p.K);
-    act.fill(p.act_q8, p.act_rows);
-    __syncthreads();
-    st.template consume<NT>(p, pipe, act, lane);
+    rows_cta<TYPE, NP, ONE, true, PAIR, false, !PAIR>(p, smem, blockIdx.x, gridDim.x, 0, 0);
 }
 
-template <int NT, bool PAIR, int NSTAGE>
-static int launch_moe_mm_ns(dc_ctx* ctx, const MoeMMParams& p, int grid, size_t smem) {
-    int st = dc_kernel_setup(ctx, (const void*)k_moe_mm<NT, PAIR, NSTAGE>, 200 * 1024, "cudaFuncSetAttribute(k_moe_mm)");
+template <int TYPE, int NP, bool ONE, bool PAIR>
+static int launch_moe_rows(dc_ctx* ctx, const RowsParams& p, size_t smem, int max_tiles) {
+    const void* f = (const void*)k_moe_rows<TYPE, NP, ONE, PAIR>;
+    int st = dc_kernel_setup(ctx, f, 220 * 1024, "cudaFuncSetAttribute(k_moe_rows)");
     if (st != DC_B200_OK) return st;
-    return dc_launch(ctx, "k_moe_mm", k_moe_mm<NT, PAIR, NSTAGE>, dim3(grid), dim3(DC_WARPS * 32), smem, p);
+    int per_sm = dc_kernel_occupancy(ctx, f, RW_THREADS, smem);
+    if (per_sm < 1) per_sm = 1;
+    const int groups = RW_WARPS / p.S, useful = (max_tiles + groups - 1) / groups;
+    const int grid = useful < ctx->num_sms * per_sm ? useful : ctx->num_sms * per_sm;
+    return dc_launch(ctx, "k_moe_rows", k_moe_rows<TYPE, NP, ONE, PAIR>, dim3(grid), dim3(RW_THREADS), smem, p);
 }
-
-// Shared memory of one CTA with `ns` stages per warp.
-static size_t moe_smem(size_t act_bytes, uint32_t stage, int ns) {
-    return DC_WARPS * DC_NSTAGE * 8 + act_bytes + (size_t)DC_WARPS * ns * stage;
-}
-// CTAs of that size an SM holds (227 KB of shared memory, 1 KB reserved per CTA), at most 4.
-static int moe_ctas_per_sm(size_t smem) {
-    const int n = (int)((227u * 1024u) / (smem + 1024));
-    return n > 4 ? 4 : n;
-}
-
-template <int NT, bool PAIR>
-static int launch_moe_mm(dc_ctx* ctx, const MoeMMParams& p, size_t act_bytes) {
-    // two stages per warp wherever that puts more CTAs on an SM, else the full depth
-    const size_t s4 = moe_smem(act_bytes, p.stage_bytes, DC_NSTAGE), s2 = moe_smem(act_bytes, p.stage_bytes, 2);
-    // resident CTAs per SM by shared memory, then by the kernel's registers (asked once per device and instance)
-    int reg_limit4 = dc_kernel_occupancy(ctx, (const void*)k_moe_mm<NT, PAIR, DC_NSTAGE>, DC_WARPS * 32, 0);
-    int reg_limit2 = dc_kernel_occupancy(ctx, (const void*)k_moe_mm<NT, PAIR, 2>, DC_WARPS * 32, 0);
-    if (reg_limit4 < 1) reg_limit4 = 1;
-    if (reg_limit2 < 1) reg_limit2 = 1;
-    int n4 = s4 <= 200 * 1024 ? moe_ctas_per_sm(s4) : 0, n2 = s2 <= 200 * 1024 ? moe_ctas_per_sm(s2) : 0;
-    if (n4 > reg_limit4) n4 = reg_limit4;
-    if (n2 > reg_limit2) n2 = reg_limit2;
-    if (n4 < 1 && n2 < 1) return dc_fail(ctx, DC_B200_UNSUPPORTED, "moe: shared memory need %zu too large", s2);
-    if (n2 > n4) return launch_moe_mm_ns<NT, PAIR, 2>(ctx, p, ctx->num_sms * n2, s2);
-    return launch_moe_mm_ns<NT, PAIR, DC_NSTAGE>(ctx, p, ctx->num_sms * n4, s4);
-}
-
-static int rows_per_stage_moe(int type, int K, int row_bytes) {
-    const int G = dc::lanes_per_row(type, K);
-    const int per_pass = 32 / G;
-    int r = DC_STAGE_TARGET / row_bytes;
-    r = r / per_pass * per_pass;
-    return r < per_pass ? per_pass : r;
+template <int TYPE, bool PAIR>
+static int launch_moe_rows_np(dc_ctx* ctx, const RowsParams& p, int np, size_t smem, int max_tiles) {
+    if (p.T == 1) return launch_moe_rows<TYPE, 1, true, PAIR>(ctx, p, smem, max_tiles);
+    if (np == 1) return launch_moe_rows<TYPE, 1, false, PAIR>(ctx, p, smem, max_tiles);
+    if (np == 2) return launch_moe_rows<TYPE, 2, false, PAIR>(ctx, p, smem, max_tiles);
+    if (np == 4) return launch_moe_rows<TYPE, 4, false, PAIR>(ctx, p, smem, max_tiles);
+    return launch_moe_rows<TYPE, 8, false, PAIR>(ctx, p, smem, max_tiles);
 }
 
 // w0/w1: expert tensors [K, N, E].  pair: gate/up + SwiGLU, activations are the T
 // token rows; else down, activations are the T*top_k assignment rows.
 int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weight* w1, const uint8_t* act_q8,
-                     int act_rows, int T, int top_k, int e_base, const dc_moe_route* rt, float* out) {
-    MoeMMParams p = {};
-    p.e_base = e_base;
+                     int T, int top_k, int e_base, const dc_moe_route* rt, float* out, const float* act_f32) {
+    RowsParams p = {};
     p.w0 = w0->dev;
     p.w1 = pair ? w1->dev : nullptr;
+    p.e_base = e_base;
     p.type = w0->type;
     p.row_bytes = (int)w0->row_bytes;
     p.N = (int)w0->N;
     p.K = (int)w0->K;
+    p.nb = p.K / DC_QK_K;
     if (p.type != DC_TYPE_Q4_K && p.type != DC_TYPE_Q6_K)
         return dc_fail(ctx, DC_B200_UNSUPPORTED, "moe: expert weight type %d is not Q4_K/Q6_K", p.type);
     if (pair && (w1->type != w0->type || w1->N != w0->N || w1->K != w0->K))
         return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "moe: gate and up tensors differ in type or shape");
     p.act_q8 = act_q8;
-    p.act_rows = act_rows;
+    p.act_f32 = act_f32;
+    p.T = T;
     p.top_k = top_k;
     p.n_active = rt->n_active;
     p.uexp = rt->uexp;
     p.uoff = rt->uoff;
     p.uassign = rt->uassign;
     p.out = out;
-    p.rpst = rows_per_stage_moe(p.type, p.K, p.row_bytes);
-    uint32_t stage = ((uint32_t)p.rpst * p.row_bytes + 32 + 127) & ~127u;
-    if (pair) {
-        p.up_off = stage;
-        stage *= 2;
-    }
-    p.stage_bytes = stage;
     p.err = ctx->d_err;
-    const size_t act_bytes = (ActSmem::bytes(act_rows, p.K) + 127) & ~(size_t)127;
-    if (pair) {
-        if (T == 1) return launch_moe_mm<1, true>(ctx, p, act_bytes);
-        if (T <= 4) return launch_moe_mm<4, true>(ctx, p, act_bytes);
-        if (T <= 8) return launch_moe_mm<8, true>(ctx, p, act_bytes);
-        return launch_moe_mm<16, true>(ctx, p, act_bytes);
-    }
-    if (T == 1) return launch_moe_mm<1, false>(ctx, p, act_bytes);
-    if (T <= 4) return launch_moe_mm<4, false>(ctx, p, act_bytes);
-    if (T <= 8) return launch_moe_mm<8, false>(ctx, p, act_bytes);
-    return launch_moe_mm<16, false>(ctx, p, act_bytes);
+    // distinct experts at most, and the experts that one CTA's neighbouring rounds touch: two where there is at least one CTA for
+    // every expert, three where there are up to twice as many experts
+    const int A = T * top_k, E = (int)w0->E, U = E < A ? E : A;
+    const int span = U <= 1 ? 1 : U <= ctx->num_sms ? 2 : 3;
+    p.act_rows = span * T < A ? span * T : A;
+    p.tiles = (p.N + 15) / 16;
+    const int np = T <= 2 ? 1 : T <= 4 ? 2 : T <= 8 ? 4 : 8, all = U * p.tiles;
+    const size_t smem = rows_plan(p, np, p.type == DC_TYPE_Q6_K, all, ctx->num_sms);
+    if (!smem) return dc_fail(ctx, DC_B200_UNSUPPORTED, "moe: K=%d needs too much shared memory for %d tokens", p.K, T);
+    if (p.type == DC_TYPE_Q4_K) return pair ? launch_moe_rows_np<DC_TYPE_Q4_K, true>(ctx, p, np, smem, all) : launch_moe_rows_np<DC_TYPE_Q4_K, false>(ctx, p, np, smem, all);
+    return pair ? launch_moe_rows_np<DC_TYPE_Q6_K, true>(ctx, p, np, smem, all) : launch_moe_rows_np<DC_TYPE_Q6_K, false>(ctx, p, np, smem, all);
 }
 
 int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_expert, int T, int top_k, float scale,
-                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode) {
+                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode, const dc_route_norm* norm) {
     // wr == nullptr: rt->logits already holds the router logits (routing only)
     if (wr && wr->type != DC_TYPE_F32) return dc_fail(ctx, DC_B200_UNSUPPORTED, "router weight must be F32");
     const int E = wr ? (int)wr->N : n_expert;
@@ -534,7 +583,15 @@ int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_ex
     p.uexp = rt->uexp;
     p.uoff = rt->uoff;
     p.uassign = rt->uassign;
-    return dc_launch(ctx, "k_router", k_router, dim3(wr ? (p.E + 1) / 2 : 1), dim3(256), 0, p);
+    size_t smem = 0;
+    if (norm) {
+        if (!wr || T > 4) return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "router: rows to be normed need router weights, and are four at most");
+        p.norm = *norm;
+        smem = (size_t)T * p.H * 4;
+        const int st = dc_kernel_setup(ctx, (const void*)k_router, 160 * 1024, "cudaFuncSetAttribute(k_router)");
+        if (st != DC_B200_OK) return st;
+    }
+    return dc_launch(ctx, "k_router", k_router, dim3(wr ? (p.E + 1) / 2 : 1), dim3(256), smem, p);
 }
 
 // ------------------------------------------------------------ combine
@@ -543,15 +600,8 @@ int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_ex
 // T <= 4 and T*top_k <= 32 (cpu_backend_moe_ops.cpp:66,1247-1248,1578-1597),
 // otherwise ascending expert id (moe_routing.cpp:647-676).  Assignments whose
 // expert lives on another GPU are skipped (their share arrives by all-reduce).
-__global__ void __launch_bounds__(256) k_moe_combine(const float* __restrict__ dn, const int32_t* __restrict__ ids,
-                                                     const float* __restrict__ weights, int T, int top_k, int H,
-                                                     int ep_lo, int ep_hi, float* __restrict__ out) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int t = blockIdx.y;
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= H) return;
-    int order[MOE_MAX_K];
+// The order in which a token's assignments are added up.
+__device__ __forceinline__ void combine_order(const int32_t* ids, int T, int top_k, int t, int (&order)[MOE_MAX_K]) {
     for (int k = 0; k < top_k; ++k) order[k] = k;
     if (!(T <= 4 && T * top_k <= 32)) {
         for (int i = 1; i < top_k; ++i) {
@@ -564,6 +614,18 @@ __global__ void __launch_bounds__(256) k_moe_combine(const float* __restrict__ d
             order[j + 1] = o;
         }
     }
+}
+
+__global__ void __launch_bounds__(256) k_moe_combine(const float* __restrict__ dn, const int32_t* __restrict__ ids,
+                                                     const float* __restrict__ weights, int T, int top_k, int H,
+                                                     int ep_lo, int ep_hi, float* __restrict__ out) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.y;
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= H) return;
+    int order[MOE_MAX_K];
+    combine_order(ids, T, top_k, t, order);
     float sum = 0.0f;
     for (int k = 0; k < top_k; ++k) {
         const int a = t * top_k + order[k], e = ids[a];
@@ -578,4 +640,78 @@ int dc_launch_moe_combine(dc_ctx* ctx, const float* dn, const int32_t* ids, cons
                           int H, int ep_lo, int ep_hi, float* out) {
     return dc_launch(ctx, "k_moe_combine", k_moe_combine, dim3((H + 255) / 256, T), dim3(256), 0, dn, ids, weights, T,
                      top_k, H, ep_lo, ep_hi, out);
+}
+
+// One CTA per token: the combine above added to the residual, then RMSNorm and Q8_K blocks (k_rmsnorm_q8k's arithmetic).  A kernel of its
+// own for the combine cost a launch of the step's chain and wrote and read the sum again.
+__global__ void __launch_bounds__(512) k_moe_combine_norm(const float* __restrict__ dn, const int32_t* __restrict__ ids, const float* __restrict__ weights,
+                                                          int T, int top_k, int H, float* __restrict__ x, const float* __restrict__ nw, float eps,
+                                                          float* __restrict__ xn_out, uint8_t* __restrict__ q8_out) {
+    extern __shared__ __align__(16) float sx[];
+    __shared__ double red[16];
+    __shared__ float s_w[MOE_MAX_K];
+    __shared__ int s_a[MOE_MAX_K];
+    pdl_launch_dependents();
+    const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n4 = H / 4;
+    float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid < n4) w0 = reinterpret_cast<const float4*>(nw)[tid];
+    pdl_wait();
+    if (tid == 0) {
+        int order[MOE_MAX_K];
+        combine_order(ids, T, top_k, t, order);
+        for (int k = 0; k < top_k; ++k) {
+            s_a[k] = t * top_k + order[k];
+            s_w[k] = weights[s_a[k]];
+        }
+    }
+    __syncthreads();
+    double ss = 0.0;
+    for (int i = tid; i < n4; i += 512) {
+        const float4 xv = reinterpret_cast<const float4*>(x + (size_t)t * H)[i];
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k0 = 0; k0 < top_k; k0 += 8) {
+            float4 r[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)     // eight rows' loads in flight
+                r[j] = reinterpret_cast<const float4*>(dn + (size_t)s_a[min(k0 + j, top_k - 1)] * H)[i];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (k0 + j >= top_k || s_w[k0 + j] == 0.0f) continue;
+                const float w = s_w[k0 + j];
+                s[0] = __fadd_rn(s[0], __fmul_rn(w, r[j].x));
+                s[1] = __fadd_rn(s[1], __fmul_rn(w, r[j].y));
+                s[2] = __fadd_rn(s[2], __fmul_rn(w, r[j].z));
+                s[3] = __fadd_rn(s[3], __fmul_rn(w, r[j].w));
+            }
+        }
+        const float4 v = make_float4(__fadd_rn(xv.x, s[0]), __fadd_rn(xv.y, s[1]), __fadd_rn(xv.z, s[2]), __fadd_rn(xv.w, s[3]));
+        reinterpret_cast<float4*>(x + (size_t)t * H)[i] = v;
+        reinterpret_cast<float4*>(sx)[i] = v;
+        ss += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    double tot = 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) tot += red[i];
+    const float mean = (float)(tot / (double)H);
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+    for (int i = tid; i < n4; i += 512) {
+        const float4 v = reinterpret_cast<const float4*>(sx)[i], w = i == tid ? w0 : reinterpret_cast<const float4*>(nw)[i];
+        const float4 y = make_float4(__fmul_rn(__fmul_rn(v.x, scale), w.x), __fmul_rn(__fmul_rn(v.y, scale), w.y),
+                                     __fmul_rn(__fmul_rn(v.z, scale), w.z), __fmul_rn(__fmul_rn(v.w, scale), w.w));
+        reinterpret_cast<float4*>(sx)[i] = y;
+        if (xn_out) reinterpret_cast<float4*>(xn_out + (size_t)t * H)[i] = y;
+    }
+    if (!q8_out) return;
+    __syncthreads();
+    const int nb = H / DC_QK_K;
+    for (int b = warp; b < nb; b += 16) quantize_block_q8k_warp<true>(sx + b * DC_QK_K, q8_out + ((size_t)t * nb + b) * DC_Q8F_BYTES, lane);
+}
+
+int dc_launch_moe_combine_norm(dc_ctx* ctx, const float* dn, const int32_t* ids, const float* weights, int T, int top_k, int H, float* x,
+                               const float* norm_w, float eps, float* xn_out, uint8_t* q8_out) {
+    return dc_launch(ctx, "k_moe_combine_norm", k_moe_combine_norm, dim3(T), dim3(512), (size_t)H * 4, dn, ids, weights, T, top_k, H, x, norm_w, eps, xn_out, q8_out);
 }

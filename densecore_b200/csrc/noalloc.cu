@@ -16,11 +16,11 @@
 #include "dc_internal.h"
 
 // Q8_K rows of one call: up to 16 activation rows of up to 16384 values
-// (64 blocks of 292 bytes each).  Every GPU that loads the library holds these
-// 299,008 bytes until the process exits.
+// (64 blocks of 320 bytes each).  Every GPU that loads the library holds these
+// 327,680 bytes until the process exits.
 #define NA_MAX_ROWS 16
 #define NA_MAX_K 16384
-#define NA_BYTES (NA_MAX_ROWS * (NA_MAX_K / DC_QK_K) * DC_Q8K_BYTES)
+#define NA_BYTES (NA_MAX_ROWS * (NA_MAX_K / DC_QK_K) * DC_Q8F_BYTES)
 static __device__ __align__(256) uint8_t g_noalloc_q8[NA_BYTES];
 
 // In host code the array's name is only a handle; the device address of each
@@ -60,8 +60,9 @@ extern "C" int dc_b200_mul_mat_dev_noalloc(dc_ctx* ctx, const dc_weight* w, cons
     if (st != DC_B200_OK) return st;
     cudaSetDevice(ctx->device);
     // the activations are fully rewritten by every call, so nothing has to be cleared first
-    st = dc_launch_quantize_q8k(ctx, x_dev, M, (int)w->K, q8);
+    const bool own = dc_rows_quantise(M, (int)w->K);
+    if (!own) st = dc_launch_quantize_q8k(ctx, x_dev, M, (int)w->K, q8, true);
     if (st != DC_B200_OK) return st;
     dc_gemv_seg seg = {w->dev, w->type, (int)w->N, (int)w->row_bytes, y_dev, (int)w->N};
-    return dc_launch_gemv(ctx, &seg, 1, DC_EPI_STORE, q8, M, (int)w->K, nullptr);
+    return dc_launch_gemv(ctx, &seg, 1, DC_EPI_STORE, q8, M, (int)w->K, nullptr, nullptr, nullptr, own ? x_dev : nullptr);
 }

@@ -124,14 +124,14 @@ static int moe_layer_dev(dc_ctx* ctx, const dc_weight* router, const float* logi
     cudaSetDevice(ctx->device);
     const int A = T * top_k;
     dc_moe_route rt_size;
-    const size_t need = (size_t)T * (H / 256) * 292 + (size_t)A * F * 4 + (size_t)A * (F / 256) * 292 + (size_t)A * H * 4 +
+    const size_t need = (size_t)T * (H / 256) * DC_Q8F_BYTES + (size_t)A * F * 4 + (size_t)A * (F / 256) * DC_Q8F_BYTES + (size_t)A * H * 4 +
                         dc_moe_route_bind(&rt_size, nullptr, T, E, top_k) + 4096;
     uint8_t* s = dc_scratch(ctx, need);
     if (!s) return DC_B200_OUT_OF_MEMORY;
     Bump b{s};
-    uint8_t* xq = b.take<uint8_t>((size_t)T * (H / 256) * 292);
+    uint8_t* xq = b.take<uint8_t>((size_t)T * (H / 256) * DC_Q8F_BYTES);
     float* h = b.take<float>((size_t)A * F);
-    uint8_t* hq = b.take<uint8_t>((size_t)A * (F / 256) * 292);
+    uint8_t* hq = b.take<uint8_t>((size_t)A * (F / 256) * DC_Q8F_BYTES);
     float* dn = b.take<float>((size_t)A * H);
     dc_moe_route rt;
     dc_moe_route_bind(&rt, s + b.off, T, E, top_k);
@@ -139,10 +139,11 @@ static int moe_layer_dev(dc_ctx* ctx, const dc_weight* router, const float* logi
     if (!router)
         DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(rt.logits, logits_dev, (size_t)T * E * 4, cudaMemcpyDeviceToDevice, ctx->stream), "logits"));
     DC_TRY(dc_launch_router(ctx, router, x_dev, E, T, top_k, routed_scale, 0, E, &rt, ctx->route_mode));
-    DC_TRY(dc_launch_quantize_q8k(ctx, x_dev, T, H, xq));
-    DC_TRY(dc_launch_moe_mm(ctx, true, gate, up, xq, T, T, top_k, 0, &rt, h));
-    DC_TRY(dc_launch_quantize_q8k(ctx, h, A, F, hq));
-    DC_TRY(dc_launch_moe_mm(ctx, false, down, nullptr, hq, A, T, top_k, 0, &rt, dn));
+    DC_TRY(dc_launch_quantize_q8k(ctx, x_dev, T, H, xq, true));
+    DC_TRY(dc_launch_moe_mm(ctx, true, gate, up, xq, T, top_k, 0, &rt, h));
+    const bool own = dc_moe_quantise_in_down(T);
+    if (!own) DC_TRY(dc_launch_quantize_q8k(ctx, h, A, F, hq, true));
+    DC_TRY(dc_launch_moe_mm(ctx, false, down, nullptr, hq, T, top_k, 0, &rt, dn, own ? h : nullptr));
     DC_TRY(dc_launch_moe_combine(ctx, dn, rt.ids, rt.weights, T, top_k, H, 0, E, y_dev));
     if (ids_dev) DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(ids_dev, rt.ids, (size_t)A * 4, cudaMemcpyDeviceToDevice, ctx->stream), "ids"));
     if (weights_dev) DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(weights_dev, rt.weights, (size_t)A * 4, cudaMemcpyDeviceToDevice, ctx->stream), "weights"));

@@ -9,7 +9,7 @@
 // (attn_prefill.cu on the tensor cores; or the decode kernels' exact chain, one grid for the chunk) -> output projection accumulated into the residual ->
 // RMSNorm -> router (logits, then one warp per token) -> assignments grouped by expert into 64-slot tiles ->
 // gate and up GEMMs with an expert per tile -> SwiGLU + tiled Q8_K -> down GEMM scattered back to
-// assignment order -> weighted combine (the decode kernel).  The last chunk ends with the decode path's
+// assignment order -> weighted combine (with the next layer's norm).  The last chunk ends with the decode path's
 // output norm, lm_head row-streaming kernel and greedy pick for its last token.
 #include <algorithm>
 
@@ -248,9 +248,14 @@ int dc_prefill_chunk_tc(dc_model* m, int seq, const int32_t* tokens, int n, bool
     const int n_tt = dc_gemm_tc_tiles(n);
     DC_TRY(dc_launch_embed(ctx, m->tok_embd, P.tokens, n, P.x));
     const float* pending = nullptr;   // MoE output of the previous layer, added in the next norm
+    bool split = false;               // the previous layer's expert outputs wait for their weighted sum, which the next norm then makes
     for (int il = 0; il < c.n_layer; ++il) {
         dc_layer& Ly = m->layers[il];
-        DC_TRY(dc_launch_rmsnorm_q8k(ctx, P.x, pending, (const float*)Ly.attn_norm->dev, n, H, c.rms_eps, P.xn, nullptr));
+        if (split)
+            DC_TRY(dc_launch_moe_combine_norm(ctx, P.dn, P.ids, P.weights, n, top_k, H, P.x, (const float*)Ly.attn_norm->dev, c.rms_eps, P.xn, nullptr));
+        else
+            DC_TRY(dc_launch_rmsnorm_q8k(ctx, P.x, pending, (const float*)Ly.attn_norm->dev, n, H, c.rms_eps, P.xn, nullptr));
+        split = false;
         pending = nullptr;
         DC_TRY(dc_launch_quantize_q8k_tiled(ctx, P.xn, H, n, H, P.act_x, n_tt, nullptr));
         {
@@ -302,6 +307,8 @@ int dc_prefill_chunk_tc(dc_model* m, int seq, const int32_t* tokens, int n, bool
             DC_TRY(launch_swiglu(ctx, P.g, P.g + F, 2 * F, F, slots, P.act_h, P.max_tiles, P.slot_assign));
             DC_TRY(dc_launch_gemm_tc(ctx, Ly.down_exps, P.act_h, slots, P.dn, H, P.tile_expert, P.slot_assign, false, P.pair_tile0,
                                      P.pair_nset, P.max_tiles));
+            split = c.ep_size == 1 && il + 1 < c.n_layer;
+            if (split) continue;
             DC_TRY(dc_launch_moe_combine(ctx, P.dn, P.ids, P.weights, n, top_k, H, m->ep_lo, m->ep_hi, P.moe_out));
             if (c.ep_size > 1) DC_TRY(dc_ep_allreduce(m, P.moe_out, (size_t)n * H));
             pending = P.moe_out;

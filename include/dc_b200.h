@@ -108,12 +108,12 @@ DC_B200_API int dc_b200_mul_mat_dev(dc_ctx* ctx, const dc_weight* w, const float
  * op callbacks running under a fixed-buffer graph executor, serving loops that
  * must not take the CUDA allocator lock after warm-up, code inside a stream
  * capture).  x_dev [M, K] and y_dev [M, N] are device buffers of the caller;
- * the Q8_K form of x lives in a 299,008-byte array built into the library
+ * the Q8_K form of x lives in a 327,680-byte array built into the library
  * (each GPU that loads the library keeps it until exit).  Limits: M <= 16 and
  * K <= 16384, larger shapes are refused with DC_B200_UNSUPPORTED.  No
  * cudaMalloc/cudaFree or allocating routine is called.  The first call on a
  * GPU looks up the array's device address (cudaGetSymbolAddress), and the first
- * call for each row-count class (1, 2-4, 5-8, 9-16) and weight shape also
+ * call for each row-count class (1, 2, 3-4, 5-8, 9-16) and weight shape also
  * configures its kernel instance (shared-memory opt-in, occupancy query) on
  * that GPU; make one such call before any stream capture begins.  All calls on a GPU share the array
  * and it keeps the previous call's contents (each call overwrites what it
@@ -386,8 +386,8 @@ DC_B200_API int dc_b200_model_read_kv(dc_model* m, int layer, int seq, int first
  * "prefill_chunk" 32..4096 (default 2048, fixed once a chunk has run); "prefill_attention" 1 (default) chunk
  * attention on the tensor cores, 0 the decode kernels' exact running-maximum chain; "prefix_cache" 0/1.
  * "persistent" 0/1/2: decode steps of MoE models run in one persistent cooperative kernel with grid
- * barriers between phases: 0 never, 1 for one stream (default: with more streams the per-op kernels are
- * faster), 2 for every stream count it supports (1-4). */
+ * barriers between phases: 0 never, 1 for one stream where that is the faster path (default: one stream of
+ * an expert-parallel model), 2 for every stream count it supports (1-4). */
 DC_B200_API int dc_b200_model_set_option(dc_model* m, const char* name, int value);
 /* Prefix-cache counters of a model (option "prefix_cache" = 1 makes dc_b200_prefill and the scheduler use
  * the cache): {lookups, blocks hit, blocks resident, evictions, prompt tokens run through the decoder}. */
