@@ -145,14 +145,15 @@ DC_PART bool dc_attn_cluster_ok(int max_blocks);
 int dc_launch_attention_prefill(dc_ctx* ctx, const float* q, const void* k_arena, const void* v_arena, const int32_t* table,
                                 int pos0, int n, int n_head, int n_kv, float scale, float* out);
 
+#define DC_MOE_PASS 4     // tokens of an expert that the expert kernels take at a time
 struct dc_moe_route {
     float* logits;     // [T][E]
     int32_t* ids;      // [T][top_k]
     float* weights;    // [T][top_k]
     int* ticket;       // zeroed once; the router resets it itself
-    int* n_active;     // number of distinct local experts hit
-    int32_t* uexp;     // [E]
-    int32_t* uoff;     // [E+1]
+    int* n_active;     // number of distinct local experts hit (k_router: of their passes)
+    int32_t* uexp;     // [E + T*top_k]
+    int32_t* uoff;     // [E + T*top_k + 1]
     int32_t* uassign;  // [T*top_k]
 };
 // mode: DC_ROUTE_STABLE = top-k on the logits with the stable comparator, weights over the picks

@@ -22,8 +22,8 @@ namespace dc {
 #define RW_WARPS 8
 #define RW_THREADS (RW_WARPS * 32)
 #define RW_STAGES 3           // units in a warp's ring; a fourth would cost an SM its second or third CTA
-#define RW_PITCH4 144u        // bytes between a unit's rows: an odd multiple of 16, so that the 32 lanes' words (8 rows x 16 bytes)
-#define RW_PITCH6 240u        // fall on distinct banks; Q6_K: 210 bytes at an even offset within the copied 224
+#define RW_PITCH4 160u        // bytes between a unit's rows, so that 16 lanes' 8-byte loads (4 rows x 32 bytes) fall on distinct banks
+#define RW_PITCH6 240u        // the same for 32 lanes' words (8 rows x 16 bytes); 210 bytes at an even offset within the copied 224
 
 // Activation blocks in fragment order (quantize_block_q8f_regs), block-major.
 struct RowAct {
@@ -97,11 +97,12 @@ __device__ __forceinline__ void rows_unit_q4k(const uint8_t* rg, const uint8_t* 
     uint32_t w[4][4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        const int o = 16 + 32 * c + 4 * t;
-        w[c][0] = ld_w(rg + o);
-        w[c][1] = ld_w(rg8 + o);
-        w[c][2] = ld_w(rg + o + 16);
-        w[c][3] = ld_w(rg8 + o + 16);
+        const int o = 16 + 32 * c + 8 * t;
+        const uint2 x = *reinterpret_cast<const uint2*>(rg + o), y = *reinterpret_cast<const uint2*>(rg8 + o);
+        w[c][0] = x.x;
+        w[c][1] = y.x;
+        w[c][2] = x.y;
+        w[c][3] = y.y;
     }
     const uint32_t sc[2] = {h.y & 0x3f3f3f3fu, (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u)};
     const uint32_t sc8[2] = {h8.y & 0x3f3f3f3fu, (h8.w & 0x0f0f0f0fu) | ((h8.y >> 2) & 0x30303030u)};
@@ -118,10 +119,10 @@ __device__ __forceinline__ void rows_unit_q4k(const uint8_t* rg, const uint8_t* 
         int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0}, ml[4], mh[4];
         mma_k16_s8(ml, m, m8, ld_w(rec + 64 + 4 * (t & 1)));
         mma_k16_s8(mh, m, m8, ld_w(rec + 72 + 4 * (t & 1)));
-        rec += 80 * t;
+        rec += 160 * (t & 1) + 16 * (t >> 1);      // words 2 t and 2 t + 1 of every sub-block: two runs, one of their groups
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const uint4 q0 = ld_v4(rec + 32 * j), q1 = ld_v4(rec + 32 * j + 16);   // quadrants of the half: words of group 0, of group 1
+            const uint4 q0 = ld_v4(rec + 32 * j), q1 = ld_v4(rec + 32 * j + 80);   // quadrants of the half: the first word, the second
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const uint32_t* x = w[2 * j + k];
@@ -505,7 +506,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
     unsigned long long best[NR];      // largest result so far of every token that the lane holds (rows g and g + 8 share one)
 #pragma unroll
     for (int i = 0; i < NR; ++i) best[i] = 0ull;
-    float acc[NA], gate[PAIR ? NR : 1];
+    float acc[NA], gate[PAIR ? NR : 1] = {};
     auto add = [&](int i, float x, float y) {
         if (Q4) acc[i] = __fsub_rn(__fadd_rn(acc[i], x), y);
         else acc[i] = __fmaf_rn(y, x, acc[i]);

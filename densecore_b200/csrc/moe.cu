@@ -32,8 +32,8 @@ struct RouterParams {
     float* weights;       // [T][top_k]
     int* ticket;          // zero-initialised, self-resetting
     int* n_active;        // U
-    int32_t* uexp;        // [E]   distinct local experts, ascending
-    int32_t* uoff;        // [E+1] offsets into uassign
+    int32_t* uexp;        // distinct local experts, ascending, once for every DC_MOE_PASS of their tokens
+    int32_t* uoff;        // their offsets into uassign, and the end
     int32_t* uassign;     // [T*top_k] assignment indices t*top_k+k, grouped by expert, routing order inside
     dc_route_norm norm;   // x given: rows still to be normed
 };
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     int cnt = 0;
     if (me < p.E && me >= p.ep_lo && me < p.ep_hi)
         for (int i = 0; i < A; ++i) cnt += (s_ids[i] == me);
-    int act = cnt > 0 ? 1 : 0;
+    int act = (cnt + DC_MOE_PASS - 1) / DC_MOE_PASS;
     // inclusive scans of (act, cnt) over the 256 threads
     int sa = act, scn = cnt;
 #pragma unroll
@@ -379,9 +379,11 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
         tot_c += s_wsum_c[w];
     }
     if (act) {
-        const int u = base_a + sa - 1, off = base_c + scn - cnt;
-        p.uexp[u] = me;
-        p.uoff[u] = off;
+        const int u = base_a + sa - act, off = base_c + scn - cnt;
+        for (int i = 0; i < act; ++i) {
+            p.uexp[u + i] = me;
+            p.uoff[u + i] = off + DC_MOE_PASS * i;
+        }
         int o = off;
         for (int i = 0; i < A; ++i)
             if (s_ids[i] == me) p.uassign[o++] = i;
@@ -492,7 +494,7 @@ int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, 
 // after its own wait, and so does the quantiser between the two, an ordinary launch), so the expert rows can be requested while this
 // kernel still waits for its predecessor's output.  Gate/up: the expert ids come from the router kernel just before.
 template <int TYPE, int NP, bool ONE, bool PAIR>
-__global__ void __launch_bounds__(RW_THREADS, NP > 4 ? 1 : TYPE == DC_TYPE_Q4_K ? 3 : 2) k_moe_rows(const RowsParams p) {
+__global__ void __launch_bounds__(RW_THREADS, TYPE == DC_TYPE_Q4_K ? 3 : 2) k_moe_rows(const RowsParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     rows_cta<TYPE, NP, ONE, true, PAIR, false, !PAIR>(p, smem, blockIdx.x, gridDim.x, 0, 0);
 }
@@ -512,9 +514,7 @@ template <int TYPE, bool PAIR>
 static int launch_moe_rows_np(dc_ctx* ctx, const RowsParams& p, int np, size_t smem, int max_tiles) {
     if (p.T == 1) return launch_moe_rows<TYPE, 1, true, PAIR>(ctx, p, smem, max_tiles);
     if (np == 1) return launch_moe_rows<TYPE, 1, false, PAIR>(ctx, p, smem, max_tiles);
-    if (np == 2) return launch_moe_rows<TYPE, 2, false, PAIR>(ctx, p, smem, max_tiles);
-    if (np == 4) return launch_moe_rows<TYPE, 4, false, PAIR>(ctx, p, smem, max_tiles);
-    return launch_moe_rows<TYPE, 8, false, PAIR>(ctx, p, smem, max_tiles);
+    return launch_moe_rows<TYPE, 2, false, PAIR>(ctx, p, smem, max_tiles);
 }
 
 // w0/w1: expert tensors [K, N, E].  pair: gate/up + SwiGLU, activations are the T
@@ -544,13 +544,14 @@ int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weigh
     p.uassign = rt->uassign;
     p.out = out;
     p.err = ctx->d_err;
-    // distinct experts at most, and the experts that one CTA's neighbouring rounds touch: two where there is at least one CTA for
-    // every expert, three where there are up to twice as many experts
-    const int A = T * top_k, E = (int)w0->E, U = E < A ? E : A;
-    const int span = U <= 1 ? 1 : U <= ctx->num_sms ? 2 : 3;
-    p.act_rows = span * T < A ? span * T : A;
+    // A kernel takes up to DC_MOE_PASS tokens of an expert; the few experts with more come several times over and are read again from
+    // L2.  (Kernels for sixteen tokens an expert hold 255 registers, eight warps an SM: 259 us for 16 tokens of 8 out of 128 experts.)
+    // act_rows: the passes that one CTA's neighbouring tiles touch are one more than its share of them, rounded up.
+    const int A = T * top_k, E = (int)w0->E, most = E + A / DC_MOE_PASS, U = most < A ? most : A;
+    const int span = U <= 1 ? 1 : (U + ctx->num_sms - 1) / ctx->num_sms + 1, per = T < DC_MOE_PASS ? T : DC_MOE_PASS;
+    p.act_rows = span * per < A ? span * per : A;
     p.tiles = (p.N + 15) / 16;
-    const int np = T <= 2 ? 1 : T <= 4 ? 2 : T <= 8 ? 4 : 8, all = U * p.tiles;
+    const int np = T <= 2 ? 1 : 2, all = U * p.tiles;
     const size_t smem = rows_plan(p, np, p.type == DC_TYPE_Q6_K, all, ctx->num_sms);
     if (!smem) return dc_fail(ctx, DC_B200_UNSUPPORTED, "moe: K=%d needs too much shared memory for %d tokens", p.K, T);
     if (p.type == DC_TYPE_Q4_K) return pair ? launch_moe_rows_np<DC_TYPE_Q4_K, true>(ctx, p, np, smem, all) : launch_moe_rows_np<DC_TYPE_Q4_K, false>(ctx, p, np, smem, all);

@@ -42,8 +42,8 @@ size_t dc_moe_route_bind(dc_moe_route* rt, uint8_t* base, int T, int E, int top_
     rt->weights = b.take<float>((size_t)T * top_k);
     rt->ticket = b.take<int>(1);
     rt->n_active = b.take<int>(1);
-    rt->uexp = b.take<int32_t>(E);
-    rt->uoff = b.take<int32_t>(E + 1);
+    rt->uexp = b.take<int32_t>(E + T * top_k);
+    rt->uoff = b.take<int32_t>(E + T * top_k + 1);
     rt->uassign = b.take<int32_t>((size_t)T * top_k);
     return b.off;
 }
