@@ -655,46 +655,55 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // ---- scores: four lanes per key, lane `sub` takes the 16-byte pieces 4 i + sub of the row
-    for (int key = tid >> 2; key < nbl * DC_KV_BLOCK; key += AC_THREADS / 4) {
+    // ---- scores: four lanes per pair of keys, lane `sub` takes the 16-byte pieces 4 i + sub of the rows; the queries' loads, which
+    // are what this part is bound by, then serve two keys
+    for (int key = 2 * (tid >> 2); key < nbl * DC_KV_BLOCK; key += AC_THREADS / 2) {
         const int sub = tid & 3;
         if (key < keys) {
-            float2 kf[16];
+            float2 kf[2][16];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint4 u = *reinterpret_cast<const uint4*>(sKV + ac_piece(key, 4 * i + sub));
-                const __half2* h2 = reinterpret_cast<const __half2*>(&u);
+            for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) kf[4 * i + j] = __half22float2(h2[j]);
-            }
+                for (int i = 0; i < 4; ++i) {      // (the row after the last key's is read as whatever it holds and not used)
+                    const uint4 u = *reinterpret_cast<const uint4*>(sKV + ac_piece(key + k, 4 * i + sub));
+                    const __half2* h2 = reinterpret_cast<const __half2*>(&u);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) kf[k][4 * i + j] = __half22float2(h2[j]);
+                }
             const uint32_t quad = 0xFu << (lane & ~3);
-            for (int h0 = 0; h0 < g; h0 += 4) {      // four heads at a time: independent chains (heads past the last are read as the last)
-                float2 d[4];
+            for (int h0 = 0; h0 < g; h0 += 2) {      // g is even
+                float2 d[2][2];
 #pragma unroll
-                for (int h = 0; h < 4; ++h) d[h] = make_float2(0.0f, 0.0f);
+                for (int h = 0; h < 2; ++h) d[h][0] = d[h][1] = make_float2(0.0f, 0.0f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        const float4* q4 = reinterpret_cast<const float4*>(sQ + min(h0 + h, g - 1) * 128 + (4 * i + sub) * 8);
+                    for (int h = 0; h < 2; ++h) {
+                        const float4* q4 = reinterpret_cast<const float4*>(sQ + (h0 + h) * 128 + (4 * i + sub) * 8);
                         const float4 a = q4[0], b = q4[1];
-                        ac_fma2(d[h], make_float2(a.x, a.y), kf[4 * i]);
-                        ac_fma2(d[h], make_float2(a.z, a.w), kf[4 * i + 1]);
-                        ac_fma2(d[h], make_float2(b.x, b.y), kf[4 * i + 2]);
-                        ac_fma2(d[h], make_float2(b.z, b.w), kf[4 * i + 3]);
-                    }
-                float mine = 0.0f;
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    float dot = d[h].x + d[h].y;
-                    dot += __shfl_xor_sync(quad, dot, 1);
-                    dot += __shfl_xor_sync(quad, dot, 2);
-                    if (h == sub) mine = dot;
-                }
-                if (h0 + sub < g) sP[ac_at(key, h0 + sub)] = __fmul_rn(mine, p.scale);
+                        for (int k = 0; k < 2; ++k) {
+                            ac_fma2(d[h][k], make_float2(a.x, a.y), kf[k][4 * i]);
+                            ac_fma2(d[h][k], make_float2(a.z, a.w), kf[k][4 * i + 1]);
+                            ac_fma2(d[h][k], make_float2(b.x, b.y), kf[k][4 * i + 2]);
+                            ac_fma2(d[h][k], make_float2(b.z, b.w), kf[k][4 * i + 3]);
+                        }
+                    }
+                float mine = 0.0f;      // lane sub keeps (head sub / 2, key sub % 2)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        float dot = d[h][k].x + d[h][k].y;
+                        dot += __shfl_xor_sync(quad, dot, 1);
+                        dot += __shfl_xor_sync(quad, dot, 2);
+                        if (2 * h + k == sub) mine = dot;
+                    }
+                const int at = key + (sub & 1);
+                sP[ac_at(at, h0 + (sub >> 1))] = at < keys ? __fmul_rn(mine, p.scale) : -INFINITY;
             }
         } else {
-            for (int h = sub; h < g; h += 4) sP[ac_at(key, h)] = -INFINITY;
+            for (int i = sub; i < 2 * g; i += 4) sP[ac_at(key + (i & 1), i >> 1)] = -INFINITY;
         }
     }
     __syncthreads();
@@ -750,9 +759,10 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
         if (lane == 0) sProd[warp] = after;
     }
     __syncthreads();
+    const int lg = g > 4 ? 3 : g > 2 ? 2 : 1;
 #pragma unroll 4
-    for (int i = tid; i < nbl * DC_KV_BLOCK * 8; i += AC_THREADS) {
-        const int key = i >> 3, h = i & 7, c = (key >> 4) * 8 + h;
+    for (int i = tid; i < nbl * DC_KV_BLOCK << lg; i += AC_THREADS) {
+        const int key = i >> lg, h = i & ((1 << lg) - 1), c = (key >> 4) * 8 + h;
         if (h < g) {
             const float s = sP[ac_at(key, h)];
             sP[ac_at(key, h)] = s == -INFINITY ? 0.0f : __fmul_rn(fast_exp_fma(s - sBm[c]), sW[c]);
@@ -777,7 +787,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
         for (int key = kg; key < keys; key += 4) {
             const float2 v = __half22float2(*reinterpret_cast<const __half2*>(sKV + key * 256 + dp * 4));
             const float4* pp = reinterpret_cast<const float4*>(sP + ac_at(key, 0));
-            const float4 x = pp[0], y = pp[1];
+            const float4 x = pp[0], y = g > 4 ? pp[1] : x;
             const float2 vx = make_float2(v.x, v.x), vy = make_float2(v.y, v.y);
             ac_fma2(a0[0], make_float2(x.x, x.y), vx);
             ac_fma2(a1[0], make_float2(x.x, x.y), vy);

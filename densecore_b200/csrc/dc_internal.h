@@ -74,10 +74,12 @@ enum { DC_EPI_STORE = 0, DC_EPI_ACC = 1, DC_EPI_SWIGLU = 2 };
 // result silu(gate.x)*(up.x) stored to seg[0].out.  argmax (optional, [T] u64 keys,
 // zeroed by the caller) receives the packed (value,row) maximum of the stored rows.
 // act_f32 (instead of act_q8): the rows before quantisation, which then is part of the kernel; pays where T * K / 256 blocks are few.
+// norm_w (with act_f32): the rows before RMSNorm, too.
 // dump_I / dump_M (parity checks, single segment): receive the exact int32 block sums the kernel forms,
 // [T][n_rows][K/256] (M for Q4_K only).
 DC_PART int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, const uint8_t* act_q8, int T, int K,
-                   unsigned long long* argmax, int32_t* dump_I = nullptr, int32_t* dump_M = nullptr, const float* act_f32 = nullptr);
+                   unsigned long long* argmax, int32_t* dump_I = nullptr, int32_t* dump_M = nullptr, const float* act_f32 = nullptr,
+                   const float* norm_w = nullptr, float norm_eps = 0.0f);
 // whether k_rows quantises its T rows itself (act_f32): each of its eight warps then has three blocks at most to quantise, about 1 us,
 // against a launch of the chain
 static inline bool dc_rows_quantise(int T, int K) { return T * (K / 256) <= 24; }

@@ -44,6 +44,8 @@ struct RowsParams {
     uint32_t off_zero, off_link, off_ring;
     const uint8_t* act_q8;
     const float* act_f32;     // given: the rows still to be quantised, which every CTA does for its own
+    const float* norm_w;      // given: and to be normed before that
+    float norm_eps;
     int T, K, nb;
     int act_rows;             // rows of activations a CTA holds
     unsigned long long* argmax;
@@ -352,6 +354,37 @@ template <class Src>
 __device__ __forceinline__ void rows_fill_act(const RowsParams& p, uint8_t* smem, int n, const Src& src) {
     constexpr int PIECES = DC_Q8F_BYTES / 16;
     const int nb = p.nb, rows = p.act_rows;
+    if (p.norm_w) {      // few rows, each of them by the whole CTA: k_rmsnorm_q8k's arithmetic
+        __shared__ double s_ss[RW_WARPS][DC_MAX_T];
+        const int lane = threadIdx.x & 31;
+        for (int row = 0; row < n; ++row) {
+            const float4* x = reinterpret_cast<const float4*>(p.act_f32 + (size_t)row * p.K);
+            double ss = 0.0;
+            for (int i = threadIdx.x; i < p.K / 4; i += RW_THREADS) {
+                const float4 v = __ldcg(x + i);
+                ss += ((double)v.x * v.x + (double)v.y * v.y) + ((double)v.z * v.z + (double)v.w * v.w);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0) s_ss[threadIdx.x >> 5][row] = ss;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x >> 5; i < n * nb; i += RW_WARPS) {
+            const int row = i / nb, b = i - row * nb;
+            const float4* x = reinterpret_cast<const float4*>(p.act_f32 + ((size_t)row * nb + b) * DC_QK_K) + 2 * lane;
+            const float4* w = reinterpret_cast<const float4*>(p.norm_w + b * DC_QK_K) + 2 * lane;
+            const float4 x0 = __ldcg(x), x1 = __ldcg(x + 1), w0 = w[0], w1 = w[1];
+            double tot = 0.0;
+#pragma unroll
+            for (int k = 0; k < RW_WARPS; ++k) tot += s_ss[k][row];
+            const float mean = (float)(tot / (double)p.K);
+            const float f = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.norm_eps)));
+            const float v[8] = {__fmul_rn(__fmul_rn(x0.x, f), w0.x), __fmul_rn(__fmul_rn(x0.y, f), w0.y), __fmul_rn(__fmul_rn(x0.z, f), w0.z), __fmul_rn(__fmul_rn(x0.w, f), w0.w),
+                                __fmul_rn(__fmul_rn(x1.x, f), w1.x), __fmul_rn(__fmul_rn(x1.y, f), w1.y), __fmul_rn(__fmul_rn(x1.z, f), w1.z), __fmul_rn(__fmul_rn(x1.w, f), w1.w)};
+            quantize_block_q8f_regs(v, smem + (b * rows + row) * DC_Q8F_BYTES, lane);
+        }
+        return;
+    }
     if (p.act_f32) {
         for (int i = threadIdx.x >> 5; i < n * nb; i += RW_WARPS) {
             const int row = i / nb, b = i - row * nb;
@@ -526,7 +559,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
     auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * S) : "memory"); };
     for (int tile = first + grp; tile < end; tile += step) {
         const RowsTile t = rows_tile<MOE>(p, tile);
-        const int nt = t.nt, row0 = t.a0 - a_lo;
+        const int nt = ONE ? 1 : t.nt, row0 = t.a0 - a_lo;
         for (int up = 0; up < (PAIR ? 2 : 1); ++up) {
 #pragma unroll
             for (int i = 0; i < NA; ++i) acc[i] = 0.0f;

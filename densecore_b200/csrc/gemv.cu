@@ -76,7 +76,7 @@ static int launch_rows_np(dc_ctx* ctx, RowsParams& p, int np, size_t smem) {
 }
 
 int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, const uint8_t* act_q8, int T, int K,
-                   unsigned long long* argmax, int32_t* dump_I, int32_t* dump_M, const float* act_f32) {
+                   unsigned long long* argmax, int32_t* dump_I, int32_t* dump_M, const float* act_f32, const float* norm_w, float norm_eps) {
     if (n_seg < 1 || n_seg > 3 || T < 1 || T > DC_MAX_T || K % DC_QK_K)
         return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "gemv: bad shape (n_seg=%d T=%d K=%d)", n_seg, T, K);
     RowsParams p = {};
@@ -84,6 +84,8 @@ int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, con
     p.epi = epi;
     p.act_q8 = act_q8;
     p.act_f32 = act_f32;
+    p.norm_w = act_f32 ? norm_w : nullptr;
+    p.norm_eps = norm_eps;
     p.T = p.act_rows = T;
     p.K = K;
     p.nb = K / DC_QK_K;
@@ -123,10 +125,10 @@ int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, con
             second[i] = segs[i];
             second[i].out = segs[i].out + (size_t)T0 * segs[i].ldo;
         }
-        int st = dc_launch_gemv(ctx, segs, n_seg, epi, act_q8, T0, K, nullptr, nullptr, nullptr, act_f32);
+        int st = dc_launch_gemv(ctx, segs, n_seg, epi, act_q8, T0, K, nullptr, nullptr, nullptr, act_f32, norm_w, norm_eps);
         if (st != DC_B200_OK) return st;
         return dc_launch_gemv(ctx, second, n_seg, epi, act_q8 + (size_t)T0 * (K / DC_QK_K) * DC_Q8F_BYTES, T - T0, K, nullptr, nullptr, nullptr,
-                              act_f32 ? act_f32 + (size_t)T0 * K : nullptr);
+                              act_f32 ? act_f32 + (size_t)T0 * K : nullptr, norm_w, norm_eps);
     }
     // parity capture of the block sums: the same kernel compiled with the stores in (never in a decoder step)
     if (dump_I) return q4 ? launch_rows<ROWS_Q4K, 8, false, false, true>(ctx, p, smem) : launch_rows<ROWS_Q6K, 8, false, false, true>(ctx, p, smem);

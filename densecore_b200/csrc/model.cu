@@ -223,14 +223,16 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
     const float* pending = nullptr;  // MoE output of the previous layer, added in the next norm
     bool split = false;              // the previous layer's expert outputs wait for their weighted sum
     const bool sum_in_norm = E > 0 && c.ep_size == 1;
+    const bool norm_in_rows = dc_rows_quantise(T, H);     // few rows: the product that reads them norms them itself, a launch less
     for (int il = 0; il < c.n_layer; ++il) {
         dc_layer& Ly = m->layers[il];
         if (split)
             L(DC_K_COMBINE, (double)T * top_k * H * 4 + xb + q8x, 1,
               dc_launch_moe_combine_norm(ctx, b.dn, b.route.ids, b.route.weights, T, top_k, H, b.x, (const float*)Ly.attn_norm->dev, c.rms_eps, nullptr, b.q8_x));
-        else
+        else if (!norm_in_rows || pending)
             L(DC_K_RMSNORM, xb + q8x + H * 4, 1,
               dc_launch_rmsnorm_q8k(ctx, b.x, pending, (const float*)Ly.attn_norm->dev, T, H, c.rms_eps, nullptr, b.q8_x));
+        const bool norm_qkv = norm_in_rows && !split && !pending;
         split = false;
         pending = nullptr;
         if (m->dbg_x)
@@ -241,7 +243,7 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
             {Ly.wv->dev, Ly.wv->type, KD, (int)Ly.wv->row_bytes, b.qkv + QD + KD, QKV},
         };
         L(DC_K_GEMV_QKV, (double)Ly.wq->bytes + Ly.wk->bytes + Ly.wv->bytes + q8x + (double)T * QKV * 4, 1,
-          dc_launch_gemv(ctx, qkv, 3, DC_EPI_STORE, b.q8_x, T, H, nullptr));
+          dc_launch_gemv(ctx, qkv, 3, DC_EPI_STORE, b.q8_x, T, H, nullptr, nullptr, nullptr, norm_qkv ? b.x : nullptr, (const float*)Ly.attn_norm->dev, c.rms_eps));
         __half* ka = m->kv.k_arena + m->kv.layer_elems * il;
         __half* va = m->kv.v_arena + m->kv.layer_elems * il;
         const dc_attn_fuse fuse = {b.qkv, Ly.q_norm ? (const float*)Ly.q_norm->dev : nullptr, Ly.k_norm ? (const float*)Ly.k_norm->dev : nullptr,
@@ -263,7 +265,8 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
         // few tokens: the router norms them itself
         const dc_route_norm rn = {b.x, (const float*)Ly.ffn_norm->dev, c.rms_eps, b.q8_x};
         const bool norm_in_router = E > 0 && T <= 4 && (size_t)T * H * 4 <= 128 * 1024;
-        if (!norm_in_router)
+        const bool norm_ffn = E == 0 && norm_in_rows;
+        if (!norm_in_router && !norm_ffn)
             L(DC_K_RMSNORM, xb * (E > 0 ? 2 : 1) + q8x + H * 4, 1,
               dc_launch_rmsnorm_q8k(ctx, b.x, nullptr, (const float*)Ly.ffn_norm->dev, T, H, c.rms_eps,
                                     E > 0 ? b.xn : nullptr, b.q8_x));
@@ -294,7 +297,7 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
                 {Ly.ffn_up->dev, Ly.ffn_up->type, c.ffn, (int)Ly.ffn_up->row_bytes, b.h, c.ffn},
             };
             L(DC_K_FFN_GATEUP, (double)Ly.ffn_gate->bytes + Ly.ffn_up->bytes + q8x + (double)T * c.ffn * 4, 1,
-              dc_launch_gemv(ctx, gu, 2, DC_EPI_SWIGLU, b.q8_x, T, H, nullptr));
+              dc_launch_gemv(ctx, gu, 2, DC_EPI_SWIGLU, b.q8_x, T, H, nullptr, nullptr, nullptr, norm_ffn ? b.x : nullptr, (const float*)Ly.ffn_norm->dev, c.rms_eps));
             const bool own = dc_rows_quantise(T, c.ffn);
             if (!own)
                 L(DC_K_QUANT_H, (double)T * c.ffn * 4 + (double)T * (c.ffn / 256) * DC_Q8F_BYTES, 1,
@@ -306,7 +309,9 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
     }
     if (lm_mode != 0) {
         const int rows = lm_mode == 1 ? 1 : T, first = lm_mode == 1 ? T - 1 : 0;
-        L(DC_K_RMSNORM, (double)rows * H * 4 * 2 + (double)rows * (H / 256) * DC_Q8F_BYTES, 1,
+        const bool norm_out = norm_in_rows && !pending;
+        if (!norm_out)
+          L(DC_K_RMSNORM, (double)rows * H * 4 * 2 + (double)rows * (H / 256) * DC_Q8F_BYTES, 1,
           dc_launch_rmsnorm_q8k(ctx, b.x + (size_t)first * H, pending ? pending + (size_t)first * H : nullptr,
                                 (const float*)m->out_norm->dev, rows, H, c.rms_eps, nullptr, b.q8_x));
         if (m->dbg_x)
@@ -314,7 +319,8 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
         const dc_weight* out_w = c.tie_embeddings ? m->tok_embd : m->output;
         dc_gemv_seg lm = {out_w->dev, out_w->type, c.vocab, (int)out_w->row_bytes, b.logits, c.vocab};
         L(DC_K_LM_HEAD, (double)out_w->bytes + (double)rows * (H / 256) * DC_Q8F_BYTES + (double)rows * c.vocab * 4, 1,
-          dc_launch_gemv(ctx, &lm, 1, DC_EPI_STORE, b.q8_x, rows, H, b.argmax_keys));
+          dc_launch_gemv(ctx, &lm, 1, DC_EPI_STORE, b.q8_x, rows, H, b.argmax_keys, nullptr, nullptr, norm_out ? b.x + (size_t)first * H : nullptr,
+                         (const float*)m->out_norm->dev, c.rms_eps));
         L(DC_K_ARGMAX, 64.0, 1,
           dc_launch_argmax_finish(ctx, b.argmax_keys, rows, b.out_tokens, feedback ? b.tokens : nullptr,
                                   feedback ? b.positions : nullptr, feedback ? b.history : nullptr,

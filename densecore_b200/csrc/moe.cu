@@ -156,24 +156,28 @@ __device__ __forceinline__ void route_token(const RouterParams& p, int t, int la
     }
 }
 
-// Routing of all T tokens by the whole CTA (DC_ROUTE_STABLE): an expert's place among a token's experts is the number of keys above its
-// own, so all experts find theirs at once; route_token's rounds of warp-wide maxima took 4.6 us a token.  Same picks, same weights.
-// s_key: 256 keys; s_sel: T * top_k picked logits.
+// Routing of all T tokens by the whole CTA (DC_ROUTE_STABLE): an expert's place among a token's experts is the number of better ones, so all
+// experts find theirs at once; route_token's rounds of warp-wide maxima took 4.6 us a token.  Same picks, same weights.
+// (Little unrolled: one CTA runs this once a launch, and instructions that are not in the SM's cache cost more than the loop.)
+// s_key: 256 keys, 16-byte aligned; s_sel: T * top_k picked logits.
 __device__ __forceinline__ void route_all_stable(const RouterParams& p, unsigned long long* s_key, float* s_sel, int32_t* s_ids) {
     const int tid = threadIdx.x, per = p.E <= 32 ? 8 : p.E <= 64 ? 4 : p.E <= 128 ? 2 : 1;     // tokens at a time
     const int width = 256 / per, slot = tid / width, e = tid % width;
+#pragma unroll 1
     for (int t0 = 0; t0 < p.T; t0 += per) {
         const int t = t0 + slot;
         const bool in = t < p.T && e < p.E;
-        const float v = in ? __ldcg(p.logits + (size_t)t * p.E + e) : 0.0f;
-        const unsigned long long key = in ? route_key(v, e) : 0ull;      // a real key is never 0
+        const unsigned long long key = in ? route_key(__ldcg(p.logits + (size_t)t * p.E + e), e) : 0ull;      // a real key is never 0
         s_key[tid] = key;
         __syncthreads();
         if (in) {
             int above = 0;
-            const unsigned long long* k = s_key + slot * width;
-#pragma unroll 8
-            for (int f = 0; f < p.E; ++f) above += k[f] > key;
+            const ulonglong2* k = reinterpret_cast<const ulonglong2*>(s_key + slot * width);
+#pragma unroll 4
+            for (int f = 0; f < (p.E + 1) / 2; ++f) {
+                const ulonglong2 x = k[f];
+                above += (x.x > key) + (x.y > key);
+            }
             if (above < p.top_k) {
                 const uint32_t ku = (uint32_t)(key >> 32);
                 s_sel[t * p.top_k + above] = __uint_as_float((ku & 0x80000000u) ? (ku & 0x7FFFFFFFu) : ~ku);    // (-0 became +0)
@@ -194,6 +198,7 @@ __device__ __forceinline__ void route_all_stable(const RouterParams& p, unsigned
         }
         float den = 0.0f, own = 0.0f;
         if (finite && isfinite(mx)) {
+#pragma unroll 1
             for (int k = 0; k < p.top_k; ++k) {
                 const float w = expf(sel[k] - mx);
                 if (k == i % p.top_k) own = w;
@@ -208,8 +213,8 @@ __device__ __forceinline__ void route_all_stable(const RouterParams& p, unsigned
 __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     __shared__ int s_last;
     __shared__ float s_prob[8][MOE_MAX_E];
-    __shared__ int32_t s_ids[DC_MAX_T * MOE_MAX_K];
-    __shared__ unsigned long long s_key[256];
+    __shared__ __align__(16) int32_t s_ids[DC_MAX_T * MOE_MAX_K + 4];
+    __shared__ __align__(16) unsigned long long s_key[256];
     __shared__ float s_sel[DC_MAX_T * MOE_MAX_K];
     __shared__ int s_wsum_a[8], s_wsum_c[8];
     pdl_launch_dependents();
@@ -271,9 +276,6 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
             }
         }
         __syncthreads();
-        const int nb = p.H / DC_QK_K;
-        for (int i = warp * gridDim.x + blockIdx.x; i < p.T * nb; i += 8 * gridDim.x)
-            quantize_block_q8k_warp<true>(s_xn + i * DC_QK_K, p.norm.q8_out + (size_t)i * DC_Q8F_BYTES, lane);
         xn = s_xn;
     }
     if (p.wr) {
@@ -338,10 +340,16 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
         s_last = old == (int)gridDim.x - 1;
         if (s_last) *p.ticket = 0;
     }
+    if (p.norm.x) {      // off the chain that the picks wait for
+        const int nb = p.H / DC_QK_K;
+        for (int i = warp * gridDim.x + blockIdx.x; i < p.T * nb; i += 8 * gridDim.x)
+            quantize_block_q8k_warp<true>(xn + i * DC_QK_K, p.norm.q8_out + (size_t)i * DC_Q8F_BYTES, lane);
+    }
     __syncthreads();
     if (!s_last) return;
 
     // ---- top-k per token
+    if (threadIdx.x < 4) s_ids[p.T * p.top_k + threadIdx.x] = -1;
     if (p.mode == DC_ROUTE_STABLE) route_all_stable(p, s_key, s_sel, s_ids);
     else
         for (int t = warp; t < p.T; t += 8) route_token(p, t, lane, s_prob[warp], s_ids);
@@ -351,7 +359,10 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     const int me = threadIdx.x;
     int cnt = 0;
     if (me < p.E && me >= p.ep_lo && me < p.ep_hi)
-        for (int i = 0; i < A; ++i) cnt += (s_ids[i] == me);
+        for (int i = 0; i < A; i += 4) {      // (s_ids is padded with -1)
+            const int4 x = *reinterpret_cast<const int4*>(s_ids + i);
+            cnt += (x.x == me) + (x.y == me) + (x.z == me) + (x.w == me);
+        }
     int act = (cnt + DC_MOE_PASS - 1) / DC_MOE_PASS;
     // inclusive scans of (act, cnt) over the 256 threads
     int sa = act, scn = cnt;
@@ -385,8 +396,13 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
             p.uoff[u + i] = off + DC_MOE_PASS * i;
         }
         int o = off;
-        for (int i = 0; i < A; ++i)
-            if (s_ids[i] == me) p.uassign[o++] = i;
+        for (int i = 0; o < off + cnt; i += 4) {
+            const int4 x = *reinterpret_cast<const int4*>(s_ids + i);
+            if (x.x == me) p.uassign[o++] = i;
+            if (x.y == me) p.uassign[o++] = i + 1;
+            if (x.z == me) p.uassign[o++] = i + 2;
+            if (x.w == me) p.uassign[o++] = i + 3;
+        }
     }
     if (threadIdx.x == 0) {
         *p.n_active = tot_a;
@@ -657,13 +673,16 @@ __global__ void __launch_bounds__(512) k_moe_combine_norm(const float* __restric
     float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (tid < n4) w0 = reinterpret_cast<const float4*>(nw)[tid];
     pdl_wait();
-    if (tid == 0) {
-        int order[MOE_MAX_K];
-        combine_order(ids, T, top_k, t, order);
-        for (int k = 0; k < top_k; ++k) {
-            s_a[k] = t * top_k + order[k];
-            s_w[k] = weights[s_a[k]];
+    if (tid < top_k) {      // combine_order's places, all at once
+        const int own = ids[t * top_k + tid];
+        const float w = weights[t * top_k + tid];
+        int at = tid;
+        if (!(T <= 4 && T * top_k <= 32)) {
+            at = 0;
+            for (int k = 0; k < top_k; ++k) at += ids[t * top_k + k] < own;
         }
+        s_a[at] = t * top_k + tid;
+        s_w[at] = w;
     }
     __syncthreads();
     double ss = 0.0;
