@@ -161,29 +161,25 @@ __device__ __forceinline__ void route_token(const RouterParams& p, int t, int la
 // (Little unrolled: one CTA runs this once a launch, and instructions that are not in the SM's cache cost more than the loop.)
 // s_key: 256 keys, 16-byte aligned; s_sel: T * top_k picked logits.
 __device__ __forceinline__ void route_all_stable(const RouterParams& p, unsigned long long* s_key, float* s_sel, int32_t* s_ids) {
-    const int tid = threadIdx.x, per = p.E <= 32 ? 8 : p.E <= 64 ? 4 : p.E <= 128 ? 2 : 1;     // tokens at a time
-    const int width = 256 / per, slot = tid / width, e = tid % width;
+    const int tid = threadIdx.x, P = p.E <= 32 ? 8 : p.E <= 64 ? 4 : p.E <= 128 ? 2 : 1;     // neighbouring threads that share an expert
+    const int e = tid / P, sub = tid % P;
+    const float* mine = p.logits + min(e, p.E - 1);
+    float v = __ldcg(mine);
 #pragma unroll 1
-    for (int t0 = 0; t0 < p.T; t0 += per) {
-        const int t = t0 + slot;
-        const bool in = t < p.T && e < p.E;
-        const unsigned long long key = in ? route_key(__ldcg(p.logits + (size_t)t * p.E + e), e) : 0ull;      // a real key is never 0
-        s_key[tid] = key;
+    for (int t = 0; t < p.T; ++t) {
+        const unsigned long long key = e < p.E ? route_key(v, e) : 0ull;      // a real key is never 0
+        if (sub == 0) s_key[e] = key;
+        if (t + 1 < p.T) v = __ldcg(mine + (size_t)(t + 1) * p.E);
         __syncthreads();
-        if (in) {
-            int above = 0;
-            const ulonglong2* k = reinterpret_cast<const ulonglong2*>(s_key + slot * width);
+        int above = 0;
 #pragma unroll 4
-            for (int f = 0; f < (p.E + 1) / 2; ++f) {
-                const ulonglong2 x = k[f];
-                above += (x.x > key) + (x.y > key);
-            }
-            if (above < p.top_k) {
-                const uint32_t ku = (uint32_t)(key >> 32);
-                s_sel[t * p.top_k + above] = __uint_as_float((ku & 0x80000000u) ? (ku & 0x7FFFFFFFu) : ~ku);    // (-0 became +0)
-                s_ids[t * p.top_k + above] = e;
-                p.ids[t * p.top_k + above] = e;
-            }
+        for (int f = sub; f < p.E; f += P) above += s_key[f] > key;
+        for (int o = 1; o < P; o <<= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
+        if (sub == 0 && e < p.E && above < p.top_k) {
+            const uint32_t ku = (uint32_t)(key >> 32);
+            s_sel[t * p.top_k + above] = __uint_as_float((ku & 0x80000000u) ? (ku & 0x7FFFFFFFu) : ~ku);    // (-0 became +0)
+            s_ids[t * p.top_k + above] = e;
+            p.ids[t * p.top_k + above] = e;
         }
         __syncthreads();
     }
@@ -354,6 +350,25 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     else
         for (int t = warp; t < p.T; t += 8) route_token(p, t, lane, s_prob[warp], s_ids);
     __syncthreads();
+    if (p.T == 1) {      // every pick is an expert's only token: the picks of this GPU's experts by ascending id
+        if (threadIdx.x < 32) {
+            const int k = threadIdx.x, own = k < p.top_k ? s_ids[k] : -1;
+            const bool local = own >= p.ep_lo && own < p.ep_hi;
+            int at = 0;
+            for (int j = 0; j < p.top_k; ++j) at += s_ids[j] >= p.ep_lo && s_ids[j] < own;
+            if (local) {
+                p.uexp[at] = own;
+                p.uoff[at] = at;
+                p.uassign[at] = k;
+            }
+            const int n = __popc(__ballot_sync(0xffffffffu, local));
+            if (k == 0) {
+                *p.n_active = n;
+                p.uoff[n] = n;
+            }
+        }
+        return;
+    }
     // ---- bucketing: thread e owns expert e
     const int A = p.T * p.top_k;
     const int me = threadIdx.x;
