@@ -7,7 +7,8 @@
 // acc = acc*alpha_b + sum_t fastexp(s_t - m_b) v_t, and finally acc/(d + 1e-6).
 // fastexp is a cubic polynomial, so the result depends on which maximum each
 // exponent is taken against.  To stay on the reference's numbers while cutting
-// the sequence into parallel runs, the work is split in two kernels:
+// the sequence into parallel runs, a cluster of CTAs shares it (k_attn_cluster,
+// below); a sequence table too long for a cluster's shared memory takes two kernels:
 //   k_attn_scores  every run computes its scores s_t and per-block maxima;
 //   k_attn_pv      every run rebuilds the reference's running-maximum chain from
 //                  ALL block maxima (so its exponents are taken against exactly
@@ -506,6 +507,8 @@ __global__ void __launch_bounds__(128) k_attn_pv_run(const AttnParams p) {
 // within a CTA; across CTAs the partials are scaled in the merge.
 // With `fuse.qkv` the kernel also norms and rotates the q heads (every CTA its own copy) and writes the new token's K and V rows
 // (k_qknorm_rope_kv); the tokens of such a step belong to different sequences.
+// What bounds it: the launch's dependency gap, the copy of K, one exchange of maxima and one of sums across the cluster.  32 Q / 4 KV
+// heads, 2304 keys, one token: 12.5 us a layer with norm, rotation and cache write, against 29 us for the three kernels it replaces.
 #define AC_THREADS 256
 #define AC_CAP 32              // KV blocks a CTA holds at most (a lane each)
 

@@ -542,8 +542,7 @@ __device__ __forceinline__ void q6k_half_ints(uint32_t blk, int j, const ActSmem
 // tok[s] = activation row of token slot s (slots >= nt are skipped).
 template <int NT, int TYPE>
 __device__ DC_HOT void rows_dot(uint32_t row, bool active, int lane, int G, const ActSmem& act, int nt,
-                                const int (&tok)[NT], float (&out)[NT], const BlockSumDump* dump = nullptr,
-                                int dump_row = 0) {
+                                const int (&tok)[NT], float (&out)[NT]) {
     const int nb = act.nb;
     const int lig = lane & (G - 1), gbase = lane & ~(G - 1);
     if (TYPE == DC_TYPE_Q4_K) {
@@ -567,11 +566,6 @@ __device__ DC_HOT void rows_dot(uint32_t row, bool active, int lane, int G, cons
                         const float yd = __int_as_float(lds32(act.dptr(tok[s], b)));
                         tI[s] = __fmul_rn(__fmul_rn(d, yd), (float)I[s]);
                         tM[s] = __fmul_rn(__fmul_rn(dmin, yd), (float)M[s]);
-                        if (dump) {
-                            const size_t di = ((size_t)tok[s] * dump->N + dump_row) * nb + b;
-                            dump->I[di] = I[s];
-                            if (dump->M) dump->M[di] = M[s];
-                        }
                     }
                 }
             }
@@ -629,12 +623,6 @@ __device__ DC_HOT void rows_dot(uint32_t row, bool active, int lane, int G, cons
                     if (s0 + s < nt) {
 #pragma unroll
                         for (int L = 0; L < 8; ++L) P[s][L] += __shfl_xor_sync(0xffffffffu, P[s][L], 1);
-                        if (dump && on && j == 0) {
-                            int tot = 0;
-#pragma unroll
-                            for (int L = 0; L < 8; ++L) tot += P[s][L];
-                            dump->I[((size_t)tok[s0 + s] * dump->N + dump_row) * nb + b] = tot;
-                        }
                     }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) x[s][k] = j ? P[s][4 + k] : P[s][k];
@@ -702,10 +690,9 @@ __device__ __forceinline__ float rows_dot1_typed(int type, uint32_t row, bool ac
 // Any token count, type decided at run time.
 template <int NT>
 __device__ __forceinline__ void rows_dot_typed(int type, uint32_t row, bool active, int lane, int G, const ActSmem& act,
-                                               int nt, const int (&tok)[NT], float (&out)[NT],
-                                               const BlockSumDump* dump = nullptr, int dump_row = 0) {
-    if (type == DC_TYPE_Q4_K) rows_dot<NT, DC_TYPE_Q4_K>(row, active, lane, G, act, nt, tok, out, dump, dump_row);
-    else rows_dot<NT, DC_TYPE_Q6_K>(row, active, lane, G, act, nt, tok, out, dump, dump_row);
+                                               int nt, const int (&tok)[NT], float (&out)[NT]) {
+    if (type == DC_TYPE_Q4_K) rows_dot<NT, DC_TYPE_Q4_K>(row, active, lane, G, act, nt, tok, out);
+    else rows_dot<NT, DC_TYPE_Q6_K>(row, active, lane, G, act, nt, tok, out);
 }
 
 // Generic-width lane-group sum (G a power of two <= 32, runtime value).

@@ -12,6 +12,12 @@
 // activations and a half-rate dp4a per four products for every token and for every row; the fragments of m16n8k32 / m16n8k16 hold
 // sixteen rows' codes once for all tokens.  Measured on B200: 8.4 cycles per instruction and scheduler for either shape, against 2
 // cycles per dp4a, i.e. 32 to 64 lanes' dp4a in the time of four.
+// What bounds it: many rows, issue slots (decoding the codes and the float terms, not the tensor instructions and not the bytes);
+// few rows, the latency of a unit's copy and decode, S units of a tile at a time.
+// Measured, microseconds at 1 / 4 / 8 / 16 tokens, rows_dot kernels before and these now (bytes alone: 11.5 and 16.8):
+//   Q4_K 65536 x 2048   25 / 60 / 158 / 337     22 / 27 / 28 / 40
+//   Q6_K 65536 x 2048   53 / 118 / 373 / 743    45 / 59 / 78 / 127
+//   Q4_K  6144 x 2048   7.5 for one token       5.9
 #pragma once
 #include "dc_common.cuh"
 #include "dc_internal.h"
@@ -426,11 +432,11 @@ struct RowsWalk {
             rows(g);
         }
     }
-    __device__ __forceinline__ void next(const RowsParams& p, int w, int g) {
-        b += p.S;
+    __device__ __forceinline__ void next(const RowsParams& p, int S, int w, int g) {
+        b += S;
         if (b < p.nb) {
-            s0 += p.S * BB;
-            s1 += p.S * BB;
+            s0 += S * BB;
+            s1 += S * BB;
             return;
         }
         b = w;
@@ -468,7 +474,7 @@ __device__ __forceinline__ void rows_copy(const uint8_t* s, uint32_t d, int t) {
 
 // The whole CTA on tiles [lo, hi) of a list, of which this is CTA `cta` of `ctas`; NP: pairs of tokens.  PREFETCH: the rows to read are
 // known before the predecessor's results are (a product's always are, an expert's where the routing is older than the predecessor).
-template <int TYPE, int NP, bool ONE, bool MOE, bool PAIR, bool DUMP, bool PREFETCH>
+template <int TYPE, int NP, bool ONE, bool ALONE, bool MOE, bool PAIR, bool DUMP, bool PREFETCH>
 __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int cta, int ctas, int lo, int hi) {
     constexpr bool Q4 = TYPE == DC_TYPE_Q4_K;
     constexpr int NS = RW_STAGES, NG = (NP + 3) / 4, NA = Q4 || ONE ? 4 * NG : 8 * NP, NR = Q4 ? 4 * NG : 2 * NP;   // sums, results of a lane
@@ -483,7 +489,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
         pdl_launch_dependents();
     }
     // expert rows: neighbouring tiles, so that a CTA meets few experts' tokens; matrices: tiles in turn
-    const int S = p.S, groups = RW_WARPS / S, w = warp & (S - 1), grp = warp / S;
+    const int S = ALONE ? 1 : p.S, groups = RW_WARPS / S, w = warp & (S - 1), grp = warp / S;      // ALONE: groups of one warp
     int first, end, step;
     if (MOE) {
         const unsigned total = (unsigned)(*p.n_active) * (unsigned)p.tiles;
@@ -509,7 +515,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
     for (int s = 0; s < NS - 1; ++s) {
         if (prod.valid) {
             copy(head);
-            prod.next(p, w, g);
+            prod.next(p, S, w, g);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         ++head;
@@ -544,9 +550,8 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
         if (Q4) acc[i] = __fsub_rn(__fadd_rn(acc[i], x), y);
         else acc[i] = __fmaf_rn(y, x, acc[i]);
     };
-    const bool alone = S == 1;
     auto sink = [&](int i, float x, float y) {
-        if (alone) {
+        if (ALONE) {
             add(i, x, y);
         } else if (Q4) {
             own[(2 * i) * 32] = x;
@@ -571,7 +576,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
                 if (b < p.nb) {
                     if (prod.valid) {
                         copy(head);
-                        prod.next(p, w, g);
+                        prod.next(p, S, w, g);
                     }
                     asm volatile("cp.async.commit_group;" ::: "memory");
                     head = head + 1 == NS ? 0 : head + 1;
@@ -588,7 +593,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
                     __syncwarp();
                     tail = tail + 1 == NS ? 0 : tail + 1;
                 }
-                if (alone) continue;
+                if (ALONE) continue;
                 meet();
                 if (w == 0) {
                     const int n = min(S, p.nb - b0);
@@ -605,7 +610,7 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
                 }
                 meet();      // the terms have been read
             }
-            if (w != 0 && !alone) continue;
+            if (w != 0) continue;
             // result i: Q4_K: token 8 (i / 4) + 2 tq + i % 2, row g + 8 (i / 2 % 2); Q6_K: token 2 (i / 2) + tq / 2, row g + 8 (i % 2)
             float v[NR];
             if constexpr (Q4) {
@@ -670,6 +675,8 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
 
 // Sizes of a launch; returns the dynamic shared memory, or 0 if the activations leave no room.  S: as many warps a tile as keep the SMs'
 // warps (two or three CTAs of eight) busy, for the tiles then run at the same time and a tile's latency is a few blocks' instead of all of them.
+// Above that line every warp has a tile of its own and the terms stay in registers: 65536 x 2048, 16 tokens, Q4_K 40 us against 46, and
+// Q6_K 127 against 143, for a kernel that also carries the code of the shared terms.
 static inline size_t rows_plan(RowsParams& p, int np, bool has_q6, long long tiles, int num_sms) {
     const long long warps = (has_q6 ? 16ll : 24ll) * num_sms;
     p.S = 1;

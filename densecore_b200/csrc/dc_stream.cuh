@@ -1,5 +1,5 @@
-// Row-streaming matmul bodies shared by the stand-alone kernels (k_gemv,
-// k_moe_mm) and the persistent decode kernel: each warp walks a contiguous
+// Row-streaming matmul bodies of the persistent decode kernel (the stand-alone
+// kernels' body is dc_rows.cuh): each warp walks a contiguous
 // range of weight rows through its bulk-copy pipeline, decodes them against the
 // Q8_K activations in shared memory and writes one float per (row, token).
 #pragma once
@@ -20,7 +20,6 @@ struct GemvParams {
     uint32_t up_off;  // SwiGLU: offset of the up rows inside a stage
     unsigned long long* argmax;
     int* err;
-    BlockSumDump dump;   // parity checks only: where the exact block sums go (I == nullptr: nowhere)
 };
 
 // Walks a warp's contiguous flattened row range stage by stage.
@@ -132,11 +131,11 @@ struct GemvStream {
     // SWIGLU = false leaves the paired gate/up path out of the generated code (callers that
     // never stream pairs).
     // SWIGLU = false leaves the paired gate/up path out of the generated code (callers that never stream
-    // pairs).  DUMP = true also stores the exact block sums (parity checks; never in the decoder's launches).
+    // pairs).
     // A warp pass runs 32 / G rows side by side, one per lane group.  Gate/up pairs: the lower half of the
     // groups takes gate rows, the upper half the up rows of the same outputs, and the two halves swap
     // results 16 lanes across (one group per row, G = 32: gate row, then up row).
-    template <int NT, bool SWIGLU = true, bool DUMP = false>
+    template <int NT, bool SWIGLU = true>
     __device__ DC_HOT void consume(const GemvParams& p, WarpPipe<NSTAGE>& pipe, const ActSmem& act, int lane) {
         int tok[NT];
 #pragma unroll
@@ -158,20 +157,19 @@ struct GemvStream {
             const uint32_t skew = (uint32_t)(((uintptr_t)s.w + (size_t)lr * s.row_bytes) & 15);
             const uint32_t skew_up = pair ? (uint32_t)(((uintptr_t)p.seg[1].w + (size_t)lr * s.row_bytes) & 15) : 0u;
             const uint32_t base = up_half ? buf + p.up_off + skew_up : buf + skew;
-            const BlockSumDump* dump = DUMP ? &p.dump : nullptr;
             for (int r = 0; r < n; r += opp) {
                 const int rr = r + (split ? grp % opp : grp);
                 const bool active = rr < n;
                 float acc[NT], acc2[NT];
-                if (NT == 1 && !DUMP) acc[0] = rows_dot1_typed(s.type, base + rr * s.row_bytes, active, lane, G, act, 0);
-                else rows_dot_typed<NT>(s.type, base + rr * s.row_bytes, active, lane, G, act, p.T, tok, acc, dump, lr + rr);
+                if (NT == 1) acc[0] = rows_dot1_typed(s.type, base + rr * s.row_bytes, active, lane, G, act, 0);
+                else rows_dot_typed<NT>(s.type, base + rr * s.row_bytes, active, lane, G, act, p.T, tok, acc);
                 if (pair) {
                     if (split) {
 #pragma unroll
                         for (int t = 0; t < NT; ++t) acc2[t] = __shfl_xor_sync(0xffffffffu, acc[t], 16);
                     } else {
                         const uint32_t urow = buf + p.up_off + skew_up + rr * s.row_bytes;
-                        if (NT == 1 && !DUMP) acc2[0] = rows_dot1_typed(s.type, urow, active, lane, G, act, 0);
+                        if (NT == 1) acc2[0] = rows_dot1_typed(s.type, urow, active, lane, G, act, 0);
                         else rows_dot_typed<NT>(s.type, urow, active, lane, G, act, p.T, tok, acc2);
                     }
                 }

@@ -36,19 +36,19 @@ int dc_launch_quantize_q8k(dc_ctx* ctx, const float* x, int rows, int K, uint8_t
 // KIND: matrices of Q4_K, of Q6_K, or of both, where every CTA works on one type.  Weights do not depend on the previous kernel:
 // they stream in while this one waits for it.
 enum { ROWS_Q4K = 0, ROWS_Q6K = 1, ROWS_BOTH = 2 };
-template <int KIND, int NP, bool ONE, bool PAIR, bool DUMP>
+template <int KIND, int NP, bool ONE, bool ALONE, bool PAIR, bool DUMP>
 __global__ void __launch_bounds__(RW_THREADS, NP > 4 ? 1 : KIND == ROWS_Q4K ? 3 : 2) k_rows(const RowsParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     if (KIND == ROWS_Q4K || (KIND == ROWS_BOTH && blockIdx.x < p.ctas4)) {
-        rows_cta<DC_TYPE_Q4_K, NP, ONE, false, PAIR, DUMP, true>(p, smem, blockIdx.x, p.ctas4, 0, p.tiles4);
+        rows_cta<DC_TYPE_Q4_K, NP, ONE, ALONE, false, PAIR, DUMP, true>(p, smem, blockIdx.x, p.ctas4, 0, p.tiles4);
     } else {
-        rows_cta<DC_TYPE_Q6_K, NP, ONE, false, PAIR, DUMP, true>(p, smem, blockIdx.x - p.ctas4, gridDim.x - p.ctas4, p.tiles4, p.tiles);
+        rows_cta<DC_TYPE_Q6_K, NP, ONE, ALONE, false, PAIR, DUMP, true>(p, smem, blockIdx.x - p.ctas4, gridDim.x - p.ctas4, p.tiles4, p.tiles);
     }
 }
 
-template <int KIND, int NP, bool ONE, bool PAIR, bool DUMP>
-static int launch_rows(dc_ctx* ctx, RowsParams& p, size_t smem) {
-    const void* f = (const void*)k_rows<KIND, NP, ONE, PAIR, DUMP>;
+template <int KIND, int NP, bool ONE, bool PAIR, bool DUMP, bool ALONE>
+static int launch_rows_as(dc_ctx* ctx, RowsParams& p, size_t smem) {
+    const void* f = (const void*)k_rows<KIND, NP, ONE, ALONE, PAIR, DUMP>;
     int st = dc_kernel_setup(ctx, f, 220 * 1024, "cudaFuncSetAttribute(k_rows)");
     if (st != DC_B200_OK) return st;
     int per_sm = dc_kernel_occupancy(ctx, f, RW_THREADS, smem);
@@ -64,7 +64,11 @@ static int launch_rows(dc_ctx* ctx, RowsParams& p, size_t smem) {
         if (c4 > n4) c4 = n4;
     }
     p.ctas4 = c4;
-    return dc_launch(ctx, "k_rows", k_rows<KIND, NP, ONE, PAIR, DUMP>, dim3(c4 + c6), dim3(RW_THREADS), smem, p);
+    return dc_launch(ctx, "k_rows", k_rows<KIND, NP, ONE, ALONE, PAIR, DUMP>, dim3(c4 + c6), dim3(RW_THREADS), smem, p);
+}
+template <int KIND, int NP, bool ONE, bool PAIR, bool DUMP>
+static int launch_rows(dc_ctx* ctx, RowsParams& p, size_t smem) {
+    return p.S == 1 ? launch_rows_as<KIND, NP, ONE, PAIR, DUMP, true>(ctx, p, smem) : launch_rows_as<KIND, NP, ONE, PAIR, DUMP, false>(ctx, p, smem);
 }
 template <int KIND, bool PAIR>
 static int launch_rows_np(dc_ctx* ctx, RowsParams& p, int np, size_t smem) {

@@ -524,22 +524,26 @@ int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, 
 // Down projection (PAIR false): the routing was final before this kernel could start (the gate/up kernel lets its successor start only
 // after its own wait, and so does the quantiser between the two, an ordinary launch), so the expert rows can be requested while this
 // kernel still waits for its predecessor's output.  Gate/up: the expert ids come from the router kernel just before.
-template <int TYPE, int NP, bool ONE, bool PAIR>
+template <int TYPE, int NP, bool ONE, bool ALONE, bool PAIR>
 __global__ void __launch_bounds__(RW_THREADS, TYPE == DC_TYPE_Q4_K ? 3 : 2) k_moe_rows(const RowsParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    rows_cta<TYPE, NP, ONE, true, PAIR, false, !PAIR>(p, smem, blockIdx.x, gridDim.x, 0, 0);
+    rows_cta<TYPE, NP, ONE, ALONE, true, PAIR, false, !PAIR>(p, smem, blockIdx.x, gridDim.x, 0, 0);
 }
 
-template <int TYPE, int NP, bool ONE, bool PAIR>
-static int launch_moe_rows(dc_ctx* ctx, const RowsParams& p, size_t smem, int max_tiles) {
-    const void* f = (const void*)k_moe_rows<TYPE, NP, ONE, PAIR>;
+template <int TYPE, int NP, bool ONE, bool PAIR, bool ALONE>
+static int launch_moe_rows_as(dc_ctx* ctx, const RowsParams& p, size_t smem, int max_tiles) {
+    const void* f = (const void*)k_moe_rows<TYPE, NP, ONE, ALONE, PAIR>;
     int st = dc_kernel_setup(ctx, f, 220 * 1024, "cudaFuncSetAttribute(k_moe_rows)");
     if (st != DC_B200_OK) return st;
     int per_sm = dc_kernel_occupancy(ctx, f, RW_THREADS, smem);
     if (per_sm < 1) per_sm = 1;
     const int groups = RW_WARPS / p.S, useful = (max_tiles + groups - 1) / groups;
     const int grid = useful < ctx->num_sms * per_sm ? useful : ctx->num_sms * per_sm;
-    return dc_launch(ctx, "k_moe_rows", k_moe_rows<TYPE, NP, ONE, PAIR>, dim3(grid), dim3(RW_THREADS), smem, p);
+    return dc_launch(ctx, "k_moe_rows", k_moe_rows<TYPE, NP, ONE, ALONE, PAIR>, dim3(grid), dim3(RW_THREADS), smem, p);
+}
+template <int TYPE, int NP, bool ONE, bool PAIR>
+static int launch_moe_rows(dc_ctx* ctx, const RowsParams& p, size_t smem, int max_tiles) {
+    return p.S == 1 ? launch_moe_rows_as<TYPE, NP, ONE, PAIR, true>(ctx, p, smem, max_tiles) : launch_moe_rows_as<TYPE, NP, ONE, PAIR, false>(ctx, p, smem, max_tiles);
 }
 template <int TYPE, bool PAIR>
 static int launch_moe_rows_np(dc_ctx* ctx, const RowsParams& p, int np, size_t smem, int max_tiles) {
@@ -577,7 +581,8 @@ int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weigh
     p.err = ctx->d_err;
     // A kernel takes up to DC_MOE_PASS tokens of an expert; the few experts with more come several times over and are read again from
     // L2.  (Kernels for sixteen tokens an expert hold 255 registers, eight warps an SM: 259 us for 16 tokens of 8 out of 128 experts.)
-    // act_rows: the passes that one CTA's neighbouring tiles touch are one more than its share of them, rounded up.
+    // act_rows: the passes that one CTA's neighbouring tiles touch are one more than its share of them, rounded up (a pass has 16 tiles at
+    // least, N being a multiple of 256, and a CTA eight or fewer where the SMs are not full).
     const int A = T * top_k, E = (int)w0->E, most = E + A / DC_MOE_PASS, U = most < A ? most : A;
     const int span = U <= 1 ? 1 : (U + ctx->num_sms - 1) / ctx->num_sms + 1, per = T < DC_MOE_PASS ? T : DC_MOE_PASS;
     p.act_rows = span * per < A ? span * per : A;
@@ -675,7 +680,8 @@ int dc_launch_moe_combine(dc_ctx* ctx, const float* dn, const int32_t* ids, cons
 }
 
 // One CTA per token: the combine above added to the residual, then RMSNorm and Q8_K blocks (k_rmsnorm_q8k's arithmetic).  A kernel of its
-// own for the combine cost a launch of the step's chain and wrote and read the sum again.
+// own for the combine cost a launch of the step's chain and wrote and read the sum again.  Bound by that chain (its bytes are 82 KB a
+// token): 4.4 us a layer at one token.
 __global__ void __launch_bounds__(512) k_moe_combine_norm(const float* __restrict__ dn, const int32_t* __restrict__ ids, const float* __restrict__ weights,
                                                           int T, int top_k, int H, float* __restrict__ x, const float* __restrict__ nw, float eps,
                                                           float* __restrict__ xn_out, uint8_t* __restrict__ q8_out) {
