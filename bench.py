@@ -627,7 +627,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--profile-classes", action="store_true", help="print the per-kernel-class table to stderr")
     ap.add_argument("--path", default="persistent", choices=["persistent", "per-op"],
-                    help="persistent: one cooperative kernel per decode run where the model fits its plan (default); "
+                    help="persistent: one cooperative kernel per decode run where that is the faster path (default); "
                          "per-op: one kernel per op, replayed as a CUDA graph")
     ap.add_argument("--phase-timing", action="store_true",
                     help="print the persistent kernel's per-phase device time (CTA 0's view) to stderr")
@@ -837,7 +837,7 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "int8 x int4/int6 block dots (dp4a), f32 accumulate", "data": "synthetic",
+        "dtype": "int8 x int4/int6 block dots, f32 accumulate", "data": "synthetic",
         "config": dict(bench_config(1, args.layers, args.prompt, world), ctx_at_timing=r1["ctx"],
                        path="persistent kernel" if persistent else "per-op CUDA graph",
                        l2="each step reads ~1.9 GB of weights, far more than the 126 MB L2, so no flush is needed"),
