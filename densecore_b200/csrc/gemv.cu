@@ -89,6 +89,7 @@ int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, con
     p.act_q8 = act_q8;
     p.act_f32 = act_f32;
     p.norm_w = act_f32 ? norm_w : nullptr;
+    if (p.norm_w && !dc_rows_quantise(T, K)) return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "gemv: too many rows to norm (T=%d K=%d)", T, K);
     p.norm_eps = norm_eps;
     p.T = p.act_rows = T;
     p.K = K;
