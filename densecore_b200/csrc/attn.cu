@@ -8,7 +8,7 @@
 // fastexp is a cubic polynomial, so the result depends on which maximum each
 // exponent is taken against.  To stay on the reference's numbers while cutting
 // the sequence into parallel runs, a cluster of CTAs shares it (k_attn_cluster,
-// below); a sequence table too long for a cluster's shared memory takes two kernels:
+// below) where that is the faster form and its keys fit into the cluster's shared memory; else two kernels do it:
 //   k_attn_scores  every run computes its scores s_t and per-block maxima;
 //   k_attn_pv      every run rebuilds the reference's running-maximum chain from
 //                  ALL block maxima (so its exponents are taken against exactly
@@ -17,6 +17,8 @@
 //                  later blocks, and the last run to finish (a ticket, no
 //                  waiting) adds the partials and emits f32 and Q8_K output.
 // Only float summation order differs from the sequential walk.
+#include <algorithm>
+
 #include "dc_common.cuh"
 #include "dc_internal.h"
 #include "dc_launch.cuh"
@@ -499,18 +501,40 @@ __global__ void __launch_bounds__(128) k_attn_pv_run(const AttnParams p) {
 
 // ------------------------------------------------------- one kernel, a cluster per (token, kv head)
 // What bounds decode attention at these lengths is not its bytes (4.7 MB of K and V at 2304 keys: 0.7 us of HBM) but the chain of
-// global round trips between score, P.V and merge kernels.  Here the CTAs of a cluster share a sequence's blocks and exchange
+// global round trips between score, P.V and merge kernels.  Here the CTAs of a cluster share a sequence's runs and exchange
 // block maxima and partial sums through each other's shared memory: K and V rows of earlier positions are copied to shared memory while
 // this kernel still waits for its predecessor, scores never leave the SM, and the merge reads all partials at once.
-// The running-maximum chain is the reference's: a block's exponents are taken against the largest score up to that block.  What the
-// reference multiplies onto its accumulator block by block (alpha) is multiplied onto the exponentials of the blocks before instead,
-// within a CTA; across CTAs the partials are scaled in the merge.
+// The runs, and the order of every float operation, are those of k_attn_scores and k_attn_pv_run, so the results are theirs bit for bit
+// and which kernels serve a call is a matter of speed alone: a key's product is four chains of 32 dimensions, a run walks its keys in
+// order and multiplies the reference's alpha onto its accumulator at every block, the alphas of later blocks are multiplied 32 at a
+// time, and the merge adds the runs in order.  (Q8_K rounding downstream turns a difference in the last bit into one of 1 % in the logits
+// of a random model, so that another order of sums would not be told from an error.)
 // With `fuse.qkv` the kernel also norms and rotates the q heads (every CTA its own copy) and writes the new token's K and V rows
 // (k_qknorm_rope_kv); the tokens of such a step belong to different sequences.
-// What bounds it: the launch's dependency gap, the copy of K, one exchange of maxima and one of sums across the cluster.  32 Q / 4 KV
-// heads, 2304 keys, one token: 12.5 us a layer with norm, rotation and cache write, against 29 us for the three kernels it replaces.
+// What bounds it: the launch's dependency gap, then the latency of its phases (scores 3 to 4 thousand cycles of 16 at one token and 2000
+// keys, P.V as long), in which instructions met for the first time cost as much as the arithmetic: loops over heads, blocks and runs
+// stay rolled.  32 Q / 4 KV heads, 2000 keys, one token, a step of three layers: 178 us; with the split kernels and k_qknorm_rope_kv 260;
+// 171 with keys dealt out over the threads in an order of sums that is not the split kernels'.
 #define AC_THREADS 256
-#define AC_CAP 32              // KV blocks a CTA holds at most (a lane each)
+#define AC_CAP 32              // KV blocks a CTA holds at most
+#define AC_SMEM (220 * 1024)
+#define AC_Q_PITCH 144         // floats of a q head: four quarters 36 apart, which fall into different banks
+
+// The runs of a sequence (split_range's, the empty ones left out) that CTA `rank` of C works on, and its blocks.
+struct AcRuns {
+    int n_blk, bps, n_run, rpc;      // blocks, blocks of a run, runs, runs of a CTA
+    int r0, r1, b0, b1;
+    __device__ __forceinline__ void set(int pos, int rank, int C, int nsplit) {
+        n_blk = (pos + 1 + DC_KV_BLOCK - 1) / DC_KV_BLOCK;
+        bps = max(1, (n_blk + nsplit - 1) / nsplit);
+        n_run = (n_blk + bps - 1) / bps;
+        rpc = max(1, (n_run + C - 1) / C);
+        r0 = min(n_run, rank * rpc);
+        r1 = min(n_run, r0 + rpc);
+        b0 = min(n_blk, r0 * bps);
+        b1 = min(n_blk, r1 * bps);
+    }
+};
 
 __device__ __forceinline__ uint32_t ac_rank() {
     uint32_t r;
@@ -520,33 +544,23 @@ __device__ __forceinline__ uint32_t ac_rank() {
 __device__ __forceinline__ void ac_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float ac_peer(const float* mine, uint32_t rank) {
+// the address of `mine` in CTA `rank`'s shared memory, and a load from such an address
+__device__ __forceinline__ uint32_t ac_map(const float* mine, uint32_t rank) {
     uint32_t a;
-    float v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(mine)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float ac_load(uint32_t a) {
+    float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ float4 ac_peer4(const float* mine, uint32_t rank) {
-    uint32_t a;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(mine)), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-    return v;
-}
-// d = a * b + d on two floats at a time (each rounded once, as two fmaf would)
-__device__ __forceinline__ void ac_fma2(float2& d, float2 a, float2 b) {
-    asm("{\n.reg .b64 ra, rb, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nmov.b64 rd, {%0, %1};\n"
-        "fma.rn.f32x2 rd, ra, rb, rd;\nmov.b64 {%0, %1}, rd;\n}"
-        : "+f"(d.x), "+f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-}
-// place of the 16-byte piece i of a key's K row: eight lanes (two keys x four pieces) fall on distinct banks
-__device__ __forceinline__ int ac_piece(int key, int i) { return key * 256 + ((i ^ ((key & 1) << 2)) << 4); }
+// place of 16-byte piece i of a key's K row: piece 4 q + i of quarter q at 4 i + q, so that eight lanes (four quarters of two
+// neighbouring keys) fall on distinct banks
+__device__ __forceinline__ int ac_piece(int key, int i) { return key * 256 + ((((i & 3) << 2 | i >> 2) ^ ((key & 1) << 2)) << 4); }
 __device__ __forceinline__ void ac_copy16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-// place of (key, head) among the scores: eight heads together, eight floats more per block so that four blocks fall on distinct banks
-__device__ __forceinline__ int ac_at(int key, int h) { return key * 8 + (key >> 4) * 8 + h; }
 
 // One head of 128 values by one warp: RMSNorm (w4 given) and rotation of interleaved pairs (c given), as k_qknorm_rope_kv.
 __device__ __forceinline__ float4 ac_norm_rope(const float* src, bool norm, float4 w4, bool turn, float4 c, float eps, int lane) {
@@ -578,22 +592,127 @@ __device__ __forceinline__ uint2 ac_half4(float4 v) {
     return r;
 }
 
-// C: CTAs of a cluster.  hs: clusters that share a kv head's query heads.
+// P.V of one run (the j-th of this CTA's): H heads from h0 on, D dimensions from d0 on a thread; the results times the alphas of all later
+// blocks.
+template <int H, int D>
+__device__ __forceinline__ void ac_pv(const AcRuns& R, const uint8_t* sKV, const float* sP, const float* sAl, const float* sSuf, int j, int h0, int d0, int g,
+                                      int cap, int ps, int keys, float (&a)[H][D]) {
+    constexpr int N = H * D > 4 ? 4 : 16;      // keys whose loads are in flight together
+    const int end = min(R.b1 - R.b0, (j + 1) * R.bps);
+    auto row = [&](const uint8_t* v, float (&f)[D]) {
+        if constexpr (D == 4) {
+            const uint2 u = *reinterpret_cast<const uint2*>(v);
+            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), y = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            f[0] = x.x, f[1] = x.y, f[2] = y.x, f[3] = y.y;
+        } else {
+            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(v));
+            f[0] = x.x, f[1] = x.y;
+        }
+    };
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int d = 0; d < D; ++d) a[h][d] = 0.0f;
+#pragma unroll 1
+    for (int bl = j * R.bps; bl < end; ++bl) {
+        const uint8_t* v = sKV + bl * DC_KV_BLOCK * 256 + d0 * 2;
+        const float* pp = sP + h0 * ps + bl * DC_KV_BLOCK;
+        const int nk = keys - bl * DC_KV_BLOCK;      // (16 or more, but for the sequence's last block)
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const float al = sAl[(h0 + h) * cap + bl];
+#pragma unroll
+            for (int d = 0; d < D; ++d) a[h][d] = __fmul_rn(a[h][d], al);
+        }
+        if (nk >= DC_KV_BLOCK) {
+#pragma unroll 1
+            for (int q = 0; q < DC_KV_BLOCK; q += N) {
+                float4 x[H][N / 4];
+                float f[N][D];
+#pragma unroll
+                for (int k = 0; k < N; ++k) row(v + (q + k) * 256, f[k]);
+#pragma unroll
+                for (int h = 0; h < H; ++h)
+#pragma unroll
+                    for (int k = 0; k < N / 4; ++k) x[h][k] = *reinterpret_cast<const float4*>(pp + h * ps + q + 4 * k);
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+#pragma unroll
+                    for (int h = 0; h < H; ++h) {
+                        const float4& y = x[h][k / 4];
+                        const float w = k % 4 == 0 ? y.x : k % 4 == 1 ? y.y : k % 4 == 2 ? y.z : y.w;
+#pragma unroll
+                        for (int d = 0; d < D; ++d) a[h][d] = fmaf(w, f[k][d], a[h][d]);
+                    }
+            }
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < nk; ++k) {
+                float f[D];
+                row(v + k * 256, f);
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const float w = pp[h * ps + k];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) a[h][d] = fmaf(w, f[d], a[h][d]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+        const float f = sSuf[j * g + h0 + h];
+#pragma unroll
+        for (int d = 0; d < D; ++d) a[h][d] = __fmul_rn(a[h][d], f);
+    }
+}
+// All of this CTA's runs by the CTA's four groups of threads.  Several runs: a group takes a run, its warps half of the heads each, and
+// leaves the sums where the run's V rows were, which nobody else reads.  At most one run: the groups share its heads, and the
+// sums go to `one`.
+template <int G>
+__device__ __forceinline__ void ac_pv_all(const AcRuns& R, uint8_t* sKV, const float* sP, const float* sAl, const float* sSuf, float* one, int cap, int rcap,
+                                          int ps, int keys) {
+    const int kg = threadIdx.x >> 6, nr = R.r1 - R.r0;
+    if (rcap == 1) {
+        constexpr int H = G == 8 || G == 6 ? 2 : 1;
+        const int d0 = 2 * (threadIdx.x & 63);
+        if (nr > 0 && kg < G / H) {
+            float a[H][2];
+            ac_pv<H, 2>(R, sKV, sP, sAl, sSuf, 0, kg * H, d0, G, cap, ps, keys, a);
+#pragma unroll
+            for (int h = 0; h < H; ++h) *reinterpret_cast<float2*>(one + (kg * H + h) * 128 + d0) = make_float2(a[h][0], a[h][1]);
+        }
+        return;
+    }
+    constexpr int H = G / 2;
+    const int h0 = (threadIdx.x >> 5 & 1) * H, d0 = 4 * (threadIdx.x & 31);
+    for (int j = kg; j < nr; j += AC_THREADS / 64) {
+        float a[H][4];
+        ac_pv<H, 4>(R, sKV, sP, sAl, sSuf, j, h0, d0, G, cap, ps, keys, a);
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + kg) : "memory");      // the group has read the run's V rows
+        float* to = reinterpret_cast<float*>(sKV + (size_t)j * R.bps * DC_KV_BLOCK * 256) + h0 * 128 + d0;
+#pragma unroll
+        for (int h = 0; h < H; ++h) *reinterpret_cast<float4*>(to + h * 128) = make_float4(a[h][0], a[h][1], a[h][2], a[h][3]);
+    }
+}
+
+// C: CTAs of a cluster.  cap, rcap: KV blocks and runs that a CTA holds at most.  hs: clusters that share a kv head's query heads.
 template <int C>
-__global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams p, const dc_attn_fuse fuse, const int cap, const int hs) {
+__global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams p, const dc_attn_fuse fuse, const int cap, const int rcap, const int hs) {
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* sKV = smem;                                           // K rows, after the scores V rows, after P.V partial sums: [key][256]
-    float* sP = reinterpret_cast<float*>(sKV + max(cap * DC_KV_BLOCK * 256, 4 * ATT_MAX_GROUP * 128 * 4));   // scores, then weighted exponentials, see ac_at
-    float* sQ = sP + cap * (DC_KV_BLOCK + 1) * 8;                  // [head][128]
-    float* sPart = sQ + ATT_MAX_GROUP * 128;                       // [head][128], read by the other CTAs
-    float* sBm = sPart + ATT_MAX_GROUP * 128;                      // [block][head]: block maximum, then the maximum to take exponents against
-    float* sW = sBm + cap * 8;                                     // [block][head]: product of the alphas of this CTA's later blocks
-    float* sMax = sW + cap * 8;                                    // [head], read by the other CTAs, as are the next two
-    float* sDen = sMax + 8;
-    float* sProd = sDen + 8;
+    __shared__ int32_t sTab[AC_CAP];                               // ids of this CTA's KV blocks
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)ac_rank(), kvh = blockIdx.x / (C * hs), part = blockIdx.x / C % hs, t = blockIdx.y, g = p.n_head / p.n_kv / hs;
     const int head0 = (kvh * hs + part) * g;                       // first of this cluster's query heads
+    const int ps = cap * DC_KV_BLOCK + 4;                          // floats between heads' scores: eight heads' pieces on distinct banks
+    uint8_t* sKV = smem;                                           // K rows, after the scores V rows: [key][256]
+    float* sP = reinterpret_cast<float*>(sKV + cap * DC_KV_BLOCK * 256);   // [head][ps] scores, then exponentials
+    float* sQ = sP + g * ps;                                       // [head][AC_Q_PITCH]
+    float* sDen = sQ + g * AC_Q_PITCH;                             // [run][head], read by the other CTAs, as is the next
+    float* sBm = sDen + rcap * g;                                  // [head][block] block maximum
+    float* sM = sBm + g * cap;                                     // [head][block] the maximum to take exponents against, then the exponentials' sum
+    float* sAl = sM + g * cap;                                     // [head][block] alpha
+    float* sSuf = sAl + g * cap;                                   // [run][head] product of the alphas of all later blocks
     pdl_launch_dependents();
     const int sid = p.seq_ids[t];
     const int32_t* table = p.block_tables + (size_t)sid * p.max_blocks;
@@ -614,11 +733,11 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
     if (!fuse.qkv)
         for (int u = 0; u < p.T; ++u)
             if (p.seq_ids[u] == sid) stable = min(stable, p.positions[u]);
-    int n_blk, b0, b1;
-    split_range(pos0, rank, C, n_blk, b0, b1);
-    const bool early = pos0 >= 0 && b1 - b0 <= cap;
+    AcRuns R;
+    R.set(pos0, rank, C, p.nsplit);
+    const bool early = pos0 >= 0 && R.b1 - R.b0 <= cap;
     if (early) {
-        const int from = b0 * DC_KV_BLOCK, to = min(b1 * DC_KV_BLOCK, stable);
+        const int from = R.b0 * DC_KV_BLOCK, to = min(R.b1 * DC_KV_BLOCK, stable);
         load_k(from, from, to);
         // V's turn in the shared buffer comes after the scores; until then its rows, two lines each, come from HBM into L2
         // (a 48-layer step at 2050 keys: 0.8 % of it)
@@ -628,8 +747,8 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
             asm volatile("prefetch.global.L2 [%0];" ::"l"(v));
         }
     }
-    auto turn_at = [&](int ps) {
-        const int rp = ps < 0 ? 0 : (fuse.max_pos > 0 && ps >= fuse.max_pos) ? fuse.max_pos - 1 : ps;
+    auto turn_at = [&](int at) {
+        const int rp = at < 0 ? 0 : (fuse.max_pos > 0 && at >= fuse.max_pos) ? fuse.max_pos - 1 : at;
         return reinterpret_cast<const float4*>(fuse.cos_sin + (size_t)rp * 128)[lane];
     };
     float4 qw = make_float4(0.f, 0.f, 0.f, 0.f), kw = qw, turn = qw;
@@ -640,20 +759,23 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
     }
     pdl_wait();
     const int pos = *reinterpret_cast<const volatile int32_t*>(p.positions + t);
-    split_range(pos, rank, C, n_blk, b0, b1);
-    const int k0 = b0 * DC_KV_BLOCK, nbl = b1 - b0, keys = max(0, min(pos + 1, b1 * DC_KV_BLOCK) - k0);
+    if (pos != pos0) R.set(pos, rank, C, p.nsplit);
+    const int k0 = R.b0 * DC_KV_BLOCK, nbl = R.b1 - R.b0, nr = R.r1 - R.r0, keys = max(0, min(pos + 1, R.b1 * DC_KV_BLOCK) - k0);
     {
         const bool same = early && pos == pos0;
+        if (tid < nbl) sTab[tid] = table[R.b0 + tid];
         if (!same) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         load_k(k0, same ? max(k0, stable) : k0, k0 + keys - (fuse.qkv && k0 + keys == pos + 1 ? 1 : 0));
     }
     uint2 new_v = make_uint2(0u, 0u);     // the new token's V row (warp 7), which has to wait for the K rows to go
     const bool mine = fuse.qkv && keys > 0 && k0 + keys == pos + 1;
+    // a lane's four values of a q head: dimensions 4 lane .. 4 lane + 3
+    auto q_at = [&](int h, int l) { return reinterpret_cast<float4*>(sQ + h * AC_Q_PITCH + (l >> 3) * 36) + (l & 7); };
     if (fuse.qkv) {
         const float* src = fuse.qkv + (size_t)t * (p.n_head + 2 * p.n_kv) * 128;
         if (pos != pos0) turn = turn_at(pos);
-        if (warp < g) reinterpret_cast<float4*>(sQ + warp * 128)[lane] = ac_norm_rope(src + (head0 + warp) * 128, fuse.qn_w != nullptr, qw, true, turn, fuse.eps, lane);
+        if (warp < g) *q_at(warp, lane) = ac_norm_rope(src + (head0 + warp) * 128, fuse.qn_w != nullptr, qw, true, turn, fuse.eps, lane);
         if (mine && warp >= 6) {       // the new token's rows: to the cache and to this CTA's tiles
             const bool is_k = warp == 6;
             const float4 v = ac_norm_rope(src + (p.n_head + (is_k ? 0 : p.n_kv) + kvh) * 128, is_k && fuse.kn_w, kw, is_k, turn, fuse.eps, lane);
@@ -664,248 +786,216 @@ __global__ void __launch_bounds__(AC_THREADS, 2) k_attn_cluster(const AttnParams
             else new_v = hv;
         }
     } else {
-        for (int i = tid; i < g * 32; i += AC_THREADS) reinterpret_cast<float4*>(sQ)[i] = reinterpret_cast<const float4*>(p.q + ((size_t)t * p.n_head + head0) * 128)[i];
+        for (int i = tid; i < g * 32; i += AC_THREADS) *q_at(i >> 5, i & 31) = reinterpret_cast<const float4*>(p.q + ((size_t)t * p.n_head + head0) * 128)[i];
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // ---- scores: four lanes per pair of keys, lane `sub` takes the 16-byte pieces 4 i + sub of the rows; the queries' loads, which
-    // are what this part is bound by, then serve two keys
-    for (int key = 2 * (tid >> 2); key < nbl * DC_KV_BLOCK; key += AC_THREADS / 2) {
-        const int sub = tid & 3;
-        if (key < keys) {
-            float2 kf[2][16];
+    // ---- scores: a warp keeps two heads' queries in registers, a quarter a lane, and takes eight keys at a time, four lanes each (queries
+    // read again for every key had the shared memory's bandwidth as their bound)
+    if (const int pairs = g / 2, turns = 8 / pairs; warp < pairs * turns) {
+        const int h0 = 2 * (warp % pairs), sub = lane & 3;
+        float q[2][32];
 #pragma unroll
-            for (int k = 0; k < 2; ++k)
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {      // (the row after the last key's is read as whatever it holds and not used)
-                    const uint4 u = *reinterpret_cast<const uint4*>(sKV + ac_piece(key + k, 4 * i + sub));
-                    const __half2* h2 = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) kf[k][4 * i + j] = __half22float2(h2[j]);
-                }
-            const uint32_t quad = 0xFu << (lane & ~3);
-            for (int h0 = 0; h0 < g; h0 += 2) {      // g is even
-                float2 d[2][2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) d[h][0] = d[h][1] = make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float4* q4 = reinterpret_cast<const float4*>(sQ + (h0 + h) * 128 + (4 * i + sub) * 8);
-                        const float4 a = q4[0], b = q4[1];
-#pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            ac_fma2(d[h][k], make_float2(a.x, a.y), kf[k][4 * i]);
-                            ac_fma2(d[h][k], make_float2(a.z, a.w), kf[k][4 * i + 1]);
-                            ac_fma2(d[h][k], make_float2(b.x, b.y), kf[k][4 * i + 2]);
-                            ac_fma2(d[h][k], make_float2(b.z, b.w), kf[k][4 * i + 3]);
-                        }
-                    }
-                float mine = 0.0f;      // lane sub keeps (head sub / 2, key sub % 2)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        float dot = d[h][k].x + d[h][k].y;
-                        dot += __shfl_xor_sync(quad, dot, 1);
-                        dot += __shfl_xor_sync(quad, dot, 2);
-                        if (2 * h + k == sub) mine = dot;
-                    }
-                const int at = key + (sub & 1);
-                sP[ac_at(at, h0 + (sub >> 1))] = at < keys ? __fmul_rn(mine, p.scale) : -INFINITY;
+            for (int i = 0; i < 8; ++i) {
+                const float4 x = reinterpret_cast<const float4*>(sQ + (h0 + h) * AC_Q_PITCH + sub * 36)[i];
+                q[h][4 * i] = x.x, q[h][4 * i + 1] = x.y, q[h][4 * i + 2] = x.z, q[h][4 * i + 3] = x.w;
             }
-        } else {
-            for (int i = sub; i < 2 * g; i += 4) sP[ac_at(key + (i & 1), i >> 1)] = -INFINITY;
+#pragma unroll 1
+        for (int key = warp / pairs * 8 + (lane >> 2); key < nbl * DC_KV_BLOCK; key += 8 * turns) {      // (16 keys a block: whole warps)
+            float d[2] = {0.0f, 0.0f};
+            uint4 u[4];      // (the rows after the last key's are read as whatever they hold and not used)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) u[i] = *reinterpret_cast<const uint4*>(sKV + ac_piece(key, 4 * sub + i));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __half2* h2 = reinterpret_cast<const __half2*>(&u[i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = __half22float2(h2[j]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) d[h] = fmaf(q[h][8 * i + 2 * j], f.x, d[h]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) d[h] = fmaf(q[h][8 * i + 2 * j + 1], f.y, d[h]);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                d[h] += __shfl_xor_sync(0xffffffffu, d[h], 1);
+                d[h] += __shfl_xor_sync(0xffffffffu, d[h], 2);
+            }
+            if (sub < 2) sP[(h0 + sub) * ps + key] = key < keys ? __fmul_rn(sub ? d[1] : d[0], p.scale) : -INFINITY;
         }
     }
     __syncthreads();
     // the V rows follow into the same memory while the block maxima make their way
     for (int key = tid >> 4; key < keys - (mine ? 1 : 0); key += AC_THREADS / 16) {
-        const int at = k0 + key;
-        const size_t off = ((size_t)table[at / DC_KV_BLOCK] * DC_KV_BLOCK + at % DC_KV_BLOCK) * row + kvh * 128 + (tid & 15) * 8;
+        const size_t off = ((size_t)sTab[key / DC_KV_BLOCK] * DC_KV_BLOCK + key % DC_KV_BLOCK) * row + kvh * 128 + (tid & 15) * 8;
         ac_copy16(aKV + key * 256 + (tid & 15) * 16, p.v_arena + off);
     }
     if (mine && warp == 7) *reinterpret_cast<uint2*>(sKV + (pos - k0) * 256 + 8 * lane) = new_v;
-    for (int i = tid; i < nbl * 8; i += AC_THREADS) {
-        const int bl = i >> 3, h = i & 7;
-        if (h < g) {
-            float mx = -1e30f;  // the reference's m_block starts at -1e30
+    // sixteen lanes per (head, block), neighbouring groups on neighbouring heads
+    const int lg = g > 4 ? 3 : g > 2 ? 2 : 1, hx = (tid >> 4) & ((1 << lg) - 1), bx = tid >> 4 >> lg, nbx = (nbl + (16 >> lg) - 1) >> (4 - lg) << (4 - lg);
+    for (int bl = bx; bl < nbx; bl += 16 >> lg) {
+        const bool in = hx < g && bl < nbl;
+        float mx = in ? fmaxf(sP[hx * ps + bl * DC_KV_BLOCK + (tid & 15)], -1e30f) : -1e30f;  // the reference's m_block starts at -1e30
 #pragma unroll
-            for (int k = 0; k < DC_KV_BLOCK; ++k) mx = fmaxf(mx, sP[ac_at(bl * DC_KV_BLOCK + k, h)]);
-            sBm[i] = mx;
-        }
-    }
-    __syncthreads();
-    // ---- the chain: warp h, lane = block
-    float incl = -1e30f, excl = -1e30f;
-    if (warp < g) {
-        if (lane < nbl) incl = sBm[lane * 8 + warp];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl = fmaxf(incl, u);
-        }
-        excl = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) excl = -1e30f;
-        if (lane == 31) sMax[warp] = incl;
+        for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (in && (tid & 15) == 0) sBm[hx * cap + bl] = mx;
     }
     ac_sync();
-    if (warp < g) {
-        float m0 = lane < rank ? ac_peer(sMax + warp, lane) : -1e30f;
+    // ---- the chain of a head by a warp, a lane per block, 32 blocks of the sequence at a time (as k_attn_pv_run)
+    if (warp < g && nr > 0) {
+        const int per = R.rpc * R.bps;         // blocks of a CTA
+        const float inv = __frcp_rn((float)per);
+        float carry = -1e30f, suf = 1.0f;      // lane j: the product of the j-th run
+        auto block_max = [&](int c) {
+            const int owner = (int)(((float)c + 0.5f) * inv);      // c / per
+            return c < R.n_blk ? ac_load(ac_map(sBm + warp * cap + (c - owner * per), owner)) : -1e30f;
+        };
+        float next = block_max(lane);
+#pragma unroll 1
+        for (int c0 = 0; c0 < R.n_blk; c0 += 32) {
+            const int c = c0 + lane;
+            float incl = next;
+            next = block_max(c + 32);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-        const float m_new = fmaxf(m0, incl);
-        const float alpha = lane < nbl ? fast_exp_fma(fmaxf(m0, excl) - m_new) : 1.0f;
-        float after = alpha;   // inclusive product from this block on
+            for (int o = 1; o < 32; o <<= 1) {
+                const float u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl = fmaxf(incl, u);
+            }
+            float excl = __shfl_up_sync(0xffffffffu, incl, 1);
+            if (lane == 0) excl = -1e30f;
+            const float m_prev = fmaxf(carry, excl), m_new = fmaxf(carry, incl);
+            carry = fmaxf(carry, __shfl_sync(0xffffffffu, incl, 31));
+            const float a = (c >= R.b0 && c < R.n_blk) ? fast_exp_fma(m_prev - m_new) : 1.0f;
+            if (c >= R.b0 && c < R.b1) {
+                sM[warp * cap + c - R.b0] = m_new;
+                sAl[warp * cap + c - R.b0] = a;
+            }
+            if (__all_sync(0xffffffffu, a == 1.0f)) continue;      // factors of one leave a product as it is
+#pragma unroll 1
+            for (int j = 0; j < nr; ++j) {
+                const int after = (R.r0 + j + 1) * R.bps;
+                if (c0 + 32 <= after) break;
+                float later = c >= after ? a : 1.0f;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float u = __shfl_down_sync(0xffffffffu, after, o);
-            if (lane + o < 32) after *= u;
+                for (int o = 16; o > 0; o >>= 1) later *= __shfl_xor_sync(0xffffffffu, later, o);
+                if (lane == j) suf *= later;
+            }
         }
-        float later = __shfl_down_sync(0xffffffffu, after, 1);
-        if (lane == 31) later = 1.0f;
-        if (lane < nbl) {
-            sBm[lane * 8 + warp] = m_new;
-            sW[lane * 8 + warp] = later;
-        }
-        if (lane == 0) sProd[warp] = after;
+        if (lane < nr) sSuf[lane * g + warp] = suf;
     }
     __syncthreads();
-    const int lg = g > 4 ? 3 : g > 2 ? 2 : 1;
-#pragma unroll 4
-    for (int i = tid; i < nbl * DC_KV_BLOCK << lg; i += AC_THREADS) {
-        const int key = i >> lg, h = i & ((1 << lg) - 1), c = (key >> 4) * 8 + h;
-        if (h < g) {
-            const float s = sP[ac_at(key, h)];
-            sP[ac_at(key, h)] = s == -INFINITY ? 0.0f : __fmul_rn(fast_exp_fma(s - sBm[c]), sW[c]);
+    // ---- exponentials and their sums over a block
+#pragma unroll 2
+    for (int bl = bx; bl < nbx; bl += 16 >> lg) {
+        const bool in = hx < g && bl < nbl;
+        float* at = sP + hx * ps + bl * DC_KV_BLOCK + (tid & 15);
+        const float s = in ? *at : -INFINITY;
+        const float pr = s == -INFINITY ? 0.0f : fast_exp_fma(s - sM[hx * cap + bl]);
+        float sum = pr;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (in) {
+            *at = pr;
+            if ((tid & 15) == 0) sM[hx * cap + bl] = sum;      // (its sixteen readers are done with the maximum)
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (warp < g) {
+    // ---- denominators of the runs by the last group of threads, which P.V keeps least busy (nr * g <= 64)
+    if (tid >= AC_THREADS - 64 && tid - (AC_THREADS - 64) < nr * g) {
+        const int i = tid - (AC_THREADS - 64), j = i / g, h = i - j * g, end = min(nbl, (j + 1) * R.bps);
         float den = 0.0f;
-        for (int key = lane; key < keys; key += 32) den += sP[ac_at(key, warp)];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-        if (lane == 0) sDen[warp] = den;
+        for (int bl = j * R.bps; bl < end; ++bl) den = fmaf(den, sAl[h * cap + bl], sM[h * cap + bl]);
+        sDen[i] = __fmul_rn(den, sSuf[i]);
     }
-    // ---- P.V: four groups of threads take every fourth key, a thread two dimensions of all heads
-    {
-        const int kg = tid >> 6, dp = tid & 63;
-        float2 a0[4], a1[4];   // head pairs, of the first and the second dimension
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a0[i] = a1[i] = make_float2(0.0f, 0.0f);
-#pragma unroll 4
-        for (int key = kg; key < keys; key += 4) {
-            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(sKV + key * 256 + dp * 4));
-            const float4* pp = reinterpret_cast<const float4*>(sP + ac_at(key, 0));
-            const float4 x = pp[0], y = g > 4 ? pp[1] : x;
-            const float2 vx = make_float2(v.x, v.x), vy = make_float2(v.y, v.y);
-            ac_fma2(a0[0], make_float2(x.x, x.y), vx);
-            ac_fma2(a1[0], make_float2(x.x, x.y), vy);
-            if (g > 2) {
-                ac_fma2(a0[1], make_float2(x.z, x.w), vx);
-                ac_fma2(a1[1], make_float2(x.z, x.w), vy);
-            }
-            if (g > 4) {
-                ac_fma2(a0[2], make_float2(y.x, y.y), vx);
-                ac_fma2(a1[2], make_float2(y.x, y.y), vy);
-            }
-            if (g > 6) {
-                ac_fma2(a0[3], make_float2(y.z, y.w), vx);
-                ac_fma2(a1[3], make_float2(y.z, y.w), vy);
-            }
-        }
-        __syncthreads();      // V has been read
-        float* red = reinterpret_cast<float*>(sKV) + kg * ATT_MAX_GROUP * 128 + 2 * dp;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (2 * i < g) {
-                *reinterpret_cast<float2*>(red + (2 * i) * 128) = make_float2(a0[i].x, a1[i].x);
-                *reinterpret_cast<float2*>(red + (2 * i + 1) * 128) = make_float2(a0[i].y, a1[i].y);
-            }
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < g * 128; i += AC_THREADS) {
-        const float* red = reinterpret_cast<const float*>(sKV) + i;
-        sPart[i] = (red[0] + red[ATT_MAX_GROUP * 128]) + (red[2 * ATT_MAX_GROUP * 128] + red[3 * ATT_MAX_GROUP * 128]);
-    }
-    ac_sync();      // (also: every thread of this CTA is done with the key groups' sums)
-    // ---- merge: CTA r writes the head pair r, the 256 values of one Q8_K block of the o-projection's input.  A warp takes C / 8 ranks'
-    // partials, times the alphas of all ranks after; the warps' sums meet in shared memory.
-    float* sSum = reinterpret_cast<float*>(sKV);                   // [warp][256], then [warp][2] denominators (the key groups' sums are done with)
+    if (g == 8) ac_pv_all<8>(R, sKV, sP, sAl, sSuf, sQ, cap, rcap, ps, keys);
+    else if (g == 6) ac_pv_all<6>(R, sKV, sP, sAl, sSuf, sQ, cap, rcap, ps, keys);
+    else if (g == 4) ac_pv_all<4>(R, sKV, sP, sAl, sSuf, sQ, cap, rcap, ps, keys);
+    else ac_pv_all<2>(R, sKV, sP, sAl, sSuf, sQ, cap, rcap, ps, keys);
+    ac_sync();
+    // ---- merge: CTA r writes the head pair r, the 256 values of one Q8_K block of the o-projection's input, a thread a value, the runs
+    // added in order
+    float* sOut = rcap == 1 ? reinterpret_cast<float*>(sKV) : sQ;      // (whichever does not hold the sums)
     if (rank < g / 2) {
-        const int head = 2 * rank + (lane >> 4), d0 = (lane & 15) * 8;
-        constexpr int R = C / 8;
-        float4 a[R], c[R];
-        float dd[R], pr = 1.0f;
+        const int head = 2 * rank + (tid >> 7), d = tid & 127;
+        const float* sums = rcap == 1 ? sQ : reinterpret_cast<const float*>(sKV);
+        const int step = R.bps * DC_KV_BLOCK * 64;      // floats between two runs' sums
+        const float per = __frcp_rn((float)R.rpc);
+        float acc = 0.0f, den = 0.0f;
+#pragma unroll 1
+        for (int r0 = 0; r0 < R.n_run; r0 += 8) {
+            float x[8], y[8];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            a[r] = ac_peer4(sPart + head * 128 + d0, warp * R + r);
-            c[r] = ac_peer4(sPart + head * 128 + d0 + 4, warp * R + r);
-            dd[r] = ac_peer(sDen + head, warp * R + r);
-        }
-        if ((lane & 15) < C) pr = ac_peer(sProd + head, lane & 15);            // lane of a half: the product of that rank's alphas
-        float after = pr;                                                      // of this rank and all later ones
+            for (int i = 0; i < 8; ++i) {      // eight runs' loads in flight
+                const int r = min(r0 + i, R.n_run - 1), owner = (int)(((float)r + 0.5f) * per), j = r - owner * R.rpc;
+                const uint32_t base = ac_map(sums, owner);
+                x[i] = ac_load(base + (uint32_t)(j * step + head * 128 + d) * 4u);
+                y[i] = ac_load(base + (uint32_t)(sDen - sums + j * g + head) * 4u);
+            }
 #pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-            const float u = __shfl_down_sync(0xffffffffu, after, o, 16);
-            if ((lane & 15) + o < 16) after *= u;
-        }
-        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, den = 0.0f;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int next = warp * R + r + 1;
-            const float suffix = __shfl_sync(0xffffffffu, after, (lane & 16) + (next & 15));
-            const float f = next < C ? suffix : 1.0f;
-            den += dd[r] * f;
-            v[0] += a[r].x * f; v[1] += a[r].y * f; v[2] += a[r].z * f; v[3] += a[r].w * f;
-            v[4] += c[r].x * f; v[5] += c[r].y * f; v[6] += c[r].z * f; v[7] += c[r].w * f;
-        }
-        float4* o = reinterpret_cast<float4*>(sSum + warp * 256 + lane * 8);
-        o[0] = make_float4(v[0], v[1], v[2], v[3]);
-        o[1] = make_float4(v[4], v[5], v[6], v[7]);
-        if ((lane & 15) == 0) sSum[8 * 256 + warp * 2 + (lane >> 4)] = den;
-    }
-    __syncthreads();
-    if (rank < g / 2 && warp == 0) {
-        const int head = 2 * rank + (lane >> 4), d0 = (lane & 15) * 8;
-        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, den = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            const float4* o = reinterpret_cast<const float4*>(sSum + w * 256 + lane * 8);
-            const float4 x = o[0], y = o[1];
-            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-            v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
-            den += sSum[8 * 256 + w * 2 + (lane >> 4)];
+            for (int i = 0; i < 8; ++i)
+                if (r0 + i < R.n_run) {
+                    acc += x[i];
+                    den += y[i];
+                }
         }
         const float inv = (den > 0.0f && isfinite(den)) ? __fdiv_rn(1.0f, __fadd_rn(den, 1e-6f)) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] *= inv;
-        if (p.out) {
-            float* o = p.out + ((size_t)t * p.n_head + head0 + head) * 128 + d0;
-            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-            *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
-        }
-        if (p.q8_out) quantize_block_q8f_regs(v, p.q8_out + ((size_t)t * (p.n_head / 2) + head0 / 2 + rank) * DC_Q8F_BYTES, lane);
+        acc *= inv;
+        if (p.out) p.out[((size_t)t * p.n_head + head0 + head) * 128 + d] = acc;
+        sOut[tid] = acc;
     }
-    ac_sync();      // nobody leaves while its shared memory is read
+    ac_sync();      // nobody leaves while its shared memory is read (and sOut is whole)
+    if (p.q8_out && rank < g / 2 && warp == 0) {
+        const float4 x = reinterpret_cast<const float4*>(sOut)[2 * lane], y = reinterpret_cast<const float4*>(sOut)[2 * lane + 1];
+        const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        quantize_block_q8f_regs(v, p.q8_out + ((size_t)t * (p.n_head / 2) + head0 / 2 + rank) * DC_Q8F_BYTES, lane);
+    }
 }
 
-static size_t attn_cluster_smem(int cap) {
-    const size_t k = (size_t)cap * DC_KV_BLOCK * 256, red = 4 * ATT_MAX_GROUP * 128 * 4;
-    return (k > red ? k : red) + ((size_t)cap * (DC_KV_BLOCK + 1) * 8 + 2 * ATT_MAX_GROUP * 128 + (size_t)cap * 16 + 24) * 4;
+// Blocks and runs that a CTA of a cluster of C meets at most, for any length up to max_blocks: with runs of a given length the longest
+// sequence has the most runs, and all lengths but the longest come with all nsplit runs.
+struct AcPlan {
+    int cap, rcap;
+    AcPlan(int C, int max_blocks, int nsplit) {
+        auto up = [](int a, int b) { return (a + b - 1) / b; };
+        const int bps = up(max_blocks, nsplit);
+        cap = up(up(max_blocks, bps), C) * bps;
+        if (bps > 1) cap = std::max(cap, up(nsplit, C) * (bps - 1));
+        rcap = up(std::min(nsplit, max_blocks), C);
+    }
+    size_t smem(int g) const {
+        return (size_t)cap * DC_KV_BLOCK * 256 + (size_t)g * (cap * DC_KV_BLOCK + 4 + AC_Q_PITCH + 2 * rcap + 3 * cap) * 4;
+    }
+};
+// few tokens: two clusters share a kv head's query heads, as long as there is an SM for every CTA
+static int attn_head_split(int C, int T, int n_kv, int g) { return g % 4 == 0 && 2 * T * n_kv * C <= 128 ? 2 : 1; }
+static bool attn_cluster_fits(int C, int T, int n_kv, int g, int max_blocks, int nsplit) {
+    const AcPlan plan(C, max_blocks, nsplit);
+    // (a thread for each of 8 x 8 denominators; runs longer than ATT_MAX_RUN take k_attn_pv, which multiplies alphas in another order)
+    return plan.cap <= AC_CAP && plan.rcap <= 8 && (max_blocks + nsplit - 1) / nsplit <= ATT_MAX_RUN &&
+           plan.smem(g / attn_head_split(C, T, n_kv, g)) <= AC_SMEM;
 }
-bool dc_attn_cluster_ok(int max_blocks) { return max_blocks <= 16 * AC_CAP; }
+// CTAs of the cluster that serves T tokens, 0: the split kernels do.  Clusters of sixteen halve a CTA's share but only one fits into a
+// group of SMs: they pay for up to eight clusters, or where eight CTAs cannot hold the keys.
+static int attn_cluster_size(int T, int n_kv, int g, int max_blocks, int nsplit) {
+    const bool eight = attn_cluster_fits(8, T, n_kv, g, max_blocks, nsplit);
+    if ((!eight || T * n_kv <= 8) && attn_cluster_fits(16, T, n_kv, g, max_blocks, nsplit)) return 16;
+    return eight ? 8 : 0;
+}
+bool dc_attn_cluster_ok(int T, int n_head, int n_kv, int max_blocks, int nsplit) {
+    return attn_cluster_size(T, n_kv, n_head / n_kv, max_blocks, nsplit) != 0;
+}
 
 template <int C>
 static int launch_attn_cluster(dc_ctx* ctx, const AttnParams& p, const dc_attn_fuse& fuse, int max_blocks) {
     const void* f = (const void*)k_attn_cluster<C>;
-    const int cap = (max_blocks + C - 1) / C, g = p.n_head / p.n_kv;
-    const size_t smem = attn_cluster_smem(cap);
-    DC_TRY(dc_kernel_setup(ctx, f, (int)attn_cluster_smem(AC_CAP), "cudaFuncSetAttribute(k_attn_cluster)"));
+    const AcPlan plan(C, max_blocks, p.nsplit);
+    const int g = p.n_head / p.n_kv;
+    DC_TRY(dc_kernel_setup(ctx, f, AC_SMEM, "cudaFuncSetAttribute(k_attn_cluster)"));
     if (C > 8) {       // more than the portable eight, which the device has to allow
         static std::mutex mu;
         static bool done[64];
@@ -914,9 +1004,9 @@ static int launch_attn_cluster(dc_ctx* ctx, const AttnParams& p, const dc_attn_f
         if (!done[d]) DC_TRY(dc_check_cuda(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "clusters of sixteen"));
         done[d] = true;
     }
-    // few tokens: two clusters share a kv head's query heads, as long as there is an SM for every CTA
-    const int hs = g % 4 == 0 && 2 * p.T * p.n_kv * C <= 128 ? 2 : 1;
-    return dc_launch_cluster(ctx, "k_attn_cluster", k_attn_cluster<C>, dim3(p.n_kv * hs * C, p.T), dim3(AC_THREADS), smem, C, p, fuse, cap, hs);
+    const int hs = attn_head_split(C, p.T, p.n_kv, g);
+    return dc_launch_cluster(ctx, "k_attn_cluster", k_attn_cluster<C>, dim3(p.n_kv * hs * C, p.T), dim3(AC_THREADS), plan.smem(g / hs), C, p, fuse, plan.cap,
+                             plan.rcap, hs);
 }
 
 size_t dc_attention_scratch_bytes(int T, int n_head, int n_kv, int max_blocks, int nsplit) {
@@ -958,13 +1048,10 @@ int dc_launch_attention(dc_ctx* ctx, const float* q, const void* k_arena, const 
     p.tickets = sc->tickets;
     p.out = out;
     p.q8_out = q8_out;
-    // The cluster's shared memory holds all keys of a sequence up to a length; longer ones take the split kernels.  Clusters of sixteen
-    // halve a CTA's share but only one fits into a group of SMs: they pay for up to eight clusters, or where eight CTAs cannot hold the keys
-    // (16 Q / 8 KV heads, 512 keys, 4 tokens: 11 us a launch with eight, 26 us with sixteen).
-    if (dc_attn_cluster_ok(max_blocks)) {
+    const int C = attn_cluster_size(T, n_kv, g, max_blocks, nsplit);
+    if (C) {
         const dc_attn_fuse none = {};
-        if (max_blocks > 8 * AC_CAP || T * n_kv <= 8) return launch_attn_cluster<16>(ctx, p, fuse ? *fuse : none, max_blocks);
-        return launch_attn_cluster<8>(ctx, p, fuse ? *fuse : none, max_blocks);
+        return C == 16 ? launch_attn_cluster<16>(ctx, p, fuse ? *fuse : none, max_blocks) : launch_attn_cluster<8>(ctx, p, fuse ? *fuse : none, max_blocks);
     }
     if (fuse) return dc_fail(ctx, DC_B200_UNSUPPORTED, "attention: %d blocks a sequence do not fit the fused kernel", max_blocks);
     int st = dc_launch(ctx, "k_attn_scores", k_attn_scores, dim3(nsplit, n_kv, T), dim3(128), 0, p);

@@ -139,8 +139,8 @@ DC_PART int dc_launch_attention(dc_ctx* ctx, const float* q, const void* k_arena
                         const int32_t* block_tables, int max_blocks, const int32_t* seq_ids, const int32_t* positions,
                         int T, int n_head, int n_kv, float scale, int nsplit, const dc_attn_scratch* sc, float* out,
                         uint8_t* q8_out, const dc_attn_fuse* fuse = nullptr);
-// whether sequences of so many KV blocks take the one-kernel form, which is what `fuse` needs
-DC_PART bool dc_attn_cluster_ok(int max_blocks);
+// whether such a call takes the one-kernel form, which is what `fuse` needs
+DC_PART bool dc_attn_cluster_ok(int T, int n_head, int n_kv, int max_blocks, int nsplit);
 
 // ---- moe.cu ----
 // causal attention of a prompt chunk (positions pos0 .. pos0 + n - 1 of one sequence) on the tensor cores
@@ -170,7 +170,7 @@ struct dc_route_norm {
     uint8_t* q8_out;
 };
 DC_PART int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_expert, int T, int top_k, float scale,
-                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode = DC_ROUTE_STABLE, const dc_route_norm* norm = nullptr);
+                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode = DC_ROUTE_STABLE, const dc_route_norm* norm = nullptr, bool sixteenths = false);
 // the same routing for any number of tokens (prompt chunks): logits [T][E], ids and weights [T][top_k]
 int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, int T, int top_k, float scale, float* logits,
                              int32_t* ids, float* weights, int mode);

@@ -193,7 +193,9 @@ static int alloc_step_buffers(dc_model* m) {
 
 // ------------------------------------------------------------- one step
 // lm_mode: 0 no logits, 1 last row only, 2 every row.  chunk: the tokens are neighbours in one sequence, not one each of several.
-static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool chunk) {
+// runs: attention runs of the persistent kernel, in whose place this step comes (its sums are then formed in that kernel's order, and
+// the results are the same bit for bit); 0: the per-op kernels' own.
+static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool chunk, int runs) {
     const dc_model_config& c = m->cfg;
     dc_ctx* ctx = m->ctx;
     dc_step_buffers& b = m->buf;
@@ -223,6 +225,8 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
     const float* pending = nullptr;  // MoE output of the previous layer, added in the next norm
     bool split = false;              // the previous layer's expert outputs wait for their weighted sum
     const bool sum_in_norm = E > 0 && c.ep_size == 1;
+    const int nsplit = runs ? runs : m->nsplit;
+    const bool cluster = dc_attn_cluster_ok(T, c.n_head, c.n_kv_head, m->kv.max_blocks_per_seq, nsplit);
     const bool norm_in_rows = dc_rows_quantise(T, H);     // few rows: the product that reads them norms them itself, a launch less
     for (int il = 0; il < c.n_layer; ++il) {
         dc_layer& Ly = m->layers[il];
@@ -249,16 +253,16 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
         const dc_attn_fuse fuse = {b.qkv, Ly.q_norm ? (const float*)Ly.q_norm->dev : nullptr, Ly.k_norm ? (const float*)Ly.k_norm->dev : nullptr,
                                    b.cos_sin, c.max_ctx, c.rms_eps};
         // one kernel where a token's attention does not read rows that the same step writes
-        const bool one = dc_attn_cluster_ok(m->kv.max_blocks_per_seq) && (!chunk || T == 1);
+        const bool one = cluster && (!chunk || T == 1);
         if (!one)
             L(DC_K_QKROPE, (double)T * QKV * 4 * 2, 1,
               dc_launch_qknorm_rope_kv(ctx, b.qkv, fuse.qn_w, fuse.kn_w, b.cos_sin, c.max_ctx, b.positions,
                                        b.seq_ids, m->kv.d_tables, m->kv.max_blocks_per_seq, ka, va, c.n_head, c.n_kv_head,
                                        c.rms_eps, T, b.q));
         // KV bytes depend on the context length; filled in by the caller of the profile
-        L(DC_K_ATTENTION, 0.0, dc_attn_cluster_ok(m->kv.max_blocks_per_seq) ? 1 : 2,
+        L(DC_K_ATTENTION, 0.0, cluster ? 1 : 2,
           dc_launch_attention(ctx, b.q, ka, va, m->kv.d_tables, m->kv.max_blocks_per_seq, b.seq_ids, b.positions, T,
-                              c.n_head, c.n_kv_head, scale, m->nsplit, &b.attn, nullptr, b.q8_attn, one ? &fuse : nullptr));
+                              c.n_head, c.n_kv_head, scale, nsplit, &b.attn, nullptr, b.q8_attn, one ? &fuse : nullptr));
         dc_gemv_seg wo = {Ly.wo->dev, Ly.wo->type, H, (int)Ly.wo->row_bytes, b.x, H};
         L(DC_K_GEMV_O, (double)Ly.wo->bytes + (double)T * (QD / 256) * DC_Q8F_BYTES + 2 * xb, 1,
           dc_launch_gemv(ctx, &wo, 1, DC_EPI_ACC, b.q8_attn, T, QD, nullptr));
@@ -276,7 +280,7 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
             const double U = T == 1 ? top_k : (A < E ? A : E);
             const double local = (double)(ep_hi - ep_lo) / E;
             L(DC_K_ROUTER, (double)Ly.router->bytes + xb, 1,
-              dc_launch_router(ctx, Ly.router, b.xn, E, T, top_k, c.routed_scale, ep_lo, ep_hi, &b.route, m->route_mode, norm_in_router ? &rn : nullptr));
+              dc_launch_router(ctx, Ly.router, b.xn, E, T, top_k, c.routed_scale, ep_lo, ep_hi, &b.route, m->route_mode, norm_in_router ? &rn : nullptr, runs != 0));
             L(DC_K_MOE_GATEUP, U * local * 2.0 * F * Ly.gate_exps->row_bytes + q8x + (double)A * F * 4, 1,
               dc_launch_moe_mm(ctx, true, Ly.gate_exps, Ly.up_exps, b.q8_x, T, top_k, ep_lo, &b.route, b.h));
             const bool own = dc_moe_quantise_in_down(T);
@@ -332,12 +336,12 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
 }
 
 // Captured once per (T, lm_mode, feedback); replayed afterwards.
-// chunk: the T tokens are consecutive positions of one sequence (otherwise one token each of T sequences).
-static int run_forward(dc_model* m, int T, int lm_mode, bool feedback, bool chunk = false) {
+// chunk: the T tokens are consecutive positions of one sequence (otherwise one token each of T sequences).  runs: see enqueue_forward.
+static int run_forward(dc_model* m, int T, int lm_mode, bool feedback, bool chunk = false, int runs = 0) {
     dc_ctx* ctx = m->ctx;
-    auto enqueue = [&]() { return m->stack ? dc_stack_enqueue_small(m, T, chunk, lm_mode, feedback) : enqueue_forward(m, T, lm_mode, feedback, chunk); };
+    auto enqueue = [&]() { return m->stack ? dc_stack_enqueue_small(m, T, chunk, lm_mode, feedback) : enqueue_forward(m, T, lm_mode, feedback, chunk, runs); };
     if (!m->use_graphs || m->dbg_x) return enqueue();
-    const int key = T * 8 + lm_mode * 2 + (feedback ? 1 : 0) + (chunk && (m->stack || T > 1) ? 1024 : 0);
+    const int key = T * 8 + lm_mode * 2 + (feedback ? 1 : 0) + (chunk && (m->stack || T > 1) ? 1024 : 0) + (runs ? 2048 : 0);      // (a model has one number of runs)
     auto it = m->graphs.find(key);
     if (it == m->graphs.end()) {
         // one eager pass first: it sets kernel attributes, which is not allowed while capturing
@@ -386,11 +390,17 @@ static int upload_step_inputs(dc_model* m, const int32_t* tokens, const int32_t*
 // model, whose ranks exchange expert outputs inside it.  Elsewhere the per-op kernels are faster: its seven grid barriers a layer cost
 // more than seven launches that overlap, and its row dots stay on dp4a.  (8-layer cut, 2048 tokens of context, us a step: one stream
 // 681 persistent, 518 per-op; four 2059 and 935.)
-static bool mega_ok(dc_model* m, int T) {
-    if (m->stack || !m->use_mega || (m->use_mega == 1 && (T > 1 || m->cfg.ep_size == 1))) return false;
+// One stream by default (use_mega 1) has the persistent kernel's results whichever serves it: *runs says how many runs its attention has,
+// for the per-op kernels to form their sums in the same order (0: in their own).
+static bool mega_ok(dc_model* m, int T, int* runs) {
+    *runs = 0;
+    if (m->stack || !m->use_mega || (m->use_mega == 1 && T > 1)) return false;
     MegaParams p;
     const char* why = "";
-    return dc_mega_plan(m, T, &p, &why);
+    if (!dc_mega_plan(m, T, &p, &why)) return false;
+    if (m->use_mega == 2 || m->cfg.ep_size > 1) return true;
+    *runs = p.nsplit;
+    return false;
 }
 
 static bool model_complete(dc_model* m, std::string* missing) {
@@ -823,8 +833,9 @@ int dc_b200_decode_step(dc_model* m, const int32_t* seqs, int n_seq, const int32
         pos[i] = s.len;
     }
     DC_TRY(upload_step_inputs(m, tokens_host, seqs, pos, n_seq));
-    if (!m->prof && mega_ok(m, n_seq)) DC_TRY(dc_mega_run(m, n_seq, 1, false));
-    else DC_TRY(run_forward(m, n_seq, 2, false));
+    int runs;
+    if (mega_ok(m, n_seq, &runs) && !m->prof) DC_TRY(dc_mega_run(m, n_seq, 1, false));
+    else DC_TRY(run_forward(m, n_seq, 2, false, false, runs));
     int32_t* pin = m->h_stage + 1000;
     DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(pin, m->buf.out_tokens, (size_t)n_seq * 4, cudaMemcpyDeviceToHost, ctx->stream), "D2H tokens"));
     if (logits_host) DC_TRY(dc_check_cuda(ctx, cudaMemcpyAsync(logits_host, m->buf.logits, (size_t)n_seq * m->cfg.vocab * 4, cudaMemcpyDeviceToHost, ctx->stream), "D2H logits"));
@@ -863,9 +874,10 @@ int dc_b200_decode_run(dc_model* m, const int32_t* seqs, int n_seq, const int32_
         cudaEventRecord(e0, ctx->stream);
     }
     int st = DC_B200_OK;
-    if (mega_ok(m, n_seq)) st = dc_mega_run(m, n_seq, n_steps, true);   // all steps in one cooperative launch
+    int runs;
+    if (mega_ok(m, n_seq, &runs)) st = dc_mega_run(m, n_seq, n_steps, true);   // all steps in one cooperative launch
     else
-        for (int i = 0; i < n_steps && st == DC_B200_OK; ++i) st = run_forward(m, n_seq, 2, true);
+        for (int i = 0; i < n_steps && st == DC_B200_OK; ++i) st = run_forward(m, n_seq, 2, true, false, runs);
     if (ms_out) {
         cudaEventRecord(e1, ctx->stream);
         cudaEventSynchronize(e1);

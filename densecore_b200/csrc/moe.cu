@@ -36,6 +36,7 @@ struct RouterParams {
     int32_t* uoff;        // their offsets into uassign, and the end
     int32_t* uassign;     // [T*top_k] assignment indices t*top_k+k, grouped by expert, routing order inside
     dc_route_norm norm;   // x given: rows still to be normed
+    bool sixteenths;      // one token: its logits as sixteen partial sums in order, as the persistent kernel forms them
 };
 
 __device__ __forceinline__ unsigned long long route_key(float v, int id) {
@@ -281,7 +282,22 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
         float acc[DC_MAX_T];
 #pragma unroll
         for (int t = 0; t < DC_MAX_T; ++t) acc[t] = 0.0f;
-        if (e < p.E) {
+        if (p.sixteenths) {
+            if (e < p.E) {
+                const int n4 = seg / 16;      // float4s of a sixteenth
+                const float4* w4 = reinterpret_cast<const float4*>(p.wr + (size_t)e * p.H + quarter * seg);
+                const float4* x4 = reinterpret_cast<const float4*>(xn + quarter * seg);
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    for (int i = lane; i < n4; i += 32) {
+                        const float4 w = n4 == 32 ? wv0[s] : w4[s * n4 + i], x = x4[s * n4 + i];
+                        acc[s] = fmaf(w.x, x.x, acc[s]);
+                        acc[s] = fmaf(w.y, x.y, acc[s]);
+                        acc[s] = fmaf(w.z, x.z, acc[s]);
+                        acc[s] = fmaf(w.w, x.w, acc[s]);
+                    }
+            }
+        } else if (e < p.E) {
             const float4* w4 = reinterpret_cast<const float4*>(p.wr + (size_t)e * p.H + quarter * seg);
             for (int i0 = 0; i0 < seg / 4; i0 += 128) {
                 float4 wv[4];
@@ -309,9 +325,10 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
                 }
             }
         }
+        const int sums = p.sixteenths ? 4 : p.T;
 #pragma unroll
         for (int t = 0; t < DC_MAX_T; ++t) {
-            if (t < p.T) {
+            if (t < sums) {
                 float v = acc[t];
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -319,7 +336,15 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
             }
         }
         __syncthreads();
-        if (threadIdx.x < 2 * p.T) {
+        if (p.sixteenths) {
+            const int which = threadIdx.x, ee = blockIdx.x * 2 + which;
+            if (which < 2 && ee < p.E) {
+                float v = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v += s_part[which * 4 + i / 4][i % 4];
+                p.logits[ee] = v;
+            }
+        } else if (threadIdx.x < 2 * p.T) {
             const int which = threadIdx.x / p.T, t = threadIdx.x % p.T, ee = blockIdx.x * 2 + which;
             if (ee < p.E)
                 p.logits[(size_t)t * p.E + ee] = (s_part[which * 4][t] + s_part[which * 4 + 1][t]) +
@@ -595,7 +620,7 @@ int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weigh
 }
 
 int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_expert, int T, int top_k, float scale,
-                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode, const dc_route_norm* norm) {
+                     int ep_lo, int ep_hi, const dc_moe_route* rt, int mode, const dc_route_norm* norm, bool sixteenths) {
     // wr == nullptr: rt->logits already holds the router logits (routing only)
     if (wr && wr->type != DC_TYPE_F32) return dc_fail(ctx, DC_B200_UNSUPPORTED, "router weight must be F32");
     const int E = wr ? (int)wr->N : n_expert;
@@ -620,6 +645,7 @@ int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_ex
     p.uexp = rt->uexp;
     p.uoff = rt->uoff;
     p.uassign = rt->uassign;
+    p.sixteenths = sixteenths && T == 1;
     size_t smem = 0;
     if (norm) {
         if (!wr || T > 4) return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "router: rows to be normed need router weights, and are four at most");

@@ -113,3 +113,79 @@ def test_decode_steps_are_the_chunk_path_bit_for_bit(ctx, moe):
     for i in range(4):
         assert np.array_equal(m.decode_step(s[:1], [toks[i, 0]], want_logits=True)[1][0], chunk[0][i]), i
     m.close()
+
+
+@pytest.mark.parametrize("n_head,n_kv,T", [(32, 4, 2), (16, 2, 4), (16, 2, 16), (12, 2, 5), (32, 8, 4), (8, 4, 1)])
+def test_cluster_attention_is_the_split_kernels_bit_for_bit(ctx, oracle, n_head, n_kv, T):
+    """A table short enough for clusters of eight or sixteen CTAs, and one that takes the split kernels (more than 64 blocks a run would
+    take the third form): the same runs, the same order of every sum, hence equal outputs.  Tokens of several sequences of unequal length,
+    and neighbours in one sequence, whose rows the call itself writes."""
+    rng = np.random.default_rng(n_head + T)
+    scale, blocks = float(128 ** -0.5), 160
+    small, large = (ctx.kv_cache(1, n_kv, 128, 17 * b, 17, b) for b in (blocks, 1024))
+    lens = [int(x) for x in np.linspace(2300, 1, T)]
+    seqs = [[c.seq_alloc() for _ in range(T + 1)] for c in (small, large)]
+    for i, n in enumerate(lens + [1500]):
+        k, v = (rng.normal(size=(n, n_kv, 128)).astype(np.float32) for _ in range(2))
+        k *= np.linspace(0.2, 1.5, n)[:, None, None].astype(np.float32)      # the running maximum keeps moving
+        for p in range(0, n, 16):
+            m = min(16, n - p)
+            for c, s in zip((small, large), seqs):
+                c.flash_attn_decode(0, np.zeros((m, n_head, 128), np.float32), k[p:p + m], v[p:p + m], [s[i]] * m, list(range(p, p + m)), scale)
+    q, k, v = (rng.normal(size=(T, h, 128)).astype(np.float32) for h in (n_head, n_kv, n_kv))
+    for step in range(2):
+        got, want = (c.flash_attn_decode(0, q, k, v, s[:T], [n + step for n in lens], scale) for c, s in zip((small, large), seqs))
+        assert np.abs(got).max() > 0 and np.array_equal(got, want), step
+    got, want = (c.flash_attn_decode(0, q, k, v, [s[T]] * T, list(range(1500, 1500 + T)), scale) for c, s in zip((small, large), seqs))
+    assert np.abs(got).max() > 0 and np.array_equal(got, want)
+    small.close()
+    large.close()
+
+
+def _prefilled(ctx, cfg, lens, seed=11):
+    m = dc.Model(ctx, cfg)
+    m.init_synthetic(5, 0.05)
+    m.finalize()
+    rng = np.random.default_rng(seed)
+    seqs = [m.seq_alloc() for _ in lens]
+    for s, n in zip(seqs, lens):
+        m.prefill(s, rng.integers(0, cfg.vocab, size=n))
+    return m, seqs
+
+
+@pytest.mark.parametrize("n_head,n_kv,streams", [(32, 8, 4), (32, 8, 1), (16, 8, 3), (64, 8, 2)])
+def test_fused_decode_steps_do_not_depend_on_the_table(ctx, n_head, n_kv, streams):
+    """Steps of streams of unequal length, several blocks a CTA, with norm, rotation and cache write inside the attention kernel (table of
+    3072 positions) and with the split kernels (16384 positions; 37 runs in both): equal logits, also for a chunk of one sequence."""
+    lens = [1900, 1130, 517, 64][:streams]
+    kw = dict(n_layer=2, hidden=512, n_head=n_head, n_kv_head=n_kv, vocab=1000, ffn=1024, max_seqs=4)
+    toks = np.random.default_rng(3).integers(0, 1000, size=(3, 4))
+    out = []
+    for max_ctx in (3072, 16384):
+        m, seqs = _prefilled(ctx, dc.Config(max_ctx=max_ctx, **kw), lens)
+        lg = [m.decode_step(seqs, t[:streams], want_logits=True)[1] for t in toks]
+        lg.append(m.forward_chunk(seqs[0], toks[0]))
+        out.append((np.concatenate(lg), m.step_stats()[0]))
+        m.close()
+    assert np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("softmax", [0, 1])
+@pytest.mark.parametrize("hidden,n_head,n_kv", [(2048, 32, 4), (512, 8, 2), (1024, 16, 8)])
+def test_one_stream_has_the_persistent_kernels_results(ctx, hidden, n_head, n_kv, softmax):
+    """By default one stream of a mixture-of-experts model runs as separate kernels, which form their sums (router logits, attention runs)
+    as the persistent kernel does: the same logits bit for bit, whichever serves the step."""
+    cfg = dc.Config(n_layer=2, hidden=hidden, n_head=n_head, n_kv_head=n_kv, vocab=1000, n_expert=24, n_expert_used=4, expert_ffn=512, max_seqs=2, max_ctx=2200)
+    m, seqs = _prefilled(ctx, cfg, [2040, 70])
+    m.set_option("route_mode", softmax)
+    toks = np.random.default_rng(4).integers(0, 1000, size=(4, 2))
+    res = {}
+    for mode in (1, 2):
+        m.set_option("persistent", mode)
+        lg = [m.decode_step([s], [t[i]], want_logits=True)[1] for i, s in enumerate(seqs) for t in toks]
+        res[mode] = (np.concatenate(lg), m.step_stats()[0])
+        for s, n in zip(seqs, (2040, 70)):
+            m.seq_truncate(s, n)
+    assert res[2][1] == 1 < res[1][1], "the two runs must have taken different paths"
+    assert np.array_equal(res[1][0], res[2][0])
+    m.close()
