@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(128) k_attn_pv_run(const AttnParams p) {
 // stay rolled.  32 Q / 4 KV heads, 2000 keys, one token, a step of three layers: 178 us; with the split kernels and k_qknorm_rope_kv 260;
 // 171 with keys dealt out over the threads in an order of sums that is not the split kernels'.
 #define AC_THREADS 256
-#define AC_CAP 32              // KV blocks a CTA holds at most
+#define AC_CAP 48              // KV blocks a CTA holds at most
 #define AC_SMEM (220 * 1024)
 #define AC_Q_PITCH 144         // floats of a q head: four quarters 36 apart, which fall into different banks
 
@@ -975,16 +975,27 @@ struct AcPlan {
 static int attn_head_split(int C, int T, int n_kv, int g) { return g % 4 == 0 && 2 * T * n_kv * C <= 128 ? 2 : 1; }
 static bool attn_cluster_fits(int C, int T, int n_kv, int g, int max_blocks, int nsplit) {
     const AcPlan plan(C, max_blocks, nsplit);
-    // (a thread for each of 8 x 8 denominators; runs longer than ATT_MAX_RUN take k_attn_pv, which multiplies alphas in another order)
-    return plan.cap <= AC_CAP && plan.rcap <= 8 && (max_blocks + nsplit - 1) / nsplit <= ATT_MAX_RUN &&
-           plan.smem(g / attn_head_split(C, T, n_kv, g)) <= AC_SMEM;
+    // a thread for each of 8 x 8 denominators; runs longer than ATT_MAX_RUN take k_attn_pv, which multiplies alphas in another order
+    if (plan.rcap > 8 || (max_blocks + nsplit - 1) / nsplit > ATT_MAX_RUN) return false;
+    // more than 32 blocks a CTA pay in clusters of sixteen alone, and not where a kv head has two query heads, whose P.V then keeps few
+    // warps busy (three layers, split kernels against clusters, us: 16 Q / 8 KV heads, table of 4096 positions, 2000 keys, four streams
+    // 192 / 213 with 35 blocks; table of 6144, 6000 keys, one stream 196 / 207 with 33)
+    if (plan.cap > (C > 8 && g > 2 ? AC_CAP : 32)) return false;
+    return plan.smem(g / attn_head_split(C, T, n_kv, g)) <= AC_SMEM;
 }
-// CTAs of the cluster that serves T tokens, 0: the split kernels do.  Clusters of sixteen halve a CTA's share but only one fits into a
-// group of SMs: they pay for up to eight clusters, or where eight CTAs cannot hold the keys.
+// CTAs of the cluster that serves T tokens, 0: the split kernels do.  An SM group holds one cluster of sixteen (two where two CTAs fit
+// into an SM), so they are for up to eight clusters.  Clusters of eight come in several waves above 32; they then pay where the runs are
+// many enough to share out evenly (10 runs keep five CTAs of eight) and two CTAs fit into an SM, or few heads make a CTA's work short.
+// Three layers, split kernels against clusters, us: 32 Q / 4 KV heads, table of 2112, 2000 keys: one stream 260 / 178, four 336 / 298,
+// sixteen 710 / 629; 500 keys and a table of 640, sixteen streams 548 / 554; 32 Q / 16 KV heads, table of 640, 500 keys, sixteen streams
+// 535 / 637; clusters of sixteen with four streams of those and a table of 4096: 216 / 372.
+// Prompt chunks of hundreds of tokens fill the SMs either way (16 Q / 8 KV heads, 2000 tokens: 106 / 118 ms).
 static int attn_cluster_size(int T, int n_kv, int g, int max_blocks, int nsplit) {
-    const bool eight = attn_cluster_fits(8, T, n_kv, g, max_blocks, nsplit);
-    if ((!eight || T * n_kv <= 8) && attn_cluster_fits(16, T, n_kv, g, max_blocks, nsplit)) return 16;
-    return eight ? 8 : 0;
+    if (T > DC_MAX_T) return 0;
+    if (T * n_kv <= 8 && attn_cluster_fits(16, T, n_kv, g, max_blocks, nsplit)) return 16;
+    if (!attn_cluster_fits(8, T, n_kv, g, max_blocks, nsplit)) return 0;
+    if (T * n_kv <= 32) return 8;
+    return nsplit >= 24 && (g <= 4 || AcPlan(8, max_blocks, nsplit).smem(g) <= 113 * 1024) ? 8 : 0;
 }
 bool dc_attn_cluster_ok(int T, int n_head, int n_kv, int max_blocks, int nsplit) {
     return attn_cluster_size(T, n_kv, n_head / n_kv, max_blocks, nsplit) != 0;

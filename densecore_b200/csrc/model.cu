@@ -389,7 +389,9 @@ static int upload_step_inputs(dc_model* m, const int32_t* tokens, const int32_t*
 // The persistent kernel serves decode steps of MoE models where it is asked for (use_mega 2), and one stream of an expert-parallel
 // model, whose ranks exchange expert outputs inside it.  Elsewhere the per-op kernels are faster: its seven grid barriers a layer cost
 // more than seven launches that overlap, and its row dots stay on dp4a.  (8-layer cut, 2048 tokens of context, us a step: one stream
-// 681 persistent, 518 per-op; four 2059 and 935.)
+// 681 persistent, 518 per-op; four 2059 and 935.)  So is one stream whose block table is too long for the cluster attention kernel: the
+// separate kernels then are two a layer more (three layers, table of 16384 positions, 2000 keys, us: 32 Q / 4 KV heads 240 persistent and
+// 260, 16 Q / 2 KV heads 176 and 198; 32 Q / 8 KV heads 231 and 216).
 // One stream by default (use_mega 1) has the persistent kernel's results whichever serves it: *runs says how many runs its attention has,
 // for the per-op kernels to form their sums in the same order (0: in their own).
 static bool mega_ok(dc_model* m, int T, int* runs) {
@@ -399,6 +401,7 @@ static bool mega_ok(dc_model* m, int T, int* runs) {
     const char* why = "";
     if (!dc_mega_plan(m, T, &p, &why)) return false;
     if (m->use_mega == 2 || m->cfg.ep_size > 1) return true;
+    if (!dc_attn_cluster_ok(T, m->cfg.n_head, m->cfg.n_kv_head, m->kv.max_blocks_per_seq, p.nsplit)) return true;
     *runs = p.nsplit;
     return false;
 }

@@ -189,3 +189,17 @@ def test_one_stream_has_the_persistent_kernels_results(ctx, hidden, n_head, n_kv
     assert res[2][1] == 1 < res[1][1], "the two runs must have taken different paths"
     assert np.array_equal(res[1][0], res[2][0])
     m.close()
+
+
+@pytest.mark.parametrize("n_head,n_kv,max_ctx,streams,cluster", [(32, 16, 640, 1, True), (32, 16, 640, 4, False), (32, 16, 4096, 2, False), (16, 8, 4096, 4, False),
+                                                                 (16, 8, 2112, 4, True), (16, 8, 2112, 16, True), (16, 8, 640, 16, False), (32, 4, 4096, 1, True)])
+def test_attention_form_of_a_step(ctx, n_head, n_kv, max_ctx, streams, cluster):
+    """The one-kernel form serves the steps for which it is the faster one, by streams, heads and length of the block table: a layer then has
+    two launches less than with a table that only the split kernels take."""
+    launches = []
+    for n in (max_ctx, 32768):
+        m, seqs = _prefilled(ctx, dc.Config(n_layer=2, hidden=512, n_head=n_head, n_kv_head=n_kv, vocab=1000, ffn=1024, max_seqs=16, max_ctx=n), [20] * streams)
+        m.decode_step(seqs, [1] * streams)
+        launches.append(m.step_stats()[0])
+        m.close()
+    assert launches[1] - launches[0] == (4 if cluster else 0)
