@@ -286,7 +286,7 @@ static int mul_mat_chunks(dc_ctx* ctx, const dc_weight* w, const float* x_dev, i
     for (int m0 = 0; m0 < M; m0 += DC_MAX_T) {
         const int T = M - m0 < DC_MAX_T ? M - m0 : DC_MAX_T;
         const float* x = x_dev + (size_t)m0 * K;
-        const bool own = dc_rows_quantise(T, K);
+        const bool own = dc_rows_quantise(T, K, x, N, y_dev + (size_t)m0 * N);
         if (!own) DC_TRY(dc_launch_quantize_q8k(ctx, x, T, K, q8, true));
         dc_gemv_seg seg = {w->dev, w->type, N, (int)w->row_bytes, y_dev + (size_t)m0 * N, N};
         DC_TRY(dc_launch_gemv(ctx, &seg, 1, DC_EPI_STORE, q8, T, K, nullptr, nullptr, nullptr, own ? x : nullptr));

@@ -83,6 +83,12 @@ DC_PART int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int 
 // whether k_rows quantises its T rows itself (act_f32): each of its eight warps then has three blocks at most to quantise, about 1 us,
 // against a launch of the chain (1.5 to 2 us).  Above the line every CTA repeats work that one small kernel does once.
 static inline bool dc_rows_quantise(int T, int K) { return T * (K / 256) <= 24; }
+// The same for rows and results at a caller's addresses: where they overlap (a product in place), the rows have to be quantised before any
+// result is stored, for a CTA may be done while another still reads.
+static inline bool dc_rows_quantise(int T, int K, const float* x, int N, const float* y) {
+    const uintptr_t x0 = (uintptr_t)x, x1 = (uintptr_t)(x + (size_t)T * K), y0 = (uintptr_t)y, y1 = (uintptr_t)(y + (size_t)T * N);
+    return dc_rows_quantise(T, K) && (x1 <= y0 || y1 <= x0);
+}
 // rows x K f32 -> native Q8_K blocks (row stride K/256*292), or blocks in fragment order (row stride K/256*320)
 DC_PART int dc_launch_quantize_q8k(dc_ctx* ctx, const float* x, int rows, int K, uint8_t* out, bool frag = false);
 // Tensor-core MUL_MAT for many token rows (gemm_tc.cu): activations quantised into 64-token tiles, then

@@ -60,7 +60,7 @@ extern "C" int dc_b200_mul_mat_dev_noalloc(dc_ctx* ctx, const dc_weight* w, cons
     if (st != DC_B200_OK) return st;
     cudaSetDevice(ctx->device);
     // the activations are fully rewritten by every call, so nothing has to be cleared first
-    const bool own = dc_rows_quantise(M, (int)w->K);
+    const bool own = dc_rows_quantise(M, (int)w->K, x_dev, (int)w->N, y_dev);
     if (!own) st = dc_launch_quantize_q8k(ctx, x_dev, M, (int)w->K, q8, true);
     if (st != DC_B200_OK) return st;
     dc_gemv_seg seg = {w->dev, w->type, (int)w->N, (int)w->row_bytes, y_dev, (int)w->N};

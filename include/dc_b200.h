@@ -100,7 +100,9 @@ DC_B200_API int dc_b200_quantize_q8k_dev(dc_ctx* ctx, const float* x_dev, int ro
  * cb_gemv_custom (M == 1, core/src/llm/matmul/gemv_exec.cpp:99) and
  * cb_gemv_batched_custom (M >= 2, core/src/llm/matmul/batched_exec.cpp:55).
  * Any M >= 1; rows are processed 16 at a time (kMaxSmallBatchColsHard,
- * core/src/llm/matmul/userdata.h:14). */
+ * core/src/llm/matmul/userdata.h:14).  With M <= 16 rows x_dev and y_dev may
+ * overlap (a product in place): the rows are then quantised before any result
+ * is stored. */
 DC_B200_API int dc_b200_mul_mat(dc_ctx* ctx, const dc_weight* w, const float* x_host, int M, float* y_host);
 DC_B200_API int dc_b200_mul_mat_dev(dc_ctx* ctx, const dc_weight* w, const float* x_dev, int M, float* y_dev);
 /* The same product for callers that may not allocate (no counterpart in

@@ -39,6 +39,25 @@ def test_rows_are_the_cpu_kernels_bit_for_bit(ctx, oracle, t, N, K):
     W.free()
 
 
+@pytest.mark.parametrize("noalloc", [False, True])
+@pytest.mark.parametrize("t,n,M", [(B.GGML_TYPE_Q4_K, 512, 12), (B.GGML_TYPE_Q6_K, 1024, 6), (B.GGML_TYPE_Q4_K, 6144, 1), (B.GGML_TYPE_Q4_K, 1024, 7)])
+def test_product_in_place(ctx, t, n, M, noalloc):
+    """Results stored over the rows themselves, and over their end: few rows (24 blocks or fewer, which the product would else quantise
+    itself while others already store) and one block more."""
+    rng = np.random.default_rng(n + M)
+    W = ctx.upload_weight(t, B.random_weight(rng, t, n, n), n, n)
+    x = rng.normal(size=(M, n)).astype(np.float32)
+    want = ctx.mul_mat(W, x)
+    buf = ctx.alloc(3 * x.nbytes)
+    for shift in (0, x.nbytes - 4096, 4096 - x.nbytes) if M > 1 else (0, 1024, -1024):
+        ctx.to_device(buf + x.nbytes, x)
+        ctx.mul_mat_dev(W, buf + x.nbytes, M, buf + x.nbytes + shift, noalloc=noalloc)
+        ctx.synchronize()
+        assert np.array_equal(ctx.from_device(buf + x.nbytes + shift, np.empty((M, n), np.float32)), want), shift
+    ctx.free(buf)
+    W.free()
+
+
 @pytest.mark.parametrize("E,F,H,k,down", [(3, 256, 512, 2, B.GGML_TYPE_Q6_K), (128, 768, 512, 8, B.GGML_TYPE_Q6_K), (200, 256, 1280, 16, B.GGML_TYPE_Q4_K)])
 def test_expert_rows_match_rows_of_single_tokens(ctx, E, F, H, k, down):
     """A token's result does not depend on the tokens beside it, up to the order in which its experts' outputs are added (routing order
