@@ -157,53 +157,57 @@ __device__ __forceinline__ void route_token(const RouterParams& p, int t, int la
     }
 }
 
-// Routing of all T tokens by the whole CTA (DC_ROUTE_STABLE): an expert's place among a token's experts is the number of better ones, so all
-// experts find theirs at once; route_token's rounds of warp-wide maxima took 4.6 us a token.  Same picks, same weights.
-// (Little unrolled: one CTA runs this once a launch, and instructions that are not in the SM's cache cost more than the loop.)
-// s_key: 256 keys, 16-byte aligned; s_sel: T * top_k picked logits.
-__device__ __forceinline__ void route_all_stable(const RouterParams& p, unsigned long long* s_key, float* s_sel, int32_t* s_ids) {
-    const int tid = threadIdx.x, P = p.E <= 32 ? 8 : p.E <= 64 ? 4 : p.E <= 128 ? 2 : 1;     // neighbouring threads that share an expert
-    const int e = tid / P, sub = tid % P;
-    const float* mine = p.logits + min(e, p.E - 1);
-    float v = __ldcg(mine);
-#pragma unroll 1
-    for (int t = 0; t < p.T; ++t) {
-        const unsigned long long key = e < p.E ? route_key(v, e) : 0ull;      // a real key is never 0
-        if (sub == 0) s_key[e] = key;
-        if (t + 1 < p.T) v = __ldcg(mine + (size_t)(t + 1) * p.E);
-        __syncthreads();
-        int above = 0;
-#pragma unroll 4
-        for (int f = sub; f < p.E; f += P) above += s_key[f] > key;
-        for (int o = 1; o < P; o <<= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
-        if (sub == 0 && e < p.E && above < p.top_k) {
-            const uint32_t ku = (uint32_t)(key >> 32);
-            s_sel[t * p.top_k + above] = __uint_as_float((ku & 0x80000000u) ? (ku & 0x7FFFFFFFu) : ~ku);    // (-0 became +0)
-            s_ids[t * p.top_k + above] = e;
-            p.ids[t * p.top_k + above] = e;
-        }
-        __syncthreads();
+// Routing of token t by one warp (DC_ROUTE_STABLE): the best expert left is found by two warp-wide reductions, of the 32-bit keys and, among
+// equal ones, of the ids; the weights are those of the persistent kernel (exponentials side by side, their sum in pick order).
+// Bound by the chain of top_k rounds.  Expert layers of 2048 columns, us at 3 / 12 tokens: 128 experts of 768 columns, 8 picks 70 / 148;
+// 256 experts of 512 65 / 135.  One CTA that compared every expert with every other, a token after the other, made these 79 / 173 and
+// 82 / 203, and route_token's rounds of 64-bit exchanges were 5 us a launch where these are 2.
+__device__ __forceinline__ void route_token_stable(const RouterParams& p, int t, int lane, int32_t* s_ids) {
+    uint32_t key[MOE_MAX_E / 32];      // order of the logits, from 1 (NaN) on; 0: none left
+#pragma unroll
+    for (int j = 0; j < MOE_MAX_E / 32; ++j) {
+        const int e = j * 32 + lane;
+        key[j] = e < p.E ? (uint32_t)(route_key(__ldcg(p.logits + (size_t)t * p.E + e), e) >> 32) + 1u : 0u;
     }
-    // weights over the selected experts only (native.cpp:649-674)
-    for (int i = tid; i < p.T * p.top_k; i += 256) {
-        const float* sel = s_sel + i / p.top_k * p.top_k;
-        float mx = -INFINITY;
-        bool finite = true;
-        for (int k = 0; k < p.top_k; ++k) {
-            finite = finite && isfinite(sel[k]);
-            if (isfinite(sel[k]) && sel[k] > mx) mx = sel[k];
-        }
-        float den = 0.0f, own = 0.0f;
-        if (finite && isfinite(mx)) {
+    int pick = 0;
+    uint32_t at = 0u;      // lane k: the k-th pick and its key
 #pragma unroll 1
-            for (int k = 0; k < p.top_k; ++k) {
-                const float w = expf(sel[k] - mx);
-                if (k == i % p.top_k) own = w;
-                den += w;
+    for (int k = 0; k < p.top_k; ++k) {
+        uint32_t best = key[0];
+        int id = lane;
+#pragma unroll
+        for (int j = 1; j < MOE_MAX_E / 32; ++j)
+            if (key[j] > best) {      // (equal: the lower id stays)
+                best = key[j];
+                id = j * 32 + lane;
             }
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        const int win = (int)__reduce_min_sync(0xffffffffu, best == top ? (uint32_t)id : 0xffffffffu);
+#pragma unroll
+        for (int j = 0; j < MOE_MAX_E / 32; ++j)
+            if (j * 32 + lane == win) key[j] = 0u;
+        if (lane == k) {
+            pick = win;
+            at = top - 1u;
         }
+    }
+    const bool own = lane < p.top_k;
+    const float v = own ? __uint_as_float((at & 0x80000000u) ? (at & 0x7FFFFFFFu) : ~at) : -INFINITY;     // the logit (-0 became +0)
+    // weights over the selected experts only (native.cpp:649-674)
+    const bool finite = __all_sync(0xffffffffu, !own || isfinite(v));
+    float mx = own && isfinite(v) ? v : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float ev = finite && isfinite(mx) && own ? expf(v - mx) : 0.0f;
+    float den = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < p.top_k; ++k) den += __shfl_sync(0xffffffffu, ev, k);
+    if (own) {
         const bool ok = den > 0.0f && isfinite(den);
-        p.weights[i] = __fmul_rn(ok ? __fdiv_rn(own, den) : __fdiv_rn(1.0f, (float)p.top_k), p.scale);
+        const int i = t * p.top_k + lane;
+        p.weights[i] = __fmul_rn(ok ? __fdiv_rn(ev, den) : __fdiv_rn(1.0f, (float)p.top_k), p.scale);
+        p.ids[i] = pick;
+        s_ids[i] = pick;
     }
 }
 
@@ -211,8 +215,6 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     __shared__ int s_last;
     __shared__ float s_prob[8][MOE_MAX_E];
     __shared__ __align__(16) int32_t s_ids[DC_MAX_T * MOE_MAX_K + 4];
-    __shared__ __align__(16) unsigned long long s_key[256];
-    __shared__ float s_sel[DC_MAX_T * MOE_MAX_K];
     __shared__ int s_wsum_a[8], s_wsum_c[8];
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -369,11 +371,12 @@ __global__ void __launch_bounds__(256) k_router(const RouterParams p) {
     __syncthreads();
     if (!s_last) return;
 
-    // ---- top-k per token
+    // ---- top-k per token, one warp per token
     if (threadIdx.x < 4) s_ids[p.T * p.top_k + threadIdx.x] = -1;
-    if (p.mode == DC_ROUTE_STABLE) route_all_stable(p, s_key, s_sel, s_ids);
-    else
-        for (int t = warp; t < p.T; t += 8) route_token(p, t, lane, s_prob[warp], s_ids);
+    for (int t = warp; t < p.T; t += 8) {
+        if (p.mode == DC_ROUTE_STABLE) route_token_stable(p, t, lane, s_ids);
+        else route_token(p, t, lane, s_prob[warp], s_ids);
+    }
     __syncthreads();
     if (p.T == 1) {      // every pick is an expert's only token: the picks of this GPU's experts by ascending id
         if (threadIdx.x < 32) {

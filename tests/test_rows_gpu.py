@@ -77,6 +77,31 @@ def test_expert_rows_match_rows_of_single_tokens(ctx, E, F, H, k, down):
         w.free()
 
 
+@pytest.mark.parametrize("E,k", [(1, 1), (2, 2), (16, 16), (31, 5), (32, 8), (33, 16), (100, 8), (128, 8), (255, 16), (256, 8)])
+def test_routing_takes_the_best_experts_in_order(ctx, E, k):
+    """Larger logit first, then lower id, NaN last: ties, both zeros, infinities and NaN at the edges of a warp's lanes.  Weights: a softmax
+    over the picks, k terms of f32 exponentials (2 ulp each) and one division; equal shares where a pick is not finite."""
+    rng = np.random.default_rng(E)
+    for T in (1, 3, 8, 9, 16):
+        lg = rng.integers(-3, 4, size=(T, E)).astype(np.float32) * np.float32(0.5)      # many ties
+        lg[lg == 0] *= rng.choice([-1, 1])
+        if T > 1:
+            lg[1] = rng.normal(size=E)
+            lg[1, rng.integers(E, size=3)] = np.nan
+        if T > 2:
+            lg[2] = rng.permutation(E)
+            lg[2, [0, -1]] = np.inf, -np.inf
+        ids, w = ctx.moe_route(lg, k)
+        key = np.where(np.isnan(lg), -np.inf, lg).astype(np.float64)
+        order = np.lexsort((np.broadcast_to(np.arange(E), lg.shape), -key, np.isnan(lg)), axis=-1)[:, :k]
+        assert np.array_equal(ids.reshape(T, k), order), T
+        v = np.take_along_axis(lg, order, 1).astype(np.float64)
+        with np.errstate(invalid="ignore"):
+            x = np.exp(v - v.max(1, keepdims=True))
+            want = np.where(np.isfinite(v).all(1, keepdims=True), x / x.sum(1, keepdims=True), 1.0 / k)
+        assert np.abs(w.reshape(T, k) - want).max() <= (k + 6) * 2.0 ** -24, T
+
+
 @pytest.mark.parametrize("n_head,n_kv,blocks", [(32, 4, 176), (16, 8, 130), (12, 2, 512), (64, 16, 256)])
 def test_cluster_attention_against_split_kernels_and_oracle(ctx, oracle, n_head, n_kv, blocks):
     """The same keys in a cache short enough for the cluster kernel and in one that is not; lengths at which a CTA of the cluster gets
