@@ -182,9 +182,10 @@ int dc_launch_router_batched(dc_ctx* ctx, const dc_weight* wr, const float* xn, 
                              int32_t* ids, float* weights, int mode);
 // carves a dc_moe_route for (T, E, top_k) out of a byte buffer; returns bytes used
 DC_PART size_t dc_moe_route_bind(dc_moe_route* rt, uint8_t* base, int T, int E, int top_k);
-// whether the down projection quantises its rows itself: a CTA then has few blocks to quantise (two tokens of an expert in most
-// CTAs, under 1 us), and a launch of the chain (2 us a layer) goes away
-static inline bool dc_moe_quantise_in_down(int T) { return T <= 4; }
+// Whether the down projection of experts of F columns quantises its rows itself: a CTA meets few tokens and thus few blocks, and a launch of
+// the chain goes away.  Expert layers at 1 / 4 tokens, us with a quantiser kernel and without: F = 768 49.5 / 97.8 and 46.2 / 94.8,
+// F = 3072 57.6 / 124.4 and 55.3 / 122.7; F = 4096 43.3 / 97.1 and 43.3 / 98.7, F = 8192 102.0 / 214.4 and 103.4 / 220.4.
+static inline bool dc_moe_quantise_in_down(int T, int F) { return T <= 4 && F < 4096; }
 DC_PART int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weight* w1, const uint8_t* act_q8,
                      int T, int top_k, int e_base, const dc_moe_route* rt, float* out, const float* act_f32 = nullptr);
 // x += the experts' weighted sum (as dc_launch_moe_combine), then RMSNorm (xn_out, optional) and Q8_K blocks in

@@ -283,7 +283,7 @@ static int enqueue_forward(dc_model* m, int T, int lm_mode, bool feedback, bool 
               dc_launch_router(ctx, Ly.router, b.xn, E, T, top_k, c.routed_scale, ep_lo, ep_hi, &b.route, m->route_mode, norm_in_router ? &rn : nullptr, runs != 0));
             L(DC_K_MOE_GATEUP, U * local * 2.0 * F * Ly.gate_exps->row_bytes + q8x + (double)A * F * 4, 1,
               dc_launch_moe_mm(ctx, true, Ly.gate_exps, Ly.up_exps, b.q8_x, T, top_k, ep_lo, &b.route, b.h));
-            const bool own = dc_moe_quantise_in_down(T);
+            const bool own = dc_moe_quantise_in_down(T, F);
             if (!own)
                 L(DC_K_QUANT_H, (double)A * F * 4 + (double)A * (F / 256) * DC_Q8F_BYTES, 1,
                   dc_launch_quantize_q8k(ctx, b.h, A, F, b.q8_h, true));

@@ -141,7 +141,7 @@ static int moe_layer_dev(dc_ctx* ctx, const dc_weight* router, const float* logi
     DC_TRY(dc_launch_router(ctx, router, x_dev, E, T, top_k, routed_scale, 0, E, &rt, ctx->route_mode));
     DC_TRY(dc_launch_quantize_q8k(ctx, x_dev, T, H, xq, true));
     DC_TRY(dc_launch_moe_mm(ctx, true, gate, up, xq, T, top_k, 0, &rt, h));
-    const bool own = dc_moe_quantise_in_down(T);
+    const bool own = dc_moe_quantise_in_down(T, F);
     if (!own) DC_TRY(dc_launch_quantize_q8k(ctx, h, A, F, hq, true));
     DC_TRY(dc_launch_moe_mm(ctx, false, down, nullptr, hq, T, top_k, 0, &rt, dn, own ? h : nullptr));
     DC_TRY(dc_launch_moe_combine(ctx, dn, rt.ids, rt.weights, T, top_k, H, 0, E, y_dev));
