@@ -252,9 +252,9 @@ __device__ __forceinline__ void rows_unit_q6k(const uint8_t* smem, uint32_t og, 
 
 // The same for a single token on m16n8k32: a 32-value quadrant of 16 rows at a time, whose eight words are the eight columns and
 // partials, so that a lane's two columns have one scale.
-template <class Sink>
+template <bool DUMP, class Sink>
 __device__ __forceinline__ void rows_unit_q6k_one(const uint8_t* smem, uint32_t og, uint32_t og8, const RowAct& act, int b, int row0, int lane,
-                                                  const RowsParams& p, const Sink& sink) {
+                                                  const RowsParams& p, int row, bool live, bool live8, const Sink& sink) {
     const int g = lane >> 2, t = lane & 3;
     const uint32_t sh = (og & 2u) * 8u, sh8 = (og8 & 2u) * 8u;
     const uint8_t *a = smem + (og & ~3u), *a8 = smem + (og8 & ~3u);
@@ -297,6 +297,16 @@ __device__ __forceinline__ void rows_unit_q6k_one(const uint8_t* smem, uint32_t 
             P[2] += s8 * d[2];
             P[3] += s8 * d[3];
         }
+    }
+    if (DUMP) {
+        int s0 = (P[0] >> 2) + (P[1] >> 2), s8 = (P[2] >> 2) + (P[3] >> 2);
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            s8 += __shfl_xor_sync(0xffffffffu, s8, o);
+        }
+        if (t == 0 && live) p.dump.I[(size_t)row * p.nb + b] = s0;
+        if (t == 0 && live8) p.dump.I[(size_t)(row + 8) * p.nb + b] = s8;
     }
     const float yd = ld_f(smem + rec + 144), f0 = __fmul_rn(yd, d0), f8 = __fmul_rn(yd, d8);
 #pragma unroll
@@ -608,7 +618,8 @@ __device__ __forceinline__ void rows_cta(const RowsParams& p, uint8_t* smem, int
                     if constexpr (Q4)
                         rows_unit_q4k<NG, ONE, DUMP>(smem + stage, smem + stage + 8 * PITCH, act, b, row0, nt, lane, p, t.row0 + g, g < t.rows, g + 8 < t.rows, sink);
                     else if constexpr (ONE)
-                        rows_unit_q6k_one(smem, stage + (sk0 + b * DC_Q6K_BYTES & 15u), stage + 8 * PITCH + (sk8 + b * DC_Q6K_BYTES & 15u), act, b, row0, lane, p, sink);
+                        rows_unit_q6k_one<DUMP>(smem, stage + (sk0 + b * DC_Q6K_BYTES & 15u), stage + 8 * PITCH + (sk8 + b * DC_Q6K_BYTES & 15u), act, b, row0, lane, p,
+                                                t.row0 + g, g < t.rows, g + 8 < t.rows, sink);
                     else
                         rows_unit_q6k<NP, DUMP>(smem, stage + (sk0 + b * DC_Q6K_BYTES & 15u), stage + 8 * PITCH + (sk8 + b * DC_Q6K_BYTES & 15u), act, b, row0, nt, lane, p,
                                                 t.row0 + g, g < t.rows, g + 8 < t.rows, sink);

@@ -70,13 +70,13 @@ template <int KIND, int NP, bool ONE, bool PAIR, bool DUMP>
 static int launch_rows(dc_ctx* ctx, RowsParams& p, size_t smem) {
     return p.S == 1 ? launch_rows_as<KIND, NP, ONE, PAIR, DUMP, true>(ctx, p, smem) : launch_rows_as<KIND, NP, ONE, PAIR, DUMP, false>(ctx, p, smem);
 }
-template <int KIND, bool PAIR>
+template <int KIND, bool PAIR, bool DUMP = false>
 static int launch_rows_np(dc_ctx* ctx, RowsParams& p, int np, size_t smem) {
-    if (p.T == 1) return launch_rows<KIND, 1, true, PAIR, false>(ctx, p, smem);
-    if (np == 1) return launch_rows<KIND, 1, false, PAIR, false>(ctx, p, smem);
-    if (np == 2) return launch_rows<KIND, 2, false, PAIR, false>(ctx, p, smem);
-    if (np == 4) return launch_rows<KIND, 4, false, PAIR, false>(ctx, p, smem);
-    return launch_rows<KIND, 8, false, PAIR, false>(ctx, p, smem);
+    if (p.T == 1) return launch_rows<KIND, 1, true, PAIR, DUMP>(ctx, p, smem);
+    if (np == 1) return launch_rows<KIND, 1, false, PAIR, DUMP>(ctx, p, smem);
+    if (np == 2) return launch_rows<KIND, 2, false, PAIR, DUMP>(ctx, p, smem);
+    if (np == 4) return launch_rows<KIND, 4, false, PAIR, DUMP>(ctx, p, smem);
+    return launch_rows<KIND, 8, false, PAIR, DUMP>(ctx, p, smem);
 }
 
 int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, const uint8_t* act_q8, int T, int K,
@@ -119,7 +119,7 @@ int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, con
         if (type == DC_TYPE_Q4_K) p.tiles4 = p.tiles;
     }
     const bool pair = epi == DC_EPI_SWIGLU;
-    const int np = dump_I ? 8 : T <= 2 ? 1 : T <= 4 ? 2 : T <= 8 ? 4 : 8;
+    const int np = T <= 2 ? 1 : T <= 4 ? 2 : T <= 8 ? 4 : 8;
     const size_t smem = rows_plan(p, np, q6, p.tiles, ctx->num_sms);
     if (!smem) {
         // activations of all T tokens do not fit beside the weight pipeline: run the tokens in two halves
@@ -135,8 +135,8 @@ int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, con
         return dc_launch_gemv(ctx, second, n_seg, epi, act_q8 + (size_t)T0 * (K / DC_QK_K) * DC_Q8F_BYTES, T - T0, K, nullptr, nullptr, nullptr,
                               act_f32 ? act_f32 + (size_t)T0 * K : nullptr, norm_w, norm_eps);
     }
-    // parity capture of the block sums: the same kernel compiled with the stores in (never in a decoder step)
-    if (dump_I) return q4 ? launch_rows<ROWS_Q4K, 8, false, false, true>(ctx, p, smem) : launch_rows<ROWS_Q6K, 8, false, false, true>(ctx, p, smem);
+    // parity capture of the block sums: the instance that serves so many tokens, compiled with the stores in (never in a decoder step)
+    if (dump_I) return q4 ? launch_rows_np<ROWS_Q4K, false, true>(ctx, p, np, smem) : launch_rows_np<ROWS_Q6K, false, true>(ctx, p, np, smem);
     if (pair) return q4 ? launch_rows_np<ROWS_Q4K, true>(ctx, p, np, smem) : launch_rows_np<ROWS_Q6K, true>(ctx, p, np, smem);
     if (q4 && q6) return launch_rows_np<ROWS_BOTH, false>(ctx, p, np, smem);
     return q4 ? launch_rows_np<ROWS_Q4K, false>(ctx, p, np, smem) : launch_rows_np<ROWS_Q6K, false>(ctx, p, np, smem);

@@ -39,6 +39,26 @@ def test_rows_are_the_cpu_kernels_bit_for_bit(ctx, oracle, t, N, K):
     W.free()
 
 
+@pytest.mark.parametrize("t", [B.GGML_TYPE_Q4_K, B.GGML_TYPE_Q6_K])
+def test_block_sums_of_every_instance(ctx, oracle, t):
+    """The exact integer sums of the instances that serve 1, 2, 3-4, 5-8 and 9-16 tokens, in groups of warps and alone."""
+    for N, K in ((37, 1280), (9000, 256)):
+        rng = np.random.default_rng(N + t)
+        w = B.random_weight(rng, t, N, K)
+        W = ctx.upload_weight(t, w, K, N)
+        x = rng.normal(size=(16, K)).astype(np.float32)
+        q8 = ctx.quantize_q8k(x).reshape(16, -1)
+        rows = np.unique(np.concatenate([np.arange(min(N, 37)), rng.integers(N, size=20), [N - 1]]))
+        want = [[oracle.block_sums(t, w.reshape(N, -1)[n], q8[m], K) for n in rows] for m in range(16)]
+        for M in (1, 2, 3, 4, 5, 8, 9, 16):
+            I, Mn = ctx.mul_mat_block_sums(W, x[:M])
+            for m in range(M):
+                assert np.array_equal(I[m][rows], np.stack([r[0] for r in want[m]])), (N, M, m)
+                if t == B.GGML_TYPE_Q4_K:
+                    assert np.array_equal(Mn[m][rows], np.stack([r[1] for r in want[m]])), (N, M, m)
+        W.free()
+
+
 @pytest.mark.parametrize("noalloc", [False, True])
 @pytest.mark.parametrize("t,n,M", [(B.GGML_TYPE_Q4_K, 512, 12), (B.GGML_TYPE_Q6_K, 1024, 6), (B.GGML_TYPE_Q4_K, 6144, 1), (B.GGML_TYPE_Q4_K, 1024, 7)])
 def test_product_in_place(ctx, t, n, M, noalloc):
