@@ -574,9 +574,9 @@ def test_decoder_two_streams_are_independent(ctx):
 
 def test_persistent_kernel_matches_per_op_kernels(ctx):
     """The persistent cooperative kernel and the per-op kernels compute the same step for 1, 2 and 4 streams.
-    Both use the same matmul bodies and rebuild the CPU kernel's running-maximum chain in attention; partial sums
-    meet in a different order in a few places (router logits, attention merge), so logits agree to float
-    rounding (1e-5 here, at short contexts) rather than bit for bit, and picked tokens agree."""
+    Their row products are different bodies with the CPU kernels' float order, and both rebuild the CPU kernel's running-maximum chain in
+    attention; in mode 0 partial sums meet in a different order in a few places (router logits, attention merge), so logits
+    agree to float rounding (1e-5 here, at short contexts) rather than bit for bit, and picked tokens agree."""
     cfg = tiny_cfg(True)
     cfg.max_seqs = 4
     m = dc.Model(ctx, cfg)

@@ -43,11 +43,14 @@ def test_contexts_on_two_gpus_in_one_process(oracle):
         m.finalize()
         s = m.seq_alloc()
         first = m.prefill(s, prompt)                                      # chunked prefill on the tensor cores
-        run, _ = m.decode_run([s], [first], 8)                            # persistent kernel
-        m.set_option("persistent", 0)
-        m.seq_truncate(s, prompt.size)
-        run2, _ = m.decode_run([s], [first], 8)                           # per-op kernels
-        assert np.array_equal(run, run2)
+        runs = {}
+        for mode in (2, 1, 0):                                            # persistent kernel, separate kernels in its order and in their own
+            m.set_option("persistent", mode)
+            runs[mode], _ = m.decode_run([s], [first], 8)
+            assert (m.step_stats()[0] == 1) == (mode == 2), "the persistent kernel serves mode 2 alone"
+            m.seq_truncate(s, prompt.size)
+        run = runs[2]
+        assert np.array_equal(run, runs[1]) and np.array_equal(run, runs[0])
         tokens.append([first] + [int(t) for t in run[:, 0]])
         m.close()
         W4.free()
