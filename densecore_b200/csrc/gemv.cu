@@ -95,7 +95,6 @@ int dc_launch_gemv(dc_ctx* ctx, const dc_gemv_seg* segs, int n_seg, int epi, con
     p.K = K;
     p.nb = K / DC_QK_K;
     p.argmax = argmax;
-    p.err = ctx->d_err;
     if (dump_I) {
         if (n_seg != 1 || epi != DC_EPI_STORE) return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "gemv: block-sum capture takes one plain segment");
         p.dump = BlockSumDump{dump_I, dump_M, segs[0].n_rows};

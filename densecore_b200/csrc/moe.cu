@@ -606,7 +606,6 @@ int dc_launch_moe_mm(dc_ctx* ctx, bool pair, const dc_weight* w0, const dc_weigh
     p.uoff = rt->uoff;
     p.uassign = rt->uassign;
     p.out = out;
-    p.err = ctx->d_err;
     // A kernel takes up to DC_MOE_PASS tokens of an expert; the few experts with more come several times over and are read again from
     // L2.  (Kernels for sixteen tokens an expert hold 255 registers, eight warps an SM: 259 us for 16 tokens of 8 out of 128 experts.)
     // act_rows: the passes that one CTA's neighbouring tiles touch are one more than its share of them, rounded up (a pass has 16 tiles at
@@ -666,10 +665,12 @@ int dc_launch_router(dc_ctx* ctx, const dc_weight* wr, const float* xn, int n_ex
 // T <= 4 and T*top_k <= 32 (cpu_backend_moe_ops.cpp:66,1247-1248,1578-1597),
 // otherwise ascending expert id (moe_routing.cpp:647-676).  Assignments whose
 // expert lives on another GPU are skipped (their share arrives by all-reduce).
-// The order in which a token's assignments are added up.
+// Whether a token's assignments are added up in routing order; else by ascending expert id.
+__device__ __forceinline__ bool combine_as_routed(int T, int top_k) { return T <= 4 && T * top_k <= 32; }
+// The order in which they are.
 __device__ __forceinline__ void combine_order(const int32_t* ids, int T, int top_k, int t, int (&order)[MOE_MAX_K]) {
     for (int k = 0; k < top_k; ++k) order[k] = k;
-    if (!(T <= 4 && T * top_k <= 32)) {
+    if (!combine_as_routed(T, top_k)) {
         for (int i = 1; i < top_k; ++i) {
             const int o = order[i], e = ids[t * top_k + o];
             int j = i - 1;
@@ -727,7 +728,7 @@ __global__ void __launch_bounds__(512) k_moe_combine_norm(const float* __restric
         const int own = ids[t * top_k + tid];
         const float w = weights[t * top_k + tid];
         int at = tid;
-        if (!(T <= 4 && T * top_k <= 32)) {
+        if (!combine_as_routed(T, top_k)) {
             at = 0;
             for (int k = 0; k < top_k; ++k) at += ids[t * top_k + k] < own;
         }
