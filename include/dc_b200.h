@@ -389,7 +389,8 @@ DC_B200_API int dc_b200_model_read_kv(dc_model* m, int layer, int seq, int first
  * attention on the tensor cores, 0 the decode kernels' exact running-maximum chain; "prefix_cache" 0/1.
  * "persistent" 0/1/2: decode steps of MoE models run in one persistent cooperative kernel with grid
  * barriers between phases: 0 never, 1 for one stream where that is the faster path (default: one stream of
- * an expert-parallel model), 2 for every stream count it supports (1-4). */
+ * an expert-parallel model, or with a block table too long for the one-kernel attention; the separate kernels
+ * that serve one stream elsewhere give the same results bit for bit), 2 for every stream count it supports (1-4). */
 DC_B200_API int dc_b200_model_set_option(dc_model* m, const char* name, int value);
 /* Prefix-cache counters of a model (option "prefix_cache" = 1 makes dc_b200_prefill and the scheduler use
  * the cache): {lookups, blocks hit, blocks resident, evictions, prompt tokens run through the decoder}. */
