@@ -6,6 +6,7 @@
 #include <cuda_profiler_api.h>
 
 #include <map>
+#include <set>
 #include <tuple>
 
 #include "dc_common.cuh"
@@ -51,6 +52,21 @@ static int kernel_setup(dc_ctx* ctx, const void* func, int max_dyn_smem, const c
 int dc_kernel_setup(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name) { return kernel_setup(ctx, func, max_dyn_smem, name, 0); }
 int dc_kernel_setup_small(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name) {
     return kernel_setup(ctx, func, max_dyn_smem, name, max_dyn_smem <= 50 * 1024 ? 45 : 0);
+}
+int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name) {
+    static std::mutex mu;
+    static std::set<const void*> good;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!good.count(func)) {
+            cudaFuncAttributes a;
+            const int st = dc_check_cuda(ctx, cudaFuncGetAttributes(&a, func), name);
+            if (st != DC_B200_OK) return st;
+            if (a.localSizeBytes) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "%s was built with %d bytes of spilled registers", name, (int)a.localSizeBytes);
+            good.insert(func);
+        }
+    }
+    return dc_kernel_setup(ctx, func, max_dyn_smem, name);
 }
 
 int dc_kernel_occupancy(dc_ctx* ctx, const void* func, int threads, size_t dyn_smem) {

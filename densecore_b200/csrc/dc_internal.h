@@ -56,6 +56,10 @@ int dc_check_device_error(dc_ctx* ctx);            // reads d_err after a sync
 int dc_kernel_setup(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name);
 // the same, asking for a split that leaves more than half of an SM's memory to L1: kernels of a decode step that overlap share one split
 int dc_kernel_setup_small(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name);
+// The same for a kernel that loads from tensor memory.  Such loads land in their registers some time after the instruction, and the code uses
+// others meanwhile.  A build that spills could store such a register too early and give it another use, which the load then overwrites: it may
+// not run.
+int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name);
 int dc_kernel_occupancy(dc_ctx* ctx, const void* func, int threads, size_t dyn_smem);
 
 // ---- launch helpers implemented in the kernel translation units ----

@@ -26,6 +26,12 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr, uint32_t sbo
     const uint32_t hi = ((sbo >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);      // version 1 (sm_100), SWIZZLE_128B
     return ((uint64_t)hi << 32) | lo;
 }
+// The same without a swizzle: core matrices of 8 rows x 16 bytes; lbo = byte distance between neighbours along K, sbo along the rows.
+__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    const uint32_t lo = ((saddr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16);
+    const uint32_t hi = ((sbo >> 4) & 0x3FFFu) | (1u << 14);
+    return ((uint64_t)hi << 32) | lo;
+}
 // 16 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16]) {
     asm volatile(
@@ -42,6 +48,15 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
                  : "r"(taddr)
                  : "memory");
 }
+// 16 consecutive 32-bit columns of this thread's TMEM lane are stored (visible to a product after tmem_st_wait and a fence).
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+        "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+        "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // The same with the loaded registers named, so that no use of them moves ahead of the wait.
 __device__ __forceinline__ void tmem_ld_wait(int (&v)[16]) {
@@ -50,6 +65,42 @@ __device__ __forceinline__ void tmem_ld_wait(int (&v)[16]) {
                    "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
                  :
                  : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait(int (&v)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+                 :
+                 : "memory");
+}
+// Names eight more registers of loads that a wait has completed.
+__device__ __forceinline__ void tmem_loaded(int (&v)[8]) {
+    asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]) : : "memory");
+}
+// One lane of a converged warp.  Code that issues products, commits and bulk copies stays in step as a whole warp and lets this lane issue:
+// measured, eight products with a commit and three waits take 419 cycles so, and 968 where a branch on the lane number encloses the loop.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(p));
+    return p != 0;
+}
+// Bounded wait of a converged warp, in as few instructions as it takes: all lanes go on or none does.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+    uint32_t left;
+    asm volatile(
+        "{\n .reg .pred P;\n mov.u32 %0, %3;\n"
+        "WAIT:\n mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n @P bra GO;\n add.u32 %0, %0, -1;\n setp.ne.u32 P, %0, 0;\n @P bra WAIT;\n"
+        "GO:\n}"
+        : "=&r"(left)
+        : "r"(bar), "r"(parity), "n"(DC_WAIT_LIMIT)
+        : "memory");
+    return __all_sync(0xffffffffu, left != 0);
+}
+// The same, telling the CTA's other waits if the limit ran out.
+__device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity, volatile int* give_up, int* err) {
+    if (mbar_wait_warp(bar, parity)) return true;
+    *give_up = 1;
+    if (err) atomicExch(err, DC_ERR_MBAR_TIMEOUT);
+    return false;
 }
 // Bounded wait that also watches the CTA's give-up flag.
 __device__ __forceinline__ bool tc_wait_raw(uint32_t bar, uint32_t parity, volatile int* give_up, int* err) {
@@ -71,7 +122,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, int x
         "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
-// D[M x N] (+)= A[M x 16] * B[16 x N], bf16 operands from shared memory, f32 accumulators in TMEM.
+// D[M x N] (+)= A[M x 16] * B[16 x N], 16-bit operands from shared memory, f32 accumulators in TMEM.
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -79,6 +130,16 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with A in tensor memory: lane = row, a 32-bit column = two neighbours along K.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Instruction descriptor: f32 accumulate, both operands f16 and K-major.
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
 // Instruction descriptor: f32 accumulate, both operands bf16 and K-major.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);

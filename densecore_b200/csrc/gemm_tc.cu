@@ -1,29 +1,23 @@
 // Batched MUL_MAT for prompt chunks (M >= 32 token rows): K-quant weights x Q8_K activations on the
-// 5th-generation tensor cores (tcgen05.mma kind::i8, accumulators in tensor memory), with the block sums
-// kept as exact integers so that the float steps per 256-value block are the CPU kernels' own
+// 5th-generation tensor cores, with block sums that are exact integers, so that the float steps per 256-value
+// block are the CPU kernels' own
 // (core/src/llm/matmul/batched_exec.cpp:1040-1240 serves these shapes on the CPU; per block
 // sumf += (d*yd)*float(I); sumf -= (dmin*yd)*float(M), core/src/kernels/hwy/hwy_moe_quant.cc:248-253).
 //
-// One CTA per SM walks work items of 128 weight rows x two 64-token tiles over the whole reduction length; its
-// warps split the three jobs of a 256-value block and overlap them, across items too (see k_gemm_tc below):
-//   1. expanders turn the raw quants of the 128 rows into 8-bit operand planes in shared memory, K-major rows
-//      of 128 bytes with the 128-byte swizzle the tensor core reads at full rate (a half block is exactly one
-//      such row):
-//        Q4_K: q4 * (sc >> 3) and q4 * (sc & 7) (2 planes, unsigned), so that I = 8 * acc0 + acc1 =
-//              sum sc_j * sum q4*q8; the minimum term M = sum m_j * (sum of the token's codes in sub-block j)
-//              needs no contraction over the values: the read-out warps form it from the eight sub-block sums
-//              that the activation tile carries per token (four two-way 16 x 8-bit dot instructions);
-//        Q6_K: sign(sc) * digit_i(|sc|) * (q6 - 32) for the four base-4 digits of |sc| (4 planes, signed),
-//              so that I = acc0 + 4 acc1 + 16 acc2 + 64 acc3;
-//      every plane entry fits 8 bits and the 32-bit accumulators are exact;
-//   2. one thread issues the UMMAs (128 rows x 128 tokens x 32 values each), two halves of 128 values per block;
-//   3. read-out warps fetch the accumulators (tcgen05.ld) and add the block's float terms in block order.
-// Q4_K's two planes x 128 token columns fit the 512 columns of tensor memory twice, so its accumulators are
-// double-buffered and the UMMAs of a block run while the block before is read out; Q6_K's four planes fit once.
-// The token side is prepared once per activation matrix by k_quantize_q8k_tiled: the Q8_K codes of every
-// (block, 64-token tile) stored as the B operand (two halves of 64 swizzled 128-byte rows), followed by the
-// 64 block scales and the tokens' sub-block sums, so that a tile half is one contiguous bulk copy.  No multicast
-// load anywhere.
+// The products are tcgen05.mma kind::f16 on whole numbers: a code times its sub-block's scale is one that fp16 holds exactly, so are the
+// activation codes, and a sum of products that stays below 2^24 is exact in the f32 accumulator.  So the read-out gets floats:
+//   Q4_K: q4 * sc (<= 945); the two halves of a block have an accumulator each (|sum| <= 945 * 127 * 128 < 2^24), whose sum rounds once: float(I).
+//         The minimum term M = sum m_j * (sum of the token's codes in sub-block j) is one more product, of length 16: the minima (each twice) times the
+//         sums of the token's codes over 16 values (<= 2048, exact), |M| <= 63 * 127 * 256.
+//   Q6_K: q6 - 32 = (ql - 8) + 8 (2 qh - 3): sc (ql - 8) (<= 1024) with an accumulator for each half (<= 1024 * 128 * 128 = 2^24), and
+//         8 sc (2 qh - 3) with one for the block, whose sums are multiples of 8 and stay below 2^27.  float(I) = the sum of the three; only where
+//         the halves' sum passes 2^24 does it round twice.
+// The weight operand lies in tensor memory (lane = row, 32 columns a quarter block, four slots), where its expander threads store it; only the
+// activations take the way through shared memory, whose 128 bytes a cycle an operand of 128 rows from there would fill alone.
+//
+// One CTA per SM walks work items of 128 weight rows x two 64-token tiles over the whole reduction length, see k_gemm_tc below.
+// The token side is prepared once per activation matrix by k_quantize_q8k_tiled (layout: dc_gemm_tc.h), so that every piece is a contiguous
+// bulk copy.  No multicast load anywhere.
 //
 // Q4_K results are bit-equal to the GEMV path and the CPU oracle.  Q6_K adds one float term per block
 // instead of the CPU small-batch kernel's eight lane partials (q6_small_batch.h:62-103): equal integers,
@@ -35,6 +29,7 @@
 #include "dc_common.cuh"
 #include "dc_gemm_tc.h"
 #include "dc_internal.h"
+#include "dc_launch.cuh"
 #include "dc_tcgen05.cuh"
 
 #define DC_TRY(expr)                       \
@@ -46,7 +41,6 @@
 namespace dc {
 
 constexpr int TC_ROWS = 128;
-constexpr int TC_PLANE = TC_ROWS * 128;               // one operand plane of a half block: 128 rows of 128 bytes
 
 struct GemmTcSeg {
     const uint8_t* w;      // rows of the matrix (expert 0)
@@ -69,24 +63,14 @@ struct GemmTcParams {
     const int* pair_tile0;    // optional [grid.x]: first tile of the CTA's pair of neighbouring tiles (< 0: none) ...
     const int* pair_nset;     // ... and how many tiles of the pair exist (1 or 2); without it CTA i owns tiles 2i, 2i + 1
     int accumulate;           // out += result (one float add) instead of out = result
+    float one;                // 1, which the compiler must not know (see fma2_rn)
     int tiles_x, tiles_y;     // work items: token-tile pairs x row tiles (of all matrices of the launch)
     int* err;
 };
 
-// D[128 x N] (+)= A[128 x 32] * B[32 x N], 8-bit operands from shared memory, int32 accumulators in TMEM.
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Instruction descriptor: int32 accumulate, A unsigned or signed 8-bit, B signed 8-bit, both K-major.
-__host__ __device__ constexpr uint32_t umma_idesc_i8(int a_signed, int M, int N) {
-    return (2u << 4) | ((uint32_t)a_signed << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-// Packed single precision (two lanes per instruction), each lane rounded to nearest like the scalar
-// instruction, never contracted with a neighbouring operation.
+// Packed single precision (two lanes per instruction), each lane rounded to nearest like the scalar instruction.  An addition behind a
+// multiplication is written as fma2_rn(product, one, sum) with a `one` from the kernel's parameters: a packed add there was seen to round
+// once, as if fused with the multiplication.
 __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
     float2 r;
     asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n mul.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}"
@@ -120,6 +104,7 @@ __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint3
 __global__ void __launch_bounds__(256) k_quantize_q8k_tiled(const float* __restrict__ x, int ldx, int n_rows, int K,
                                                             uint8_t* __restrict__ act, int n_tt,
                                                             const int* __restrict__ slot_token) {
+    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = K / DC_QK_K;
     const long long total = (long long)n_tt * TC_NTOK * nb;
@@ -141,69 +126,40 @@ __global__ void __launch_bounds__(256) k_quantize_q8k_tiled(const float* __restr
     }
 }
 
-// ---- weight side ---------------------------------------------------------------------------------------
-template <int TYPE>
-struct TcTraits;
-template <>
-struct TcTraits<DC_TYPE_Q4_K> {
-    // two operand planes and two sets of accumulators (the minimum term comes from the tokens' sub-block sums)
-    static constexpr int NP = 2, NSET = 2, BB = DC_Q4K_BYTES, A_SIGNED = 0, TAIL_COPY = TC_ACT_TAIL;
-    static constexpr int RO_TOK = 32;         // tokens per read-out warp: 16 read-out warps, four per scheduler
-    static constexpr int A_STAGES = 2;        // half blocks of operand planes in shared memory
-};
-template <>
-struct TcTraits<DC_TYPE_Q6_K> {
-    static constexpr int NP = 4, NSET = 1, BB = DC_Q6K_BYTES, A_SIGNED = 1, TAIL_COPY = TC_ACT_SCALES;
-    static constexpr int RO_TOK = 32;
-    static constexpr int A_STAGES = 2;
-};
+// ---- the kernel -----------------------------------------------------------------------------------------
+// The three jobs of a block (expanding the weight operand, issuing products, reading the accumulators out) run on different warps of one CTA per
+// SM and overlap.  A work item is 128 rows x two 64-token tiles; the CTA walks its items round robin, and every ring slot and barrier phase is
+// picked by the number of the block, which runs on across items, so an item's first blocks are expanded while the item before is read out.
+//   warps 0-7    expanders: thread r of four warps turns its row's quarter block into the 32 columns of an operand slot.  Q4_K: either four take
+//                every second quarter, expanded in registers before the slot is free; Q6_K: the lower four bits, the upper two
+//   warps 8-23   read-out: warp w owns TMEM lane quarter w % 4 and sixteen tokens of either tile
+//   warps 24, 25 issue the products
+//   warp 26      loads the token tiles (three blocks ahead)
+// Tensor memory: two sets of three 64-column accumulators, one per token tile (a lone tile takes them in turn), so that one is read out while the
+// other's products run, and the four operand slots.
+// What bounds it: the chain of a block (operand slot free, stored, multiplied, read out, accumulators free), each hand-over 150 to 400 cycles, while every SM
+// sub-partition is about half busy (packed multiply-adds of the read-out, expansion); without the read-out's work a block takes 10 % less, without the
+// expansion's 16 %, without either 28 %.  Measured, us, against the int8 form of this kernel (operands in shared memory, 13 instead of 4 instructions per element
+// and block in the read-out): Q4_K 4096 x 2048 by 1531 tokens 69 -> 47, Q6_K 113 -> 89; Q4_K 2048 x 4096 by 300 tokens 44 -> 29, 2048 x 768 by 64 11 -> 8.  Tried:
+// accumulators of 128 tokens (one set only, 63 us); eight read-out warps, or four expanders (61); one issuing warp (48); operand slots of half a block (60).
+constexpr int TC_EXPANDERS = 8, TC_READERS = 16;
+constexpr int TC_WARP_MMA = TC_EXPANDERS + TC_READERS;
+constexpr int TC_THREADS = (TC_WARP_MMA + 4) * 32;         // (the last warp only gives its registers)
+constexpr int TC_READ_REGS = 80, TC_REST_REGS = 40;        // 256 x 72 + 512 x 80 + 128 x 40 = 896 x 72, the launch's
+constexpr int TC_B_STAGES = 3;
+constexpr uint32_t TC_SET = 3 * TC_NTOK;                   // columns of a set of accumulators
+constexpr uint32_t TC_COL_A = 2 * TC_SET;                  // first operand column
 
-// ---- the kernel: the three jobs of a block (expanding operand planes, issuing UMMAs, reading the accumulators
-// out) run on different warps of one CTA per SM and overlap.  A work item is 128 rows x two 64-token tiles, so
-// that a block's planes are expanded once for 128 tokens and every UMMA is 128 tokens wide (a stand-alone loop
-// runs the instruction in 49 cycles at N = 64 and 65 at N = 128); the CTA walks its items round robin.
-//   warps 0-3   expanders: thread r turns its row's half block into the planes of a stage (two stages)
-//   warp 4      one thread issues the UMMAs (stage x 128 tokens -> accumulators in TMEM), commits
-//               "stage free", "token codes free" and "accumulators full"
-//   warp 5      one thread loads the token tiles (codes double-buffered, interleaved so that the two tiles
-//               form one 128-row operand; block scales and sub-block sums in a ring of four)
-//   warps 6-21  read-out: warp w owns TMEM lane quarter w % 4 and tokens 32 ((w - 6) / 4) .. + 31: adds the
-//               block's float terms for its row, then frees the accumulators
-// Q4_K: two sets of accumulators (2 planes x 128 columns each) alternate by block.  Q6_K: one set (4 planes x 128
-// columns of the 512): the UMMAs of the next block wait for the read-out, the expansion does not.  Every wait is
-// bounded and watches a CTA-wide give-up flag.
-template <int TYPE>
-constexpr int tc_threads() {
-    return (6 + 4 * (128 / TcTraits<TYPE>::RO_TOK)) * 32;
-}
-constexpr int TC_EXPAND = 128;
-constexpr int TC_N = 128;                  // tokens per CTA
+// mbarriers of the kernel, as indexes from the first one
+enum TcBar { A_FULL = 0, A_FREE = 4, B_FULL = 8, B_FREE = 11, S_FULL = 14, D_FULL = 22, ACC_FULL = 26, ACC_FREE = 28, DRAIN = 30, TC_NBARS = 32 };
 
-// mbarriers of the kernel, as word offsets from the first one (addresses are computed, not looked up: several are
-// indexed with run-time values)
-enum TcBar { A_FULL = 0, A_FREE = 4, B_FULL = 8, B_FREE = 10, S_FULL = 12, D_FULL = 16, ACC_FULL = 20, ACC_FREE = 22, TC_NBARS = 24 };
-
-#ifdef DC_TC_TIMING
-// instrumented build: cycles one thread of every role spends in each kind of wait, summed over CTAs
-// 0 a_free (expander)  1 b_full  2 a_full  3 acc_free (issuer)  4 b_free (loader)  5 d/s_full  6 acc_full (read-out)
-// 7 whole kernel (thread 0)
-__device__ unsigned long long g_tc_wait[8];
-__device__ __forceinline__ bool tc_wait_k(int kind, uint32_t bar, uint32_t parity, volatile int* give_up, int* err) {
-    const long long t0 = clock64();
-    const bool ok = tc_wait_raw(bar, parity, give_up, err);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&g_tc_wait[kind], (unsigned long long)(clock64() - t0));
-    return ok;
-}
-#else
-#define tc_wait_k(kind, bar, parity, give_up, err) tc_wait_raw(bar, parity, give_up, err)
-#endif
-template <int TYPE>
-constexpr size_t tc_smem_bytes() {
-    using T = TcTraits<TYPE>;
-    // planes: 2 stages; token codes: 2 buffers x 2 tiles; tile tails (block scales, sub-block sums): 4 x 2 tiles;
-    // row constants: 4 x 128 x 16 bytes; 1024 bytes of slack to start the swizzled tiles on a 1024-byte boundary
-    return (size_t)T::A_STAGES * T::NP * TC_PLANE + (size_t)4 * TC_B_Q + 4 * 2 * TC_ACT_TAIL + 4 * 128 * 16 + 384 + 1024;
-}
+constexpr uint32_t TC_TILE = TC_B_Q + 2 * TC_SUM_HALF;                     // a token tile without its scales
+constexpr uint32_t TC_SB = 0;                                              // [3][two tiles]
+constexpr uint32_t TC_SM = TC_SB + TC_B_STAGES * 2 * TC_TILE;              // the rows' minima as an operand: [half][row][16 bytes]
+constexpr uint32_t TC_SSC = TC_SM + 4096;                                  // [8][two tiles] block scales
+constexpr uint32_t TC_SD = TC_SSC + 8 * 2 * TC_ACT_SCALES;                 // [4][128] d, -dmin of the rows
+constexpr uint32_t TC_SBAR = TC_SD + 4 * 128 * 8;
+constexpr size_t TC_SMEM = TC_SBAR + TC_NBARS * 8 + 16 + 1024;             // the swizzled tiles start on a 1024-byte boundary
 
 struct TcTile {       // one work item: 128 rows of one matrix x a pair of neighbouring 64-token tiles of one expert
     bool live;
@@ -237,377 +193,458 @@ __device__ __forceinline__ TcTile tc_tile_at(const GemmTcParams& p, int t) {
     return ti;
 }
 
-template <int TYPE>
-__global__ void __launch_bounds__(tc_threads<TYPE>(), 1) k_gemm_tc(GemmTcParams p) {
-    using T = TcTraits<TYPE>;
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    __shared__ int s_give_up;
-    const uint32_t sA = (smem_u32(smem_raw) + 1023u) & ~1023u;   // [A_STAGES][NP planes][16 KB], swizzle-aligned
-    const uint32_t sBq = sA + T::A_STAGES * T::NP * TC_PLANE;    // [2 buffers][2 halves][2 tiles][8 KB]
-    const uint32_t sS = sBq + 4 * TC_B_Q;                        // [4][2 tiles] tails: 64 block scales, 64 x 8 sub-block sums
-    const uint32_t sD = sS + 4 * 2 * TC_ACT_TAIL;                // [4][128] d, dmin, the eight sub-block minima of the rows
-    const uint32_t sBar = sD + 4 * 128 * 16;
-    auto bar = [sBar](int which, int i) -> uint32_t { return sBar + 8u * (uint32_t)(which + i); };
-    const uint32_t tmem_slot = sBar + TC_NBARS * 8;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nb = p.K / DC_QK_K, total = p.tiles_x * p.tiles_y;
-    constexpr uint32_t NCOLS = 512;
-    constexpr int RO_THREADS = 4 * (128 / T::RO_TOK) * 32;
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+__device__ __forceinline__ __half2 h2_of(float x) { return __float2half2_rn(x); }
 
-    if (warp == 4) {
-        tmem_alloc(tmem_slot, NCOLS);
+// 4 x 8 nibbles of a Q4_K row -> 16 operand columns.  0x6400 + n are the bits of 1024 + n, and (1024 + n) * s - 1024 * s is n * s exactly in one
+// fused multiply-add (s <= 63; high nibbles stay in place: (1024 + 16 n) * (s / 16) - 64 s).
+struct Q4Scale {
+    __half2 s, n, s16, n16;      // of the low nibbles' sub-block: s, -1024 s; of the high nibbles': s / 16, -64 s
+    __device__ __forceinline__ void set(uint32_t scw) {      // the scales in the lower two bytes
+        const __half2 k = h2_of(-1024.0f);
+        const __half2 lo = __hadd2(bits_h2(__byte_perm(scw, 0x64u, 0x4040)), k), hi = __hadd2(bits_h2(__byte_perm(scw, 0x64u, 0x4141)), k);
+        s = lo;
+        n = __hmul2(lo, k);
+        s16 = __hmul2(hi, h2_of(0.0625f));
+        n16 = __hmul2(hi, h2_of(-64.0f));
+    }
+};
+__device__ __forceinline__ void q4_columns(uint4 q, const Q4Scale& c, uint32_t (&v)[16]) {
+    const uint32_t in[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t w = in[k], w8 = w >> 8;
+        v[4 * k] = h2_bits(__hfma2(bits_h2((w & 0x000F000Fu) | 0x64006400u), c.s, c.n));
+        v[4 * k + 1] = h2_bits(__hfma2(bits_h2((w8 & 0x000F000Fu) | 0x64006400u), c.s, c.n));
+        v[4 * k + 2] = h2_bits(__hfma2(bits_h2((w & 0x00F000F0u) | 0x64006400u), c.s16, c.n16));
+        v[4 * k + 3] = h2_bits(__hfma2(bits_h2((w8 & 0x00F000F0u) | 0x64006400u), c.s16, c.n16));
+    }
+}
+// Eight words of either 32-value run of a quarter (`second`: the later quarter of a half block), four at a time: w the words of the first run,
+// x of the second, with 16-value scales s0 and s1 -> 16 columns of sc (ql - 8); nibbles stay in place.
+__device__ __forceinline__ void q6_low_columns(const uint32_t* w, const uint32_t* x, float s0, float s1, bool second, uint32_t (&v)[16]) {
+    const __half2 f0 = h2_of(second ? s0 * 0.0625f : s0), f1 = h2_of(second ? s1 * 0.0625f : s1), k = h2_of(second ? -1152.0f : -1032.0f);
+    const uint32_t m = second ? 0x00F000F0u : 0x000F000Fu;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        v[4 * i] = h2_bits(__hmul2(__hadd2(bits_h2((w[i] & m) | 0x64006400u), k), f0));
+        v[4 * i + 1] = h2_bits(__hmul2(__hadd2(bits_h2(((w[i] >> 8) & m) | 0x64006400u), k), f0));
+        v[4 * i + 2] = h2_bits(__hmul2(__hadd2(bits_h2((x[i] & m) | 0x64006400u), k), f1));
+        v[4 * i + 3] = h2_bits(__hmul2(__hadd2(bits_h2(((x[i] >> 8) & m) | 0x64006400u), k), f1));
+    }
+}
+// The same of 8 sc (2 qh - 3).  The two bits of quadrant i of a half block lie at bits 2 i of a byte: u (2 qh - 3) with u = 1 << (2 i - 1) (quadrant 0
+// moved up a bit) after the bias 1024 + 3 u, then times 8 sc / u.
+__device__ __forceinline__ void q6_high_columns(const uint32_t* w, float s0, float s1, bool second, uint32_t (&v)[16]) {
+    const __half2 k0 = h2_of(second ? -1048.0f : -1027.0f), k1 = h2_of(second ? -1120.0f : -1030.0f);
+    const __half2 f0 = h2_of(second ? s0 : 8.0f * s0), f1 = h2_of(second ? 0.25f * s1 : 4.0f * s1);
+    const uint32_t m0 = second ? 0x00300030u : 0x00060006u, m1 = second ? 0x00C000C0u : 0x000C000Cu;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t a = second ? w[i] : w[i] << 1, a8 = second ? w[i] >> 8 : w[i] >> 7;
+        v[4 * i] = h2_bits(__hmul2(__hadd2(bits_h2((a & m0) | 0x64006400u), k0), f0));
+        v[4 * i + 1] = h2_bits(__hmul2(__hadd2(bits_h2((a8 & m0) | 0x64006400u), k0), f0));
+        v[4 * i + 2] = h2_bits(__hmul2(__hadd2(bits_h2((w[i] & m1) | 0x64006400u), k1), f1));
+        v[4 * i + 3] = h2_bits(__hmul2(__hadd2(bits_h2(((w[i] >> 8) & m1) | 0x64006400u), k1), f1));
+    }
+}
+
+template <int TYPE>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const GemmTcParams p) {
+    constexpr bool Q4 = TYPE == DC_TYPE_Q4_K;
+    constexpr int BB = Q4 ? DC_Q4K_BYTES : DC_Q6K_BYTES;
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    __shared__ uint32_t s_tmem;
+    const uint32_t sm = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    auto bar = [sm](int which, int i = 0) -> uint32_t { return sm + TC_SBAR + 8u * (uint32_t)(which + i); };
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int nb = p.K / DC_QK_K, total = p.tiles_x * p.tiles_y;
+
+    if (warp == TC_WARP_MMA) {
+        tmem_alloc(smem_u32(&s_tmem), 512);
         tmem_relinquish();
     }
     if (tid == 0) {
-        s_give_up = 0;
-        for (int i = 0; i < 4; ++i) {
-            mbar_init(bar(A_FULL, i), TC_EXPAND);
-            mbar_init(bar(A_FREE, i), 1);
-            mbar_init(bar(S_FULL, i), 1);
-            mbar_init(bar(D_FULL, i), TC_EXPAND);
-        }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(bar(B_FULL, i), 1);
-            mbar_init(bar(B_FREE, i), 1);
-            mbar_init(bar(ACC_FULL, i), 1);
-            mbar_init(bar(ACC_FREE, i), RO_THREADS);   // every read-out thread arrives, with or without tokens of its own
-        }
+        for (int i = 0; i < TC_NBARS; ++i) mbar_init(bar(i), i < A_FREE || (i >= D_FULL && i < ACC_FULL) ? 4 : i >= ACC_FREE && i < DRAIN ? TC_READERS : (i >= B_FREE && i < S_FULL) || (i >= ACC_FULL && i < ACC_FREE) ? 2 : 1);
         mbar_fence_init();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = lds32(tmem_slot);
-    volatile int* give_up = &s_give_up;
-#ifdef DC_TC_TIMING
-    const long long t_kernel0 = clock64();
-#endif
-    // Every role walks the same list of tiles (this CTA's share, round robin) and counts 256-value blocks across
-    // tiles: g = blocks before this tile + block index picks ring slots, accumulator sets and barrier phases, so
-    // the expansion of a tile's first blocks overlaps the read-out and the stores of the tile before.
-
-    if (warp < 4) {
+    const uint32_t tmem = s_tmem;
+    pdl_wait();      // (the set-up above overlaps the quantiser's end)
+    auto wait = [](uint32_t b, uint32_t parity) { return mbar_wait_warp(b, parity); };
+    // Every role walks the same list of items (this CTA's share, round robin) and counts blocks across them (g).  Why no slot is overwritten too
+    // early: products of block g run only when the read-out has released the last block of that set of accumulators, g - 1 or, in a lone tile, g - 2,
+    // behind its last reads of that block's d, dmin and scales.  Row constants of block g are stored behind products of g - 1, so those
+    // of g - 3 and before are free: a ring of four.  Scales of block g are loaded behind products of g - 3: those of g - 5 and before are free: a ring of eight.
+    if (warp < TC_EXPANDERS) {
         // ------------------------------------------------------------------ expanders
-        const int r = tid;
-        int g0 = 0;
+        const int r = tid & 127, grp = warp >> 2;
+        const uint32_t t_a = tmem + TC_COL_A + ((uint32_t)(32 * (warp & 3)) << 16);
+        auto filled = [&](int slot) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(A_FULL, slot));
+        };
+        int g = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x) {
             const TcTile ti = tc_tile_at(p, t);
             if (!ti.live) continue;
             const uint8_t* rp = ti.wbase + (size_t)min(ti.row0 + r, ti.N - 1) * p.row_bytes;
-            if (TYPE == DC_TYPE_Q4_K) {
-                // the raw quants of a half block (header + 64 bytes) are requested two halves ahead of their expansion:
-                // one half of expansion work is shorter than a round trip to memory
-                struct HalfRaw { uint4 hdr, q[4]; };
-                HalfRaw n1, n2;
-                auto fetch = [&](HalfRaw& f, int idx) {
-                    const uint4* b = reinterpret_cast<const uint4*>(rp + (size_t)(idx >> 1) * T::BB);
-                    f.hdr = __ldg(b);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) f.q[i] = __ldg(b + 1 + 4 * (idx & 1) + i);
-                };
-                fetch(n1, 0);
-                fetch(n2, 1);
-                for (int kb = 0; kb < nb; ++kb) {
-                    const int g = g0 + kb;
+            if constexpr (Q4) {
+                // this warp's quarters of a block: grp and grp + 2; a quarter's raw quants are requested one turn ahead
+                const uint4* b = reinterpret_cast<const uint4*>(rp);
+                const uint4* from = b + 1 + 2 * grp;
+                uint4 H = __ldg(b), q0 = __ldg(from), q1 = __ldg(from + 1);
 #pragma unroll 1
-                    for (int h = 0; h < 2; ++h) {
-                        const uint4 H = n1.hdr;
-                        uint4 Q[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) Q[i] = n1.q[i];
-                        n1 = n2;
-                        if (2 * kb + h + 2 < 2 * nb) fetch(n2, 2 * kb + h + 2);
-                        const int hg = 2 * g + h, stg = hg % T::A_STAGES, use = hg / T::A_STAGES;   // stage of this half, its use count
-                        if (use > 0 && !tc_wait_k(0, bar(A_FREE, stg), (use - 1) & 1, give_up, p.err)) goto done;
-                        // the 6-bit scales and minima of the eight sub-blocks, four to a word (get_scale_min_k4 of ggml's
-                        // K-quants on packed bytes)
-                        const uint32_t scw = h ? ((H.w & 0x0F0F0F0Fu) | (((H.y >> 6) & 0x03030303u) << 4)) : (H.y & 0x3F3F3F3Fu);
-                        if (h == 0) {
-                            // this row's scales and minima for the read-out warps (the minima negated: the read-out
-                            // subtracts their term)
-                            const uint32_t mA = __vneg4(H.z & 0x3F3F3F3Fu),
-                                           mB = __vneg4(((H.w >> 4) & 0x0F0F0F0Fu) | (((H.z >> 6) & 0x03030303u) << 4));
-                            sts128(sD + ((g & 3) * 128 + r) * 16, __float_as_uint(fp16_bits_to_float((uint16_t)(H.x & 0xFFFF))),
-                                   __float_as_uint(fp16_bits_to_float((uint16_t)(H.x >> 16))), mA, mB);
-                            mbar_arrive(bar(D_FULL, g & 3));
-                        }
-                        // row r of the stage's planes; chunk c of the row goes to chunk position c ^ (r % 8)
-                        const uint32_t stage = sA + stg * (T::NP * TC_PLANE) + (r >> 3) * 1024 + (r & 7) * 128;
-                        const uint32_t rx = (uint32_t)(r & 7);
-#pragma unroll
-                        for (int gl = 0; gl < 2; ++gl) {          // sub-blocks 4h + 2gl (low nibbles) and 4h + 2gl + 1 (high nibbles)
-                            const uint32_t sc0 = (scw >> (16 * gl)) & 0xFFu, sc1 = (scw >> (16 * gl + 8)) & 0xFFu;
-                            const uint32_t a0 = sc0 >> 3, a1 = sc0 & 7u, b0 = sc1 >> 3, b1 = sc1 & 7u;
-#pragma unroll
-                            for (int hf = 0; hf < 2; ++hf) {
-                                const uint4 qv = Q[2 * gl + hf];
-                                const uint32_t in[4] = {qv.x, qv.y, qv.z, qv.w};
-                                uint32_t lo[4], hi[4];
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    lo[k] = in[k] & 0x0F0F0F0Fu;
-                                    hi[k] = (in[k] >> 4) & 0x0F0F0F0Fu;
-                                }
-                                const uint32_t c_lo = stage + (((uint32_t)(4 * gl + hf) ^ rx) << 4);
-                                const uint32_t c_hi = stage + (((uint32_t)(4 * gl + hf + 2) ^ rx) << 4);
-                                sts128(c_lo, lo[0] * a0, lo[1] * a0, lo[2] * a0, lo[3] * a0);
-                                sts128(c_lo + TC_PLANE, lo[0] * a1, lo[1] * a1, lo[2] * a1, lo[3] * a1);
-                                sts128(c_hi, hi[0] * b0, hi[1] * b0, hi[2] * b0, hi[3] * b0);
-                                sts128(c_hi + TC_PLANE, hi[0] * b1, hi[1] * b1, hi[2] * b1, hi[3] * b1);
-                            }
-                        }
-                        fence_async_smem();
-                        mbar_arrive(bar(A_FULL, stg));
+                for (int i = 0; i < 2 * nb; ++i) {
+                    const int j = i & 1, slot = grp + 2 * j;
+                    // the 6-bit scales of sub-blocks 4 j .. 4 j + 3, four to a word (get_scale_min_k4 of ggml's K-quants on packed bytes)
+                    const uint32_t scw = j ? ((H.w & 0x0F0F0F0Fu) | (((H.y >> 6) & 0x03030303u) << 4)) : (H.y & 0x3F3F3F3Fu);
+                    Q4Scale sc;
+                    sc.set(scw >> (16 * grp));
+                    uint32_t v[2][16];
+                    q4_columns(q0, sc, v[0]);
+                    q4_columns(q1, sc, v[1]);
+                    const bool more = i + 1 < 2 * nb;
+                    from += j ? 5 : 4;
+                    if (more) {
+                        q0 = __ldg(from);
+                        q1 = __ldg(from + 1);
                     }
+                    if (!wait(bar(A_FREE, slot), (g & 1) ^ 1)) goto gave_up;      // (the first passes)
+                    tc_fence_after();
+                    tmem_st16(t_a + 32 * slot, v[0]);
+                    tmem_st16(t_a + 32 * slot + 16, v[1]);
+                    if (!j && grp == 0) {
+                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sm + TC_SD + ((g & 3) * 128 + r) * 8), "f"(fp16_bits_to_float((uint16_t)(H.x & 0xFFFF))),
+                                     "f"(-fp16_bits_to_float((uint16_t)(H.x >> 16)))
+                                     : "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar(D_FULL, g & 3));
+                    }
+                    if (j) {
+                        if (grp == 1) {
+                            // minima of sub-blocks 0..3, 4..7 as pairs of equal fp16 numbers (the product that read the last ones is done, as the slot's is)
+                            const uint32_t mw[2] = {H.z & 0x3F3F3F3Fu, ((H.w >> 4) & 0x0F0F0F0Fu) | (((H.z >> 6) & 0x03030303u) << 4)};
+                            const __half2 k = h2_of(-1024.0f);
+#pragma unroll
+                            for (int n = 0; n < 2; ++n)
+                                sts128(sm + TC_SM + n * 2048 + (r >> 3) * 128 + (r & 7) * 16, h2_bits(__hadd2(bits_h2(__byte_perm(mw[n], 0x64u, 0x4040)), k)),
+                                       h2_bits(__hadd2(bits_h2(__byte_perm(mw[n], 0x64u, 0x4141)), k)), h2_bits(__hadd2(bits_h2(__byte_perm(mw[n], 0x64u, 0x4242)), k)),
+                                       h2_bits(__hadd2(bits_h2(__byte_perm(mw[n], 0x64u, 0x4343)), k)));
+                            fence_async_smem();
+                        }
+                        ++g;
+                        b += 9;
+                        if (more) H = __ldg(b);
+                    }
+                    filled(slot);
                 }
             } else {
-                // Q6_K: 210-byte blocks at 2-byte aligned addresses: aligned 32-bit loads and a funnel shift
-                uint32_t wl[17], wh[9], ws[3], wd = 0;
-                auto fetch = [&](int kb, int h) {
-                    const uintptr_t a = (uintptr_t)(rp + (size_t)kb * T::BB);
-                    const uint32_t* bl = reinterpret_cast<const uint32_t*>((a + 64 * h) & ~(uintptr_t)3);
-                    const uint32_t* bh = reinterpret_cast<const uint32_t*>((a + 128 + 32 * h) & ~(uintptr_t)3);
+                // 210-byte blocks at 2-byte aligned addresses: aligned 32-bit loads and a funnel shift; a half block is requested ahead
+                uint32_t raw[17], ws[3], wd = 0;      // 17 words of lower bits, or 9 of upper
+                auto fetch = [&](int i) {      // half i & 1 of block i / 2
+                    const uintptr_t a = (uintptr_t)(rp + (size_t)(i >> 1) * BB);
+                    const int h = i & 1;
                     const uint32_t* bs = reinterpret_cast<const uint32_t*>((a + 192 + 8 * h) & ~(uintptr_t)3);
 #pragma unroll
-                    for (int i = 0; i < 17; ++i) wl[i] = __ldg(bl + i);
+                    for (int k = 0; k < 3; ++k) ws[k] = __ldg(bs + k);
+                    if (grp == 0) {
+                        const uint32_t* bl = reinterpret_cast<const uint32_t*>((a + 64 * h) & ~(uintptr_t)3);
 #pragma unroll
-                    for (int i = 0; i < 9; ++i) wh[i] = __ldg(bh + i);
+                        for (int k = 0; k < 17; ++k) raw[k] = __ldg(bl + k);
+                        wd = __ldg(reinterpret_cast<const uint32_t*>((a + 208) & ~(uintptr_t)3));
+                    } else {
+                        const uint32_t* bh = reinterpret_cast<const uint32_t*>((a + 128 + 32 * h) & ~(uintptr_t)3);
 #pragma unroll
-                    for (int i = 0; i < 3; ++i) ws[i] = __ldg(bs + i);
-                    wd = __ldg(reinterpret_cast<const uint32_t*>((a + 208) & ~(uintptr_t)3));
-                };
-                fetch(0, 0);
-                for (int kb = 0; kb < nb; ++kb) {
-                    const int g = g0 + kb;
-#pragma unroll 1
-                    for (int h = 0; h < 2; ++h) {
-                        const uintptr_t a = (uintptr_t)(rp + (size_t)kb * T::BB);
-                        const uint32_t sh = (uint32_t)(a & 2u) * 8u;       // every field of the block shares the 2-byte phase
-                        uint32_t ql[16], qh[8], scw[2];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) ql[i] = __funnelshift_r(wl[i], wl[i + 1], sh);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) qh[i] = __funnelshift_r(wh[i], wh[i + 1], sh);
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) scw[i] = __funnelshift_r(ws[i], ws[i + 1], sh);
-                        const float d = fp16_bits_to_float((uint16_t)((wd >> sh) & 0xFFFFu));
-                        if (h == 0) fetch(kb, 1);
-                        else if (kb + 1 < nb) fetch(kb + 1, 0);
-                        const int hg = 2 * g + h, stg = hg % T::A_STAGES, use = hg / T::A_STAGES;
-                        if (use > 0 && !tc_wait_k(0, bar(A_FREE, stg), (use - 1) & 1, give_up, p.err)) goto done;
-                        if (h == 0) {
-                            sts128(sD + ((g & 3) * 128 + r) * 16, __float_as_uint(d), 0u, 0u, 0u);
-                            mbar_arrive(bar(D_FULL, g & 3));
-                        }
-                        const uint32_t stage = sA + stg * (T::NP * TC_PLANE) + (r >> 3) * 1024 + (r & 7) * 128;
-                        const uint32_t rx = (uint32_t)(r & 7);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {                       // chunk i of the half: quadrant i / 2, words 4 (i & 1)..
-                            const int qd = i >> 1, w0 = 4 * (i & 1);
-                            const int sc = (int)(int8_t)((scw[i >> 2] >> (8 * (i & 3))) & 0xFFu);
-                            const uint32_t mag = (uint32_t)(sc < 0 ? -sc : sc);
-                            uint32_t u[4];
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                u[k] = ((ql[8 * (qd & 1) + w0 + k] >> (4 * (qd >> 1))) & 0x0F0F0F0Fu) |
-                                       (((qh[w0 + k] >> (2 * qd)) & 0x03030303u) << 4);
-#pragma unroll
-                            for (int di = 0; di < 4; ++di) {
-                                // signed digit m in -3..3; per byte m * (u - 32) + 128 = m * u + (128 - 32 m) lies in 32..224, so
-                                // one 32-bit multiply-add does the four bytes without carries between them, and flipping
-                                // each byte's top bit turns the biased value into the two's-complement byte m * (u - 32)
-                                const int dg = (int)((mag >> (2 * di)) & 3u);
-                                const int m = sc < 0 ? -dg : dg;
-                                const uint32_t K = (uint32_t)(128 - 32 * m) * 0x01010101u;
-                                sts128(stage + (((uint32_t)i ^ rx) << 4) + di * TC_PLANE, (u[0] * (uint32_t)m + K) ^ 0x80808080u,
-                                       (u[1] * (uint32_t)m + K) ^ 0x80808080u, (u[2] * (uint32_t)m + K) ^ 0x80808080u,
-                                       (u[3] * (uint32_t)m + K) ^ 0x80808080u);
-                            }
-                        }
-                        fence_async_smem();
-                        mbar_arrive(bar(A_FULL, stg));
+                        for (int k = 0; k < 9; ++k) raw[k] = __ldg(bh + k);
                     }
-                }
-            }
-            g0 += nb;
-        }
-    } else if (warp == 4) {
-        // ------------------------------------------------------------------ UMMA issue
-        if (lane == 0) {
-            int g0 = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                const TcTile ti = tc_tile_at(p, t);
-                if (!ti.live) continue;
-                const uint32_t idesc = umma_idesc_i8(T::A_SIGNED, TC_ROWS, TC_NTOK * ti.nset);
-                for (int kb = 0; kb < nb && ok; ++kb) {
-                    const int g = g0 + kb;
-                    if (!tc_wait_k(1, bar(B_FULL, g & 1), (g >> 1) & 1, give_up, p.err)) { ok = false; break; }
-                    const uint32_t sBcur = sBq + (g & 1) * (2 * TC_B_Q);
-                    const int set = g % T::NSET;
-                    const uint32_t tmem_set = tmem + set * (T::NP * TC_N);
-                    for (int h = 0; h < 2 && ok; ++h) {
-                        const int hg = 2 * g + h, stg = hg % T::A_STAGES, use = hg / T::A_STAGES;
-                        if (!tc_wait_k(2, bar(A_FULL, stg), use & 1, give_up, p.err)) { ok = false; break; }
-                        // the read-out of the block that used this set of accumulators last must have drained them
-                        if (h == 0 && g >= T::NSET && !tc_wait_k(3, bar(ACC_FREE, set), (g / T::NSET - 1) & 1, give_up, p.err)) { ok = false; break; }
+                };
+                fetch(0);
+#pragma unroll 1
+                for (int i = 0; i < 2 * nb; ++i) {
+                    const int h = i & 1;
+                    const uint32_t sh = (uint32_t)((uintptr_t)(rp + (size_t)(i >> 1) * BB) & 2u) * 8u;       // every field of the block shares the 2-byte phase
+                    uint32_t w[16], scw[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) scw[k] = __funnelshift_r(ws[k], ws[k + 1], sh);
+                    if (grp == 0) {
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) w[k] = __funnelshift_r(raw[k], raw[k + 1], sh);
+                        if (h == 0) {
+                            asm volatile("st.shared.f32 [%0], %1;" ::"r"(sm + TC_SD + ((g & 3) * 128 + r) * 8), "f"(fp16_bits_to_float((uint16_t)((wd >> sh) & 0xFFFFu))) : "memory");
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar(D_FULL, g & 3));
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) w[k] = __funnelshift_r(raw[k], raw[k + 1], sh);
+                    }
+                    if (i + 1 < 2 * nb) fetch(i + 1);
+#pragma unroll
+                    for (int gl = 0; gl < 2; ++gl) {      // quarter 2 h + gl: quadrants 2 gl and 2 gl + 1 of the half
+                        const int slot = 2 * gl + grp;      // filled twice a block
+                        if (!wait(bar(A_FREE, slot), h ^ 1)) goto gave_up;      // (the first passes)
                         tc_fence_after();
 #pragma unroll
-                        for (int pl = 0; pl < T::NP; ++pl)
-#pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)
-                                umma_i8(tmem_set + pl * TC_N, umma_desc_sw128(sA + stg * (T::NP * TC_PLANE) + pl * TC_PLANE + 32 * kk, 1024),
-                                        umma_desc_sw128(sBcur + h * (2 * TC_B_HALF) + 32 * kk, 1024), idesc, (h | kk) ? 1u : 0u);
-                        if (h == 1) umma_commit(bar(ACC_FULL, set));
-                        umma_commit(bar(A_FREE, stg));
+                        for (int hf = 0; hf < 2; ++hf) {      // words 0..3, 4..7: one 16-value group of either quadrant
+                            const float s0 = (float)(int8_t)(scw[gl] >> (8 * hf)), s1 = (float)(int8_t)(scw[gl] >> (16 + 8 * hf));
+                            uint32_t v[16];
+                            if (grp == 0) q6_low_columns(w + 4 * hf, w + 8 + 4 * hf, s0, s1, gl, v);
+                            else q6_high_columns(w + 4 * hf, s0, s1, gl, v);
+                            tmem_st16(t_a + 32 * slot + 16 * hf, v);
+                        }
+                        filled(slot);
                     }
-                    if (!ok) break;
-                    umma_commit(bar(B_FREE, g & 1));
+                    g += h;
                 }
-                g0 += nb;
             }
         }
-    } else if (warp == 5) {
-        // ------------------------------------------------------------------ token tiles
-        if (lane == 0) {
-            int g0 = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+    } else if (warp < TC_WARP_MMA) {
+        // ------------------------------------------------------------------ read-out
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_READ_REGS));
+        // every warp reads sixteen tokens of either tile: a set of accumulators is free again sooner than with eight warps for each tile
+        const int tok0 = 16 * ((warp - TC_EXPANDERS) >> 2);
+        const uint32_t t_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + tok0;
+        const float2 one = make_float2(p.one, p.one);
+        int g = 0;
+        uint32_t phase = 0;      // bit i: of set i's next use
+        for (int t = blockIdx.x; t < total; t += gridDim.x) {
+            bool two;
+            {
                 const TcTile ti = tc_tile_at(p, t);
                 if (!ti.live) continue;
-                for (int kb = 0; kb < nb; ++kb) {
-                    const int g = g0 + kb;
-                    if (g >= 2 && !tc_wait_k(4, bar(B_FREE, g & 1), ((g - 2) >> 1) & 1, give_up, p.err)) { ok = false; break; }
-                    const uint8_t* src = p.act + ((size_t)kb * p.n_tt + ti.tt0) * TC_ACT_TILE;
-                    mbar_expect_tx(bar(B_FULL, g & 1), (uint32_t)ti.nset * TC_B_Q);
-                    mbar_expect_tx(bar(S_FULL, g & 3), (uint32_t)ti.nset * T::TAIL_COPY);
-                    // operand rows 0..63 come from the first tile, 64..127 from the second: per half block, the two tiles'
-                    // 8 KB of swizzled rows back to back
-                    const uint32_t dst = sBq + (g & 1) * (2 * TC_B_Q);
-                    for (int th = 0; th < ti.nset; ++th) {
-                        for (int hh = 0; hh < 2; ++hh)
-                            bulk_g2s(dst + hh * (2 * TC_B_HALF) + th * TC_B_HALF, src + (size_t)th * TC_ACT_TILE + hh * TC_B_HALF, TC_B_HALF,
-                                     bar(B_FULL, g & 1));
-                        bulk_g2s(sS + ((g & 3) * 2 + th) * TC_ACT_TAIL, src + (size_t)th * TC_ACT_TILE + TC_B_Q, T::TAIL_COPY, bar(S_FULL, g & 3));
+                two = ti.nset == 2;
+            }
+            float2 sum[2][8];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sum[i >> 3][i & 7] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+            for (int kb = 0; kb < nb; ++kb, ++g) {
+                float2 d2, dm2;
+#pragma unroll
+                for (int th = 0; th < 2; ++th) {
+                    if (th && !two) break;
+                    const int set = th ? 1 : two ? 0 : kb & 1;
+                    // some lanes wait for the accumulators, some for d and dmin, some for the scales
+                    const uint32_t b = th || lane & 1 ? bar(ACC_FULL, set) : lane & 2 ? bar(D_FULL, g & 3) : bar(S_FULL, g & 7);
+                    if (!wait(b, th || lane & 1 ? (phase >> set) & 1 : lane & 2 ? (g >> 2) & 1 : (g >> 3) & 1)) goto gave_up;
+                    phase ^= 1u << set;
+                    tc_fence_after();
+                    const uint32_t yds = sm + TC_SSC + ((g & 7) * 2 + th) * TC_ACT_SCALES + 4 * tok0, col = t_lane + set * TC_SET;
+                    // eight tokens at a time; the next loads are on their way while the float terms of the last are made
+                    int x0[8], x1[8];
+                    tmem_ld8(col, x0);
+                    tmem_ld8(col + TC_NTOK, x1);
+                    if (th == 0) {
+                        const uint2 dd = lds64(sm + TC_SD + ((g & 3) * 128 + 32 * (warp & 3) + lane) * 8);
+                        d2 = make_float2(__uint_as_float(dd.x), __uint_as_float(dd.x));
+                        dm2 = make_float2(__uint_as_float(dd.y), __uint_as_float(dd.y));
+                    }
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        int x2[8];
+                        const uint4 ya = lds128(yds + 32 * c), yb = lds128(yds + 32 * c + 16);
+                        const float2 yd[4] = {make_float2(__uint_as_float(ya.x), __uint_as_float(ya.y)), make_float2(__uint_as_float(ya.z), __uint_as_float(ya.w)),
+                                              make_float2(__uint_as_float(yb.x), __uint_as_float(yb.y)), make_float2(__uint_as_float(yb.z), __uint_as_float(yb.w))};
+                        auto pair = [](const int (&v)[8], int i) { return make_float2(__int_as_float(v[2 * i]), __int_as_float(v[2 * i + 1])); };
+                        tmem_ld_wait(x0);
+                        tmem_loaded(x1);
+                        tmem_ld8(col + 2 * TC_NTOK + 8 * c, x2);
+                        float2 x[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float2& s = sum[th][4 * c + i];
+                            x[i] = add2_rn(pair(x0, i), pair(x1, i));
+                            if (Q4) s = fma2_rn(mul2_rn(mul2_rn(d2, yd[i]), x[i]), one, s);
+                        }
+                        tmem_ld_wait(x2);
+                        if (c == 0) {
+                            tmem_ld8(col + 8, x0);
+                            tmem_ld8(col + TC_NTOK + 8, x1);
+                        } else {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar(ACC_FREE, set));
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float2& s = sum[th][4 * c + i];
+                            const float2 m = pair(x2, i);
+                            if (Q4) s = fma2_rn(mul2_rn(mul2_rn(dm2, yd[i]), m), one, s);
+                            else s = fma2_rn(mul2_rn(mul2_rn(d2, yd[i]), add2_rn(x[i], m)), one, s);
+                        }
                     }
                 }
-                g0 += nb;
+            }
+            int again = t;      // (the item looked up anew: its values would hold registers through the loop)
+            asm volatile("" : "+r"(again));
+            const TcTile ti = tc_tile_at(p, again);
+            const int row = ti.row0 + 32 * (warp & 3) + lane;
+            const uint64_t out = reinterpret_cast<uint64_t>(p.out + p.seg[ti.seg].out_off + row);
+            const uint32_t pitch = 4u * (uint32_t)p.ldo;
+            // output rows of the sixteen slots of either tile, one to a lane (little code: what the blocks' loops need stays in the instruction caches)
+            const int slot = ti.tt0 * TC_NTOK + (lane & 16 ? TC_NTOK : 0) + tok0 + (lane & 15);
+            const int at = slot < p.n_slots && (two || lane < 16) ? (p.slot_row ? p.slot_row[slot] : slot) : -1;
+            const bool live = row < ti.N;
+#pragma unroll
+            for (int th = 0; th < 2; ++th) {
+                if (th && !two) break;
+                float old[16];
+                if (p.accumulate) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const int to = __shfl_sync(0xffffffffu, at, 16 * th + i);
+                        if (live && to >= 0) old[i] = *reinterpret_cast<const float*>(out + (uint64_t)(uint32_t)to * pitch);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float& x = i & 1 ? sum[th][i >> 1].y : sum[th][i >> 1].x;
+                        x = __fadd_rn(old[i], x);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int to = __shfl_sync(0xffffffffu, at, 16 * th + i);
+                    if (live && to >= 0) *reinterpret_cast<float*>(out + (uint64_t)(uint32_t)to * pitch) = i & 1 ? sum[th][i >> 1].y : sum[th][i >> 1].x;
+                }
             }
         }
     } else {
-        // ------------------------------------------------------------------ read-out
-        // a warp reaches the TMEM lanes 32 (warp index % 4) .. + 31: warps 6..9 read the first token tile, 10..13 the second
-        constexpr int RO_TOK = T::RO_TOK;
-        const int q = warp & 3, tok0 = ((warp - 6) >> 2) * RO_TOK, th = tok0 / TC_NTOK, tin = tok0 % TC_NTOK;
-        const uint32_t t_lane0 = tmem + ((uint32_t)(32 * q) << 16) + tok0;
-        const int r = 32 * q + lane;
-        int g0 = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-            const TcTile ti = tc_tile_at(p, t);
-            if (!ti.live) continue;
-            const bool mine = th < ti.nset;      // (a lone tile: the second tile's warps only keep the barrier counts)
-            float2 sumf[RO_TOK / 2];
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REST_REGS));
+        const bool one = elect_one();
+        if (warp < TC_WARP_MMA + 2) {
+            // ------------------------------------------------------------------ products
+            // Two warps: Q4_K: the halves of a block; Q6_K: the lower and the upper bits.  Either has accumulators of its own, so they need no order.  (A wait takes 100
+            // cycles and more even where nothing is to wait for, and a warp has six a block.)
+            const int h = warp - TC_WARP_MMA;
+            int st = 0;
+            uint32_t st_phase = 0, a_phase = 0, phase = 3;      // of the stage, of the operand slots, bit i: of set i's last use (the first passes)
+            bool ok = true;
+            constexpr uint32_t idesc = umma_idesc_f16(TC_ROWS, TC_NTOK);
+            auto set_free = [&](int set) {
+                const bool is = wait(bar(ACC_FREE, set), (phase >> set) & 1);
+                phase ^= 1u << set;
+                return is;
+            };
+            // a quarter block of a tile (its descriptor) from an operand slot into the accumulator at d
+            auto part = [&](uint32_t d, uint64_t tile, int slot, bool first) {
 #pragma unroll
-            for (int i = 0; i < RO_TOK / 2; ++i) sumf[i] = make_float2(0.0f, 0.0f);
-            for (int kb = 0; kb < nb && ok; ++kb) {
-                const int g = g0 + kb;
-                if ((mine && (!tc_wait_k(5, bar(D_FULL, g & 3), (g >> 2) & 1, give_up, p.err) ||
-                              !tc_wait_k(5, bar(S_FULL, g & 3), (g >> 2) & 1, give_up, p.err))) ||
-                    !tc_wait_k(6, bar(ACC_FULL, g % T::NSET), (g / T::NSET) & 1, give_up, p.err)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                if (mine) {
-                    const uint4 dd = lds128(sD + ((g & 3) * 128 + r) * 16);
-                    const float d = __uint_as_float(dd.x), dmin = __uint_as_float(dd.y);
-                    const uint32_t tail = sS + ((g & 3) * 2 + th) * TC_ACT_TAIL;
-                    const uint32_t yd_base = tail + 4 * tin, ys_base = tail + TC_ACT_SCALES + 16 * tin;
-                    const uint32_t t_lane = t_lane0 + (g % T::NSET) * (T::NP * TC_N);
-                    // eight tokens at a time: few enough live registers beside the 64 running sums for the compiler to
-                    // keep several token pairs in flight (the read-out is a chain of dependent short operations)
-                    const float2 d2 = make_float2(d, d), dm2 = make_float2(dmin, dmin);
+                for (int k = 0; k < 4; ++k) umma_f16_ts(d, tmem + TC_COL_A + 32 * slot + 8 * k, tile + 2 * k, idesc, !first || k > 0);
+            };
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                const TcTile ti = tc_tile_at(p, t);
+                if (!ti.live) continue;
+                const bool two = ti.nset == 2;
+#pragma unroll 1
+                for (int kb = 0; kb < nb && ok; ++kb) {
+                    const int set = two ? 0 : kb & 1;      // of the first tile
+                    const uint32_t at = sm + TC_SB + st * (2 * TC_TILE), d0 = tmem + set * TC_SET, d1 = tmem + TC_SET;
+                    const uint64_t tiles = umma_desc_sw128(at, 1024);
+                    ok = wait(bar(B_FULL, st), st_phase) && set_free(set);
+                    if constexpr (Q4) {
+                        const uint64_t mine = tiles + h * (2 * TC_QUARTER / 16), sums = umma_desc_plain(at + TC_B_Q, TC_SUM_HALF, 128), m = umma_desc_plain(sm + TC_SM, 2048, 128);
+                        const uint32_t to = h * TC_NTOK;
 #pragma unroll
-                    for (int piece = 0; piece < RO_TOK / 8; ++piece) {
-                        int a0[8], a1[8], a2[8], a3[8];
-                        tmem_ld8(t_lane + 8 * piece, a0);
-                        tmem_ld8(t_lane + TC_N + 8 * piece, a1);
-                        if (T::NP == 4) {
-                            tmem_ld8(t_lane + 2 * TC_N + 8 * piece, a2);
-                            tmem_ld8(t_lane + 3 * TC_N + 8 * piece, a3);
+                        for (int th = 0; th < 2; ++th) {
+                            if (th && !two) break;
+                            if (th) ok = ok && set_free(1);
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                if (th == 0) ok = ok && wait(bar(A_FULL, 2 * h + j), a_phase);
+                                if (!ok) break;
+                                tc_fence_after();
+                                if (one) {
+                                    const uint32_t d = th ? d1 : d0;
+                                    part(d + to, mine + (th * TC_TILE + j * TC_QUARTER) / 16, 2 * h + j, j == 0);
+                                    if (j == 1) {
+                                        if (h == 1) umma_f16(d + 2 * TC_NTOK, m, sums + th * TC_TILE / 16, idesc, 0);
+                                        umma_commit(bar(ACC_FULL, th ? 1 : set));
+                                    }
+                                    if (th || !two) umma_commit(bar(A_FREE, 2 * h + j));
+                                }
+                            }
                         }
-                        tmem_ld_wait();
+                    } else {
+                        // an operand slot serves both tiles before it is filled anew
+                        if (two) ok = ok && set_free(1);
 #pragma unroll
-                        for (int i = 0; i < 8; i += 2) {
-                            const uint2 yw = lds64(yd_base + 4 * (8 * piece + i));
-                            const float2 yd = make_float2(__uint_as_float(yw.x), __uint_as_float(yw.y));
-                            float2& s = sumf[4 * piece + (i >> 1)];
-                            if (TYPE == DC_TYPE_Q4_K) {
-                                // |acc0|, |acc1| <= 7 * 15 * 127 * 256 and |M| <= 63 * 127 * 256 stay below 2^22: adding the
-                                // integer to the bits of 1.5 * 2^23 and subtracting that constant converts it exactly without
-                                // the conversion unit; 8 * acc0 + acc1 then rounds once, in the fused multiply-add: float(I).
-                                // -M = sum over sub-blocks of (-minimum) x (sum of the token's codes there), accumulated on
-                                // top of the constant's bits.
-                                const uint4 ya = lds128(ys_base + 16 * (8 * piece + i)), yb = lds128(ys_base + 16 * (8 * piece + i + 1));
-                                int Ma = __dp2a_lo((int)ya.x, (int)dd.z, 0x4B400000);
-                                int Mb = __dp2a_lo((int)yb.x, (int)dd.z, 0x4B400000);
-                                Ma = __dp2a_hi((int)ya.y, (int)dd.z, Ma);
-                                Mb = __dp2a_hi((int)yb.y, (int)dd.z, Mb);
-                                Ma = __dp2a_lo((int)ya.z, (int)dd.w, Ma);
-                                Mb = __dp2a_lo((int)yb.z, (int)dd.w, Mb);
-                                Ma = __dp2a_hi((int)ya.w, (int)dd.w, Ma);
-                                Mb = __dp2a_hi((int)yb.w, (int)dd.w, Mb);
-                                const float2 kc = make_float2(-12582912.0f, -12582912.0f);
-                                const float2 f0 = add2_rn(make_float2(__int_as_float(0x4B400000 + a0[i]), __int_as_float(0x4B400000 + a0[i + 1])), kc);
-                                const float2 f1 = add2_rn(make_float2(__int_as_float(0x4B400000 + a1[i]), __int_as_float(0x4B400000 + a1[i + 1])), kc);
-                                const float2 fMn = add2_rn(make_float2(__int_as_float(Ma), __int_as_float(Mb)), kc);
-                                const float2 fI = fma2_rn(f0, make_float2(8.0f, 8.0f), f1);
-                                const float2 tI = mul2_rn(mul2_rn(d2, yd), fI);
-                                const float2 tMn = mul2_rn(mul2_rn(dm2, yd), fMn);     // -(dmin * yd) * float(M), exactly
-                                // (the two additions stay scalar: behind a packed multiply, a packed add or 1 * x + y was seen
-                                // to round once instead of twice, as if fused with the multiply)
-                                s.x = __fadd_rn(__fadd_rn(s.x, tI.x), tMn.x);
-                                s.y = __fadd_rn(__fadd_rn(s.y, tI.y), tMn.y);
-                            } else {
-                                const int Ia = a0[i] + 4 * a1[i] + 16 * a2[i] + 64 * a3[i];
-                                const int Ib = a0[i + 1] + 4 * a1[i + 1] + 16 * a2[i + 1] + 64 * a3[i + 1];
-                                const float2 tt = mul2_rn(mul2_rn(d2, yd), make_float2((float)Ia, (float)Ib));
-                                s.x = __fadd_rn(s.x, tt.x);
-                                s.y = __fadd_rn(s.y, tt.y);
+                        for (int q = 0; q < 4; ++q) {
+                            const int slot = 2 * (q & 1) + h;
+                            ok = ok && wait(bar(A_FULL, slot), q >> 1);
+                            if (!ok) break;
+                            tc_fence_after();
+                            if (one) {
+                                const uint32_t to = (h ? 2 : q >> 1) * TC_NTOK;
+                                const bool first = q == 0 || (h == 0 && q == 2);
+                                part(d0 + to, tiles + q * (TC_QUARTER / 16), slot, first);
+                                if (q == 3) umma_commit(bar(ACC_FULL, set));
+                                if (two) {
+                                    part(d1 + to, tiles + (TC_TILE + q * TC_QUARTER) / 16, slot, first);
+                                    if (q == 3) umma_commit(bar(ACC_FULL, 1));
+                                }
+                                umma_commit(bar(A_FREE, slot));
                             }
                         }
                     }
-                }
-                tc_fence_before();
-                mbar_arrive(bar(ACC_FREE, g % T::NSET));
-            }
-            if (ok && mine) {
-                const int row = ti.row0 + r;
-                if (row < ti.N) {
-                    float* out = p.out + p.seg[ti.seg].out_off;
-#pragma unroll
-                    for (int i = 0; i < RO_TOK; ++i) {
-                        const int slot = ti.tt0 * TC_NTOK + tok0 + i;
-                        if (slot >= p.n_slots) continue;
-                        const int orow = p.slot_row ? p.slot_row[slot] : slot;
-                        if (orow < 0) continue;
-                        float* o = out + (size_t)orow * p.ldo + row;
-                        const float v = (i & 1) ? sumf[i >> 1].y : sumf[i >> 1].x;
-                        *o = p.accumulate ? __fadd_rn(*o, v) : v;
+                    if (ok && one) umma_commit(bar(B_FREE, st));
+                    a_phase ^= 1;
+                    if (++st == TC_B_STAGES) {
+                        st = 0;
+                        st_phase ^= 1;
                     }
                 }
             }
-            g0 += nb;
+            if (!ok) {      // products in flight still read shared and tensor memory
+                if (one) umma_commit(bar(DRAIN, h));
+                mbar_wait(bar(DRAIN, h), 0, nullptr);
+                goto gave_up;
+            }
+        } else if (warp == TC_WARP_MMA + 2) {
+            // ------------------------------------------------------------------ token tiles
+            int g = 0, st = 0;
+            uint32_t st_phase = 1;      // of the stage's last use (the first passes)
+            for (int t = blockIdx.x; t < total; t += gridDim.x) {
+                const TcTile ti = tc_tile_at(p, t);
+                if (!ti.live) continue;
+                for (int kb = 0; kb < nb; ++kb, ++g) {
+                    if (!wait(bar(B_FREE, st), st_phase)) {
+                        // copies of the last blocks may still be on their way
+                        for (int o = max(0, g - TC_B_STAGES); o < g; ++o) mbar_wait(bar(B_FULL, o % TC_B_STAGES), (o / TC_B_STAGES) & 1, nullptr);
+                        goto gave_up;
+                    }
+                    if (one) {
+                        const uint8_t* src = p.act + ((size_t)kb * p.n_tt + ti.tt0) * TC_ACT_TILE;
+                        const uint32_t dst = sm + TC_SB + st * (2 * TC_TILE), dss = sm + TC_SSC + (g & 7) * (2 * TC_ACT_SCALES);
+                        constexpr uint32_t n = Q4 ? TC_TILE : TC_B_Q;
+                        mbar_expect_tx(bar(B_FULL, st), ti.nset * n);
+                        mbar_expect_tx(bar(S_FULL, g & 7), ti.nset * TC_ACT_SCALES);
+                        bulk_g2s(dst, src, n, bar(B_FULL, st));
+                        bulk_g2s(dss, src + TC_TILE, TC_ACT_SCALES, bar(S_FULL, g & 7));
+                        if (ti.nset == 2) {
+                            bulk_g2s(dst + TC_TILE, src + TC_ACT_TILE, n, bar(B_FULL, st));
+                            bulk_g2s(dss + TC_ACT_SCALES, src + TC_ACT_TILE + TC_TILE, TC_ACT_SCALES, bar(S_FULL, g & 7));
+                        }
+                    }
+                    if (++st == TC_B_STAGES) {
+                        st = 0;
+                        st_phase ^= 1;
+                    }
+                }
+            }
         }
     }
-done:
+    if (false) {
+    gave_up:
+        if (p.err) atomicExch(p.err, DC_ERR_MBAR_TIMEOUT);
+    }
     tc_fence_before();
     __syncthreads();
-#ifdef DC_TC_TIMING
-    if (tid == 0) atomicAdd(&g_tc_wait[7], (unsigned long long)(clock64() - t_kernel0));
-#endif
-    if (warp == 4) tmem_dealloc(tmem, NCOLS);
+    if (warp == TC_WARP_MMA) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace dc
@@ -668,17 +705,8 @@ int dc_launch_gemm_tc_multi(dc_ctx* ctx, const dc_weight* const* ws, const int* 
     p.slot_row = slot_row;
     p.accumulate = accumulate ? 1 : 0;
     p.estride = (size_t)w->N * w->row_bytes;
+    p.one = 1.0f;
     p.err = ctx->d_err;
-#ifdef DC_TC_TIMING
-    {
-        if (getenv("DC_TC_TIMING_DUMP")) {
-            unsigned long long w2[8];
-            cudaMemcpyFromSymbol(w2, g_tc_wait, sizeof(w2));
-            fprintf(stderr, "gemm_tc wait cycles so far: a_free %llu b_full %llu a_full %llu acc_free %llu b_free %llu d/s_full %llu acc_full %llu kernel %llu\n",
-                    w2[0], w2[1], w2[2], w2[3], w2[4], w2[5], w2[6], w2[7]);
-        }
-    }
-#endif
     if (tile_expert && !pair_tile0) return dc_fail(ctx, DC_B200_INVALID_ARGUMENT, "gemm_tc: grouped matmul without its tile pairs");
     p.pair_tile0 = pair_tile0;
     p.pair_nset = pair_nset;
@@ -687,15 +715,12 @@ int dc_launch_gemm_tc_multi(dc_ctx* ctx, const dc_weight* const* ws, const int* 
     // one CTA per SM walks its share of the tiles
     const dim3 grid((unsigned)std::min(p.tiles_x * p.tiles_y, ctx->num_sms));
     if (w->type == DC_TYPE_Q4_K) {
-        constexpr size_t smem = tc_smem_bytes<DC_TYPE_Q4_K>();
-        DC_TRY(dc_kernel_setup(ctx, (const void*)k_gemm_tc<DC_TYPE_Q4_K>, smem, "k_gemm_tc<Q4_K>"));
-        k_gemm_tc<DC_TYPE_Q4_K><<<grid, tc_threads<DC_TYPE_Q4_K>(), smem, ctx->stream>>>(p);
+        DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gemm_tc<DC_TYPE_Q4_K>, (int)TC_SMEM, "k_gemm_tc<Q4_K>"));
+        return dc_launch(ctx, "k_gemm_tc", k_gemm_tc<DC_TYPE_Q4_K>, grid, dim3(TC_THREADS), TC_SMEM, p);
     } else {
-        constexpr size_t smem = tc_smem_bytes<DC_TYPE_Q6_K>();
-        DC_TRY(dc_kernel_setup(ctx, (const void*)k_gemm_tc<DC_TYPE_Q6_K>, smem, "k_gemm_tc<Q6_K>"));
-        k_gemm_tc<DC_TYPE_Q6_K><<<grid, tc_threads<DC_TYPE_Q6_K>(), smem, ctx->stream>>>(p);
+        DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gemm_tc<DC_TYPE_Q6_K>, (int)TC_SMEM, "k_gemm_tc<Q6_K>"));
+        return dc_launch(ctx, "k_gemm_tc", k_gemm_tc<DC_TYPE_Q6_K>, grid, dim3(TC_THREADS), TC_SMEM, p);
     }
-    return dc_check_cuda(ctx, cudaGetLastError(), "k_gemm_tc");
 }
 
 int dc_launch_gemm_tc(dc_ctx* ctx, const dc_weight* w, const uint8_t* act, int n_slots, float* out, int ldo,

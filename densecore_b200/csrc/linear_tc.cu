@@ -12,8 +12,6 @@
 // CTA has its tensor memory.  Columns beyond K and rows beyond the matrix are the zeros that TMA fills in.  Every wait is
 // bounded; a CTA that gives up drains its copies, frees its tensor memory and leaves.
 #include <algorithm>
-#include <mutex>
-#include <set>
 
 #include "dc_common.cuh"
 #include "dc_launch.cuh"
@@ -444,24 +442,6 @@ EncodeFn encode_fn() {
 
 }  // namespace
 
-// Loads from tensor memory land in their registers some time after the instruction; each16 uses others meanwhile.  A build that
-// spills could store such a register too early and give it another use, which the load then overwrites: it may not run.
-static int setup_unspilled(dc_ctx* ctx, const void* f, int smem, const char* name) {
-    static std::mutex mu;
-    static std::set<const void*> good;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!good.count(f)) {
-            cudaFuncAttributes a;
-            const int st = dc_check_cuda(ctx, cudaFuncGetAttributes(&a, f), name);
-            if (st != DC_B200_OK) return st;
-            if (a.localSizeBytes) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "%s was built with %d bytes of spilled registers", name, (int)a.localSizeBytes);
-            good.insert(f);
-        }
-    }
-    return dc_kernel_setup(ctx, f, smem, name);
-}
-
 // Tensor map of a bf16 matrix [rows][ld] whose first K columns count: boxes of 128 rows x 64 columns.
 int dc_lin_encode(dc_ctx* ctx, CUtensorMap* map, const __nv_bfloat16* base, int rows, int K, int ld) {
     EncodeFn f = encode_fn();
@@ -482,13 +462,13 @@ int dc_launch_linear_tc(dc_ctx* ctx, const dc_lin& w, const dc_tc_in& x, int T, 
     p.e.n_pairs = std::max(0, std::min(epi.n_pairs, (w.N - epi.pair0) / 2));
     const int row_tiles = (w.N + 127) / 128, tok_tiles = (T + 255) / 256, tiles = row_tiles * tok_tiles;
     if (T > 128 && tiles >= ctx->num_sms / 2) {
-        int st = setup_unspilled(ctx, (const void*)k_linear_tc_wide<false>, (int)LW_SMEM, "k_linear_tc_wide");
+        int st = dc_kernel_setup_unspilled(ctx, (const void*)k_linear_tc_wide<false>, (int)LW_SMEM, "k_linear_tc_wide");
         if (st != DC_B200_OK) return st;
         const LwTiles tl = {row_tiles, tok_tiles, 0, 0, nullptr};
         return dc_launch(ctx, "k_linear_tc_wide", k_linear_tc_wide<false>, dim3(tiles < ctx->num_sms ? tiles : ctx->num_sms), dim3(LW_THREADS), LW_SMEM,
                          w.map, x.map, p, tl);
     }
-    int st = setup_unspilled(ctx, (const void*)k_linear_tc, (int)LT_SMEM, "k_linear_tc");
+    int st = dc_kernel_setup_unspilled(ctx, (const void*)k_linear_tc, (int)LT_SMEM, "k_linear_tc");
     if (st != DC_B200_OK) return st;
     return dc_launch(ctx, "k_linear_tc", k_linear_tc, dim3((w.N + 127) / 128, (T + 127) / 128), dim3(LT_THREADS), LT_SMEM, w.map, x.map, p);
 }
@@ -503,7 +483,7 @@ int dc_launch_linear_grouped_tc(dc_ctx* ctx, const dc_lin& w, int groups, int gr
     p.e.n_store = std::min(epi.n_store, std::min(group_rows, epi.pair0));
     p.e.n_pairs = std::max(0, std::min(epi.n_pairs, (group_rows - epi.pair0) / 2));
     const LwTiles tl = {(group_rows + 127) / 128, 0, groups, group_rows, group_off};
-    const int st = setup_unspilled(ctx, (const void*)k_linear_tc_wide<true>, (int)LW_SMEM, "k_linear_tc_grouped");
+    const int st = dc_kernel_setup_unspilled(ctx, (const void*)k_linear_tc_wide<true>, (int)LW_SMEM, "k_linear_tc_grouped");
     if (st != DC_B200_OK) return st;
     const long long most = (long long)tl.row_tiles * (max_rows / 256 + std::min(groups, max_rows));
     return dc_launch(ctx, "k_linear_tc_grouped", k_linear_tc_wide<true>, dim3((int)std::min<long long>(most, ctx->num_sms)), dim3(LW_THREADS), LW_SMEM, w.map, x.map,

@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(1024) k_moe_group(const int32_t* __restrict__ 
 __global__ void __launch_bounds__(256) k_swiglu_q8k_tiled(const float* __restrict__ g, const float* __restrict__ u, int ld, int F,
                                                           int n_slots_data, uint8_t* __restrict__ act, int n_tt,
                                                           const int32_t* __restrict__ slot_valid) {
+    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = F / DC_QK_K;
     const long long total = (long long)n_tt * 64 * nb;

@@ -1,0 +1,51 @@
+"""The prompt-sized products of K-quant matrices at the edges of their tiles, and where their sums are largest."""
+import numpy as np
+import pytest
+
+from densecore_b200 import blocks as B
+
+pytestmark = pytest.mark.gpu
+
+Q4, Q6 = B.GGML_TYPE_Q4_K, B.GGML_TYPE_Q6_K
+
+
+def check(got, want, t):
+    if t == Q4:
+        assert np.array_equal(got, want)
+    else:       # equal integers, one float term per block where the oracle keeps eight partials: a few roundings of 2^-24 for each of up to eight blocks
+        assert np.abs(got - want).max() <= 2e-6 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("t", [Q4, Q6])
+@pytest.mark.parametrize("N,K", [(1, 256), (127, 768), (129, 512), (300, 1280)])
+def test_edges_of_rows_tokens_and_blocks(ctx, oracle, t, N, K):
+    """Lone and paired token tiles, full, ragged and empty at the end; rows on either side of the 128-row tile; even and odd numbers of blocks."""
+    rng = np.random.default_rng(N + K)
+    w = B.random_weight(rng, t, N, K)
+    W = ctx.upload_weight(t, w, K, N)
+    for M in (32, 33, 64, 65, 127, 128, 129, 193, 257):
+        x = rng.normal(size=(M, K)).astype(np.float32)
+        check(ctx.mul_mat(W, x), oracle.mul_mat(t, w, N, K, x), t)
+    W.free()
+
+
+@pytest.mark.parametrize("t", [Q4, Q6])
+def test_largest_sums(ctx, oracle, t):
+    """Codes, scales and minima at the ends of their ranges with activations that are all one value: block sums beyond 2^24."""
+    N, K, M = 130, 512, 70
+    rng = np.random.default_rng(7)
+    nb = K // 256
+    if t == Q4:
+        blk = B.random_q4k(rng, N, K).reshape(N, nb, 144)
+        hi = rng.integers(60, 64, size=(N, nb, 8), dtype=np.uint8)
+        blk[:, :, 4:16] = B.pack_q4k_scales(hi, hi)
+        blk[:, :, 16:] = rng.choice(np.array([0xFF, 0xFE, 0xEF], np.uint8), size=(N, nb, 128))
+    else:
+        blk = B.random_q6k(rng, N, K).reshape(N, nb, 210)
+        blk[:, :, :192] = rng.choice(np.array([0x00, 0xFF], np.uint8), size=(N, nb, 1))      # every code -32 or every code 31
+        blk[:, :, 192:208] = rng.choice(np.array([-128, -127, 127], np.int8), size=(N, nb, 1)).view(np.uint8)
+    w = blk.reshape(N, -1)
+    x = np.where(rng.random((M, K)) < 0.002, 0.5, 1.0).astype(np.float32) * rng.choice([-1.0, 1.0], size=(M, 1)).astype(np.float32)
+    W = ctx.upload_weight(t, w, K, N)
+    check(ctx.mul_mat(W, x), oracle.mul_mat(t, w, N, K, x), t)
+    W.free()
