@@ -9,7 +9,8 @@
 // out by eight warps; the wider tile reads shared memory less often per product.  Its grouped form multiplies runs of sorted tokens with
 // a matrix of their own each (experts); the runs' ends are device data, so every CTA lists the tiles itself, and a tile
 // of few tokens takes narrower products.  All let the next kernel start only after every
-// CTA has its tensor memory.  Columns beyond K and rows beyond the matrix are the zeros that TMA fills in.  Every wait is
+// CTA has its tensor memory.  The loading and the issuing warp run as whole warps of which one lane issues: with a branch on the lane number around their
+// loops a stage's wait, four products and commit took as long as the products themselves (prompts 1 to 2 % longer).  Columns beyond K and rows beyond the matrix are the zeros that TMA fills in.  Every wait is
 // bounded; a CTA that gives up drains its copies, frees its tensor memory and leaves.
 #include <algorithm>
 
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(LT_THREADS, 2) k_linear_tc(const __grid_consta
     __shared__ int s_give_up;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t full = smem_u32(s_bar), empty = full + 8 * LT_STAGES, acc = empty + 8 * LT_STAGES;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int row0 = blockIdx.x * 128, t0 = blockIdx.y * 128;
     const int nk = (p.K + 63) / 64;
     volatile int* give_up = &s_give_up;
@@ -232,36 +233,39 @@ __global__ void __launch_bounds__(LT_THREADS, 2) k_linear_tc(const __grid_consta
     pdl_launch_dependents();
     pdl_wait();
     if (warp == 0) {
-        if (lane == 0) {
-            int issued = 0;
-            for (; issued < nk; ++issued) {
-                const int s = issued % LT_STAGES, use = issued / LT_STAGES;
-                if (use > 0 && !tc_wait_raw(empty + 8 * s, (use - 1) & 1, give_up, p.err)) break;
-                mbar_expect_tx(full + 8 * s, 2 * LT_TILE);
-                tma_load_2d(base + s * 2 * LT_TILE, &wmap, issued * 64, row0, full + 8 * s);
-                tma_load_2d(base + s * 2 * LT_TILE + LT_TILE, &xmap, issued * 64, t0, full + 8 * s);
+        const bool one = elect_one();
+        int issued = 0, s = 0;
+        uint32_t phase = 1;      // of the stage's last use (the first passes)
+        for (; issued < nk; ++issued) {
+            if (!tc_wait_warp(empty + 8 * s, phase, give_up, p.err)) break;
+            if (one) {
+                const uint32_t to = base + s * 2 * LT_TILE, bar = full + 8 * s;
+                mbar_expect_tx(bar, 2 * LT_TILE);
+                tma_load_2d(to, &wmap, issued * 64, row0, bar);
+                tma_load_2d(to + LT_TILE, &xmap, issued * 64, t0, bar);
             }
-            // no copy may still be in flight when the CTA leaves (at once unless someone gave up)
-            for (int s = 0; s < LT_STAGES; ++s) {
-                const int uses = (issued - s + LT_STAGES - 1) / LT_STAGES;
-                if (issued > s)
-                    for (uint32_t i = 0; i < DC_WAIT_LIMIT && !mbar_try_wait(full + 8 * s, (uses - 1) & 1); ++i) {}
-            }
+            if (++s == LT_STAGES) s = 0, phase ^= 1;
         }
+        // no copy may still be in flight when the CTA leaves (at once unless someone gave up)
+        for (int i = 0; i < LT_STAGES; ++i)
+            if (issued > i) mbar_wait_warp(full + 8 * i, ((issued - i + LT_STAGES - 1) / LT_STAGES - 1) & 1);
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16(128, 128);
-            for (int k = 0; k < nk; ++k) {
-                const int s = k % LT_STAGES;
-                if (!tc_wait_raw(full + 8 * s, (k / LT_STAGES) & 1, give_up, p.err)) break;
-                tc_fence_after();
-                const uint32_t a = base + s * 2 * LT_TILE, b = a + LT_TILE;
+        const bool one = elect_one();
+        constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
+        int s = 0;
+        uint32_t phase = 0;
+        for (int k = 0; k < nk; ++k) {
+            if (!tc_wait_warp(full + 8 * s, phase, give_up, p.err)) break;
+            tc_fence_after();
+            const uint64_t a = umma_desc_sw128(base + s * 2 * LT_TILE, 1024), b = umma_desc_sw128(base + s * 2 * LT_TILE + LT_TILE, 1024);
+            if (one) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_f16(tmem, umma_desc_sw128(a + 32 * j, 1024), umma_desc_sw128(b + 32 * j, 1024), idesc, k > 0 || j > 0);
+                for (int j = 0; j < 4; ++j) umma_f16(tmem, a + 2 * j, b + 2 * j, idesc, k > 0 || j > 0);
                 umma_commit(empty + 8 * s);
             }
-            umma_commit(acc);
+            if (++s == LT_STAGES) s = 0, phase ^= 1;
         }
+        if (one) umma_commit(acc);
     } else {
         const bool ok = tc_wait_raw(acc, 0, give_up, p.err) && !*give_up;
         tc_fence_after();
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(LW_THREADS, 1) k_linear_tc_wide(const __grid_c
     __shared__ int s_off[GROUPED ? DC_MOE_MAX_EXPERTS + 1 : 1], s_first[GROUPED ? DC_MOE_MAX_EXPERTS + 1 : 1];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t full = smem_u32(s_bar), empty = full + 8 * LW_STAGES, acc_full = empty + 8 * LW_STAGES, acc_free = acc_full + 16;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nk = (p.K + 63) / 64;
     volatile int* give_up = &s_give_up;
     if (warp == 1) {
@@ -356,56 +360,52 @@ __global__ void __launch_bounds__(LW_THREADS, 1) k_linear_tc_wide(const __grid_c
     };
     // Every role walks the same tiles; stages are counted on across tiles.
     if (warp == 0) {
-        if (lane == 0) {
-            int issued = 0, group = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-                const Place at = place(tile, group);
-                const bool both = !GROUPED || at.cols() > 128;
-                for (int k = 0; k < nk; ++k, ++issued) {
-                    const int s = issued % LW_STAGES, use = issued / LW_STAGES;
-                    if (use > 0 && !tc_wait_raw(empty + 8 * s, (use - 1) & 1, give_up, p.err)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t to = base + s * LW_STAGE;
-                    mbar_expect_tx(full + 8 * s, both ? LW_STAGE : 2 * LT_TILE);
-                    tma_load_2d(to, &wmap, k * 64, at.wrow, full + 8 * s);
-                    tma_load_2d(to + LT_TILE, &xmap, k * 64, at.t0, full + 8 * s);
-                    if (both) tma_load_2d(to + 2 * LT_TILE, &xmap, k * 64, at.t0 + 128, full + 8 * s);
+        const bool one = elect_one();
+        int issued = 0, group = 0, s = 0;
+        uint32_t phase = 1;      // of the stage's last use (the first passes)
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+            const Place at = place(tile, group);
+            const bool both = !GROUPED || at.cols() > 128;
+            for (int k = 0; k < nk; ++k, ++issued) {
+                ok = tc_wait_warp(empty + 8 * s, phase, give_up, p.err);
+                if (!ok) break;
+                if (one) {
+                    const uint32_t to = base + s * LW_STAGE, bar = full + 8 * s;
+                    mbar_expect_tx(bar, both ? LW_STAGE : 2 * LT_TILE);
+                    tma_load_2d(to, &wmap, k * 64, at.wrow, bar);
+                    tma_load_2d(to + LT_TILE, &xmap, k * 64, at.t0, bar);
+                    if (both) tma_load_2d(to + 2 * LT_TILE, &xmap, k * 64, at.t0 + 128, bar);
                 }
-            }
-            // no copy may still be in flight when the CTA leaves (at once unless someone gave up)
-            for (int s = 0; s < LW_STAGES; ++s) {
-                const int uses = (issued - s + LW_STAGES - 1) / LW_STAGES;
-                if (issued > s)
-                    for (uint32_t i = 0; i < DC_WAIT_LIMIT && !mbar_try_wait(full + 8 * s, (uses - 1) & 1); ++i) {}
+                if (++s == LW_STAGES) s = 0, phase ^= 1;
             }
         }
+        // no copy may still be in flight when the CTA leaves (at once unless someone gave up)
+        for (int i = 0; i < LW_STAGES; ++i)
+            if (issued > i) mbar_wait_warp(full + 8 * i, ((issued - i + LW_STAGES - 1) / LW_STAGES - 1) & 1);
     } else if (warp == 1) {
-        if (lane == 0) {
-            int it = 0, j = 0, group = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++j) {
-                const int set = j & 1;
-                const uint32_t idesc = umma_idesc_bf16(128, GROUPED ? (place(tile, group).cols() + 15) & ~15 : 256);
-                if (j >= 2 && !tc_wait_raw(acc_free + 8 * set, ((j >> 1) - 1) & 1, give_up, p.err)) break;
+        const bool one = elect_one();
+        int j = 0, group = 0, s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++j) {
+            const int set = j & 1;
+            const uint32_t idesc = umma_idesc_bf16(128, GROUPED ? (place(tile, group).cols() + 15) & ~15 : 256), d = tmem + 256 * set;
+            if (j >= 2 && !tc_wait_warp(acc_free + 8 * set, ((j >> 1) - 1) & 1, give_up, p.err)) break;
+            tc_fence_after();
+            for (int k = 0; k < nk; ++k) {
+                ok = tc_wait_warp(full + 8 * s, phase, give_up, p.err);
+                if (!ok) break;
                 tc_fence_after();
-                for (int k = 0; k < nk; ++k, ++it) {
-                    const int s = it % LW_STAGES;
-                    if (!tc_wait_raw(full + 8 * s, (it / LW_STAGES) & 1, give_up, p.err)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a = base + s * LW_STAGE, b = a + LT_TILE;
+                const uint64_t a = umma_desc_sw128(base + s * LW_STAGE, 1024), b = umma_desc_sw128(base + s * LW_STAGE + LT_TILE, 1024);
+                if (one) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        umma_f16(tmem + 256 * set, umma_desc_sw128(a + 32 * q, 1024), umma_desc_sw128(b + 32 * q, 1024), idesc, k > 0 || q > 0);
+                    for (int q = 0; q < 4; ++q) umma_f16(d, a + 2 * q, b + 2 * q, idesc, k > 0 || q > 0);
                     umma_commit(empty + 8 * s);
                 }
-                umma_commit(acc_full + 8 * set);
+                if (++s == LW_STAGES) s = 0, phase ^= 1;
             }
+            if (one) umma_commit(acc_full + 8 * set);
         }
     } else {
         int j = 0, group = 0;
