@@ -111,31 +111,42 @@ __global__ void __launch_bounds__(1024) k_moe_group(const int32_t* __restrict__ 
                                                     int ep_lo, int ep_hi, int32_t* __restrict__ slot_assign,
                                                     int32_t* __restrict__ slot_token, int32_t* __restrict__ tile_expert,
                                                     int32_t* __restrict__ pair_tile0, int32_t* __restrict__ pair_nset) {
-    __shared__ int s_cnt[256], s_off[256], s_fill[256], s_total, s_pairs;
-    const int tid = threadIdx.x;
+    __shared__ int s_cnt[256], s_off[256], s_fill[256], s_warp[8], s_total, s_pairs;
+    const int tid = threadIdx.x, lane = tid & 31;
     if (tid < 256) s_cnt[tid] = s_fill[tid] = 0;
     __syncthreads();
     for (int i = tid; i < A; i += blockDim.x) atomicAdd(&s_cnt[ids[i]], 1);
     __syncthreads();
+    // tiles and pairs of tiles (the work items of the matmul kernel) ahead of every expert's, as the two halves of one running sum (at most 2^15 of either)
+    int tiles = 0, pairs = 0, sum = 0;
     if (tid < 256) {
-        int off = 0;
-        for (int i = 0; i < tid; ++i) off += (s_cnt[i] + 63) / 64;
+        tiles = tid < E ? (s_cnt[tid] + 63) / 64 : 0;
+        pairs = (tiles + 1) / 2;
+        sum = tiles | pairs << 16;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        if (lane == 31) s_warp[tid >> 5] = sum;
+    }
+    __syncthreads();
+    if (tid < 256) {
+        for (int w = 0; w < tid >> 5; ++w) sum += s_warp[w];
+        const int off = (sum & 0xFFFF) - tiles, poff = (sum >> 16) - pairs;
         s_off[tid] = off;
-        const int tiles = tid < E ? (s_cnt[tid] + 63) / 64 : 0;
         // expert parallel: this GPU stores experts [ep_lo, ep_hi) only, as slabs 0 .. ep_hi - ep_lo - 1; tiles of the
         // others are skipped here and their share of the layer arrives by all-reduce
         const int local = (tid >= ep_lo && tid < ep_hi) ? tid - ep_lo : -1;
         for (int t = 0; t < tiles; ++t) tile_expert[off + t] = local;
-        if (tid == 255) s_total = off + tiles;
-        // pairs of neighbouring tiles of one expert (the work items of the matmul kernel's second form)
-        int poff = 0;
-        for (int i = 0; i < tid; ++i) poff += ((s_cnt[i] + 63) / 64 + 1) / 2;
-        const int pairs = (tiles + 1) / 2;
         for (int j = 0; j < pairs; ++j) {
             pair_tile0[poff + j] = local >= 0 ? off + 2 * j : -1;
             pair_nset[poff + j] = min(2, tiles - 2 * j);
         }
-        if (tid == 255) s_pairs = poff + pairs;
+        if (tid == 255) {
+            s_total = off + tiles;
+            s_pairs = poff + pairs;
+        }
     }
     for (int sl = tid; sl < max_tiles * 64; sl += blockDim.x) {
         slot_assign[sl] = -1;
@@ -154,7 +165,7 @@ __global__ void __launch_bounds__(1024) k_moe_group(const int32_t* __restrict__ 
 
 // h = silu(g) * u per slot (the production SwiGLU of the CPU kernels, see silu_fast), quantised to the
 // tiled Q8_K layout of the down projection's activations.  One warp per (slot, 256-value block);
-// slot_valid (optional): slots whose entry is negative hold zeros.
+// slot_valid (optional): slots whose entry is negative are left as they are, and so are those beyond the data (see k_quantize_q8k_tiled).
 __global__ void __launch_bounds__(256) k_swiglu_q8k_tiled(const float* __restrict__ g, const float* __restrict__ u, int ld, int F,
                                                           int n_slots_data, uint8_t* __restrict__ act, int n_tt,
                                                           const int32_t* __restrict__ slot_valid) {
@@ -164,20 +175,18 @@ __global__ void __launch_bounds__(256) k_swiglu_q8k_tiled(const float* __restric
     const long long total = (long long)n_tt * 64 * nb;
     for (long long item = (long long)blockIdx.x * 8 + warp; item < total; item += (long long)gridDim.x * 8) {
         const int b = (int)(item % nb), slot = (int)(item / nb);
-        const bool live = slot < n_slots_data && (!slot_valid || slot_valid[slot] >= 0);
+        if (slot >= n_slots_data || (slot_valid && slot_valid[slot] < 0)) continue;
         uint8_t* tile = act + ((size_t)b * n_tt + slot / TC_NTOK) * TC_ACT_TILE;
-        uint32_t w0 = 0, w1 = 0, bw = 0;
-        float d = 0.0f;
-        if (live) {
-            const size_t base = (size_t)slot * ld + (size_t)b * DC_QK_K + 8 * lane;
-            const float4 g0 = *reinterpret_cast<const float4*>(g + base), g1 = *reinterpret_cast<const float4*>(g + base + 4);
-            const float4 u0 = *reinterpret_cast<const float4*>(u + base), u1 = *reinterpret_cast<const float4*>(u + base + 4);
-            const float v[8] = {__fmul_rn(silu_fast(g0.x), u0.x), __fmul_rn(silu_fast(g0.y), u0.y),
-                                __fmul_rn(silu_fast(g0.z), u0.z), __fmul_rn(silu_fast(g0.w), u0.w),
-                                __fmul_rn(silu_fast(g1.x), u1.x), __fmul_rn(silu_fast(g1.y), u1.y),
-                                __fmul_rn(silu_fast(g1.z), u1.z), __fmul_rn(silu_fast(g1.w), u1.w)};
-            q8k_block_core(v, lane, w0, w1, bw, d);
-        }
+        uint32_t w0, w1, bw;
+        float d;
+        const size_t base = (size_t)slot * ld + (size_t)b * DC_QK_K + 8 * lane;
+        const float4 g0 = *reinterpret_cast<const float4*>(g + base), g1 = *reinterpret_cast<const float4*>(g + base + 4);
+        const float4 u0 = *reinterpret_cast<const float4*>(u + base), u1 = *reinterpret_cast<const float4*>(u + base + 4);
+        const float v[8] = {__fmul_rn(silu_fast(g0.x), u0.x), __fmul_rn(silu_fast(g0.y), u0.y),
+                            __fmul_rn(silu_fast(g0.z), u0.z), __fmul_rn(silu_fast(g0.w), u0.w),
+                            __fmul_rn(silu_fast(g1.x), u1.x), __fmul_rn(silu_fast(g1.y), u1.y),
+                            __fmul_rn(silu_fast(g1.z), u1.z), __fmul_rn(silu_fast(g1.w), u1.w)};
+        q8k_block_core(v, lane, w0, w1, bw, d);
         tc_act_store(tile, slot % TC_NTOK, lane, w0, w1, bw, d);
     }
 }
