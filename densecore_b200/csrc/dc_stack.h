@@ -321,7 +321,7 @@ void dc_stack_stats(dc_model* m, double* weight_bytes, double* kv_bytes_per_toke
 
 // ---- linear.cu / linear_tc.cu: y = W x
 // T <= DC_MAX_T tokens, bf16 or f32 inputs: one pass over the weights
-int dc_launch_linear_mma(dc_ctx* ctx, const dc_lin& w, const __nv_bfloat16* x, int ldx, int T, const dc_lin_epi& epi);
+int dc_launch_linear_mma(dc_ctx* ctx, const dc_lin& w, const __nv_bfloat16* x, int ldx, int T, const dc_lin_epi& epi, const dc_lin* next = nullptr);     // next: the product whose weights are to come into L2 meanwhile
 int dc_launch_linear_rows(dc_ctx* ctx, const dc_lin& w, const float* x, int ldx, int T, const dc_lin_epi& epi);
 // any T, f32 inputs (f32 models)
 int dc_launch_linear_f32(dc_ctx* ctx, const dc_lin& w, const float* x, int ldx, int T, const dc_lin_epi& epi);

@@ -148,7 +148,18 @@ struct MmaParams {
     const __nv_bfloat16* x;
     int ldx, T;
     dc_lin_epi e;
+    const char* next;        // weights of the product after this one ...
+    uint32_t next_slice, next_bytes;      // ... a CTA's share of them, all
 };
+
+// One thread: this CTA's share of the next product's weights on its way into L2, while memory would idle: in this kernel's sums and the small
+// kernels in between.
+__device__ __forceinline__ void fetch_next(const MmaParams& p) {
+    if (threadIdx.x != 0 || !p.next_slice) return;
+    const uint32_t from = blockIdx.x * p.next_slice, to = min(from + p.next_slice, p.next_bytes);
+    for (uint32_t at = from; at < to; at += 16384)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.next + at), "r"(min(16384u, to - at)) : "memory");
+}
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -160,7 +171,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // KS: CTAs of a cluster that share sixteen rows, each with its part of the columns; the first adds the parts up.
 // With KS 1 a CTA walks over its tiles of sixteen rows and fetches the next tile's first runs ahead of a tile's sum.
 template <int NT, int AHEAD, int KS>
-__global__ void __launch_bounds__(LM_WARPS * 32) k_linear_mma(const MmaParams p) {
+__global__ void __launch_bounds__(LM_WARPS * 32, AHEAD > 2 ? 1 : LM_CTAS) k_linear_mma(const MmaParams p) {
     __shared__ float red[2][LM_WARPS][16][8 * NT + 1];
     __shared__ float other[KS > 1 ? KS - 1 : 1][KS > 1 ? 128 * NT : 1];
     if (KS > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");       // waited for ahead of the first remote store
@@ -181,9 +192,11 @@ __global__ void __launch_bounds__(LM_WARPS * 32) k_linear_mma(const MmaParams p)
     const int step = gridDim.x / KS;
 #pragma unroll
     for (int j = 0; j < AHEAD; ++j) fetch(j, tile, first + warp * AHEAD + j);
+    if (KS > 1) fetch_next(p);
     dc::pdl_wait();
     for (int buf = 0; tile < tiles; tile += step, buf ^= 1) {
         const int row0 = 16 * tile;
+        if (KS == 1 && tile + step >= tiles) fetch_next(p);
         float acc[NT][4];
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
@@ -296,12 +309,14 @@ __global__ void __launch_bounds__(256) k_linear_f32(const RowsParams p) {
 }
 
 template <int NT, int AHEAD, int KS>
-int launch_mma(dc_ctx* ctx, const MmaParams& p) {
+int launch_mma(dc_ctx* ctx, MmaParams p) {
     const int tiles = (p.N + 15) / 16;
     const dim3 block(LM_WARPS * 32);
-    if (KS > 1) return dc_launch_cluster(ctx, "k_linear_mma", k_linear_mma<NT, AHEAD, KS>, dim3(tiles * KS), block, 0, KS, p);
-    const int room = LM_CTAS * ctx->num_sms, rounds = (tiles + room - 1) / room;
-    return dc_launch(ctx, "k_linear_mma", k_linear_mma<NT, AHEAD, 1>, dim3((tiles + rounds - 1) / rounds), block, 0, p);
+    const int room = LM_CTAS * ctx->num_sms, rounds = (tiles + room - 1) / room, grid = KS > 1 ? tiles * KS : (tiles + rounds - 1) / rounds;
+    p.next_slice = (p.next_bytes / grid + 511) / 256 * 256;
+    if (!p.next_bytes) p.next_slice = 0;
+    if (KS > 1) return dc_launch_cluster(ctx, "k_linear_mma", k_linear_mma<NT, AHEAD, KS>, dim3(grid), block, 0, KS, p);
+    return dc_launch(ctx, "k_linear_mma", k_linear_mma<NT, AHEAD, 1>, dim3(grid), block, 0, p);
 }
 
 dc_lin_epi clipped(const dc_lin& w, dc_lin_epi e) {
@@ -313,9 +328,13 @@ bool epi_ok(const dc_lin_epi& e) { return e.pair0 >= (1 << 30) || e.pair0 % DC_P
 
 }  // namespace
 
-int dc_launch_linear_mma(dc_ctx* ctx, const dc_lin& w, const __nv_bfloat16* x, int ldx, int T, const dc_lin_epi& epi) {
+int dc_launch_linear_mma(dc_ctx* ctx, const dc_lin& w, const __nv_bfloat16* x, int ldx, int T, const dc_lin_epi& epi, const dc_lin* next) {
     if (T < 1 || T > DC_MAX_T || ((uintptr_t)x & 15) || (ldx & 7) || (w.N & 7) || !epi_ok(epi)) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "linear_mma: bad operand");
-    MmaParams p = {w.w, w.N, w.K, w.ld, x, ldx, T, clipped(w, epi)};
+    MmaParams p = {w.w, w.N, w.K, w.ld, x, ldx, T, clipped(w, epi), nullptr, 0, 0};
+    if (next && !((uintptr_t)next->w & 15)) {
+        p.next = (const char*)next->w;
+        p.next_bytes = (uint32_t)std::min<size_t>((size_t)next->N * next->ld * 2, 6u << 20) & ~15u;
+    }
     // fewer tiles than SMs: long rows are shared by a cluster, short ones need more in flight per warp
     const int tiles = (w.N + 15) / 16;
     if (2 * tiles <= ctx->num_sms && w.K >= 2048) return T <= 8 ? launch_mma<1, 2, 4>(ctx, p) : launch_mma<2, 2, 4>(ctx, p);

@@ -455,8 +455,9 @@ int tc_in(dc_model* m, dc_tc_in* out, const __nv_bfloat16* x, int K, int ld, int
 }
 
 // y = W x for the step's tokens: xf is the input of f32 models, xb that of bf16 models, same pitch.
-int linear(dc_model* m, const dc_step& st, const dc_lin& w, const float* xf, const __nv_bfloat16* xb, int ldx, const dc_lin_epi& epi) {
-    if (st.b16 && st.T <= DC_MAX_T) return dc_launch_linear_mma(m->ctx, w, xb, ldx, st.T, epi);
+// next: the product after it.
+int linear(dc_model* m, const dc_step& st, const dc_lin& w, const float* xf, const __nv_bfloat16* xb, int ldx, const dc_lin_epi& epi, const dc_lin* next = nullptr) {
+    if (st.b16 && st.T <= DC_MAX_T) return dc_launch_linear_mma(m->ctx, w, xb, ldx, st.T, epi, next);
     if (st.b16) {
         dc_tc_in in;
         DC_TRY(tc_in(m, &in, xb, w.K, ldx, m->stack->b.cap));
@@ -581,9 +582,18 @@ int mix_lightning(dc_model* m, const dc_step& st, const dc_stack_run& run, dc_st
     return dc_launch_lightning_norm(m->ctx, d, st, b.scan, ldy, b.proj, actb, lda, m->stack->cfg.eps, b.mix, st.b16 ? b.mixb : nullptr, ldm);
 }
 
+// A layer's first and last products around its mixer; the product that a layer run begins with (behind the last: the output matrix).
+const dc_lin& mixer_in(const dc_stack_layer& Ly) {
+    return Ly.kind == DC_MIX_DELTA ? Ly.dl.in : Ly.kind == DC_MIX_SSD ? Ly.ssd.in : Ly.kind == DC_MIX_LATENT ? Ly.la.in : Ly.in;
+}
+const dc_lin& mixer_out(const dc_stack_layer& Ly) {
+    return Ly.kind == DC_MIX_DELTA ? Ly.dl.o : Ly.kind == DC_MIX_SSD ? Ly.ssd.o : Ly.kind == DC_MIX_LATENT ? Ly.la.o : Ly.out;
+}
+const dc_lin* run_begin(const dc_stack* s, size_t il) { return il < s->runs.size() ? &mixer_in(s->layers[s->runs[il].layer]) : &s->head; }
+
 // x += mixer(h) + ff(h) with h = norm1(x): one product from h, the mixer, one product back into the residual.  The
 // feed-forward's hidden values lie beside the mixer's output.
-int parallel_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_stack_run& run, dc_stack_layer& Ly) {
+int parallel_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_stack_run& run, dc_stack_layer& Ly, const dc_lin* after) {
     dc_stack* s = m->stack;
     dc_ctx* ctx = m->ctx;
     dc_stack_buffers& b = s->b;
@@ -594,13 +604,13 @@ int parallel_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_
     if (light) in.act_rows = Ly.li.off_g;
     else in.bias = Ly.ga.bias;
     if (Ly.ff) in.pairs(Ly.pair0, DC_PAIR_CLAMPED, Ly.limit, b.mix + Ly.out_ff, st.b16 ? b.mixb + Ly.out_ff : nullptr, ldm, Ly.ff);
-    L(DC_K_MIX_IN, lin_bytes(Ly.in, T), 1, linear(m, st, Ly.in, b.y, b.xb, H, in));
+    L(DC_K_MIX_IN, lin_bytes(Ly.in, T), 1, linear(m, st, Ly.in, b.y, b.xb, H, in, &Ly.out));
     if (light) L(DC_K_MIX_LIGHTNING, 8.0 * st.E * Ly.li.heads * Ly.li.dim * Ly.li.vdim, st.single && !st.tc ? 2 : 4, mix_lightning(m, st, run, Ly));
     else L(DC_K_MIX_GQA, 4.0 * T * Ly.in.N, st.tc ? 2 : 3, mix_gqa(m, st, sk, run, Ly));
     dc_lin_epi out = to(b.x, H);
     out.add = true;
     out.bias = Ly.out_bias;
-    L(DC_K_MIX_OUT, lin_bytes(Ly.out, T), 1, linear(m, st, Ly.out, b.mix, b.mixb, ldm, out));
+    L(DC_K_MIX_OUT, lin_bytes(Ly.out, T), 1, linear(m, st, Ly.out, b.mix, b.mixb, ldm, out, after));
     return DC_B200_OK;
 }
 
@@ -651,7 +661,7 @@ int moe_layer(dc_model* m, const dc_step& st, dc_stack_layer& Ly, const dc_hyper
 }
 
 // x += mixer(norm1(x)), then x += experts(norm2(x)).  *owed: rows that the feed-forward before has not added yet.
-int pre_norm_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_stack_run& run, dc_stack_layer& Ly, dc_row_sum* owed) {
+int pre_norm_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_stack_run& run, dc_stack_layer& Ly, dc_row_sum* owed, const dc_lin* after) {
     dc_stack* s = m->stack;
     dc_ctx* ctx = m->ctx;
     dc_stack_buffers& b = s->b;
@@ -663,12 +673,12 @@ int pre_norm_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_
     *owed = dc_row_sum();
     dc_lin_epi proj = to(b.proj, in.N);
     if (!latent) proj.bias = Ly.ga.bias;
-    L(DC_K_MIX_IN, lin_bytes(in, T), 1, linear(m, st, in, b.y, b.xb, H, proj));
+    L(DC_K_MIX_IN, lin_bytes(in, T), 1, linear(m, st, in, b.y, b.xb, H, proj, &o));
     if (latent) L(DC_K_MIX_LATENT, (double)Ly.la.ukv.N * Ly.la.ukv.ld * 2, 4, mix_latent(m, st, sk, run, Ly));
     else L(DC_K_MIX_GQA, 4.0 * T * in.N, st.tc ? 2 : 3, mix_gqa(m, st, sk, run, Ly));
     dc_lin_epi out = to(b.x, H);
     out.add = true;
-    L(DC_K_MIX_OUT, lin_bytes(o, T), 1, linear(m, st, o, b.mix, b.mixb, dc_pad8(o.K), out));
+    L(DC_K_MIX_OUT, lin_bytes(o, T), 1, linear(m, st, o, b.mix, b.mixb, dc_pad8(o.K), out, after));
     return Ly.moe.experts ? moe_layer(m, st, Ly, nullptr, owed) : DC_B200_OK;
 }
 
@@ -683,17 +693,17 @@ dc_hyper hyper_next(dc_model* m, dc_hyper* hy, const float* next) {
 }
 
 // Hyper-connected sublayers, mixer and feed-forward: u from the streams, y = f(norm(u)), which the streams then owe.
-int hyper_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_stack_run& run, dc_stack_layer& Ly, dc_hyper* hy) {
+int hyper_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_stack_run& run, dc_stack_layer& Ly, dc_hyper* hy, const dc_lin* after) {
     dc_stack* s = m->stack;
     dc_ctx* ctx = m->ctx;
     dc_stack_buffers& b = s->b;
     const int W = s->cfg.width, H = dc_pad8(W), T = st.T;
     __nv_bfloat16* xb = st.b16 ? b.xb : nullptr;
     L(DC_K_PRE_NORM, hyper_bytes(m, T), 1, dc_launch_hyper_norm(ctx, hyper_next(m, hy, Ly.hyper[0]), Ly.norm1, nullptr, 0, T, W, H, s->cfg.eps, b.h, xb));
-    L(DC_K_MIX_IN, lin_bytes(Ly.in, T), 1, linear(m, st, Ly.in, b.h, b.xb, H, to(b.proj, Ly.in.N)));
+    L(DC_K_MIX_IN, lin_bytes(Ly.in, T), 1, linear(m, st, Ly.in, b.h, b.xb, H, to(b.proj, Ly.in.N), &Ly.out));
     if (Ly.kind == DC_MIX_GENERAL) L(DC_K_MIX_GENERAL, 8.0 * st.E * Ly.ge.heads * Ly.ge.dim * Ly.ge.dim, st.single && !st.tc ? 1 : 5, mix_general(m, st, run, Ly));
     else L(DC_K_MIX_GQA, 4.0 * T * Ly.in.N, st.tc ? 2 : 3, mix_gqa(m, st, sk, run, Ly));
-    L(DC_K_MIX_OUT, lin_bytes(Ly.out, T), 1, linear(m, st, Ly.out, b.mix, b.mixb, dc_pad8(Ly.out.K), to(b.y, H)));
+    L(DC_K_MIX_OUT, lin_bytes(Ly.out, T), 1, linear(m, st, Ly.out, b.mix, b.mixb, dc_pad8(Ly.out.K), to(b.y, H), Ly.moe.experts || !Ly.ff ? after : &Ly.gate_up));
     if (Ly.moe.experts) {
         const dc_hyper now = hyper_next(m, hy, Ly.hyper[1]);
         return moe_layer(m, st, Ly, &now, &hy->sum);
@@ -701,8 +711,8 @@ int hyper_layer(dc_model* m, const dc_step& st, const StepKeys& sk, const dc_sta
     if (!Ly.ff) return DC_B200_OK;
     const int F = dc_pad8(Ly.ff);
     L(DC_K_PRE_NORM, hyper_bytes(m, T), 1, dc_launch_hyper_norm(ctx, hyper_next(m, hy, Ly.hyper[1]), Ly.norm2, nullptr, 0, T, W, H, s->cfg.eps, b.h, xb));
-    L(DC_K_FFN_GATEUP, lin_bytes(Ly.gate_up, T), 1, linear(m, st, Ly.gate_up, b.h, b.xb, H, dc_lin_epi().pairs(0, Ly.ff_pair, 0.0f, b.ff, st.b16 ? b.ffb : nullptr, F, F)));
-    L(DC_K_FFN_DOWN, lin_bytes(Ly.down, T), 1, linear(m, st, Ly.down, b.ff, b.ffb, F, to(b.y, H)));
+    L(DC_K_FFN_GATEUP, lin_bytes(Ly.gate_up, T), 1, linear(m, st, Ly.gate_up, b.h, b.xb, H, dc_lin_epi().pairs(0, Ly.ff_pair, 0.0f, b.ff, st.b16 ? b.ffb : nullptr, F, F), &Ly.down));
+    L(DC_K_FFN_DOWN, lin_bytes(Ly.down, T), 1, linear(m, st, Ly.down, b.ff, b.ffb, F, to(b.y, H), after));
     return DC_B200_OK;
 }
 
@@ -738,32 +748,32 @@ int run_layers(dc_model* m, const dc_step& st, const StepKeys& sk, dc_hyper* hy)
     for (size_t il = 0; il < s->runs.size(); ++il) {
         const dc_stack_run& run = s->runs[il];
         dc_stack_layer& Ly = s->layers[run.layer];
+        const dc_lin* after = run_begin(s, il + 1);
         if (m->dbg_x) DC_TRY(settle());
         DC_TRY(capture((int)il));
         if (hyper) {
-            DC_TRY(hyper_layer(m, st, sk, run, Ly, hy));
+            DC_TRY(hyper_layer(m, st, sk, run, Ly, hy, after));
             continue;
         }
         if (s->cfg.block == DC_BLOCK_PARALLEL) {
-            DC_TRY(parallel_layer(m, st, sk, run, Ly));
+            DC_TRY(parallel_layer(m, st, sk, run, Ly, after));
             continue;
         }
         if (s->cfg.block == DC_BLOCK_PRE_NORM) {
-            DC_TRY(pre_norm_layer(m, st, sk, run, Ly, &owed));
+            DC_TRY(pre_norm_layer(m, st, sk, run, Ly, &owed, after));
             continue;
         }
-        const dc_lin& in = Ly.kind == DC_MIX_DELTA ? Ly.dl.in : Ly.kind == DC_MIX_SSD ? Ly.ssd.in : Ly.la.in;
-        const dc_lin& o = Ly.kind == DC_MIX_DELTA ? Ly.dl.o : Ly.kind == DC_MIX_SSD ? Ly.ssd.o : Ly.la.o;
-        L(DC_K_MIX_IN, lin_bytes(in, T), 1, linear(m, st, in, b.x, xb, H, to(b.proj, in.N)));
+        const dc_lin &in = mixer_in(Ly), &o = mixer_out(Ly);
+        L(DC_K_MIX_IN, lin_bytes(in, T), 1, linear(m, st, in, b.x, xb, H, to(b.proj, in.N), &o));
         if (Ly.kind == DC_MIX_DELTA) L(DC_K_MIX_DELTA, 8.0 * st.E * Ly.dl.heads * Ly.dl.dim * Ly.dl.vdim, st.single && !st.tc ? 1 : 7, mix_delta(m, st, run, Ly));
         else if (Ly.kind == DC_MIX_SSD) L(DC_K_MIX_SSD, 8.0 * st.E * Ly.ssd.heads * Ly.ssd.state * Ly.ssd.vdim, st.single && !st.tc ? 2 : 5, mix_ssd(m, st, run, Ly));
         else L(DC_K_MIX_LATENT, (double)Ly.la.ukv.N * Ly.la.ukv.ld * 2, 4, mix_latent(m, st, sk, run, Ly));
-        L(DC_K_MIX_OUT, lin_bytes(o, T), 1, linear(m, st, o, b.mix, b.mixb, dc_pad8(o.K), to(b.y, H)));
+        L(DC_K_MIX_OUT, lin_bytes(o, T), 1, linear(m, st, o, b.mix, b.mixb, dc_pad8(o.K), to(b.y, H), Ly.ff ? &Ly.gate_up : after));
         L(DC_K_POST_NORM, 12.0 * T * W, 1, dc_launch_post_norm(ctx, b.x, b.y, Ly.norm1, T, W, H, eps, xb));
         if (!Ly.ff) continue;
         const int F = dc_pad8(Ly.ff);
-        L(DC_K_FFN_GATEUP, lin_bytes(Ly.gate_up, T), 1, linear(m, st, Ly.gate_up, b.x, xb, H, dc_lin_epi().pairs(0, Ly.ff_pair, 0.0f, b.ff, st.b16 ? b.ffb : nullptr, F, F)));
-        L(DC_K_FFN_DOWN, lin_bytes(Ly.down, T), 1, linear(m, st, Ly.down, b.ff, b.ffb, F, to(b.y, H)));
+        L(DC_K_FFN_GATEUP, lin_bytes(Ly.gate_up, T), 1, linear(m, st, Ly.gate_up, b.x, xb, H, dc_lin_epi().pairs(0, Ly.ff_pair, 0.0f, b.ff, st.b16 ? b.ffb : nullptr, F, F), &Ly.down));
+        L(DC_K_FFN_DOWN, lin_bytes(Ly.down, T), 1, linear(m, st, Ly.down, b.ff, b.ffb, F, to(b.y, H), after));
         L(DC_K_POST_NORM, 12.0 * T * W, 1, dc_launch_post_norm(ctx, b.x, b.y, Ly.norm2, T, W, H, eps, xb));
     }
     DC_TRY(settle());
