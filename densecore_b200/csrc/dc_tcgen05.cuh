@@ -26,6 +26,12 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr, uint32_t sbo
     const uint32_t hi = ((sbo >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);      // version 1 (sm_100), SWIZZLE_128B
     return ((uint64_t)hi << 32) | lo;
 }
+// The same of an operand whose rows run along N: K rows of 64 16-bit values each, 8-row groups sbo bytes apart; lbo = byte distance to the next 64 of N.
+__device__ __forceinline__ uint64_t umma_desc_sw128_n(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    const uint32_t lo = ((saddr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16);
+    const uint32_t hi = ((sbo >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
+    return ((uint64_t)hi << 32) | lo;
+}
 // The same without a swizzle: core matrices of 8 rows x 16 bytes; lbo = byte distance between neighbours along K, sbo along the rows.
 __device__ __forceinline__ uint64_t umma_desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     const uint32_t lo = ((saddr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16);

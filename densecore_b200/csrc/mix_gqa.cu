@@ -14,6 +14,7 @@
 #include "dc_launch.cuh"
 #include "dc_stack.h"
 #include "dc_stack.cuh"
+#include "dc_tcgen05.cuh"
 
 #define DC_TRY(expr)                       \
     do {                                   \
@@ -880,6 +881,271 @@ __global__ void __launch_bounds__(2 * PQ, PQ == 128 ? 2 : 1) k_gqa_prompt(const 
     }
 }
 
+// ---- the same on the 5th-generation tensor cores: head sizes up to 128, one map, an even number of query heads per key head
+// One CTA per (128 queries of one entry, two query heads of a key head), which share key and value tiles of 64 keys.  Scores and P V are tcgen05.mma with f32
+// accumulators in tensor memory: per head two sets of scores of 64 columns, whose first 32 then hold the weights as bf16 pairs, and 128 columns of answers.
+// So the next tile's scores are made while a thread per query weights this one's, and one head's products run during the other's weights.
+//   warps 0-7    weights: four a head, thread = query = tensor-memory lane (no sums across lanes)
+//   warps 8-11   load key and value rows by asynchronous copies into the operands' 128-byte swizzle
+//   warp 12      issues the products
+// Bound: the weights' arithmetic (about ten instructions per score) and the chain scores, weights, answers of a tile, one CTA per SM.
+constexpr int TP_Q = 128, TP_STAGES = 4, TP_THREADS = 13 * 32;
+constexpr uint32_t TP_QHEAD = TP_Q * 256, TP_TILE = PK * 256;      // a head's queries, keys or values of a tile: two halves of 64 columns
+constexpr uint32_t TP_KV = 2 * TP_QHEAD, TP_BARS = TP_KV + TP_STAGES * 2 * TP_TILE;
+enum TpBar { TP_FULL = 0, TP_FREE = 4, TP_S = 8, TP_P = 12, TP_O = 16, TP_DRAIN = 18, TP_NBARS };
+constexpr size_t TP_SMEM = TP_BARS + TP_NBARS * 8 + 1024;
+
+template <bool SIGMOID>
+__global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptParams p, int* err) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_give_up;
+    pdl_wait();
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, head0 = 2 * blockIdx.y;
+    const int tile0 = (int)(gridDim.x - 1 - blockIdx.x);           // later queries see more keys: they start first
+    const int e = p.tiles[2 * tile0], q0 = p.tiles[2 * tile0 + 1];
+    const int t0 = p.starts[e], n = p.starts[e + 1] - t0, pos0 = p.positions[t0], seq = p.seq_ids[t0];
+    if (q0 % TP_Q || q0 >= n) return;                               // tiles are listed per DC_LATENT_QTILE queries
+    const uint32_t sm = (smem_u32(smem) + 1023u) & ~1023u;
+    auto bar = [sm](int which, int i = 0) -> uint32_t { return sm + TP_BARS + 8u * (uint32_t)(which + i); };
+    const int last = pos0 + min(q0 + TP_Q, n) - 1;
+    const Keys keys = keys_of(pos0 + q0, last, p.window, p.keep);
+    const int n_tiles = (keys.n + PK - 1) / PK;
+    volatile int* give_up = &s_give_up;
+    if (warp == 12) {
+        tmem_alloc(smem_u32(&s_tmem), 512);
+        tmem_relinquish();
+    }
+    if (tid == 0) {
+        s_give_up = 0;
+        for (int i = 0; i < TP_NBARS; ++i) mbar_init(bar(i), i < TP_FREE ? 128 : i >= TP_P && i < TP_O ? 4 : 1);
+        mbar_fence_init();
+    }
+    for (int i = tid; i < 2 * TP_Q * 16; i += TP_THREADS) {        // both heads' queries; what is beyond the entry or the head is zero
+        const int u = i >> 11, row = (i >> 4) & 127, c = i & 15;
+        const bool in = q0 + row < n && 8 * c < p.ldq;
+        cp_async16z(sm + u * TP_QHEAD + (c >> 3) * (TP_Q * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4),
+                    p.q + ((size_t)(t0 + q0 + (in ? row : 0)) * p.heads + head0 + u) * p.ldq + (in ? 8 * c : 0), in);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_launch_dependents();      // (not before the tensor memory is there: a successor that held some and waited for this kernel would never give it back)
+    const uint32_t tmem = s_tmem;
+    auto wait = [&](uint32_t b, uint32_t parity) { return tc_wait_warp(b, parity, give_up, err); };
+    if (warp < 8) {
+        // ------------------------------------------------------------------ weights
+        const int u = warp >> 2, row = 32 * (warp & 3) + lane, head = head0 + u;
+        const uint32_t t_unit = tmem + u * 256 + ((uint32_t)(32 * (warp & 3)) << 16), t_o = t_unit + 128;
+        const bool capped = p.softcap > 0.0f;
+        const float cap = p.softcap * 1.4426950408889634f, to_cap = capped ? p.scale / p.softcap : 0.0f;
+        const float sl2 = capped ? 1.0f : p.scale * 1.4426950408889634f, sink2 = p.sink * 1.4426950408889634f;
+        const float bias2 = SIGMOID ? p.score_bias[head] * 1.4426950408889634f : 0.0f;
+        const int wq0 = pos0 + q0 + 32 * (warp & 3), qp = wq0 + lane, window = p.window > 0 ? p.window : 0x7fffffff;
+        const bool sink = p.sink > -INFINITY;      // the first term of the sum
+        float m_run = sink ? sink2 : -1e30f, l_run = sink ? 1.0f : 0.0f;
+        bool ok = true;
+        for (int t = 0; t < n_tiles; ++t) {
+            const uint32_t t_s = t_unit + 64 * (t & 1);
+            ok = wait(bar(TP_S, 2 * u + (t & 1)), (t >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            int x[4][16];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tmem_ld16(t_s + 16 * c, x[c]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tmem_ld_wait(x[c]);
+            auto s = [&](int i) -> float { return __int_as_float(x[i >> 4][i & 15]); };
+            auto set = [&](int i, float v) { x[i >> 4][i & 15] = __float_as_int(v); };
+            if (capped) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) set(i, soft_cap(s(i) * to_cap, cap));
+            }
+            if constexpr (SIGMOID) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) set(i, __fdividef(1.0f, 1.0f + ex2(-fmaf(s(i), sl2, bias2))));
+            }
+            // the warp's queries see the whole tile, or the mask decides key by key
+            const int k0 = keys.at(t * PK), k1 = keys.at(t * PK + PK - 1);
+            if (!(k1 <= wq0 && wq0 + 31 - k0 < window)) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) {
+                    const int kp = keys.at(t * PK + i);
+                    if (!(kp <= qp && (qp - kp < window || kp < p.keep))) set(i, SIGMOID ? 0.0f : -INFINITY);
+                }
+            }
+            if constexpr (!SIGMOID) {
+                float mx[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    mx[c] = s(16 * c);
+#pragma unroll
+                    for (int i = 1; i < 16; ++i) mx[c] = fmaxf(mx[c], s(16 * c + i));
+                }
+                const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2);
+                if (__any_sync(0xffffffffu, m_new > m_run)) {
+                    const float corr = ex2(m_run - m_new);
+                    m_run = m_new;
+                    l_run *= corr;
+                    if (t > 0) {
+                        ok = wait(bar(TP_O, u), (t - 1) & 1);
+                        if (!ok) break;
+                        tc_fence_after();
+#pragma unroll 1
+                        for (int c = 0; c < 8; ++c) {
+                            int o[16];
+                            uint32_t r[16];
+                            tmem_ld16(t_o + 16 * c, o);
+                            tmem_ld_wait(o);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__int_as_float(o[i]) * corr);
+                            tmem_st16(t_o + 16 * c, r);
+                        }
+                    }
+                }
+            }
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t w[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float a = s(32 * h + 2 * i), b = s(32 * h + 2 * i + 1);
+                    if constexpr (!SIGMOID) {
+                        a = ex2(fmaf(a, sl2, -m_run)), b = ex2(fmaf(b, sl2, -m_run));
+                        sum[i & 1] += a;
+                        sum[2 + (i & 1)] += b;
+                    }
+                    w[i] = pack_bf2(a, b);
+                }
+                tmem_st16(t_s + 16 * h, w);
+            }
+            l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(TP_P, 2 * u + (t & 1)));      // (two barriers: a warp may be done with the next tile before another is with this one)
+        }
+        // (phase by phase: the parity of the last alone also stands for the one before the last but one; tile t's scores come behind phase t - 2)
+        if (ok && n_tiles > 1) ok = wait(bar(TP_O, u), (n_tiles - 2) & 1);
+        if (ok) ok = wait(bar(TP_O, u), (n_tiles - 1) & 1);
+        if (ok) {
+            tc_fence_after();
+            const bool in = q0 + row < n;
+            float mul = SIGMOID ? 1.0f : 1.0f / l_run;
+            if (p.gate && in) mul *= sigmoid(p.gate[(size_t)(t0 + q0 + row) * p.ldg + head]);
+            __nv_bfloat16* dst = p.out + (size_t)(t0 + q0 + row) * p.ldm + (size_t)head * p.vdim;
+            const bool vec = p.vdim % 8 == 0 && p.ldm % 8 == 0 && ((uintptr_t)p.out & 15) == 0;
+#pragma unroll 1
+            for (int c = 0; c < 8; ++c) {
+                int o[16];
+                tmem_ld16(t_o + 16 * c, o);
+                tmem_ld_wait(o);
+                if (!in) continue;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int at = 16 * c + 8 * j;
+                    auto v = [&](int i) { return __int_as_float(o[8 * j + i]) * mul; };
+                    if (vec) {
+                        if (at < p.vdim) *reinterpret_cast<uint4*>(dst + at) = make_uint4(pack_bf2(v(0), v(1)), pack_bf2(v(2), v(3)), pack_bf2(v(4), v(5)), pack_bf2(v(6), v(7)));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (at + i < p.vdim) dst[at + i] = __float2bfloat16_rn(v(i));
+                    }
+                }
+            }
+        }
+    } else if (warp < 12) {
+        // ------------------------------------------------------------------ key and value tiles
+        const int lt = tid - 256, kc = p.dim_p / 8, vc = p.vdim_p / 8;
+        const __nv_bfloat16* cache = reinterpret_cast<const __nv_bfloat16*>(p.c.arena);
+        const int k_at = head0 / p.per * p.dim_p, v_at = p.v_at + head0 / p.per * p.vdim_p;
+        // tile t's copies are waited for once those of the next are on their way (the products want tile t + 1 before they are done with tile t)
+        for (int t = 0; t <= n_tiles; ++t) {
+            if (t < n_tiles) {
+                if (t >= TP_STAGES && !wait(bar(TP_FREE, t % TP_STAGES), (t / TP_STAGES - 1) & 1)) break;
+                const uint32_t to = sm + TP_KV + (t % TP_STAGES) * (2 * TP_TILE);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int key = (lt >> 4) + 8 * i, c = lt & 15, at = t * PK + key;      // sixteen threads a row
+                    const bool in = at < keys.n;
+                    const __nv_bfloat16* src = cache + p.c.at(seq, in ? keys.at(at) : last);
+                    const uint32_t dst = to + (c >> 3) * (PK * 128) + key * 128 + (((c & 7) ^ (key & 7)) << 4);
+                    cp_async16z(dst, in && c < kc ? src + k_at + 8 * c : src, in && c < kc);
+                    cp_async16z(dst + TP_TILE, in && c < vc ? src + v_at + 8 * c : src, in && c < vc);
+                }
+            }
+            cp_async_commit();
+            if (t == 0) continue;
+            cp_async_wait<1>();
+            fence_async_smem();
+            mbar_arrive(bar(TP_FULL, (t - 1) % TP_STAGES));
+        }
+        cp_async_wait<0>();
+    } else {
+        // ------------------------------------------------------------------ products
+        const bool one = elect_one();
+        constexpr uint32_t id_s = umma_idesc_bf16(TP_Q, PK), id_o = umma_idesc_bf16(TP_Q, 128) | (1u << 16);      // a value tile's rows are keys: N-major
+        auto scores = [&](int u, int t) {
+            if (one) {
+                const uint64_t q = umma_desc_sw128(sm + u * TP_QHEAD, 1024), k = umma_desc_sw128(sm + TP_KV + (t % TP_STAGES) * (2 * TP_TILE), 1024);
+                const uint32_t d = tmem + u * 256 + 64 * (t & 1);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) umma_f16(d, q + ((i >> 2) * (TP_Q * 128) + 32 * (i & 3)) / 16, k + ((i >> 2) * (PK * 128) + 32 * (i & 3)) / 16, id_s, i > 0);
+                umma_commit(bar(TP_S, 2 * u + (t & 1)));
+            }
+        };
+        auto values = [&](int u, int t) {
+            if (one) {
+                const uint64_t v = umma_desc_sw128_n(sm + TP_KV + (t % TP_STAGES) * (2 * TP_TILE) + TP_TILE, PK * 128, 1024);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) umma_f16_ts(tmem + u * 256 + 128, tmem + u * 256 + 64 * (t & 1) + 8 * i, v + (16 * 128 * i) / 16, id_o, t > 0 || i > 0);
+                umma_commit(bar(TP_O, u));
+            }
+        };
+        bool ok = wait(bar(TP_FULL, 0), 0);
+        if (ok) {
+            tc_fence_after();
+            scores(0, 0);
+            scores(1, 0);
+        }
+        // scores of tile t + 1 go where the weights of tile t - 1 were, once the product that reads those is complete (products of another shape need not
+        // run in order)
+        for (int t = 0; t < n_tiles && ok; ++t) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (ok && t + 1 < n_tiles) {
+                    if (u == 0) ok = wait(bar(TP_FULL, (t + 1) % TP_STAGES), ((t + 1) / TP_STAGES) & 1);
+                    if (ok && t > 0) ok = wait(bar(TP_O, u), (t - 1) & 1);
+                    tc_fence_after();
+                    if (ok) scores(u, t + 1);
+                }
+                ok = ok && wait(bar(TP_P, 2 * u + (t & 1)), (t >> 1) & 1);
+                tc_fence_after();
+                if (ok) values(u, t);
+            }
+            if (ok && one) umma_commit(bar(TP_FREE, t % TP_STAGES));
+        }
+        if (!ok) {      // products in flight still read shared and tensor memory
+            if (one) umma_commit(bar(TP_DRAIN));
+            mbar_wait_warp(bar(TP_DRAIN), 0);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 12) tmem_dealloc(tmem, 512);
+}
+
+template <bool SIGMOID>
+int launch_prompt_tc(dc_ctx* ctx, const PromptParams& p, int n_tiles) {
+    DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gqa_prompt_tc<SIGMOID>, (int)TP_SMEM, "k_gqa_prompt_tc"));
+    return dc_launch(ctx, "k_gqa_prompt_tc", k_gqa_prompt_tc<SIGMOID>, dim3(n_tiles, p.heads / 2), dim3(TP_THREADS), TP_SMEM, p, ctx->d_err);
+}
+
 template <int DP, int VP, int PQ, int ST, int MAPS, bool SIGMOID>
 int launch_prompt(dc_ctx* ctx, const PromptParams& p, int n_tiles) {
     constexpr int QT = PQ / MAPS, bytes = (PQ * (DP + 8) + ST * PK * (MAPS * DP + VP + 16)) * 2;
@@ -966,10 +1232,18 @@ int dc_launch_gqa_tokens(dc_ctx* ctx, const dc_gqa_mixer& m, const dc_step& st, 
                      gate, ldp, mix, mixb, ldm);
 }
 
+// Head sizes of 65 to 128 whose key heads serve pairs of query heads take the tcgen05 kernel, whatever the step's length: 16 heads of 128, window 1024, us, mma.sync
+// against tcgen05: 2048 tokens 88 / 36, 900 68 / 28, 300 22 / 15; 8 heads, 600 tokens 36 / 20; sigmoid weights, 1357 tokens 88 / 40; soft cap and kept tokens, 1500
+// tokens 102 / 56, 8 heads and 400 tokens 45 / 26.  Smaller heads would leave half of its operands empty.
+static bool gqa_prompt_tc_ok(const dc_gqa_mixer& m) {
+    return m.maps == 1 && m.dim_p <= 128 && m.vdim_p <= 128 && (m.dim > 64 || m.vdim > 64) && m.heads / m.kv_heads % 2 == 0;
+}
+
 int dc_launch_gqa_prompt(dc_ctx* ctx, const dc_gqa_mixer& m, const dc_step& st, const dc_gqa_cache& c, const int32_t* tiles, int n_tiles,
                          const __nv_bfloat16* qb, const float* proj, int ldp, float eps, __nv_bfloat16* mixb, int ldm) {
     PromptParams p = {qb, dc_gqa_ldq(m), m.heads, m.heads / m.kv_heads, m.dim, m.vdim, m.dim_p, m.vdim_p, m.v_at, m.window, m.keep, m.scale, m.softcap, sink_of(m),
                       m.lambda, 1.0f - m.diff, eps, m.score_bias, m.off_g < 0 ? nullptr : proj + m.off_g, ldp, st.seq_ids, st.positions, st.starts, tiles, cache_ref(c, m.row), mixb, ldm};
+    if (gqa_prompt_tc_ok(m)) return m.score_bias ? launch_prompt_tc<true>(ctx, p, n_tiles) : launch_prompt_tc<false>(ctx, p, n_tiles);
     // the smallest pair of padded key and value sizes that holds the head
 #define DC_PROMPT(DP, VP, PQ, ST, MAPS)                                                                  \
     if (m.maps == MAPS && !m.score_bias && m.dim <= DP && m.vdim <= VP) return launch_prompt<DP, VP, PQ, ST, MAPS, false>(ctx, p, n_tiles)
