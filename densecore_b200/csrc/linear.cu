@@ -169,6 +169,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 
 // NT: groups of eight tokens; AHEAD: neighbouring runs of 32 columns that a warp keeps in flight.  Column 8 q + 4 s + e of a run (q: lane % 4) is k-slot 2 q + e % 2 + 8 (e / 2) of product s.
 // KS: CTAs of a cluster that share sixteen rows, each with its part of the columns; the first adds the parts up.
+// Two CTAs an SM by declaration (four runs ahead need the registers of one): eight decode steps of Garilix at width 2048 take 5645 us without, 5510 with it.
 // With KS 1 a CTA walks over its tiles of sixteen rows and fetches the next tile's first runs ahead of a tile's sum.
 template <int NT, int AHEAD, int KS>
 __global__ void __launch_bounds__(LM_WARPS * 32, AHEAD > 2 ? 1 : LM_CTAS) k_linear_mma(const MmaParams p) {
@@ -331,6 +332,8 @@ bool epi_ok(const dc_lin_epi& e) { return e.pair0 >= (1 << 30) || e.pair0 % DC_P
 int dc_launch_linear_mma(dc_ctx* ctx, const dc_lin& w, const __nv_bfloat16* x, int ldx, int T, const dc_lin_epi& epi, const dc_lin* next) {
     if (T < 1 || T > DC_MAX_T || ((uintptr_t)x & 15) || (ldx & 7) || (w.N & 7) || !epi_ok(epi)) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "linear_mma: bad operand");
     MmaParams p = {w.w, w.N, w.K, w.ld, x, ldx, T, clipped(w, epi), nullptr, 0, 0};
+    // 6 MB ahead: eight steps of Garilix at width 2048 take 5437 us; none 5510, 2 MB 5475, 32 MB 5598, which delays what the small kernels in between wait for.
+    // Gomuzen with four sequences, where expert products lie in between, gains nothing (8.10 and 8.12 ms).
     if (next && !((uintptr_t)next->w & 15)) {
         p.next = (const char*)next->w;
         p.next_bytes = (uint32_t)std::min<size_t>((size_t)next->N * next->ld * 2, 6u << 20) & ~15u;
