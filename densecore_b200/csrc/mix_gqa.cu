@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
         const float bias2 = SIGMOID ? p.score_bias[head] * 1.4426950408889634f : 0.0f;
         const int wq0 = pos0 + q0 + 32 * (warp & 3), qp = wq0 + lane, window = p.window > 0 ? p.window : 0x7fffffff;
         const bool sink = p.sink > -INFINITY;      // the first term of the sum
-        float m_run = sink ? sink2 : -1e30f, l_run = sink ? 1.0f : 0.0f;
+        float m_run = sink ? sink2 : -1e30f, l_run[4] = {sink ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};      // the sums of k_gqa_prompt, in its order: one for each pair of eight columns
         bool ok = true;
         for (int t = 0; t < n_tiles; ++t) {
             const uint32_t t_s = t_unit + 64 * (t & 1);
@@ -989,7 +989,8 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
                 if (__any_sync(0xffffffffu, m_new > m_run)) {
                     const float corr = ex2(m_run - m_new);
                     m_run = m_new;
-                    l_run *= corr;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) l_run[i] *= corr;
                     if (t > 0) {
                         ok = wait(bar(TP_O, u), (t - 1) & 1);
                         if (!ok) break;
@@ -1007,7 +1008,6 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
                     }
                 }
             }
-            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t w[16];
@@ -1016,14 +1016,13 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
                     float a = s(32 * h + 2 * i), b = s(32 * h + 2 * i + 1);
                     if constexpr (!SIGMOID) {
                         a = ex2(fmaf(a, sl2, -m_run)), b = ex2(fmaf(b, sl2, -m_run));
-                        sum[i & 1] += a;
-                        sum[2 + (i & 1)] += b;
+                        l_run[i & 3] += a;
+                        l_run[i & 3] += b;
                     }
                     w[i] = pack_bf2(a, b);
                 }
                 tmem_st16(t_s + 16 * h, w);
             }
-            l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -1035,7 +1034,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
         if (ok) {
             tc_fence_after();
             const bool in = q0 + row < n;
-            float mul = SIGMOID ? 1.0f : 1.0f / l_run;
+            float mul = SIGMOID ? 1.0f : 1.0f / ((l_run[0] + l_run[1]) + (l_run[2] + l_run[3]));
             if (p.gate && in) mul *= sigmoid(p.gate[(size_t)(t0 + q0 + row) * p.ldg + head]);
             __nv_bfloat16* dst = p.out + (size_t)(t0 + q0 + row) * p.ldm + (size_t)head * p.vdim;
             const bool vec = p.vdim % 8 == 0 && p.ldm % 8 == 0 && ((uintptr_t)p.out & 15) == 0;

@@ -1,4 +1,7 @@
 """Prompt attention of grouped-query layers on the tensor cores at the edges of its tiles: 128 queries, 64 keys, head sizes of 65 to 128."""
+import copy
+import re
+
 import numpy as np
 import pytest
 
@@ -46,3 +49,50 @@ def test_prompt_attention_at_tile_edges(ctx, tmp_path, name, window):
             assert first is None or np.array_equal(got, first)
             first = got
     m.close()
+
+
+def with_own_key_heads(cfg, t):
+    """The same model with a key head for every query head: copies of the key and value rows that it shares.  Such layers keep k_gqa_prompt."""
+    cfg, t = copy.deepcopy(cfg), dict(t)
+    for i, ly in enumerate(cfg["layers"]):
+        m = ly["mixer"]
+        for n in [n for n in t if re.fullmatch(rf"l{i}\.mix\.[kv](\.\w+)?", n)]:
+            t[n] = np.repeat(t[n].reshape(m["kv_heads"], -1, *t[n].shape[1:]), m["heads"] // m["kv_heads"], axis=0).reshape(-1, *t[n].shape[1:])
+        m["kv_heads"] = m["heads"]
+    return cfg, t
+
+
+def logits_in_steps(ctx, path, cfg, t, steps):
+    """Logits of all tokens of all steps; a step: (sequence, tokens) pairs."""
+    m = dc.Model.from_dir(ctx, write_model(path, cfg, t), "bfloat16", max_seqs=8, max_ctx=512)
+    m.finalize()
+    seqs = [m.seq_alloc() for _ in range(8)]
+    out = [m.forward_batch([(seqs[i], tok) for i, tok in step], np.arange(sum(len(tok) for _, tok in step))) for step in steps]
+    m.close()
+    return np.concatenate(out)
+
+
+def several_prompts(rng, vocab):
+    """Steps of several entries: whole prompts, their next portions, single tokens among them."""
+    lengths = ([300, 5, 130, 64, 1], [90, 123, 1, 65, 127], [1, 130, 129, 1, 17])
+    return [[(i, rng.integers(0, vocab, size=n)) for i, n in enumerate(step)] for step in lengths]
+
+
+BOTH = {
+    "softmax": (gu, lambda w: gu.config([gu.kept(heads=4, kv_heads=1, dim=72, vdim=128, softcap=None, window=w, keep=3)])),
+    "capped": (gu, lambda w: gu.config([gu.kept(heads=4, kv_heads=2, dim=128, vdim=96, window=w, keep=70)])),
+    "sigmoid": (vu, lambda w: vu.config([vu.attention(heads=8, kv_heads=2, dim=128, vdim=72, window=w)], [vu.dense(48)])),
+}
+
+
+@pytest.mark.parametrize("window", [1, 40, 1000])
+@pytest.mark.parametrize("name", list(BOTH))
+def test_both_prompt_kernels_agree_bit_for_bit(ctx, tmp_path, name, window):
+    """Shared key heads (tcgen05) against copies of them (mma.sync): the same products, weights and sums in the same order."""
+    util, make = BOTH[name]
+    cfg = make(window)
+    t = util.make_tensors(cfg, 6)
+    steps = several_prompts(np.random.default_rng(window), cfg["vocab"])
+    shared = logits_in_steps(ctx, tmp_path / "shared", cfg, t, steps)
+    own = logits_in_steps(ctx, tmp_path / "own", *with_own_key_heads(cfg, t), steps)
+    assert np.isfinite(shared).all() and np.array_equal(shared, own)
