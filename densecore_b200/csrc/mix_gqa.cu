@@ -885,6 +885,8 @@ __global__ void __launch_bounds__(2 * PQ, PQ == 128 ? 2 : 1) k_gqa_prompt(const 
 // One CTA per (128 queries of one entry, two query heads of a key head), which share key and value tiles of 64 keys.  Scores and P V are tcgen05.mma with f32
 // accumulators in tensor memory: per head two sets of scores of 64 columns, whose first 32 then hold the weights as bf16 pairs, and 128 columns of answers.
 // So the next tile's scores are made while a thread per query weights this one's, and one head's products run during the other's weights.
+// Sixteen queries that see nothing of a tile take no part in its answers (their lanes of the product are off), as in k_gqa_prompt: with weights of zero alone, a
+// value that is infinite or NaN would reach every query of the CTA.
 //   warps 0-7    weights: four a head, thread = query = tensor-memory lane (no sums across lanes)
 //   warps 8-11   load key and value rows by asynchronous copies into the operands' 128-byte swizzle
 //   warp 12      issues the products
@@ -948,6 +950,11 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
         const bool sink = p.sink > -INFINITY;      // the first term of the sum
         float m_run = sink ? sink2 : -1e30f, l_run[4] = {sink ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};      // the sums of k_gqa_prompt, in its order: one for each pair of eight columns
         bool ok = true;
+        {
+            const uint32_t zero[16] = {};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) tmem_st16(t_o + 16 * c, zero);      // (complete and ordered with the first tile's weights)
+        }
         for (int t = 0; t < n_tiles; ++t) {
             const uint32_t t_s = t_unit + 64 * (t & 1);
             ok = wait(bar(TP_S, 2 * u + (t & 1)), (t >> 1) & 1);
@@ -1098,14 +1105,24 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
                 umma_commit(bar(TP_S, 2 * u + (t & 1)));
             }
         };
-        auto values = [&](int u, int t) {
+        auto values = [&](int u, int t, uint32_t seen) {
             if (one) {
                 const uint64_t v = umma_desc_sw128_n(sm + TP_KV + (t % TP_STAGES) * (2 * TP_TILE) + TP_TILE, PK * 128, 1024);
+                const uint32_t d = tmem + u * 256 + 128, w = tmem + u * 256 + 64 * (t & 1);
+                if (seen == 0xFFu) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) umma_f16_ts(tmem + u * 256 + 128, tmem + u * 256 + 64 * (t & 1) + 8 * i, v + (16 * 128 * i) / 16, id_o, t > 0 || i > 0);
+                    for (int i = 0; i < 4; ++i) umma_f16_ts(d, w + 8 * i, v + (16 * 128 * i) / 16, id_o, 1);
+                } else {
+                    uint32_t off[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) off[i] = (seen >> (2 * i) & 1u ? 0u : 0x0000FFFFu) | (seen >> (2 * i + 1) & 1u ? 0u : 0xFFFF0000u);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) umma_f16_ts_lanes(d, w + 8 * i, v + (16 * 128 * i) / 16, id_o, 1, off);
+                }
                 umma_commit(bar(TP_O, u));
             }
         };
+        const int window = p.window > 0 ? p.window : 0x7fffffff;
         bool ok = wait(bar(TP_FULL, 0), 0);
         if (ok) {
             tc_fence_after();
@@ -1115,6 +1132,9 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
         // scores of tile t + 1 go where the weights of tile t - 1 were, once the product that reads those is complete (products of another shape need not
         // run in order)
         for (int t = 0; t < n_tiles && ok; ++t) {
+            // bit i: queries 16 i .. 16 i + 15 see some of the tile
+            const int wq0 = pos0 + q0 + 16 * (lane & 7), k0 = keys.at(t * PK), k1 = keys.at(t * PK + PK - 1);
+            const uint32_t seen = __ballot_sync(0xffffffffu, !(k0 > wq0 + 15 || (k1 <= wq0 - window && k0 >= p.keep))) & 0xFFu;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 if (ok && t + 1 < n_tiles) {
@@ -1125,7 +1145,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
                 }
                 ok = ok && wait(bar(TP_P, 2 * u + (t & 1)), (t >> 1) & 1);
                 tc_fence_after();
-                if (ok) values(u, t);
+                if (ok) values(u, t, seen);
             }
             if (ok && one) umma_commit(bar(TP_FREE, t % TP_STAGES));
         }

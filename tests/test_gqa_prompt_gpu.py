@@ -96,3 +96,27 @@ def test_both_prompt_kernels_agree_bit_for_bit(ctx, tmp_path, name, window):
     shared = logits_in_steps(ctx, tmp_path / "shared", cfg, t, steps)
     own = logits_in_steps(ctx, tmp_path / "own", *with_own_key_heads(cfg, t), steps)
     assert np.isfinite(shared).all() and np.array_equal(shared, own)
+
+
+@pytest.mark.parametrize("window", [1, 40, 1000])
+@pytest.mark.parametrize("name", list(BOTH))
+def test_infinite_values_stay_where_they_are_seen(ctx, tmp_path, name, window):
+    """Token 0 has an infinite value row, which weights of zero turn into NaN: only queries that share its tile with keys that they see may meet it, in either kernel."""
+    util, make = BOTH[name]
+    cfg = make(window)
+    t = util.make_tensors(cfg, 6)
+    rng = np.random.default_rng(window)
+    t["embed"][:, :2] = 0
+    t["embed"][0, :2] = 4
+    for n in t:
+        if re.fullmatch(r"l0\.mix\.[qkg]", n):
+            t[n][:, :2] = 0
+    t["l0.mix.v"][:, :2] = 2.0 ** 127
+    steps = [[(i, 1 + tok % (cfg["vocab"] - 1)) for i, tok in step] for step in several_prompts(rng, cfg["vocab"])]
+    bad = {(0, 0): 250, (0, 2): 3, (1, 1): 100, (2, 2): 128}      # (step, entry): place of token 0
+    for (i, j), at in bad.items():
+        steps[i][j][1][at] = 0
+    shared = logits_in_steps(ctx, tmp_path / "shared", cfg, t, steps)
+    own = logits_in_steps(ctx, tmp_path / "own", *with_own_key_heads(cfg, t), steps)
+    assert np.array_equal(shared, own, equal_nan=True)
+    assert not np.isfinite(shared[250]).all() and np.isfinite(shared[:250 - 64 - 16]).all() and (window > 1 or np.isfinite(shared[256:300]).all())
