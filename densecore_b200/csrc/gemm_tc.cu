@@ -10,8 +10,8 @@
 //         The minimum term M = sum m_j * (sum of the token's codes in sub-block j) is one more product, of length 16: the minima (each twice) times the
 //         sums of the token's codes over 16 values (<= 2048, exact), |M| <= 63 * 127 * 256.
 //   Q6_K: q6 - 32 = (ql - 8) + 8 (2 qh - 3): sc (ql - 8) (<= 1024) with an accumulator for each half (<= 1024 * 128 * 128 = 2^24), and
-//         8 sc (2 qh - 3) with one for the block, whose sums are multiples of 8 and stay below 2^27.  float(I) = the sum of the three; only where
-//         the halves' sum passes 2^24 does it round twice.
+//         8 sc (2 qh - 3) with one for the block, whose sums are multiples of 8 and stay below 2^27.  float(I) = the sum of the three, rounded once: where the
+//         halves' sum reaches 2^24, a warp adds the three as integers.
 // The weight operand lies in tensor memory (lane = row, 32 columns a quarter block, four slots), where its expander threads store it; only the
 // activations take the way through shared memory, whose 128 bytes a cycle an operand of 128 rows from there would fill alone.
 //
@@ -448,21 +448,47 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const GemmTcParams p)
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
                         int x2[8];
-                        const uint4 ya = lds128(yds + 32 * c), yb = lds128(yds + 32 * c + 16);
-                        const float2 yd[4] = {make_float2(__uint_as_float(ya.x), __uint_as_float(ya.y)), make_float2(__uint_as_float(ya.z), __uint_as_float(ya.w)),
-                                              make_float2(__uint_as_float(yb.x), __uint_as_float(yb.y)), make_float2(__uint_as_float(yb.z), __uint_as_float(yb.w))};
+                        float2 yd[4];
+                        auto scales = [&]() {
+                            const uint4 ya = lds128(yds + 32 * c), yb = lds128(yds + 32 * c + 16);
+                            yd[0] = make_float2(__uint_as_float(ya.x), __uint_as_float(ya.y)), yd[1] = make_float2(__uint_as_float(ya.z), __uint_as_float(ya.w));
+                            yd[2] = make_float2(__uint_as_float(yb.x), __uint_as_float(yb.y)), yd[3] = make_float2(__uint_as_float(yb.z), __uint_as_float(yb.w));
+                        };
+                        if (Q4) scales();
                         auto pair = [](const int (&v)[8], int i) { return make_float2(__int_as_float(v[2 * i]), __int_as_float(v[2 * i + 1])); };
                         tmem_ld_wait(x0);
                         tmem_loaded(x1);
                         tmem_ld8(col + 2 * TC_NTOK + 8 * c, x2);
                         float2 x[4];
+                        float most = 0.0f;
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             float2& s = sum[th][4 * c + i];
                             x[i] = add2_rn(pair(x0, i), pair(x1, i));
+                            if (!Q4) most = fmaxf(most, fmaxf(fabsf(x[i].x), fabsf(x[i].y)));
                             if (Q4) s = fma2_rn(mul2_rn(mul2_rn(d2, yd[i]), x[i]), one, s);
                         }
                         tmem_ld_wait(x2);
+                        if constexpr (!Q4) {
+                            if (__any_sync(0xffffffffu, most >= 16777216.0f)) {      // a sum of the halves may have been rounded: all three anew, as integers
+                                int I[8];
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) I[i] = __float2int_rn(__int_as_float(x2[i]));
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    tmem_ld8(col + h * TC_NTOK + 8 * c, x0);
+                                    tmem_ld_wait(x0);
+#pragma unroll
+                                    for (int i = 0; i < 8; ++i) I[i] += __float2int_rn(__int_as_float(x0[i]));
+                                }
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) x[i] = make_float2(__int2float_rn(I[2 * i]), __int2float_rn(I[2 * i + 1]));
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) x[i] = add2_rn(x[i], pair(x2, i));
+                            }
+                            scales();
+                        }
                         if (c == 0) {
                             tmem_ld8(col + 8, x0);
                             tmem_ld8(col + TC_NTOK + 8, x1);
@@ -474,9 +500,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const GemmTcParams p)
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             float2& s = sum[th][4 * c + i];
-                            const float2 m = pair(x2, i);
-                            if (Q4) s = fma2_rn(mul2_rn(mul2_rn(dm2, yd[i]), m), one, s);
-                            else s = fma2_rn(mul2_rn(mul2_rn(d2, yd[i]), add2_rn(x[i], m)), one, s);
+                            if (Q4) s = fma2_rn(mul2_rn(mul2_rn(dm2, yd[i]), pair(x2, i)), one, s);
+                            else s = fma2_rn(mul2_rn(mul2_rn(d2, yd[i]), x[i]), one, s);
                         }
                     }
                 }

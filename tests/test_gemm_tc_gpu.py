@@ -49,3 +49,35 @@ def test_largest_sums(ctx, oracle, t):
     W = ctx.upload_weight(t, w, K, N)
     check(ctx.mul_mat(W, x), oracle.mul_mat(t, w, N, K, x), t)
     W.free()
+
+
+@pytest.mark.parametrize("M", [70, 128, 200])
+def test_q6k_block_sums_round_once(ctx, oracle, M):
+    """Codes of 0, 1 and few others: a block's sum is small beside its parts (lower and upper bits), which pass 2^24.  The whole result, step by step:
+    the sum as an integer, rounded once, times d yd, added in block order; to the bit."""
+    N, K = 150, 768
+    rng = np.random.default_rng(M)
+    nb = K // 256
+    blk = np.zeros((N, nb, 210), np.uint8)
+    codes = rng.choice(np.array([32, 33, 34, 47, 31, 63]), p=[0.5, 0.4, 0.06, 0.02, 0.01, 0.01], size=(N, nb, 256))
+    codes[N // 2:] = np.maximum(codes[N // 2:] - 32 * (rng.random((N - N // 2, nb, 1)) < 0.5), 0)        # and sums beyond 2^26
+    q = codes.reshape(N, nb, 2, 4, 32)       # a half block's quadrants: lower bits of 0 and 2, 1 and 3 share bytes, upper bits of all four
+    low, up = q & 15, q >> 4
+    blk[:, :, :128] = np.stack([low[:, :, :, 0] | low[:, :, :, 2] << 4, low[:, :, :, 1] | low[:, :, :, 3] << 4], 3).reshape(N, nb, 128)
+    blk[:, :, 128:192] = (up[:, :, :, 0] | up[:, :, :, 1] << 2 | up[:, :, :, 2] << 4 | up[:, :, :, 3] << 6).reshape(N, nb, 64)
+    scale = rng.choice(np.array([127, 126, 125, -128], np.int8), p=[0.5, 0.3, 0.1, 0.1], size=(N, nb, 16))
+    blk[:, :, 192:208] = scale.view(np.uint8)
+    d = np.abs(rng.normal(0.0, 0.01, size=(N, nb))).astype(np.float16)
+    blk[:, :, 208:] = d[:, :, None].view(np.uint8)
+    x = np.abs(rng.normal(1.0, 0.1, size=(M, K))).astype(np.float32)
+    yd, y, _ = oracle.q8k_fields(oracle.quantize_q8k(x))
+    sums = np.einsum("nbv,mbv->nmb", ((codes - 32).reshape(N, nb, 16, 16) * scale[:, :, :, None].astype(np.int64)).reshape(N, nb, 256), y.astype(np.int64))
+    lower = np.einsum("nbv,mbv->nmb", (((codes & 15) - 8).reshape(N, nb, 16, 16) * scale[:, :, :, None].astype(np.int64)).reshape(N, nb, 256), y.astype(np.int64))
+    assert (np.abs(lower) > 1 << 24).mean() > 0.2 and (np.abs(sums) > 1 << 26).any() and (np.abs(sums) < 1 << 24).any()
+    want = np.zeros((N, M), np.float32)
+    for b in range(nb):
+        want += d[:, None, b].astype(np.float32) * yd[None, :, b] * sums[:, :, b].astype(np.float32)
+    W = ctx.upload_weight(Q6, blk.reshape(N, -1), K, N)
+    got = ctx.mul_mat(W, x)
+    W.free()
+    assert np.array_equal(got, want.T)
