@@ -1048,19 +1048,21 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
 #pragma unroll 1
             for (int c = 0; c < 8; ++c) {
                 int o[16];
+                __syncwarp();      // lanes without a query have skipped the gate or the last stores: the load is the whole warp's
                 tmem_ld16(t_o + 16 * c, o);
                 tmem_ld_wait(o);
-                if (!in) continue;
+                if (in) {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int at = 16 * c + 8 * j;
-                    auto v = [&](int i) { return __int_as_float(o[8 * j + i]) * mul; };
-                    if (vec) {
-                        if (at < p.vdim) *reinterpret_cast<uint4*>(dst + at) = make_uint4(pack_bf2(v(0), v(1)), pack_bf2(v(2), v(3)), pack_bf2(v(4), v(5)), pack_bf2(v(6), v(7)));
-                    } else {
+                    for (int j = 0; j < 2; ++j) {
+                        const int at = 16 * c + 8 * j;
+                        auto v = [&](int i) { return __int_as_float(o[8 * j + i]) * mul; };
+                        if (vec) {
+                            if (at < p.vdim) *reinterpret_cast<uint4*>(dst + at) = make_uint4(pack_bf2(v(0), v(1)), pack_bf2(v(2), v(3)), pack_bf2(v(4), v(5)), pack_bf2(v(6), v(7)));
+                        } else {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (at + i < p.vdim) dst[at + i] = __float2bfloat16_rn(v(i));
+                            for (int i = 0; i < 8; ++i)
+                                if (at + i < p.vdim) dst[at + i] = __float2bfloat16_rn(v(i));
+                        }
                     }
                 }
             }
