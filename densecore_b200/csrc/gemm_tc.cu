@@ -641,6 +641,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const GemmTcParams p)
                     if (!wait(bar(B_FREE, st), st_phase)) {
                         // copies of the last blocks may still be on their way
                         for (int o = max(0, g - TC_B_STAGES); o < g; ++o) mbar_wait(bar(B_FULL, o % TC_B_STAGES), (o / TC_B_STAGES) & 1, nullptr);
+                        for (int o = max(0, g - 8); o < g; ++o) mbar_wait(bar(S_FULL, o & 7), (o >> 3) & 1, nullptr);
                         goto gave_up;
                     }
                     if (one) {
