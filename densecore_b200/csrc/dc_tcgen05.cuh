@@ -63,8 +63,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// The same with the loaded registers named, so that no use of them moves ahead of the wait.
+// The wait for this thread's loads, with the loaded registers named, so that no use of them moves ahead of it.
 __device__ __forceinline__ void tmem_ld_wait(int (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]),
@@ -101,7 +100,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
         : "memory");
     return __all_sync(0xffffffffu, left != 0);
 }
-// The same, telling the CTA's other waits if the limit ran out.
+// The same, setting the CTA's give-up flag, which tc_wait_raw watches, if the limit ran out.
 __device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity, volatile int* give_up, int* err) {
     if (mbar_wait_warp(bar, parity)) return true;
     *give_up = 1;

@@ -901,7 +901,6 @@ template <bool SIGMOID>
 __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptParams p, int* err) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_give_up;
     pdl_wait();
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, head0 = 2 * blockIdx.y;
     const int tile0 = (int)(gridDim.x - 1 - blockIdx.x);           // later queries see more keys: they start first
@@ -913,13 +912,11 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
     const int last = pos0 + min(q0 + TP_Q, n) - 1;
     const Keys keys = keys_of(pos0 + q0, last, p.window, p.keep);
     const int n_tiles = (keys.n + PK - 1) / PK;
-    volatile int* give_up = &s_give_up;
     if (warp == 12) {
         tmem_alloc(smem_u32(&s_tmem), 512);
         tmem_relinquish();
     }
     if (tid == 0) {
-        s_give_up = 0;
         for (int i = 0; i < TP_NBARS; ++i) mbar_init(bar(i), i < TP_FREE ? 128 : i >= TP_P && i < TP_O ? 4 : 1);
         mbar_fence_init();
     }
@@ -937,7 +934,11 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
     tc_fence_after();
     pdl_launch_dependents();      // (not before the tensor memory is there: a successor that held some and waited for this kernel would never give it back)
     const uint32_t tmem = s_tmem;
-    auto wait = [&](uint32_t b, uint32_t parity) { return tc_wait_warp(b, parity, give_up, err); };
+    auto wait = [&](uint32_t b, uint32_t parity) {      // (a role that gives up lets the others run into limits of their own)
+        const bool is = mbar_wait_warp(b, parity);
+        if (!is && err) atomicExch(err, DC_ERR_MBAR_TIMEOUT);
+        return is;
+    };
     if (warp < 8) {
         // ------------------------------------------------------------------ weights
         const int u = warp >> 2, row = 32 * (warp & 3) + lane, head = head0 + u;
