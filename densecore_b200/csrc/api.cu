@@ -11,6 +11,7 @@
 
 #include "dc_common.cuh"
 #include "dc_internal.h"
+#include "dc_registers.h"
 
 int dc_fail(dc_ctx* ctx, int status, const char* fmt, ...) {
     char buf[512];
@@ -53,7 +54,7 @@ int dc_kernel_setup(dc_ctx* ctx, const void* func, int max_dyn_smem, const char*
 int dc_kernel_setup_small(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name) {
     return kernel_setup(ctx, func, max_dyn_smem, name, max_dyn_smem <= 50 * 1024 ? 45 : 0);
 }
-int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name) {
+int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name, int launch_regs) {
     static std::mutex mu;
     static std::set<const void*> good;
     {
@@ -63,6 +64,7 @@ int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, c
             const int st = dc_check_cuda(ctx, cudaFuncGetAttributes(&a, func), name);
             if (st != DC_B200_OK) return st;
             if (a.localSizeBytes) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "%s was built with %d bytes of spilled registers", name, (int)a.localSizeBytes);
+            if (!dc_registers_match(a.numRegs, launch_regs)) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "%s was built with %d registers a thread instead of %d", name, a.numRegs, launch_regs);
             good.insert(func);
         }
     }

@@ -58,8 +58,8 @@ int dc_kernel_setup(dc_ctx* ctx, const void* func, int max_dyn_smem, const char*
 int dc_kernel_setup_small(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name);
 // The same for a kernel that loads from tensor memory.  Such loads land in their registers some time after the instruction, and the code uses
 // others meanwhile.  A build that spills could store such a register too early and give it another use, which the load then overwrites: it may
-// not run.
-int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name);
+// not run.  launch_regs: registers a thread that the kernel has to start with (one that shares them out anew among its warps), 0: any number.
+int dc_kernel_setup_unspilled(dc_ctx* ctx, const void* func, int max_dyn_smem, const char* name, int launch_regs = 0);
 int dc_kernel_occupancy(dc_ctx* ctx, const void* func, int threads, size_t dyn_smem);
 
 // ---- launch helpers implemented in the kernel translation units ----

@@ -145,7 +145,11 @@ __global__ void __launch_bounds__(256) k_quantize_q8k_tiled(const float* __restr
 constexpr int TC_EXPANDERS = 8, TC_READERS = 16;
 constexpr int TC_WARP_MMA = TC_EXPANDERS + TC_READERS;
 constexpr int TC_THREADS = (TC_WARP_MMA + 4) * 32;         // (the last warp only gives its registers)
-constexpr int TC_READ_REGS = 80, TC_REST_REGS = 40;        // 256 x 72 + 512 x 80 + 128 x 40 = 896 x 72, the launch's
+// Registers a thread at launch, of the read-out and of the last four warps once they have shared theirs out anew; expanders keep the launch's.  What the read-out takes has
+// to be what the others give: from a launch with fewer registers it would wait for more without end, so the launcher refuses any other build.
+constexpr int TC_LAUNCH_REGS = 72, TC_READ_REGS = 80, TC_REST_REGS = 40;
+static_assert(TC_EXPANDERS * TC_LAUNCH_REGS + TC_READERS * TC_READ_REGS + 4 * TC_REST_REGS <= (TC_THREADS / 32) * TC_LAUNCH_REGS, "the launch's registers");
+static_assert(TC_EXPANDERS % 4 == 0 && TC_READERS % 4 == 0, "whole warpgroups");
 constexpr int TC_B_STAGES = 3;
 constexpr uint32_t TC_SET = 3 * TC_NTOK;                   // columns of a set of accumulators
 constexpr uint32_t TC_COL_A = 2 * TC_SET;                  // first operand column
@@ -742,10 +746,10 @@ int dc_launch_gemm_tc_multi(dc_ctx* ctx, const dc_weight* const* ws, const int* 
     // one CTA per SM walks its share of the tiles
     const dim3 grid((unsigned)std::min(p.tiles_x * p.tiles_y, ctx->num_sms));
     if (w->type == DC_TYPE_Q4_K) {
-        DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gemm_tc<DC_TYPE_Q4_K>, (int)TC_SMEM, "k_gemm_tc<Q4_K>"));
+        DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gemm_tc<DC_TYPE_Q4_K>, (int)TC_SMEM, "k_gemm_tc<Q4_K>", TC_LAUNCH_REGS));
         return dc_launch(ctx, "k_gemm_tc", k_gemm_tc<DC_TYPE_Q4_K>, grid, dim3(TC_THREADS), TC_SMEM, p);
     } else {
-        DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gemm_tc<DC_TYPE_Q6_K>, (int)TC_SMEM, "k_gemm_tc<Q6_K>"));
+        DC_TRY(dc_kernel_setup_unspilled(ctx, (const void*)k_gemm_tc<DC_TYPE_Q6_K>, (int)TC_SMEM, "k_gemm_tc<Q6_K>", TC_LAUNCH_REGS));
         return dc_launch(ctx, "k_gemm_tc", k_gemm_tc<DC_TYPE_Q6_K>, grid, dim3(TC_THREADS), TC_SMEM, p);
     }
 }
