@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+import densecore_b200 as dc
 from densecore_b200 import blocks as B
 
 pytestmark = pytest.mark.gpu
@@ -81,3 +82,40 @@ def test_q6k_block_sums_round_once(ctx, oracle, M):
     got = ctx.mul_mat(W, x)
     W.free()
     assert np.array_equal(got, want.T)
+
+
+@pytest.mark.parametrize("t", [Q4, Q6])
+def test_unused_slots_may_hold_anything(ctx, oracle, t):
+    """The last token tile's slots beyond the rows are not written: with the scratch full of NaN patterns (of f32 and of fp16) the results are the same bits."""
+    N, K = 200, 512
+    rng = np.random.default_rng(3)
+    w = B.random_weight(rng, t, N, K)
+    W = ctx.upload_weight(t, w, K, N)
+    for M in (33, 65, 190):
+        x = rng.normal(size=(M, K)).astype(np.float32)
+        first = ctx.mul_mat(W, x)
+        ctx.mul_mat(W, np.full((1024, K), 0xFFFFFFFF, np.uint32).view(np.float32))      # its inputs lie where the next call's activations will
+        again = ctx.mul_mat(W, x)
+        check(again, oracle.mul_mat(t, w, N, K, x), t)
+        assert np.array_equal(again, first)
+    W.free()
+
+
+def test_unused_expert_slots_may_hold_anything(ctx):
+    """A prompt through a mixture of experts whose buffers come out of memory full of NaN patterns, and out of zeros."""
+    cfg = dc.Config(max_seqs=1, max_ctx=512, n_layer=2, hidden=512, n_head=4, n_kv_head=2, vocab=1000, n_expert=8, n_expert_used=2, expert_ffn=256)
+    prompt = np.random.default_rng(5).integers(0, cfg.vocab, size=300)
+    out = []
+    for fill in (0, 0xFFFFFFFF):
+        m = dc.Model(ctx, cfg)
+        m.init_synthetic(11, 0.05)
+        m.finalize()
+        pattern = np.full(1 << 24, fill, np.uint32)
+        blocks = [ctx.alloc(pattern.nbytes) for _ in range(16)]      # 1 GB, given back ahead of the prompt's buffers
+        for b in blocks:
+            ctx.to_device(b, pattern)
+        for b in blocks:
+            ctx.free(b)
+        out.append(m.prefill(m.seq_alloc(), prompt, want_logits=True)[1].copy())
+        m.close()
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])

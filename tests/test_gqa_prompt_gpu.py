@@ -18,6 +18,12 @@ CASES = {
     "sink": (du, lambda w: du.config([du.attention(heads=4, kv_heads=2, dim=96, window=w)], ff=48)),
     "sigmoid": (vu, lambda w: vu.config([vu.attention(heads=8, kv_heads=2, dim=128, vdim=72, window=w)], [vu.dense(48)])),
     "kept": (gu, lambda w: gu.config([gu.kept(heads=4, kv_heads=1, dim=72, vdim=128, window=w, keep=3)], gu.moe())),
+    # odd numbers of query heads a key head: the mma.sync kernel, which serves these head sizes too
+    "sink_own_128": (du, lambda w: du.config([du.attention(heads=2, kv_heads=2, dim=128, window=w)], ff=48)),
+    "kept_odd_64_128": (gu, lambda w: gu.config([gu.kept(heads=3, kv_heads=1, dim=56, vdim=128, window=w, keep=3)])),
+    "kept_odd_128": (gu, lambda w: gu.config([gu.kept(heads=3, kv_heads=1, dim=128, vdim=128, window=w, keep=3)])),
+    "sigmoid_odd_96": (vu, lambda w: vu.config([vu.attention(heads=3, kv_heads=1, dim=96, vdim=80, window=w)], [vu.dense(48)])),
+    "sigmoid_odd_128": (vu, lambda w: vu.config([vu.attention(heads=3, kv_heads=1, dim=128, vdim=128, window=w)], [vu.dense(48)])),
 }
 
 
