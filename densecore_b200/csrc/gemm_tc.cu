@@ -100,8 +100,9 @@ __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint3
 // ---- activation side ---------------------------------------------------------------------------------
 // One warp per (token slot, 256-value block): Q8_K codes (bit-equal to the row quantiser) into the tile
 // layout of dc_gemm_tc.h, block scale into the tile's tail.  slot_token (optional) maps a slot to its source
-// row, < 0 or beyond n_rows: the slot is left as it is.  (What an unused slot holds stays in its own column of the products, which nobody stores;
-// a third of a prompt's expert slots are such; with zeros written there the three launches of a layer took 80 us for 2011 tokens, now 73.)
+// row, < 0 or beyond n_rows: the slot is left as it is.  (What an unused slot holds stays in its own column of the products: gate and up store it into the
+// slot's own row, which nobody reads, the down product stores nothing of it.  A third of a prompt's expert slots are such; with zeros written there the three
+// launches of a layer took 80 us for 2011 tokens, now 73.)
 __global__ void __launch_bounds__(256) k_quantize_q8k_tiled(const float* __restrict__ x, int ldx, int n_rows, int K,
                                                             uint8_t* __restrict__ act, int n_tt,
                                                             const int* __restrict__ slot_token) {
