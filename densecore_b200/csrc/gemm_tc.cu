@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) k_quantize_q8k_tiled(const float* __restr
 // What bounds it: the chain of a block (operand slot free, stored, multiplied, read out, accumulators free), each hand-over 150 to 400 cycles, while every SM
 // sub-partition is about half busy (packed multiply-adds of the read-out, expansion); without the read-out's work a block takes 10 % less, without the
 // expansion's 16 %, without either 28 %.  Measured, us, against the int8 form of this kernel (operands in shared memory, 13 instead of 4 instructions per element
-// and block in the read-out): Q4_K 4096 x 2048 by 1531 tokens 69 -> 47, Q6_K 113 -> 89; Q4_K 2048 x 4096 by 300 tokens 44 -> 29, 2048 x 768 by 64 11 -> 8.  Tried:
+// and block in the read-out): Q4_K 4096 x 2048 by 1531 tokens 70 -> 47, Q6_K 114 -> 92; 2048 x 4096 by 300 tokens 45 -> 29 and 82 -> 62, 2048 x 768 by 64 11 -> 8 and 18 -> 13.  Tried:
 // accumulators of 128 tokens (one set only, 63 us); eight read-out warps, or four expanders (61); one issuing warp (48); operand slots of half a block (60).
 constexpr int TC_EXPANDERS = 8, TC_READERS = 16;
 constexpr int TC_WARP_MMA = TC_EXPANDERS + TC_READERS;

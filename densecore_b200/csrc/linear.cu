@@ -332,8 +332,10 @@ bool epi_ok(const dc_lin_epi& e) { return e.pair0 >= (1 << 30) || e.pair0 % DC_P
 int dc_launch_linear_mma(dc_ctx* ctx, const dc_lin& w, const __nv_bfloat16* x, int ldx, int T, const dc_lin_epi& epi, const dc_lin* next) {
     if (T < 1 || T > DC_MAX_T || ((uintptr_t)x & 15) || (ldx & 7) || (w.N & 7) || !epi_ok(epi)) return dc_fail(ctx, DC_B200_INTERNAL_ERROR, "linear_mma: bad operand");
     MmaParams p = {w.w, w.N, w.K, w.ld, x, ldx, T, clipped(w, epi), nullptr, 0, 0};
-    // 6 MB ahead: eight steps of Garilix at width 2048 take 5437 us; none 5510, 2 MB 5475, 32 MB 5598, which delays what the small kernels in between wait for.
-    // Gomuzen with four sequences, where expert products lie in between, gains nothing (8.10 and 8.12 ms).
+    // 6 MB ahead; more delays what the small kernels in between wait for.  Us a step with none, 3, 6 and 12 MB: Garilix of width 2048, one sequence 689, 678, 677, 689,
+    // sixteen 912, 904, 900, 912; of width 1024, one 455, 445, 443, 443; Datasun of width 2048, one 518, 511, 507, 516; of width 1024, sixteen 371, 370, 363, 357.
+    // Where expert products lie in between, it gives less: none and 6 MB: Vepitar of width 1024, one sequence 469 and 466, Gomuzen of width 1024, two 601 and 592, sixteen
+    // 822 and 817, of width 2048, four 973 and 974, sixteen 1446 and 1453.
     if (next && !((uintptr_t)next->w & 15)) {
         p.next = (const char*)next->w;
         p.next_bytes = (uint32_t)std::min<size_t>((size_t)next->N * next->ld * 2, 6u << 20) & ~15u;

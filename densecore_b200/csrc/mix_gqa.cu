@@ -1255,8 +1255,8 @@ int dc_launch_gqa_tokens(dc_ctx* ctx, const dc_gqa_mixer& m, const dc_step& st, 
 }
 
 // Head sizes of 65 to 128 whose key heads serve pairs of query heads take the tcgen05 kernel, whatever the step's length: 16 heads of 128, window 1024, us, mma.sync
-// against tcgen05: 2048 tokens 88 / 36, 900 68 / 28, 300 22 / 15; 8 heads, 600 tokens 36 / 20; sigmoid weights, 1357 tokens 88 / 40; soft cap and kept tokens, 1500
-// tokens 102 / 56, 8 heads and 400 tokens 45 / 26.  Smaller heads would leave half of its operands empty.
+// against tcgen05: 2048 tokens 88 / 36, 900 67 / 28, 300 20 / 14; 8 heads, 600 tokens 35 / 22; sigmoid weights, 1357 tokens 82 / 34; soft cap and kept tokens, 1500
+// tokens 101 / 54, 8 heads and 400 tokens 28 / 23.  Chunks of 17 to 300 tokens behind 0 to 4000 others take 0 to 33 % less in decoders of eight such layers.  Smaller heads would leave half of its operands empty.
 static bool gqa_prompt_tc_ok(const dc_gqa_mixer& m) {
     return m.maps == 1 && m.dim_p <= 128 && m.vdim_p <= 128 && (m.dim > 64 || m.vdim > 64) && m.heads / m.kv_heads % 2 == 0;
 }
