@@ -88,7 +88,8 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(p));
     return p != 0;
 }
-// Bounded wait of a converged warp, in as few instructions as it takes: all lanes go on or none does.
+// Bounded wait of a converged warp, in as few instructions as it takes: all lanes go on or none does.  Lanes may wait for barriers of their own: what one has waited for
+// holds for the others too (a vote alone orders no memory and need not leave the warp whole).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
     uint32_t left;
     asm volatile(
@@ -98,7 +99,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
         : "=&r"(left)
         : "r"(bar), "r"(parity), "n"(DC_WAIT_LIMIT)
         : "memory");
-    return __all_sync(0xffffffffu, left != 0);
+    const bool all = __all_sync(0xffffffffu, left != 0);
+    __syncwarp();
+    return all;
 }
 // The same, setting the CTA's give-up flag, which tc_wait_raw watches, if the limit ran out.
 __device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity, volatile int* give_up, int* err) {

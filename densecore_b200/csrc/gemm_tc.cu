@@ -289,6 +289,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const GemmTcParams p)
         const int r = tid & 127, grp = warp >> 2;
         const uint32_t t_a = tmem + TC_COL_A + ((uint32_t)(32 * (warp & 3)) << 16);
         auto filled = [&](int slot) {
+            __syncwarp();
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -439,7 +440,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const GemmTcParams p)
                     const uint32_t b = th || lane & 1 ? bar(ACC_FULL, set) : lane & 2 ? bar(D_FULL, g & 3) : bar(S_FULL, g & 7);
                     if (!wait(b, th || lane & 1 ? (phase >> set) & 1 : lane & 2 ? (g >> 2) & 1 : (g >> 3) & 1)) goto gave_up;
                     phase ^= 1u << set;
-                    __syncwarp();      // what a lane has waited for holds for the others too (a vote alone orders no memory)
                     tc_fence_after();
                     const uint32_t yds = sm + TC_SSC + ((g & 7) * 2 + th) * TC_ACT_SCALES + 4 * tok0, col = t_lane + set * TC_SET;
                     // eight tokens at a time; the next loads are on their way while the float terms of the last are made

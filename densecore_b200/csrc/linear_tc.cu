@@ -47,6 +47,7 @@ __device__ __forceinline__ float quick_clamped(float limit, float gate, float up
 template <int COLS, typename F>
 __device__ __forceinline__ void each16(uint32_t tmem, int n, F f) {
     int v[2][16];
+    __syncwarp();
     tmem_ld16(tmem, v[0]);
 #pragma unroll 1
     for (int c0 = 0; c0 < COLS && c0 < n; c0 += 32) {
@@ -54,6 +55,7 @@ __device__ __forceinline__ void each16(uint32_t tmem, int n, F f) {
         for (int i = 0; i < 2; ++i) {
             const int c = c0 + 16 * i;
             if (c >= n) break;
+            __syncwarp();      // lanes store or skip what is theirs, but loads are the whole warp's
             tmem_ld_wait(v[i]);
             if (c + 16 < COLS && c + 16 < n) tmem_ld16(tmem + c + 16, v[i ^ 1]);
             f(v[i], c);

@@ -1016,6 +1016,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_gqa_prompt_tc(const PromptPar
                     }
                 }
             }
+            __syncwarp();      // masks are a lane's own, the stores are the whole warp's
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t w[16];
