@@ -256,8 +256,10 @@ __global__ void __launch_bounds__(LT_THREADS, 2) k_linear_tc(const __grid_consta
         constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
         int s = 0;
         uint32_t phase = 0;
+        bool ok = true;
         for (int k = 0; k < nk; ++k) {
-            if (!tc_wait_warp(full + 8 * s, phase, give_up, p.err)) break;
+            ok = tc_wait_warp(full + 8 * s, phase, give_up, p.err);
+            if (!ok) break;
             tc_fence_after();
             const uint64_t a = umma_desc_sw128(base + s * 2 * LT_TILE, 1024), b = umma_desc_sw128(base + s * 2 * LT_TILE + LT_TILE, 1024);
             if (one) {
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(LT_THREADS, 2) k_linear_tc(const __grid_consta
             if (++s == LT_STAGES) s = 0, phase ^= 1;
         }
         if (one) umma_commit(acc);
+        if (!ok) mbar_wait_warp(acc, 0);      // products in flight still use shared and tensor memory
     } else {
         const bool ok = tc_wait_raw(acc, 0, give_up, p.err) && !*give_up;
         tc_fence_after();
@@ -294,12 +297,12 @@ template <bool GROUPED>
 __global__ void __launch_bounds__(LW_THREADS, 1) k_linear_tc_wide(const __grid_constant__ CUtensorMap wmap,
                                                                   const __grid_constant__ CUtensorMap xmap, const LtParams p, const LwTiles tl) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t s_bar[2 * LW_STAGES + 4];
+    __shared__ __align__(8) uint64_t s_bar[2 * LW_STAGES + 5];
     __shared__ uint32_t s_tmem;
     __shared__ int s_give_up;
     __shared__ int s_off[GROUPED ? DC_MOE_MAX_EXPERTS + 1 : 1], s_first[GROUPED ? DC_MOE_MAX_EXPERTS + 1 : 1];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t full = smem_u32(s_bar), empty = full + 8 * LW_STAGES, acc_full = empty + 8 * LW_STAGES, acc_free = acc_full + 16;
+    const uint32_t full = smem_u32(s_bar), empty = full + 8 * LW_STAGES, acc_full = empty + 8 * LW_STAGES, acc_free = acc_full + 16, drain = acc_free + 16;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nk = (p.K + 63) / 64;
     volatile int* give_up = &s_give_up;
@@ -317,6 +320,7 @@ __global__ void __launch_bounds__(LW_THREADS, 1) k_linear_tc_wide(const __grid_c
             mbar_init(acc_full + 8 * i, 1);
             mbar_init(acc_free + 8 * i, 128 * LW_READERS);
         }
+        mbar_init(drain, 1);
         mbar_fence_init();
     }
     tc_fence_before();
@@ -393,7 +397,8 @@ __global__ void __launch_bounds__(LW_THREADS, 1) k_linear_tc_wide(const __grid_c
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++j) {
             const int set = j & 1;
             const uint32_t idesc = umma_idesc_bf16(128, GROUPED ? (place(tile, group).cols() + 15) & ~15 : 256), d = tmem + 256 * set;
-            if (j >= 2 && !tc_wait_warp(acc_free + 8 * set, ((j >> 1) - 1) & 1, give_up, p.err)) break;
+            if (j >= 2) ok = tc_wait_warp(acc_free + 8 * set, ((j >> 1) - 1) & 1, give_up, p.err);
+            if (!ok) break;
             tc_fence_after();
             for (int k = 0; k < nk; ++k) {
                 ok = tc_wait_warp(full + 8 * s, phase, give_up, p.err);
@@ -408,6 +413,10 @@ __global__ void __launch_bounds__(LW_THREADS, 1) k_linear_tc_wide(const __grid_c
                 if (++s == LW_STAGES) s = 0, phase ^= 1;
             }
             if (one) umma_commit(acc_full + 8 * set);
+        }
+        if (!ok) {      // products in flight still use shared and tensor memory
+            if (one) umma_commit(drain);
+            mbar_wait_warp(drain, 0);
         }
     } else {
         int j = 0, group = 0;
