@@ -11,7 +11,7 @@
 // of few tokens takes narrower products.  All let the next kernel start only after every
 // CTA has its tensor memory.  The loading and the issuing warp run as whole warps of which one lane issues: with a branch on the lane number around their
 // loops a stage's wait, four products and commit took as long as the products themselves (prompts 1 to 2 % longer).  Columns beyond K and rows beyond the matrix are the zeros that TMA fills in.  Every wait is
-// bounded; a CTA that gives up drains its copies, frees its tensor memory and leaves.
+// bounded; a CTA that gives up drains its copies and products, frees its tensor memory and leaves.
 #include <algorithm>
 
 #include "dc_common.cuh"
